@@ -84,6 +84,23 @@ def load():
     return _lib
 
 
+_host_module = None
+
+
+def host():
+    """The native host path (_host.so), loaded once.  Raises RuntimeError when it has not been built."""
+    global _host_module
+    if _host_module is None:
+        load()
+        try:
+            from . import _host
+        except ImportError as e:
+            raise RuntimeError(f"qtip_b200/_host.so cannot be loaded ({e}): build it with `python -m qtip_b200.build` "
+                               "(qtip_b200 has no fallback path)") from e
+        _host_module = _host
+    return _host_module
+
+
 def check_desc_layout(lib):
     """The ctypes mirror of qtip_linear_desc against the compiled struct (size and every field offset): a mirror that is
     out of step would hand the kernels pointer bits as counts and limits."""

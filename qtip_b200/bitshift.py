@@ -4,12 +4,10 @@ Same constructor and forward signature as upstream's BitshiftLinear (bitshift.py
 QuantizedLinear (or upstream's own) can hold it unchanged.  Only the inference modes are built:
 the Viterbi quantizer and the training modes are outside this package.
 """
-import math
-
 import torch
 from torch import nn
 
-from . import ops
+from . import _lib, ops
 
 _CODE_OF_MODE = {"quantlut_sym": ops.CODE_HYB, "3inst": ops.CODE_3INST, "1mad": ops.CODE_1MAD}
 
@@ -44,6 +42,7 @@ class BitshiftLinear(nn.Module):
         self.has_kernel = has_kernel
         self.scale = 32
         self._sv_cache = {}
+        self._bits = [None, None]
         self.workspace = None  # optional caller-owned workspace for the fused matvec
 
     # -- decoders ------------------------------------------------------------------------------
@@ -82,46 +81,29 @@ class BitshiftLinear(nn.Module):
             self._sv_cache[key] = hit
         return hit
 
+    def _hadk_bits(self, side, had, device):
+        """Packed signs of a factor matrix on `device`, remembered per side (0 in, 1 out) while the matrix stays the same."""
+        if had is None:
+            return None
+        hit = self._bits[side]
+        if hit is None or hit[0] is not had or hit[1] != had._version or hit[2] != device:
+            hit = self._bits[side] = (had, had._version, device, ops.hadk_bits_for(had, device))
+        return hit[3]
+
     def forward(self, input, trellis, SU, SV, had_left, had_right, K_left, K_right, rcp, tp_rank, mode='eval',
                 **kwargs):
-        n, m = len(SU), len(SV)
-        tp = int(tp_rank)
-        x = input.reshape(-1, n)
-        bs = x.shape[0]
-        if x.dtype not in (torch.float16, torch.float32):
-            x = x.float()
-        if mode == 'train-fixW':
-            y = ((x.float() * SU).to(self.internal_dtype) @ self.hatW.T).float() * self._sv_scaled(SV)
-            return y.view(*input.shape[:-1], m).to(input.dtype)
-        if mode != 'eval':
+        if mode == 'eval':
+            # x * SU -> Hadamard^T (per chunk when row-parallel) -> / 32 -> fp16; decode + product; Hadamard (per chunk when
+            # column-parallel) -> * SV * 32: one native call (csrc/host.cpp), whose cost the host does not notice
+            cb, dev = self._modules['cb'], input.device
+            out, launches = _lib.host().linear_forward(input, trellis, cb.tlut, SU, SV, self._hadk_bits(0, had_left, dev), K_left or 1,
+                                                       self._hadk_bits(1, had_right, dev), K_right or 1, cb.code, cb.K, self.has_kernel,
+                                                       rcp, int(tp_rank), self.workspace)
+            ops.launch_count += launches
+            return out
+        if mode != 'train-fixW':
             raise NotImplementedError(f"mode {mode!r}: only 'eval' and 'train-fixW' are built")
-
-        # input side: x * SU -> Hadamard^T (per chunk when row-parallel) -> / 32 -> fp16
-        seg_n = n // tp if rcp == 1 else n
-        xh = ops.rht(x.reshape(-1, seg_n), sign_in=SU, hadk_bits=ops.hadk_bits_for(had_left, x.device),
-                     kfac=K_left or 1, transpose=True, scale=1.0 / (math.sqrt(seg_n) * self.scale),
-                     out_dtype=torch.float16).reshape(bs, n)
-
-        v1 = self.cb.code in (ops.CODE_3INST, ops.CODE_1MAD)
-        if v1 and ops.gemm_plain_supported(m, n, bs):
-            # compute codes: the tensor-core kernel decodes eight states per 44-bit window and is the faster one at
-            # every batch size it takes (it needs whole 128 x 64 tiles)
-            y = ops.decompress_gemm_plain(trellis, xh, self.cb.code, self.cb.K, m, n)
-        elif bs <= ops.MAX_MATVEC_BATCH:
-            if self.has_kernel:
-                y = ops.decompress_matvec(trellis, xh, self.cb.tlut, self.cb.K, m, n, workspace=self.workspace)
-            else:
-                y = ops.decompress_matvec_plain(trellis, xh, self.cb.code, self.cb.K, m, n, workspace=self.workspace)
-        elif self.has_kernel and ops.gemm_supported(m, n, bs):
-            # batches 9..128: decode inside the tensor-core GEMM, the dense matrix never exists
-            y = ops.decompress_gemm(trellis, xh, self.cb.tlut, self.cb.K, m, n)
-        else:
-            # anything else: decode once, dense fp16 GEMM (BitshiftLinearKernelAG upstream, bitshift.py:476-489)
-            y = (xh @ self.decode(trellis, m, n).T).float()
-
-        # output side: Hadamard (per chunk when column-parallel) -> * SV * 32
-        seg_m = m // tp if rcp == 2 else m
-        out = ops.rht(y.reshape(-1, seg_m), sign_out=self._sv_scaled(SV), hadk_bits=ops.hadk_bits_for(had_right, x.device),
-                      kfac=K_right or 1, transpose=False, scale=1.0 / math.sqrt(seg_m),
-                      out_dtype=input.dtype if input.dtype in (torch.float16, torch.float32) else torch.float32)
-        return out.reshape(*input.shape[:-1], m).to(input.dtype)
+        n, m = len(SU), len(SV)
+        x = input.reshape(-1, n)
+        y = ((x.float() * SU).to(self.internal_dtype) @ self.hatW.T).float() * self._sv_scaled(SV)
+        return y.view(*input.shape[:-1], m).to(input.dtype)

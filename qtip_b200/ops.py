@@ -111,18 +111,10 @@ def hadk_bits_for(hadK, device):
 # ---------------------------------------------------------------------------------------------
 # workspace for the fused matvec (ticket counters + partial sums), zeroed once at allocation
 # ---------------------------------------------------------------------------------------------
-_workspaces = {}
-
-
 def matvec_workspace(m, n, bs, device):
     """A zero-initialised workspace tensor private to (device, current stream)."""
-    need = _lib.load().qtip_matvec_workspace_bytes(m, n, bs)
-    key = (torch.device(device).index, _stream())
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(max(need, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    index = torch.device(device).index
+    return _lib.host().matvec_workspace(torch.cuda.current_device() if index is None else index, m, n, bs)
 
 
 # ---------------------------------------------------------------------------------------------
@@ -510,13 +502,10 @@ def linear_fused(descs, K, m, n, bs=1):
     launch_count += 1
 
 
-_gemm_status = {}
-
-
 def gemm_status(device):
     """The status word of decompress_gemm on `device` (0 = every launch so far completed its waits)."""
-    t = _gemm_status.get(torch.device(device).index)
-    return 0 if t is None else int(t.item())
+    index = torch.device(device).index
+    return int(_lib.host().gemm_status(torch.cuda.current_device() if index is None else index).item())
 
 
 def decompress_gemm(codes, x, tlut, K, m, n, out=None):
@@ -528,12 +517,10 @@ def decompress_gemm(codes, x, tlut, K, m, n, out=None):
     bs = x.shape[0]
     if out is None:
         out = torch.empty(bs, m, dtype=torch.float32, device=x.device)
-    key = x.device.index
-    if key not in _gemm_status:
-        _gemm_status[key] = torch.zeros(1, dtype=torch.int32, device=x.device)
+    status = _lib.host().gemm_status(x.device.index)
     with torch.cuda.device(x.device):
         st = _lib.load().qtip_decompress_gemm(out.data_ptr(), codes.data_ptr(), x.data_ptr(), tlut.data_ptr(), K, m, n, bs,
-                                              _gemm_status[key].data_ptr(), _stream())
+                                              status.data_ptr(), _stream())
     _lib.check(st, "qtip_decompress_gemm")
     global launch_count
     launch_count += 1
@@ -550,12 +537,10 @@ def decompress_gemm_plain(codes, x, code, K, m, n, out=None):
     bs = x.shape[0]
     if out is None:
         out = torch.empty(bs, m, dtype=torch.float32, device=x.device)
-    key = x.device.index
-    if key not in _gemm_status:
-        _gemm_status[key] = torch.zeros(1, dtype=torch.int32, device=x.device)
+    status = _lib.host().gemm_status(x.device.index)
     with torch.cuda.device(x.device):
         st = _lib.load().qtip_decompress_gemm_plain(out.data_ptr(), codes.data_ptr(), x.data_ptr(), code, K, m, n, bs,
-                                                    _gemm_status[key].data_ptr(), _stream())
+                                                    status.data_ptr(), _stream())
     _lib.check(st, "qtip_decompress_gemm_plain")
     global launch_count
     launch_count += 1

@@ -507,3 +507,24 @@ def test_cache_hatw_dense_path_matches_fused_path():
         mod.SU.copy_(torch.from_numpy(lay["SU"])); mod.SV.copy_(torch.from_numpy(lay["SV"]))
     x = torch.from_numpy(lay["x"]).to(DEV)
     assert rel_l2(qd(x).float().cpu().numpy(), q(x).float().cpu().numpy()) < 3e-3
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(0, 256), (256,), (3, 256), (2, 6, 256), (150, 256)])
+def test_native_layer_call_input_forms(dtype, shape):
+    """Every form of input the module takes: empty, one vector, leading dimensions, a strided view, each dtype."""
+    m, n, K = 384, 256, 2
+    lay = synth.make_layer(m, n, K, seed=31)
+    q = QuantizedLinear(n, m, 16, 16, 16, K, 2, 9, "quantlut_sym").to(DEV)
+    for name in ("tlut", "SU", "SV"):
+        getattr(q, name).copy_(torch.from_numpy(lay[name]))
+    q.trellis.copy_(t16(lay["codes"]))
+    x = torch.randn(*shape[:-1], 2 * n, device=DEV).to(dtype)[..., ::2]
+    y = q(x)
+    assert y.dtype == dtype and y.shape == (*shape[:-1], m)
+    if y.numel():
+        want = C.layer_forward(x.reshape(-1, n).float().cpu().numpy(), lay["codes"], m, n, K, lay["tlut"], lay["SU"].astype(np.float32),
+                               lay["SV"], q.had_left, q.had_right.cpu().numpy())
+        assert rel_l2(y.reshape(-1, m).float().cpu().numpy(), want) < (4e-3 if dtype == torch.bfloat16 else 1e-3)
+    with pytest.raises(RuntimeError):
+        q(x.cpu())
