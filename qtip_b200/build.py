@@ -12,7 +12,7 @@ SO = os.path.join(HERE, "libqtip_b200.so")
 HOST_SRC = os.path.join(CSRC, "host.cpp")
 HOST_SO = os.path.join(HERE, "_host.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
-              "-Xcompiler", "-fPIC", "-shared"]
+              "-Xcompiler", "-fPIC", "-shared", "--threads", "0"]
 
 
 def sources():

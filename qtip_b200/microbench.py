@@ -128,9 +128,9 @@ def time_viterbi(N):
     g = torch.Generator(device=dev).manual_seed(11)
     X = torch.randn(N, 256, generator=g, device=dev).half()
     tlut = torch.randn(512, 2, generator=g, device=dev)
-    for mode, Ks in (("quantlut_sym", (2, 3, 4)), ("3inst", (2, 3, 4)), ("1mad", (2,))):
+    for mode, Ks in (("quantlut_sym", (2, 3, 4)), ("3inst", (2, 3, 4)), ("1mad", (2, 3, 4))):
         for K in Ks:
-            ops.viterbi_quantize(X[:256], mode, K, tlut=tlut)
+            ops.viterbi_quantize(X, mode, K, tlut=tlut)      # warm-up, and the workspace of this size
             torch.cuda.synchronize()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()

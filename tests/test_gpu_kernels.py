@@ -108,6 +108,21 @@ def test_viterbi_quantize_short_and_long_sequences(mode, K, T, N):
     assert np.array_equal(cost.cpu().numpy().view(np.uint32), want_cost.view(np.uint32))
 
 
+@pytest.mark.parametrize("mode,K,T", [("quantlut_sym", 2, 12), ("quantlut_sym", 2, 20), ("quantlut_sym", 3, 28), ("quantlut_sym", 4, 36),
+                                      ("3inst", 2, 22), ("3inst", 3, 14), ("3inst", 4, 10), ("1mad", 2, 18), ("1mad", 3, 26), ("1mad", 4, 6)])
+def test_viterbi_quantize_trace_depths(mode, K, T):
+    """Walk lengths whose back-trace starts and stops inside a tree of stored rows (odd halves, partial depths), with tied
+    candidates (repeated values), against the C restatement."""
+    rng = np.random.default_rng(T * K)
+    V = 2 if mode == "quantlut_sym" else 1
+    tlut32 = np.round(rng.standard_normal((512, 2)) * 2).astype(np.float32) / 2
+    X = (np.round(rng.standard_normal((5, T)) * 2) / 2).astype(np.float16)
+    want, want_cost = C.viterbi_quantize(X, K, V, O.recons_table(ops.CODE_IDS[mode], tlut32))
+    got, cost = ops.viterbi_quantize(torch.from_numpy(X).to(DEV), mode, K, tlut=torch.from_numpy(tlut32), return_cost=True)
+    assert np.array_equal(got.cpu().numpy(), want)
+    assert np.array_equal(cost.cpu().numpy().view(np.uint32), want_cost.view(np.uint32))
+
+
 def test_producers_smallest_shapes():
     """One tile / one block: pack_trellis on a single tile, the layout shuffles on a single 32 x 32 block."""
     rng = np.random.default_rng(3)
