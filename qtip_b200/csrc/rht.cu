@@ -19,39 +19,12 @@
 //
 // Launched with programmatic stream serialization: the hadK sign table (weights) is expanded
 // before griddepcontrol.wait, activations are touched after it.
-#include "fwht.cuh"
+#include "rht.cuh"
 
 namespace qtip {
 namespace {
 
 constexpr int kRhtThreads = 1024;
-
-struct RhtArgs {
-    void *out; const void *in; const void *sign_in; const float *sign_out; const uint32_t *hadk_bits;
-    const __half *residual; __half *residual_out; const __half *norm_weight; const __half *gate;
-    long in_row_stride;  // elements between input rows (0 = every row reads the same input)
-    int out_dtype, in_dtype, sign_in_dtype;
-    int n, p, sign_rep, kfac, transpose;
-    int rpc;             // hadK output rows per CTA (4, 8 or 16)
-    int part_offset;     // float offset in shared memory of the partial-product buffer (short rows only)
-    int sgn_offset;      // float offset of the staged sign_out slice (short rows only, else 0)
-    int vec_ok;          // every buffer is 16-byte aligned and n, strides are multiples of 8: 8-wide loads / stores
-    float scale, eps;
-};
-
-__device__ __forceinline__ float load_elem(const void *p, int dtype, size_t i) {
-    return dtype == QTIP_F16 ? __half2float(static_cast<const __half *>(p)[i]) : static_cast<const float *>(p)[i];
-}
-
-// 8 consecutive elements starting at element i (i % 8 == 0, base pointers 16-byte aligned)
-__device__ __forceinline__ void load8(const void *p, int dtype, size_t i, float (&o)[8]) {
-    if (dtype == QTIP_F16) load8_f16(static_cast<const __half *>(p), i, o);
-    else load8_f32(static_cast<const float *>(p), i, o);
-}
-__device__ __forceinline__ void store8(void *p, int dtype, size_t i, const float (&o)[8]) {
-    if (dtype == QTIP_F16) store8_f16(static_cast<__half *>(p), i, o);
-    else store8_f32(static_cast<float *>(p), i, o);
-}
 
 // 8 values from one (fp16) or two (fp32) raw 16-byte registers
 __device__ __forceinline__ void unpack_raw(const uint4 *r, int dtype, float (&o)[8]) {
@@ -399,6 +372,15 @@ int launch_rht(RhtArgs a, long rows, void *stream) {
     int p = 0;
     while ((1 << p) < len) p++;
     a.p = p;
+    {
+        const void *ptrs[] = {a.out, a.in, a.residual, a.residual_out, a.gate, a.sign_in, a.sign_out, a.norm_weight};
+        bool ok = (a.n % 8 == 0) && (a.in_row_stride % 8 == 0);
+        for (const void *q : ptrs) ok = ok && aligned(q, 16);
+        a.vec_ok = ok ? 1 : 0;
+    }
+    int status = QTIP_OK;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (launch_rht_cluster(a, rows, s, status) || launch_rht_rows(a, rows, s, status)) return status;
     // rows of the factor matrix per CTA: 8, or 4 when a row is long - a thread keeps at most 4 x 4 products
     // in registers, so (rpc / 4) * len <= 4 * kRhtThreads
     a.rpc = len >= 1024 ? 4 : 8;
@@ -415,12 +397,6 @@ int launch_rht(RhtArgs a, long rows, void *stream) {
         words += (size_t)a.rpc * len;
     }
     const size_t smem = words * sizeof(float);
-    {
-        const void *ptrs[] = {a.out, a.in, a.residual, a.residual_out, a.gate, a.sign_in, a.sign_out, a.norm_weight};
-        bool ok = (a.n % 8 == 0) && (a.in_row_stride % 8 == 0);
-        for (const void *q : ptrs) ok = ok && aligned(q, 16);
-        a.vec_ok = ok ? 1 : 0;
-    }
     if (smem > 227 * 1024) return QTIP_ERR_BAD_SHAPE;
     static bool attr_set[64] = {};
     int dev = 0;

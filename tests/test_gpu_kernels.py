@@ -326,6 +326,34 @@ def test_rht_vs_oracle(n):
     assert rel_l2(got.cpu().numpy(), O.hadamard(xh.astype(np.float32), hkn)) < 1e-5
 
 
+@pytest.mark.parametrize("n", [96, 1376, 2240, 2496, 3328, 5120, 11008, 13824, 14336, 22016, 24576, 28672, 53248])
+@pytest.mark.parametrize("rows", [1, 3, 28, 75, 151])
+@pytest.mark.parametrize("kind", ["fp16", "fp32", "wide"])
+def test_rht_factor_rows(n, rows, kind):
+    """Factor widths over every split of the work (rows of the view of 8..2048 columns, parts of a row, clusters, whole rows),
+    both directions: fp16 activations with signs (exact operands), fp32 values, and fp32 rows whose magnitudes differ by
+    many orders (scaled heads and remainders)."""
+    g = torch.Generator(device=DEV).manual_seed(n + rows)
+    k = ops.had_factor(n)
+    H = ops.get_hadK(n)[0].to(DEV)
+    bits = ops.pack_hadk(H)
+    x = torch.randn(rows, n, generator=g, device=DEV)
+    if kind == "wide":
+        x = x * 10.0 ** torch.linspace(-30, 30, rows, device=DEV)[:, None] * 10.0 ** torch.linspace(-4, 0, n, device=DEV)
+    x = x.half() if kind == "fp16" else x
+    su = (torch.randn(n, generator=g, device=DEV).sign() + 1e-5).sign().half()
+    sv = torch.randn(n, generator=g, device=DEV)
+    hh = torch.ones(1, 1, dtype=torch.float64, device=DEV)
+    while hh.shape[0] < n // k:
+        hh = torch.cat([torch.cat([hh, hh], 1), torch.cat([hh, -hh], 1)], 0)
+    for transpose in (False, True):
+        F = (H.T if transpose else H).double()
+        want = torch.einsum("ik,rkj,jl->ril", F, (x.double() * su.double()).view(rows, k, n // k), hh).reshape(rows, n) * sv.double() / n**0.5
+        got = ops.rht(x, sign_in=su, sign_out=sv, hadk_bits=bits, kfac=k, transpose=transpose, scale=1 / n**0.5, out_dtype=torch.float32)
+        err = (got.double() - want).norm(dim=1) / want.norm(dim=1)
+        assert float(err.max()) < 1e-6
+
+
 def test_rht_chunked_signs():
     """Per-chunk transforms of the tensor-parallel layouts: rows cycle through the chunks of the sign vector."""
     rng = np.random.default_rng(0)
