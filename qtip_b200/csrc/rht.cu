@@ -17,6 +17,10 @@
 // prologue options replace the residual add, LlamaRMSNorm (model/llama.py:129-136) and the
 // SwiGLU product (model/llama.py:399-400) kernels that would otherwise run in between.
 //
+// This kernel takes every width and alignment; launch_rht hands the aligned widths of layers to the kernels of rht_pow2.cu and
+// rht_factor.cu, so what remains are rows below 1024, unaligned buffers, and factor widths with rows of the view below 8 or
+// above 2048 values.
+//
 // Launched with programmatic stream serialization: the hadK sign table (weights) is expanded
 // before griddepcontrol.wait, activations are touched after it.
 #include "rht.cuh"
@@ -37,55 +41,6 @@ __device__ __forceinline__ void unpack_raw(const uint4 *r, int dtype, float (&o)
 #pragma unroll
         for (int k = 0; k < 8; k++) o[k] = f[k];
     }
-}
-
-// Power-of-two n = 1024*E with vector-aligned buffers: a thread owns E consecutive values and the whole
-// row stays in registers (fwht_regs); shared memory is used for one transpose only.
-template <int E>
-__device__ __forceinline__ void rht_regs(const RhtArgs &a, float *buf, float *scratch) {
-    const int n = a.n;
-    const long row = blockIdx.y;
-    const size_t sign_off = (size_t)(row % a.sign_rep) * n;
-    const size_t in_off = (size_t)row * a.in_row_stride, out_off = (size_t)row * n;
-    const size_t j = (size_t)threadIdx.x * E;
-    const size_t jo = (size_t)((threadIdx.x & 31) * 32 + (threadIdx.x >> 5)) * E;   // ownership after the transform
-    float v[E], rs[E], wn[E], gt[E], sg[E], so[E];
-    if (a.in_dtype == QTIP_F16) loadE_f16<E>(static_cast<const __half *>(a.in), in_off + j, v);
-    else loadE_f32<E>(static_cast<const float *>(a.in), in_off + j, v, false);
-    if (a.residual) loadE_f16<E>(a.residual, in_off + j, rs);
-    if (a.norm_weight) loadE_f16<E>(a.norm_weight, j, wn);
-    if (a.gate) loadE_f16<E>(a.gate, in_off + j, gt);
-    if (a.sign_in) {
-        if (a.sign_in_dtype == QTIP_F16) loadE_f16<E>(static_cast<const __half *>(a.sign_in), sign_off + j, sg);
-        else loadE_f32<E>(static_cast<const float *>(a.sign_in), sign_off + j, sg, false);
-    }
-    if (a.sign_out) loadE_f32<E>(a.sign_out, sign_off + jo, so, false);
-    if (a.residual) {
-#pragma unroll
-        for (int k = 0; k < E; k++) v[k] = __half2float(__float2half_rn(v[k] + rs[k]));
-        if (a.residual_out && (a.in_row_stride != 0 || row == 0)) storeE_f16<E>(a.residual_out, in_off + j, v);
-    }
-    if (a.norm_weight) {
-        float ss = 0.f;
-#pragma unroll
-        for (int k = 0; k < E; k++) ss += v[k] * v[k];
-        const float r = rsqrtf(block_sum(ss, scratch) / (float)n + a.eps);
-#pragma unroll
-        for (int k = 0; k < E; k++) v[k] = __half2float(__hmul(__float2half_rn(wn[k]), __float2half_rn(v[k] * r)));
-    }
-#pragma unroll
-    for (int k = 0; k < E; k++) {
-        if (a.gate) v[k] = swiglu_fp16(gt[k], v[k]);
-        if (a.sign_in) v[k] *= sg[k];
-    }
-    fwht_regs<E>(v, buf);
-#pragma unroll
-    for (int k = 0; k < E; k++) {
-        v[k] *= a.scale;
-        if (a.sign_out) v[k] *= so[k];
-    }
-    if (a.out_dtype == QTIP_F16) storeE_f16<E>(static_cast<__half *>(a.out), out_off + jo, v);
-    else storeE_f32<E>(static_cast<float *>(a.out), out_off + jo, v);
 }
 
 __global__ void __launch_bounds__(kRhtThreads) rht_kernel(const RhtArgs a) {
@@ -134,11 +89,6 @@ __global__ void __launch_bounds__(kRhtThreads) rht_kernel(const RhtArgs a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    if (kfac == 1 && vec && (n == 4096 || n == 8192)) {
-        if (n == 4096) rht_regs<4>(a, v, scratch);
-        else rht_regs<8>(a, v, scratch);
-        return;
-    }
     const bool write_res = a.residual_out && blockIdx.x == 0 && (a.in_row_stride != 0 || row == 0);
     float ss = 0.f;
     if (vec && !a.residual && !a.norm_weight) {
@@ -380,7 +330,7 @@ int launch_rht(RhtArgs a, long rows, void *stream) {
     }
     int status = QTIP_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (launch_rht_cluster(a, rows, s, status) || launch_rht_rows(a, rows, s, status)) return status;
+    if (launch_rht_pow2(a, rows, s, status) || launch_rht_cluster(a, rows, s, status) || launch_rht_rows(a, rows, s, status)) return status;
     // rows of the factor matrix per CTA: 8, or 4 when a row is long - a thread keeps at most 4 x 4 products
     // in registers, so (rpc / 4) * len <= 4 * kRhtThreads
     a.rpc = len >= 1024 ? 4 : 8;

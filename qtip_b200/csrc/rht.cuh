@@ -1,4 +1,4 @@
-// Arguments and element helpers shared by the Hadamard-transform kernels (rht.cu, rht_factor.cu).
+// Arguments and element helpers shared by the Hadamard-transform kernels (rht.cu, rht_factor.cu, rht_pow2.cu).
 #pragma once
 
 #include "fwht.cuh"
@@ -98,7 +98,12 @@ __device__ __forceinline__ float cluster_sum(float x, float *scratch, int csize)
     return t;
 }
 
+// Shared memory that only one CTA per SM can have.  A launch of about one CTA per SM asks for it: with programmatic stream
+// serialization it is placed while its predecessor still occupies most SMs, and would otherwise crowd onto the free ones.
+constexpr int kOnePerSm = 120 * 1024;
+
 // Launchers of the specialised kernels: false if the kernel does not apply, else `status` is the launch's result.
+bool launch_rht_pow2(const RhtArgs &a, long rows, cudaStream_t s, int &status);       // rht_pow2.cu
 bool launch_rht_cluster(const RhtArgs &a, long rows, cudaStream_t s, int &status);    // rht_factor.cu: few rows
 bool launch_rht_rows(const RhtArgs &a, long rows, cudaStream_t s, int &status);       // rht_factor.cu: many rows
 

@@ -637,7 +637,7 @@ bool launch_rht_rows(const RhtArgs &a, long rows, cudaStream_t s, int &status) {
     // Threads: a row's vector pairs spread so that a thread holds at most four of them in registers.  Few rows: more
     // threads, to have more of the row in flight at once.
     const long want_parts = sm_count() / rows;
-    const bool few = want_parts > 1;
+    const bool few = want_parts >= 1;
     const int threads = a.n > 16384 || (few && a.n > 4096) ? 512 : (a.n > 4096 || few ? 256 : 128), warps = threads / 32;
     const int npairs = a.n / 16, hold = (npairs + threads - 1) / threads;
     // Columns of a warp's task: the whole row of the view or 64 of it; fewer when the CTA would have idle warps otherwise.

@@ -354,6 +354,36 @@ def test_rht_factor_rows(n, rows, kind):
         assert float(err.max()) < 1e-6
 
 
+@pytest.mark.parametrize("n", [1024, 2048, 4096, 8192, 16384, 32768, 65536])
+@pytest.mark.parametrize("rows", [1, 5, 28, 149])
+def test_rht_pow2_rows(n, rows):
+    """Power-of-two rows over every split (several rows per CTA with a partly filled last one, one row per CTA, clusters), with
+    the whole prologue: residual add, RMSNorm, SwiGLU gate and signs."""
+    g = torch.Generator(device=DEV).manual_seed(n + rows)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    x, res, gate = r(rows, n).half(), r(rows, n).half(), r(rows, n).half()
+    w, su, sv = (1 + 0.1 * r(n)).half(), (r(n).sign() + 1e-5).sign().half(), r(n)
+
+    def transform(v):
+        v, h = v.double().clone(), 1
+        while h < n:
+            v = v.view(-1, n // (2 * h), 2, h)
+            v = torch.stack((v[:, :, 0] + v[:, :, 1], v[:, :, 0] - v[:, :, 1]), 2).reshape(-1, n)
+            h *= 2
+        return v / n**0.5
+    got = ops.rht(x.float(), sign_in=su, sign_out=sv, scale=1 / n**0.5)
+    want = transform(x.double() * su.double()) * sv.double()
+    assert float(((got - want).norm(dim=1) / want.norm(dim=1)).max()) < 1e-6
+    out, res_out = torch.empty(rows, n, device=DEV), torch.empty_like(x)
+    ops.rht_fused(x, rows, n, out, residual=res, residual_out=res_out, norm_weight=w, eps=1e-5, gate=gate, sign_in=su, scale=1 / n**0.5)
+    s = x + res
+    assert torch.equal(res_out, s)
+    v = w * (s.float() * torch.rsqrt(s.float().pow(2).mean(-1, keepdim=True) + 1e-5)).half()
+    v = torch.nn.functional.silu(gate.float()).half() * v
+    want = transform(v.double() * su.double())
+    assert float(((out - want).norm(dim=1) / want.norm(dim=1)).max()) < 1e-3
+
+
 def test_rht_chunked_signs():
     """Per-chunk transforms of the tensor-parallel layouts: rows cycle through the chunks of the sign vector."""
     rng = np.random.default_rng(0)
