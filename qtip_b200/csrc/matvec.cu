@@ -4,34 +4,31 @@
 // 16x16 tiles, 128*K contiguous bytes; the blocks of one 32-row block are contiguous).  The grid
 // has at most one CTA (32 warps) per SM.  Two schedules exist and the host picks the cheaper one:
 //   rows     CTA c owns whole 32-row blocks c, c+G, ...: no cross-CTA reduction at all;
-//   stream-K CTA c owns the contiguous block range [c*B/G, (c+1)*B/G), cut into segments at
-//            row-block boundaries: perfectly balanced bytes, but row blocks shared by several
-//            CTAs need the ticket reduction below.
+//   stream-K CTA c owns the contiguous block range [c*B/G, (c+1)*B/G): perfectly balanced, but row blocks shared
+//            by two CTAs need the ticket reduction below.
+// The warps of a CTA share its blocks without meeting until the end of a round of several row blocks: each owns either a
+// fixed 32nd of every row block or one contiguous run (see PIECES), and leaves its sums of a row block in a slot of its own.
 //
-// Data path.  Inside a segment warp w owns a CONTIGUOUS run of blocks (1/32 of the segment).  It pulls the
-// run in chunks of up to 1 KiB with one bulk copy (cp.async.bulk, the 1-D form of TMA) per chunk into a
-// two-slot ring of its own in shared memory, completion on an mbarrier of its own; the next chunk -
-// of this or of the following segment - is always in flight while one is decoded (up to 64 KiB in
-// flight per SM, no registers held, no load-latency stalls in the loop).  A lane reads its 4K bytes of a
-// block and those of lane+1 (the wrap-around bits of the tail-biting stream) from the ring, so the loop
-// has no shuffles.  A lane decodes its 16 trellis states into four mma.m16n8k16 A
-// fragments in registers - HYB: h = s*(s+1), entry (h>>6)&1023 of a 1024-entry table (the 512-entry
-// LUT and its sign-flipped twin) kept as 32 lane-private copies in shared memory, so gathers never
-// conflict - and multiplies them with x held in the B fragment (column j of B = batch row j, so up
-// to 8 batch rows share one decode).  fp32 accumulation in the MMA.  x is staged once per CTA
-// in shared memory in fragment order (one 16-byte load per block and lane) when it fits beside the
-// table; 8 rows of a wide layer do not, and are then read from L1/L2 per block (about 1.5x the time
-// of a single row).
+// Data path.  A warp pulls its blocks in chunks of up to 1 KiB with one bulk copy (cp.async.bulk, the 1-D form of TMA) per
+// chunk into a two-slot ring of its own in shared memory, completion on an mbarrier of its own; the next chunk is always in
+// flight while one is decoded (up to 64 KiB in flight per SM, no registers held, no load-latency stalls in the loop).  A lane
+// reads its 4K bytes of a block and those of lane+1 (the wrap-around bits of the tail-biting stream) from the ring, so the loop
+// has no shuffles.  A lane decodes its 16 trellis states into four mma.m16n8k16 A fragments in registers - HYB: h = s*(s+1),
+// entry (h>>6)&1023 of a 1024-entry table (the 512-entry LUT and its sign-flipped twin) kept as 32 lane-private copies in
+// shared memory, so gathers never conflict - and multiplies them with x held in the B fragment (column j of B = batch row j,
+// so up to 8 batch rows share one decode).  fp32 accumulation in the MMA.  x is staged once per CTA in shared memory in
+// fragment order (one 16-byte load per block and lane) when it fits beside the table; longer x is put into that order once per
+// launch in global memory and travels through the ring with the codes.
 //
-// The kernel is instruction-issue bound, not HBM bound (about 5 instructions per state are
-// irreducible: shift, multiply-add hash, mask, multiply-add address, shared load; multiply-add, logic
-// and shift instructions each issue once per two cycles per sub-partition on this part).  The ring costs about one instruction per block because it is
-// private to a warp: no producer warp, no CTA barrier, one bounded mbarrier wait per chunk.
+// The kernel is instruction-issue bound, not HBM bound (about 5 instructions per state are irreducible: shift, multiply-add
+// hash, mask, multiply-add address, shared load).  The decode loop alone, on resident data, takes 28 cycles per block and SM
+// (K = 2), with the ring 31; in the kernel 35.  A launch adds about 4000 cycles before the loop (table, x) and, for shared
+// row blocks, 4500 after it.  Measured, K = 2, against one CTA barrier and reduction per row block and four blocks unrolled
+// (microseconds): 28672 x 8192 1 row 43.1 -> 38.7, 5 rows 58.1 -> 47.8; 22016 x 4096 18.3 -> 16.2; 4096 x 4096 5.6 -> 5.4.
 //
-// Reduction.  Warps of a CTA are summed through shared memory at the end of a segment.  When a
-// row block is shared by several CTAs each stores its partial sums to the workspace and takes a
-// ticket; the CTA that draws the last ticket adds the partials in CTA order and writes the result,
-// so the output is deterministic and is overwritten, never accumulated into.
+// Reduction.  Slots are summed in warp order at the end of a round.  When a row block is shared by several CTAs each stores
+// its partial sums to the workspace and takes a ticket; the CTA that draws the last ticket adds the partials in CTA order and
+// writes the result, so the output is deterministic and is overwritten, never accumulated into.
 //
 // Launch overlap.  The kernel is launched with programmatic stream serialization: everything that
 // touches only weights (the first code loads, the table build) runs before griddepcontrol.wait,
@@ -66,7 +63,8 @@ constexpr int kMaxBatch = 8;
 // [0, 64 KiB)   ticket counters, one uint32 per 32-row block (m <= 524288); zero between calls
 // [64 KiB, +256) word 0: counter of finished CTAs (fused output transform); zero between calls
 //               word 1: sticky flag, set if a wait for a bulk copy ever ran out (never cleared by the kernels)
-// [.., end)     partial sums: [row block][contributor][8 batch x 32 rows] fp32
+// [.., ..)      partial sums: [row block][contributor][8 batch x 32 rows] fp32
+// [.., end)     x of the call in fragment order, when it is too long for shared memory
 constexpr size_t kCounterBytes = 64 * 1024;
 constexpr size_t kPartialOffset = kCounterBytes + 256;
 constexpr int kMaxGrid = 1024;  // sizing bound for the number of CTAs
@@ -86,19 +84,19 @@ struct Partition {
     int mode;
 };
 
-// Cost model in bytes streamed by the busiest SM; the ticket reduction of a shared row block costs
-// about as much time as streaming kTailBytes.
-constexpr long kTailBytes = 40 * 1024;
+// Cost in blocks decoded by the busiest warp.  A row block shared by several CTAs costs a round trip through the workspace at the
+// end (partials, fence, ticket, sum: 4500 cycles, the time of kTailBlocks blocks per warp).
+constexpr long kTailBlocks = 4;
 
 // nprob problems of the same shape share one launch: each gets sm_count / nprob CTAs.
-Partition make_partition(int m, int n, int K, int nprob = 1) {
+Partition make_partition(int m, int n, int nprob = 1) {
     Partition p;
-    const long mb = m >> 5, nb = n >> 5, B = mb * nb, bb = 128 * K;
+    const long mb = m >> 5, nb = n >> 5, B = mb * nb, W = kConsumerWarps;
     const long sms = sm_count() / nprob > 0 ? sm_count() / nprob : 1;
     const long g_stream = B < sms ? B : sms, g_rows = mb < sms ? mb : sms;
-    const long cost_rows = ((mb + g_rows - 1) / g_rows) * nb * bb;
+    const long cost_rows = ((mb + g_rows - 1) / g_rows * nb + W - 1) / W;
     const bool shared_rows = (B % g_stream) != 0 || ((B / g_stream) % nb) != 0;
-    const long cost_stream = ((B + g_stream - 1) / g_stream) * bb + (shared_rows ? kTailBytes : 0);
+    const long cost_stream = ((B + g_stream - 1) / g_stream + W - 1) / W + (shared_rows ? kTailBlocks : 0);
     p.mode = cost_rows <= cost_stream ? kModeRows : kModeStreamK;
     p.grid = (int)(p.mode == kModeRows ? g_rows : g_stream);
     p.kmax = max_contributors(nb, B, g_stream);
@@ -161,7 +159,8 @@ constexpr unsigned long long kPeerWaitNs = 200ull * 1000ull * 1000ull;
 
 struct Shared {            // control block at the start of dynamic shared memory
     int is_last;
-    int pad_[7];
+    int last_of[2];        // reduce_round: contributors of a shared row block this CTA has to add, or 0
+    int pad_[5];
     float warp_sums[32];   // scratch of block_sum
 };
 static_assert(sizeof(Shared) <= kCtrlBytes, "control block too large");
@@ -312,9 +311,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// One bulk copy global -> shared (addresses and size multiples of 16 bytes), completion counted on `bar`.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
+// Bulk copy global -> shared (addresses and size multiples of 16 bytes), completion counted on `bar`; the bytes of all copies
+// of a phase are announced once.
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
@@ -477,27 +479,118 @@ __device__ __forceinline__ void fused_output_regs(const FusedOut &O, const float
     }
 }
 
-// XS: x is staged once per CTA in shared memory, permuted so that a lane's four B-fragment words of
-// a block are one 16-byte load; otherwise they are read from global memory (L1-resident) per block.
-// db: the cross-warp reduction buffer is double-buffered, which drops one CTA barrier per segment.
+// Eight values of x (quad i of row b) into fragment order: block N, row b, lane t of four, four words
+// { x[32N + 2t], x[.. + 8], x[.. + 16], x[.. + 24] } (pairs); the rows of a block lie together.
+__device__ __forceinline__ void put_fragment(uint32_t *dst, const uint4 *row, int i, int b, int bs) {
+    const uint4 q = __ldg(row + i);
+    const uint32_t wv[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int wi = i * 4 + k, blk = wi >> 4, w = wi & 15;   // 16 words per 32-column block
+        dst[(blk * bs + b) * 16 + (w & 3) * 4 + (w >> 2)] = wv[k];
+    }
+}
+
+// x of a launch whose activations travel through the ring, once for all CTAs
+struct FragmentArgs {
+    const __half *x[kMaxProblems];
+    uint32_t *frag[kMaxProblems];
+};
+__global__ void __launch_bounds__(256) x_fragment_kernel(const __grid_constant__ FragmentArgs a, int n, int bs) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < (n >> 3)) put_fragment(a.frag[blockIdx.z], reinterpret_cast<const uint4 *>(a.x[blockIdx.z] + (size_t)blockIdx.y * n), i, blockIdx.y, bs);
+}
+
+// The end of a round without pieces: every warp has left the sums of the row blocks it met in slot warp + (row block - rbase) -
+// a warp's blocks are contiguous, so the (warp, row block) pairs that occur are distinct slots - and a row block is the sum
+// over consecutive warps, in warp order.
+template <int NW>
+__device__ __forceinline__ void reduce_round(const float *red, Shared *sh, float *__restrict__ out, float *__restrict__ partial,
+                                             unsigned *__restrict__ counters, int p, int e, int v_begin, int v_end, int rbase, int nb, int B, int G,
+                                             int row0, int rstep, int kmax, int m, int bs, const OutCopies &copies, unsigned stamp) {
+    const int stride = 32 * bs, rows = (e - 1) / nb - rbase + 1;
+    const unsigned cnt = e - p;
+    // the warp that decoded block a of the round: the largest w with w * cnt / NW <= a
+    auto warp_of = [&](int a) { return cnt < (1u << 26) ? (int)(((unsigned)(a + 1) * NW - 1) / cnt) : (int)(((unsigned long long)(a + 1) * NW - 1) / cnt); };
+    for (int idx = threadIdx.x; idx < rows * stride; idx += NW * 32) {
+        const int rr = idx / stride, q = idx - rr * stride, row = rbase + rr;
+        const int a = max(p, row * nb) - p, b = min(e, (row + 1) * nb) - p;
+        const int w_lo = warp_of(a), w_hi = warp_of(b - 1);
+        float v = 0.f;
+        for (int w = w_lo; w <= w_hi; w++) v += red[(w + rr) * stride + q];
+        const long M = row0 + (long)row * rstep;
+        if (row * nb >= v_begin && (row + 1) * nb <= v_end) {
+            const size_t o = (size_t)(q >> 5) * m + 32 * M + (q & 31);
+            out[o] = v;
+            for (int c = 0; c < copies.n; c++) store_stamped(copies.dst[c] + o, v, stamp);
+        } else {
+            const int k = (int)(blockIdx.x - cta_of_block(M * nb, B, G));
+            __stcg(partial + ((size_t)M * kmax + k) * 256 + q, v);
+        }
+    }
+    // at most the first and the last row block of a CTA are shared; their tickets are taken when all blocks are done
+    const int first = v_begin / nb, last = (v_end - 1) / nb;
+    const bool first_shared = first * nb < v_begin || (first + 1) * nb > v_end, last_shared = last != first && (last + 1) * nb > v_end;
+    if (e != v_end || !(first_shared || last_shared)) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const long M = row0 + (threadIdx.x ? last : first);       // stream-K: rstep is 1
+        int contributors = 0;
+        if (threadIdx.x ? last_shared : first_shared) {
+            contributors = (int)(cta_of_block((M + 1) * nb - 1, B, G) - cta_of_block(M * nb, B, G)) + 1;
+            if (atomicAdd(&counters[M], 1u) == (unsigned)(contributors - 1)) counters[M] = 0;      // ready for the next call
+            else contributors = 0;
+        }
+        sh->last_of[threadIdx.x] = contributors;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int contributors = sh->last_of[k];
+        if (contributors == 0) continue;
+        const long M = row0 + (k ? last : first);
+        __threadfence();
+        for (int q = threadIdx.x; q < stride; q += NW * 32) {
+            float s = 0.f;
+            for (int c = 0; c < contributors; c++) s += __ldcg(partial + ((size_t)M * kmax + c) * 256 + q);
+            const size_t o = (size_t)(q >> 5) * m + 32 * M + (q & 31);
+            out[o] = s;
+            for (int c = 0; c < copies.n; c++) store_stamped(copies.dst[c] + o, s, stamp);
+        }
+    }
+}
+
+// How a warp's blocks are cut:
+//   PIECES  (rows mode; one row of x, or one row block per CTA) the w-th 32nd of every row block: the order of the sums depends
+//           on n alone, not on the grid;
+//   else    contiguous runs over the CTA's blocks.
+// Where x comes from:
+//   XS      staged once per CTA in shared memory in fragment order (a lane's four B-fragment words of a block are one 16-byte load);
+//   else    x is too long for that: it lies in global memory in fragment order and every chunk of codes brings its own x along
+//           through the ring.
 // blockIdx.y selects the problem of the batch (all problems have the same m, n, K, bs).
 // TP: the tensor-parallel fields (PeerIn / Signal) are live; the single-GPU instantiation carries none of that code.
-// NW: warps per CTA (32: the register transforms of the fused sides are written for 1024 threads).
-// C:  blocks per bulk copy; xs_offset: byte offset of the staged x in shared memory (the host fits the ring, the
-// reduction buffers, x and the scratch of the fused input side into 227 KiB and picks C accordingly).
-template <int K, bool XS, bool TP, int NW, int C>
-__global__ void __launch_bounds__(NW * 32, 1)
-    matvec_hyb_kernel(const __grid_constant__ MatvecBatch batch, int m, int n, int bs, int kmax, int mode, int db,
-                      int xs_offset, int scratch_offset) {
+// C:  blocks per bulk copy; xs_offset: byte offset of the staged x in shared memory (the host fits the ring, the partial-sum
+// slots, x and the scratch of the fused input side into 227 KiB and picks C accordingly); max_rows: row blocks whose partial sums
+// fit the slots at once.
+enum { kStagedX = 1, kPieces = 2 };
+struct HybLaunch {
+    int kmax, mode, max_rows, xs_offset, scratch_offset;
+    int rows_each, rows_extra;     // rows mode: row blocks per CTA, and how many CTAs have one more
+};
+template <int K, int MODE, bool TP, int C>
+__global__ void __launch_bounds__(kConsumerWarps * 32, 1)
+    matvec_hyb_kernel(const __grid_constant__ MatvecBatch batch, int m, int n, int bs, const __grid_constant__ HybLaunch L) {
+    constexpr bool XS = (MODE & kStagedX) != 0, PIECES = (MODE & kPieces) != 0;
+    const int xs_offset = L.xs_offset, scratch_offset = L.scratch_offset, max_rows = L.max_rows;
     constexpr int kBlockBytes = 128 * K;
-    constexpr int chunk_blocks = C;
-    const bool DB = db != 0;
-    constexpr int kConsumerWarps = NW, kThreads = NW * 32;     // shadow the file-scope defaults
-    constexpr int kWarpShift = NW == 32 ? 5 : 4;
-    static_assert(NW == 32 || NW == 16, "a segment is split over 16 or 32 warps");
+    constexpr int NW = kConsumerWarps, kThreads = NW * 32;
     extern __shared__ __align__(128) uint8_t smem[];
-    // layout: control block (incl. two mbarriers per warp) | LUT | ring slot 0 [NW][chunk] | ring slot 1 [NW][chunk] |
-    //         reduction buffer(s) [NW][bs][32] fp32 | (padding) | x (bs, n) fp16 permuted
+    // layout: control block (incl. two mbarriers per warp) | LUT | ring slot 0 [NW][slot] | ring slot 1 [NW][slot] |
+    //         partial sums [NW + max_rows, or NW * max_rows with pieces][bs][32] fp32 | (padding) | x (bs, n) fp16 permuted
     // The fp32 scratch of the fused input transform lies behind x when everything fits (scratch_offset > 0); otherwise
     // it overlays ring slot 1 and what follows it up to x, and slot 1 is first filled after the transform is done.
     const MatvecProblem &P = batch.p[blockIdx.y];
@@ -507,11 +600,11 @@ __global__ void __launch_bounds__(NW * 32, 1)
     const uint32_t *__restrict__ tlut = P.tlut;
     Shared *sh = reinterpret_cast<Shared *>(smem);
     uint32_t *lut = reinterpret_cast<uint32_t *>(smem + kCtrlBytes);
-    const int slot_bytes = chunk_blocks * kBlockBytes;             // per warp
+    const int xblk_bytes = XS ? 0 : bs * 64;                       // x of a block of columns, when it travels with the codes
+    const int slot_bytes = C * (kBlockBytes + xblk_bytes);         // per warp
     uint8_t *ring = smem + kCtrlBytes + kLutBytes;
-    const int red_floats = kConsumerWarps * 32 * bs;
+    const int stride = 32 * bs;                                    // floats of a partial-sum slot
     float *red = reinterpret_cast<float *>(ring + 2 * NW * slot_bytes);
-    (void)chunk_blocks;
     uint4 *xs = reinterpret_cast<uint4 *>(smem + xs_offset);
     float *fscratch = reinterpret_cast<float *>(scratch_offset > 0 ? smem + scratch_offset : ring + NW * slot_bytes);
 
@@ -523,24 +616,40 @@ __global__ void __launch_bounds__(NW * 32, 1)
     const int G = gridDim.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    // Segment bookkeeping in 32-bit block indices (B = mb*nb < 2^30 is checked by the host).
-    // rows mode: segments are whole row blocks c, c+G, ...; stream-K: [r0, r1) cut at row boundaries.  Both are
-    // "the part of row block M from pos up to min(end, (M+1)*nb), then on to row block M + mstep at seg_end + gap",
-    // so the loops below carry no mode branches and no divisions.
+    // Blocks are numbered row block by row block (B = mb*nb < 2^30 is checked by the host).  stream-K: this CTA's blocks are
+    // [c*B/G, (c+1)*B/G); rows mode: the row blocks c, c + G, ... as if they were consecutive ("virtual" numbering: block v is
+    // column v % nb of row block row0 + (v / nb) * rstep).  A round is as many row blocks as the partial-sum slots hold; without
+    // pieces warp w decodes the w-th 32nd of the round (contiguous memory except across row blocks in rows mode).
     const int B = mb * nb;
-    int pos, end, M, mstep, gap;
-    if (mode == kModeRows) { pos = blockIdx.x * nb; end = B; M = blockIdx.x; mstep = G; gap = (G - 1) * nb; }
-    else {
-        pos = (int)range_start(blockIdx.x, B, G); end = (int)range_start(blockIdx.x + 1, B, G);
-        M = pos / nb; mstep = 1; gap = 0;
+    const bool by_rows = PIECES || L.mode == kModeRows;
+    const int rows_total = L.rows_each + ((int)blockIdx.x < L.rows_extra ? 1 : 0);     // (rows mode)
+    int v_begin, v_end, row0, rstep;
+    if (by_rows) {
+        row0 = blockIdx.x; rstep = G;
+        v_begin = 0; v_end = rows_total * nb;
+    } else {
+        const int r0 = (int)range_start(blockIdx.x, B, G);
+        row0 = r0 / nb; rstep = 1;
+        v_begin = r0 - row0 * nb; v_end = (int)range_start(blockIdx.x + 1, B, G) - row0 * nb;
     }
-    // warp w's run of a segment [p, e): an even split of its blocks, contiguous in memory
-    auto run_of = [&](int p, int e, int &r0, int &r1) {
-        const int cnt = e - p;
-        r0 = p + ((warp * cnt) >> kWarpShift);
-        r1 = p + (((warp + 1) * cnt) >> kWarpShift);
+    int p = v_begin, e = min(v_end, max_rows * nb), rbase = 0;     // the round's blocks [p, e), its first row block rbase
+    const int piece_lo = (int)(((long)warp * nb) >> 5), piece_n = (int)(((long)(warp + 1) * nb) >> 5) - piece_lo;
+    const int seg_n = PIECES ? piece_n : nb;                       // blocks of a segment (what lies in one row block), but for ends
+    // this warp's blocks of a round: first block v (column col of its row block), `left` of the first segment, `total`
+    auto run_of = [&](int &v, int &col, int &left, int &total) {
+        if (PIECES) {
+            col = piece_lo;
+            v = p + piece_lo;
+            left = piece_n;
+            total = min(max_rows, rows_total - rbase) * piece_n;
+        } else {
+            const int cnt = e - p;
+            v = p + (int)(((long)warp * cnt) >> 5);
+            total = p + (int)(((long)(warp + 1) * cnt) >> 5) - v;
+            col = v - v / nb * nb;
+            left = min(total, nb - col);
+        }
     };
-    int seg_end = min(end, (M + 1) * nb);
 
     // The ring of this warp: slot s at ring + (s*NW + warp)*slot_bytes, its barrier at bar_w + 8s.
     const uint32_t ring_w = smem_u32(ring) + warp * slot_bytes;
@@ -549,32 +658,49 @@ __global__ void __launch_bounds__(NW * 32, 1)
     if (lane == 0) { mbar_init(bar_w, 1); mbar_init(bar_w + 8, 1); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncwarp();
-    // Issue cursor: walks this warp's chunks (over all segments of the CTA, in order) one or two chunks ahead of
-    // the decoding; uniform over the warp, lane 0 issues the copy.
-    int i_M = M, i_seg_end = seg_end, i_blk = 0, i_run_end = 0;
-    bool i_valid = pos < end;
+    // Issue cursor: this warp's chunks in order, one or two ahead of the decoding; a chunk does not cross a segment.
+    // Uniform over the warp, lane 0 issues the copies.
+    int i_left, i_total, i_col;
+    const uint8_t *i_ptr;
+    const size_t i_jump = ((size_t)rstep * nb - seg_n) * kBlockBytes;
     unsigned ichunk = 0;
-    if (i_valid) run_of(pos, i_seg_end, i_blk, i_run_end);
-    auto issue = [&]() {
-        while (i_valid && i_blk >= i_run_end) {
-            const int i_pos = i_seg_end + gap;
-            i_M += mstep;
-            if (i_pos >= end) { i_valid = false; break; }
-            i_seg_end = min(end, (i_M + 1) * nb);
-            run_of(i_pos, i_seg_end, i_blk, i_run_end);
-        }
-        if (!i_valid) return;
-        const int nblk = min(chunk_blocks, i_run_end - i_blk);
-        if (lane == 0)
-            bulk_load(ring_w + (ichunk & 1u) * slot_stride, codes + (size_t)i_blk * kBlockBytes, (uint32_t)(nblk * kBlockBytes),
-                      bar_w + (ichunk & 1u) * 8);
-        i_blk += nblk;
-        ichunk++;
+    auto start_issue = [&]() {
+        int v;
+        run_of(v, i_col, i_left, i_total);
+        const int row = PIECES ? 0 : (v - i_col) / nb;             // pieces: the cursor runs on through all rounds
+        i_ptr = codes + ((size_t)(row0 + row * rstep) * nb + i_col) * kBlockBytes;
+        if (PIECES) i_total = rows_total * piece_n;
     };
+    // codes: the packed weights (any time); with x through the ring the x part follows separately for the chunk issued
+    // before the activations may be read
+    auto issue = [&](bool with_x) {
+        if (i_left <= 0) return;
+        const int nblk = min(C, i_left);
+        if (lane == 0) {
+            const uint32_t dst = ring_w + (ichunk & 1u) * slot_stride, bar = bar_w + (ichunk & 1u) * 8;
+            mbar_expect(bar, (uint32_t)(nblk * (kBlockBytes + xblk_bytes)));
+            bulk_copy(dst, i_ptr, (uint32_t)(nblk * kBlockBytes), bar);
+            if (!XS && with_x)
+                bulk_copy(dst + C * kBlockBytes, reinterpret_cast<const uint8_t *>(x) + (size_t)i_col * xblk_bytes,
+                          (uint32_t)(nblk * xblk_bytes), bar);
+        }
+        ichunk++;
+        i_left -= nblk;
+        i_total -= nblk;
+        i_ptr += nblk * kBlockBytes;
+        if (!XS) i_col += nblk;
+        if (i_left == 0) {
+            i_left = min(seg_n, i_total);
+            i_ptr += i_jump;
+            i_col = PIECES ? piece_lo : 0;
+        }
+    };
+    start_issue();
+    const int first_n = min(C, i_left), first_col = i_col;
     // First chunk of this warp: packed codes are weights, so the copy starts before the table build and before
     // waiting for the previous kernel of the stream.
-    issue();
-    if (scratch_offset > 0) issue();      // ring slot 1 is free from the start: second chunk in flight as well
+    issue(false);
+    if (XS && scratch_offset > 0) issue(false);      // ring slot 1 is free from the start: second chunk in flight as well
     if (threadIdx.x == 0) sh->is_last = 0;
     // lane-private LUT copies: entry e = sign << 9 | index, copy l at byte e*128 + l*4; the sign bit
     // flips the sign of the first (low) half of the pair.  Thread t writes the 16-byte groups t, t + kThreads, ...:
@@ -598,18 +724,14 @@ __global__ void __launch_bounds__(NW * 32, 1)
     unsigned stamp = 0u;
     if constexpr (TP) stamp = P.sig.seq ? *reinterpret_cast<const volatile unsigned *>(P.sig.seq) + 1u : 0u;
     if constexpr (XS) {
-        // xs[(b*nb + N)*4 + t] = { x[b][32N+2t..+1], x[..+8..], x[..+16..], x[..+24..] }
-        if (NW == 32 && (P.in.x_raw || P.in.y_prev || (TP && P.peer.n > 0))) {
+        if ((P.in.x_raw || P.in.y_prev || (TP && P.peer.n > 0))) {
             // fused input side (bs == 1, n a power of two): every CTA transforms the activation itself.
             // A thread owns 8 consecutive values; the loads of all operand vectors are issued together so
             // the whole prologue costs one L2 round trip, not one per array.
             const FusedIn &I = P.in;
-#ifndef QTIP_PROLOGUE_SMEM
-            if (NW == 32 && n == 4096) fused_input_regs<4, TP>(I, P.peer, n, xs, fscratch, sh->warp_sums);
-            else if (NW == 32 && n == 8192) fused_input_regs<8, TP>(I, P.peer, n, xs, fscratch, sh->warp_sums);
-            else
-#endif
-            {
+            if (n == 4096) fused_input_regs<4, TP>(I, P.peer, n, xs, fscratch, sh->warp_sums);
+            else if (n == 8192) fused_input_regs<8, TP>(I, P.peer, n, xs, fscratch, sh->warp_sums);
+            else {
             const int nvec = n >> 3;
             int p = 0;
             while ((1 << p) < n) p++;
@@ -716,43 +838,46 @@ __global__ void __launch_bounds__(NW * 32, 1)
             }
             }
         } else {
-            // 4 words (8 values) per thread and trip
-            const uint4 *xw = reinterpret_cast<const uint4 *>(x);
-            const int quads = bs * (n >> 3);
-            for (int i = threadIdx.x; i < quads; i += kThreads) {
-                const uint4 q = __ldg(xw + i);
-                const uint32_t wv[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    const int wi = i * 4 + k, blk = wi >> 4, w = wi & 15;   // 16 words per 32-column block
-                    reinterpret_cast<uint32_t *>(xs)[blk * 16 + (w & 3) * 4 + (w >> 2)] = wv[k];
-                }
+            const int per_row = n >> 3;
+#pragma unroll 2
+            for (int i = threadIdx.x; i < bs * per_row; i += kThreads) {
+                const int b = bs == 1 ? 0 : i / per_row;
+                put_fragment(reinterpret_cast<uint32_t *>(xs), reinterpret_cast<const uint4 *>(x) + (size_t)b * per_row, i - b * per_row, b, bs);
             }
         }
     }
+    else {
+        // the x part of the chunk whose codes were requested above
+        if (lane == 0 && first_n > 0)
+            bulk_copy(ring_w + C * kBlockBytes, reinterpret_cast<const uint8_t *>(x) + (size_t)first_col * xblk_bytes,
+                      (uint32_t)(first_n * xblk_bytes), bar_w);
+    }
     __syncthreads();
-    if (scratch_offset <= 0) issue();   // second chunk: ring slot 1 (the scratch of the fused input side lay over it until now)
+    if (ichunk < 2) issue(true);        // second chunk: x may be read now, and the scratch no longer lies over ring slot 1
 
     const int g = lane >> 2, t = lane & 3;
-    const int xg = g < bs ? g : 0;  // lanes of unused batch columns alias row 0; their results are never stored
-    const uint32_t *xrow = reinterpret_cast<const uint32_t *>(x + (size_t)xg * n + 2 * t);
-    const uint32_t xsrow = smem_u32(xs) + (uint32_t)(xg * nb * 4 + t) * 16u;   // shared-memory address of this lane's fragments
+    const int xg = g < bs ? g : 0;      // lanes of unused batch columns alias row 0; their results are never stored
+    const uint32_t xlane = (uint32_t)(xg * 64 + t * 16);           // this lane's fragment words within a block's x
+    const uint32_t xs_step = (uint32_t)bs * 64u, xs_base = smem_u32(xs) + xlane;
     const uint32_t lut_lane = smem_u32(lut) + lane * 4;
     const uint32_t own_off = lane * (4 * K), nxt_off = ((lane + 1) & 31) * (4 * K);   // lane 31 wraps to lane 0: tail-biting
 
-    uint32_t segno = 0;
     unsigned cchunk = 0;       // chunks consumed so far: slot cchunk & 1, barrier phase (cchunk >> 1) & 1
     bool ring_dead = false;    // a wait ran out: stop waiting (the results are meaningless, the kernel terminates)
-    while (pos < end) {
-        int r0, r1;
-        run_of(pos, seg_end, r0, r1);
-        const int row0 = M * nb;
+    for (;;) {
+        if (!PIECES && e - p < NW) {      // some warps have no block: what they do not write counts as zero
+            for (int i = threadIdx.x; i < (NW + (e - 1) / nb - rbase) * stride; i += kThreads) red[i] = 0.f;
+            __syncthreads();
+        }
+        int v, col, left, total;
+        run_of(v, col, left, total);
+        float *slot_out = red + (PIECES ? warp : warp + (v - col) / nb - rbase) * stride;
+        uint32_t xsp = xs_base + (uint32_t)col * xs_step;
+        const uint32_t xs_next = PIECES ? xsp : xs_base;           // x at the start of the segments that follow
         float acc[2][4] = {};
-        uint32_t xsp = xsrow + (uint32_t)(r0 - row0) * 64u;    // x fragments of the block being decoded (64 bytes per block)
-        const uint32_t *xgp = xrow + 16 * (r0 - row0);
-        for (int blk = r0; blk < r1; blk += C) {
-            const int nblk = min(C, r1 - blk);
-            const uint32_t slot = ring_w + (cchunk & 1u) * slot_stride;
+        while (total > 0) {
+            const int nblk = min(C, left);
+            uint32_t slot = ring_w + (cchunk & 1u) * slot_stride;
             if (!ring_dead) {
                 const uint32_t bar = bar_w + (cchunk & 1u) * 8, parity = (cchunk >> 1) & 1u;
                 unsigned spins = 0;
@@ -764,33 +889,62 @@ __global__ void __launch_bounds__(NW * 32, 1)
                     }
                 }
             }
-#pragma unroll
-            for (int i = 0; i < C; i++) {
-                if (i < nblk) {
-                    const LaneCodes<K> own = lds_lane_codes<K>(slot + i * kBlockBytes + own_off);
-                    const LaneCodes<K> nxt = lds_lane_codes<K>(slot + i * kBlockBytes + nxt_off);
-                    uint32_t xb[4];
-                    if constexpr (XS) {
-                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(xb[0]), "=r"(xb[1]), "=r"(xb[2]), "=r"(xb[3]) : "r"(xsp + i * 64));
-                    }
-                    else { const uint32_t *xp = xgp + 16 * i; xb[0] = __ldg(xp); xb[1] = __ldg(xp + 4); xb[2] = __ldg(xp + 8); xb[3] = __ldg(xp + 12); }
-                    decode_block<K>(own, nxt, xb, acc, lut_lane);
-                }
+            uint32_t xa = XS ? xsp : slot + C * kBlockBytes + xlane;
+            // One block per trip, not unrolled: the body (about 95 instructions) stays in the instruction buffers of the
+            // sub-partitions; four blocks unrolled ran 17 % slower on the same data (32.6 against 28 cycles per block and SM).
+#pragma unroll 1
+            for (int i = 0; i < nblk; i++) {
+                const LaneCodes<K> own = lds_lane_codes<K>(slot + own_off);
+                const LaneCodes<K> nxt = lds_lane_codes<K>(slot + nxt_off);
+                uint32_t xb[4];
+                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(xb[0]), "=r"(xb[1]), "=r"(xb[2]), "=r"(xb[3]) : "r"(xa));
+                xa += xs_step;
+                slot += kBlockBytes;
+                decode_block<K>(own, nxt, xb, acc, lut_lane);
             }
-            if constexpr (XS) xsp += C * 64;
-            else xgp += C * 16;
+            xsp = xa;
+            left -= nblk;
+            total -= nblk;
             __syncwarp();      // every lane has read the slot before it is filled again
-            issue();
+            issue(true);
             cchunk++;
+            if (left == 0) {
+                // accumulator (ms, i): row = 16*ms + g + 8*(i>>1), batch = 2*t + (i&1); slot word = batch*32 + row
+#pragma unroll
+                for (int ms = 0; ms < 2; ms++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const int b = 2 * t + (i & 1);
+                        if (b < bs) slot_out[b * 32 + 16 * ms + g + 8 * (i >> 1)] = acc[ms][i];
+                        acc[ms][i] = 0.f;
+                    }
+                slot_out += PIECES ? NW * stride : stride;
+                left = min(seg_n, total);
+                xsp = xs_next;
+            }
         }
-        // a segment that covers its whole row block has no other contributor (true for every segment in rows mode)
-        const bool whole = pos == row0 && seg_end - pos == nb;
-        finish_segment<kConsumerWarps>(acc, DB ? red + (segno & 1) * red_floats : red, sh, out, partial, counters, M, nb,
-                                       (long)B, G, kmax, m, bs, whole, !DB, TP ? P.sig.copies : OutCopies{}, stamp);
-        segno++;
-        pos = seg_end + gap;
-        M += mstep;
-        seg_end = min(end, (M + 1) * nb);
+        __syncthreads();
+        if constexpr (PIECES) {
+            // a warp adds one row block and row of x: lane = output row, 32 pieces in order
+            const int outputs = min(max_rows, rows_total - rbase) * bs;
+            for (int k = warp; k < outputs; k += NW) {
+                const int rr = bs == 1 ? k : k / bs, b = k - rr * bs;
+                float y = 0.f;
+#pragma unroll
+                for (int w = 0; w < NW; w++) y += red[(rr * NW + w) * stride + b * 32 + lane];
+                const size_t o = (size_t)b * m + 32 * (size_t)(row0 + (rbase + rr) * rstep) + lane;
+                out[o] = y;
+                if constexpr (TP)
+                    for (int c = 0; c < P.sig.copies.n; c++) store_stamped(P.sig.copies.dst[c] + o, y, stamp);
+            }
+        } else {
+            reduce_round<NW>(red, sh, out, partial, counters, p, e, v_begin, v_end, rbase, nb, B, G, row0, rstep, L.kmax, m, bs,
+                             TP ? P.sig.copies : OutCopies{}, stamp);
+        }
+        if (e == v_end) break;
+        p = e; e = min(v_end, e + max_rows * nb); rbase += max_rows;
+        if (!PIECES) { start_issue(); issue(true); issue(true); }
+        __syncthreads();       // the slots are read before the next round writes them
     }
 
     if (TP && P.sig.seq) {
@@ -803,7 +957,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
                 *done_counter = 0;
             }
         }
-    } else if (NW == 32 && P.ep.final) {
+    } else if (P.ep.final) {
         // fused output side (m a power of two): the CTA that finishes last transforms the whole result
         __threadfence();
         __syncthreads();
@@ -950,11 +1104,11 @@ int check_common(const void *out, const void *codes, const void *x, int K, int m
 }
 
 struct SmemPlan {
-    int chunk_blocks, xs_offset, total, db, scratch_offset;
+    int chunk_blocks, xs_offset, total, max_rows, scratch_offset;
 };
 
-template <int K, bool XS, bool TP, int NW, int C>
-int launch_hyb_variant_tp(const MatvecBatch &batch, int nprob, int m, int n, int bs, const SmemPlan &plan, cudaStream_t s) {
+template <int K, int MODE, bool TP, int C>
+int launch_hyb_variant_tp(const MatvecBatch &batch, int nprob, int m, int n, int bs, const Partition &p, const SmemPlan &plan, cudaStream_t s) {
     static bool attr_set[64] = {};
     static std::mutex attr_mutex;
     int dev = 0;
@@ -963,15 +1117,14 @@ int launch_hyb_variant_tp(const MatvecBatch &batch, int nprob, int m, int n, int
     {
         std::lock_guard<std::mutex> lock(attr_mutex);
         if (!attr_set[dev]) {
-            QTIP_CUDA_TRY(cudaFuncSetAttribute(matvec_hyb_kernel<K, XS, TP, NW, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               kSmemLimit));
+            QTIP_CUDA_TRY(cudaFuncSetAttribute(matvec_hyb_kernel<K, MODE, TP, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit));
             attr_set[dev] = true;
         }
     }
-    const Partition p = make_partition(m, n, K, nprob);
+    const HybLaunch L = {p.kmax, p.mode, plan.max_rows, plan.xs_offset, plan.scratch_offset, (m >> 5) / p.grid, (m >> 5) % p.grid};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.grid, nprob);
-    cfg.blockDim = dim3(NW * 32);
+    cfg.blockDim = dim3(kConsumerWarps * 32);
     cfg.dynamicSmemBytes = plan.total;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -979,46 +1132,48 @@ int launch_hyb_variant_tp(const MatvecBatch &batch, int nprob, int m, int n, int
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, matvec_hyb_kernel<K, XS, TP, NW, C>, batch, m, n, bs, p.kmax, p.mode, plan.db,
-                                     plan.xs_offset, plan.scratch_offset));
+    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, matvec_hyb_kernel<K, MODE, TP, C>, batch, m, n, bs, L));
     return check_launch();
 }
 
-template <int K, bool XS, int C>
-int launch_hyb_variant_c(const MatvecBatch &batch, int nprob, int m, int n, int bs, const SmemPlan &plan, cudaStream_t s) {
+template <int K, int MODE, int C>
+int launch_hyb_variant_c(const MatvecBatch &batch, int nprob, int m, int n, int bs, const Partition &p, const SmemPlan &plan, cudaStream_t s) {
     bool tp = false;
     for (int i = 0; i < nprob; i++) {
         const MatvecProblem &q = batch.p[i];
         tp = tp || q.peer.n > 0 || q.sig.seq != nullptr;
     }
-    if (tp) return launch_hyb_variant_tp<K, XS, true, 32, C>(batch, nprob, m, n, bs, plan, s);
-    return launch_hyb_variant_tp<K, XS, false, 32, C>(batch, nprob, m, n, bs, plan, s);
+    if (tp) return launch_hyb_variant_tp<K, MODE, true, C>(batch, nprob, m, n, bs, p, plan, s);
+    return launch_hyb_variant_tp<K, MODE, false, C>(batch, nprob, m, n, bs, p, plan, s);
 }
 
-template <int K, bool XS>
-int launch_hyb_variant(const MatvecBatch &batch, int nprob, int m, int n, int bs, const SmemPlan &plan, cudaStream_t s) {
+template <int K, int MODE>
+int launch_hyb_variant(const MatvecBatch &batch, int nprob, int m, int n, int bs, const Partition &p, const SmemPlan &plan, cudaStream_t s) {
     constexpr int kMaxC = kMaxChunkBytes / (128 * K);      // 4 for K = 2, 2 for K = 3 and 4
     if constexpr (kMaxC >= 4) {
-        if (plan.chunk_blocks >= 4) return launch_hyb_variant_c<K, XS, 4>(batch, nprob, m, n, bs, plan, s);
+        if (plan.chunk_blocks >= 4) return launch_hyb_variant_c<K, MODE, 4>(batch, nprob, m, n, bs, p, plan, s);
     }
-    if (plan.chunk_blocks >= 2) return launch_hyb_variant_c<K, XS, 2>(batch, nprob, m, n, bs, plan, s);
-    return launch_hyb_variant_c<K, XS, 1>(batch, nprob, m, n, bs, plan, s);
+    if (plan.chunk_blocks >= 2) return launch_hyb_variant_c<K, MODE, 2>(batch, nprob, m, n, bs, p, plan, s);
+    return launch_hyb_variant_c<K, MODE, 1>(batch, nprob, m, n, bs, p, plan, s);
 }
 
-// Fit ring, reduction buffer(s), x and the scratch of the fused input side into the shared memory left beside
-// the table.  Returns false if not even a one-block ring fits.
+// Fit ring, partial-sum slots, x and the scratch of the fused input side into the shared memory left beside the table.
+// cta_rows: row blocks a CTA meets; they share the slots in rounds of max_rows: up to `pieces` with a slot per warp and row
+// block, or (pieces = 0) up to 32 for contiguous runs.  Returns false if not even a one-block ring fits.
 template <int K>
-bool plan_smem(int n, int bs, bool xs, bool db, bool fused_in, SmemPlan &plan) {
+bool plan_smem(int n, int bs, int cta_rows, int pieces, bool xs, bool fused_in, SmemPlan &plan) {
     constexpr int NW = kConsumerWarps, BB = 128 * K;
-    const int red_bytes = (db ? 2 : 1) * NW * 32 * bs * (int)sizeof(float);
-    const int x_bytes = xs ? bs * n * 2 : 0;
+    const int cap = pieces ? pieces : 32;
+    plan.max_rows = cta_rows < cap ? cta_rows : cap;
+    const int red_bytes = (pieces ? NW * plan.max_rows : NW + plan.max_rows) * 32 * bs * (int)sizeof(float);
+    const int x_bytes = xs ? bs * n * 2 : 0, ring_x = xs ? 0 : bs * 64;
     // fwht_shared wants n + n/32 + 8 floats, fwht_regs 32 rows of n/32 + 4
     const int scratch_bytes = fused_in ? (n + (n >> 5) + 136) * (int)sizeof(float) : 0;
     const int avail = kSmemLimit - kCtrlBytes - kLutBytes;
-    plan.db = db ? 1 : 0;
+    if ((long)bs * n * 2 > avail && xs) return false;
     plan.scratch_offset = 0;
     for (int c = kMaxChunkBytes / BB; c >= 1; c >>= 1) {          // 4, 2, 1: the instantiated chunk sizes
-        const int slot = NW * c * BB;                                   // one ring slot, all warps
+        const int slot = NW * c * (BB + ring_x);                        // one ring slot, all warps
         if (2 * slot + red_bytes + x_bytes + scratch_bytes <= avail) {  // room for a scratch area of its own
             plan.chunk_blocks = c;
             plan.xs_offset = kCtrlBytes + kLutBytes + 2 * slot + red_bytes;
@@ -1040,18 +1195,55 @@ bool plan_smem(int n, int bs, bool xs, bool db, bool fused_in, SmemPlan &plan) {
     return false;
 }
 
+// Where the fragment-ordered x lies in the workspace.
+size_t partials_end(int m, int n) {
+    const long nb = n >> 5, B = (long)(m >> 5) * nb;
+    const long G = B < kMaxGrid ? B : kMaxGrid;
+    return kPartialOffset + (size_t)(m >> 5) * max_contributors(nb, B, G) * 256 * sizeof(float);
+}
+
+int launch_fragments(const FragmentArgs &a, int nprob, int n, int bs, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(((n >> 3) + 255) / 256, bs, nprob);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, x_fragment_kernel, a, n, bs));
+    return check_launch();
+}
+
 // fused_in: the batch uses the fused input transform (needs x staged in shared memory plus fp32 scratch)
 template <int K>
 int launch_hyb_batch(const MatvecBatch &batch, int nprob, int m, int n, int bs, bool fused_in, cudaStream_t s) {
-    // shared memory: control + table are fixed; then the ring, the reduction buffer(s) and, when it fits, x.
-    // Preference: x staged and double-buffered reduction; then give up the second reduction buffer; then x.
+    // shared memory: control + table are fixed; then the ring, the partial-sum slots and, when it fits, x.
+    const Partition p = make_partition(m, n, nprob);
+    const int mb = m >> 5, nb = n >> 5;
+    const int cta_rows = p.mode == kModeRows ? (mb + p.grid - 1) / p.grid : (int)((((long)mb * nb + p.grid - 1) / p.grid + nb - 2) / nb) + 1;
+    // More rows of x need several times the slots, which the ring then lacks (22016 x 4096, 5 rows: 24.6 us with pieces, 19.8
+    // with runs); with one row block per CTA the slots are few and pieces save the run arithmetic (4096 x 4096: 7.1 against 8.2)
+    const bool pieces = (bs == 1 || cta_rows == 1) && p.mode == kModeRows && nb >= kConsumerWarps;
     SmemPlan plan;
-    if (plan_smem<K>(n, bs, true, true, fused_in, plan)) return launch_hyb_variant<K, true>(batch, nprob, m, n, bs, plan, s);
-    if (plan_smem<K>(n, bs, true, false, fused_in, plan)) return launch_hyb_variant<K, true>(batch, nprob, m, n, bs, plan, s);
+    // slots of up to four row blocks at once, fewer where memory is short
+    for (int rows = pieces ? 4 : 1; rows >= 1; rows >>= 1)
+        if (plan_smem<K>(n, bs, cta_rows, pieces ? rows : 0, true, fused_in, plan))
+            return pieces ? launch_hyb_variant<K, kStagedX | kPieces>(batch, nprob, m, n, bs, p, plan, s)
+                          : launch_hyb_variant<K, kStagedX>(batch, nprob, m, n, bs, p, plan, s);
     if (fused_in) return QTIP_ERR_BAD_SHAPE;      // the fused input side leaves x in shared memory
-    if (plan_smem<K>(n, bs, false, true, false, plan)) return launch_hyb_variant<K, false>(batch, nprob, m, n, bs, plan, s);
-    if (plan_smem<K>(n, bs, false, false, false, plan)) return launch_hyb_variant<K, false>(batch, nprob, m, n, bs, plan, s);
-    return QTIP_ERR_BAD_SHAPE;
+    MatvecBatch ring = batch;
+    FragmentArgs a = {};
+    for (int i = 0; i < nprob; i++) {
+        a.x[i] = batch.p[i].x;
+        a.frag[i] = reinterpret_cast<uint32_t *>(batch.p[i].workspace + partials_end(m, n));
+        ring.p[i].x = reinterpret_cast<const __half *>(a.frag[i]);
+    }
+    if (!plan_smem<K>(n, bs, cta_rows, 0, false, false, plan)) return QTIP_ERR_BAD_SHAPE;
+    const int st = launch_fragments(a, nprob, n, bs, s);
+    if (st != QTIP_OK) return st;
+    return launch_hyb_variant<K, 0>(ring, nprob, m, n, bs, p, plan, s);
 }
 
 template <int K>
@@ -1069,11 +1261,8 @@ int launch_hyb(float *out, const uint8_t *codes, const __half *x, const uint32_t
 using namespace qtip;
 
 extern "C" size_t qtip_matvec_workspace_bytes(int m, int n, int bs) {
-    (void)bs;
     if (m < 32 || n < 32) return kPartialOffset;
-    const long nb = n >> 5, B = (long)(m >> 5) * nb;
-    const long G = B < kMaxGrid ? B : kMaxGrid;
-    return kPartialOffset + (size_t)(m >> 5) * max_contributors(nb, B, G) * 256 * sizeof(float);
+    return partials_end(m, n) + (size_t)(bs < 1 ? 1 : bs) * n * sizeof(__half);
 }
 
 extern "C" int qtip_decompress_matvec(float *out, const void *codes, const void *x, const void *tlut, int K, int m,
@@ -1097,7 +1286,7 @@ extern "C" int qtip_decompress_matvec_plain(float *out, const void *codes, const
     if (code != QTIP_CODE_3INST && code != QTIP_CODE_1MAD) return QTIP_ERR_BAD_ARG;
     int st = check_common(out, codes, x, K, m, n, bs, workspace, workspace_bytes);
     if (st != QTIP_OK) return st;
-    Partition p = make_partition(m, n, K);
+    Partition p = make_partition(m, n);
     // two CTAs of 16 warps per SM
     if (p.mode == kModeStreamK) {
         const long B = (long)(m >> 5) * (n >> 5);
@@ -1203,12 +1392,12 @@ extern "C" int qtip_linear_fused(const qtip_linear_desc *descs, int count, int K
 
 // ---- allocation-free variant ------------------------------------------------------------------------------
 // Scratch (ticket counters + partial sums) of qtip_decompress_matvec_static: a fixed array in the
-// library's device image.  Every GPU that loads the library carries these 4 MiB + 64.25 KiB until the
+// library's device image.  Every GPU that loads the library carries these 8 MiB + 64.25 KiB until the
 // process exits.  In host code the name below is only a stand-in for the symbol; the address a kernel
 // can use comes from cudaGetSymbolAddress, looked up once per device.
 namespace qtip {
 namespace {
-constexpr size_t kStaticScratchBytes = kPartialOffset + 4u * 1024u * 1024u;
+constexpr size_t kStaticScratchBytes = kPartialOffset + 8u * 1024u * 1024u;    // partial sums, and x in fragment order
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
 std::mutex g_static_scratch_mutex;
 void *g_static_scratch_ptr[64] = {};

@@ -519,3 +519,17 @@ def test_embed_and_sampler():
     for _ in range(50):
         ops.sample_top_k(tok, out2, pos, logits, temperature=0.6, top_k=k, seed=77)
     assert torch.equal(out2[1:51], out[1:51])
+
+
+@pytest.mark.parametrize("K", [2, 3, 4])
+@pytest.mark.parametrize("m,n,bs", [(32, 32, 1), (32, 992, 1), (64, 32, 3), (9600, 64, 1), (4736, 1024, 1), (4768, 1056, 1), (9472, 1024, 2),
+                                    (5000 * 32, 32, 1), (64, 65536, 1), (96, 32768, 8), (14208, 4096, 7), (512, 16384, 5)])
+def test_matvec_hyb_partitions(K, m, n, bs):
+    """Every way of cutting the work: rows shorter than a warp each, pieces and contiguous runs, several rounds of row blocks,
+    shared row blocks, x staged and x through the ring - against the decoded matrix."""
+    lay = synth.make_layer(m, n, K, seed=m + n + bs, bs=bs, device=DEV)
+    codes = lay["codes"].view(torch.int16)
+    got = ops.decompress_matvec(codes, lay["x"], lay["tlut"], K, m, n)
+    want = lay["x"].double() @ ops.decode_hyb(codes, lay["tlut"], K, m, n).double().T
+    assert float((got.double() - want).norm() / want.norm()) < 2e-6
+    assert torch.equal(got, ops.decompress_matvec(codes, lay["x"], lay["tlut"], K, m, n))
