@@ -205,7 +205,7 @@ int qtip_linear_desc_layout(size_t *out, int capacity);
  * workspace - a serving loop that froze its memory pool at start-up, a plug-in whose host owns every
  * allocation, code running where a cudaMalloc would synchronise the device.  (No counterpart in the
  * reference, whose kernel needs no scratch.)  Same arguments and result as qtip_decompress_matvec minus
- * the workspace: the ticket counters and partial sums live in a 4 MiB + 64.25 KiB array built into the
+ * the workspace: the ticket counters and partial sums live in a 8 MiB + 64.25 KiB array built into the
  * library's device image (each GPU that loads the library holds it until the process exits).  Problems
  * whose qtip_matvec_workspace_bytes(m, n, bs) exceeds that size return QTIP_ERR_TOO_LARGE; every
  * Llama-2/3 layer shape up to 53248 x 16384 fits.  The call itself performs no cudaMalloc / cudaFree
