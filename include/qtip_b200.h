@@ -311,6 +311,11 @@ int qtip_lm_head(float *logits, const void *res, const void *delta, const void *
 int qtip_sample_top_k(long long *token, long long *out_tokens, int *pos, const float *logits, int vocab,
                       float temperature, int top_k, unsigned long long seed, int max_tokens, unsigned *status,
                       void *stream);
+/* The same for `batch` sequences in one launch: token, pos (batch), out_tokens (batch, max_tokens), logits (batch, vocab)
+ * contiguous; sequence b draws with seed + b. */
+int qtip_sample_top_k_batch(long long *token, long long *out_tokens, int *pos, const float *logits, int vocab, int batch,
+                            float temperature, int top_k, unsigned long long seed, int max_tokens, unsigned *status,
+                            void *stream);
 
 /* Rotary embedding of q (n_heads, head_dim; in place) and k (n_kv_heads, head_dim), and append of the
  * rotated k and of v to the caches at row *pos (caches are (max_positions, n_kv_heads*head_dim)).
@@ -346,6 +351,15 @@ int qtip_attn_decode_fused(void *out, const float *y_q, const float *y_k, const 
  * for a single new token. */
 int qtip_attn_decode(void *out, const void *q, const void *cache_k, const void *cache_v, const int *pos, int n_heads,
                      int n_kv_heads, int head_dim, int max_positions, unsigned *status, void *stream);
+
+/* qtip_rope_kv_append / qtip_attn_decode for `batch` sequences in one launch: q, k, v, out are (batch, heads * head_dim) contiguous,
+ * pos (batch), and the caches of consecutive sequences are cache_stride elements apart (a multiple of 8). */
+int qtip_rope_kv_append_batch(void *q, const void *k, const void *v, void *cache_k, void *cache_v, const int *pos, int n_heads,
+                              int n_kv_heads, int head_dim, float theta, int max_positions, int batch, long cache_stride,
+                              unsigned *status, void *stream);
+int qtip_attn_decode_batch(void *out, const void *q, const void *cache_k, const void *cache_v, const int *pos, int n_heads,
+                           int n_kv_heads, int head_dim, int max_positions, int batch, long cache_stride, unsigned *status,
+                           void *stream);
 
 #ifdef __cplusplus
 }

@@ -62,6 +62,9 @@ SIGNATURES = {
     "qtip_rope_kv_append_fused": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _f, _vp, _vp, _vp, _i, _i, _i, _f, _i, _vp,
                                        _vp]),
     "qtip_attn_decode_fused": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _f, _f, _vp, _vp, _vp, _i, _i, _i, _f, _i, _vp, _vp]),
+    "qtip_sample_top_k_batch": (_i, [_vp, _vp, _vp, _vp, _i, _i, _f, _i, ctypes.c_ulonglong, _i, _vp, _vp]),
+    "qtip_rope_kv_append_batch": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _f, _i, _i, _l, _vp, _vp]),
+    "qtip_attn_decode_batch": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _l, _vp, _vp]),
     "qtip_attn_decode": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp]),
 }
 

@@ -130,29 +130,47 @@ __device__ __forceinline__ unsigned long long splitmix64(unsigned long long x) {
     return x ^ (x >> 31);
 }
 
-// One CTA.  top_k rounds of a block-wide arg-max over the logits not yet taken (ties: lower index), then
-// softmax(top / temperature) and one draw by inverse CDF from a counter-based generator keyed by (seed, *pos).
-// Writes the token to `token` and to out_tokens[*pos + 1], then advances *pos.
-__global__ void __launch_bounds__(kSampleThreads)
-    sample_kernel(long long *__restrict__ token, long long *__restrict__ out_tokens, int *__restrict__ pos,
-                  const float *__restrict__ logits, int vocab, float inv_temperature, int top_k, unsigned long long seed,
-                  int max_tokens, unsigned *status) {
+// A cluster of eight CTAs per sequence (blockIdx.y).  Every CTA finds the top_k of its eighth of the vocabulary by top_k rounds
+// of a block-wide arg-max over the logits not yet taken (ties: lower index), held in registers; one warp merges the eight
+// lists, then softmax(top / temperature) and one draw by inverse CDF from a counter-based generator keyed by (seed, *pos).
+// Writes the token to `token` and to out_tokens[*pos + 1], then advances *pos.  Bound by the rounds' latency (one CTA that
+// re-read a 128256-entry vocabulary every round took 100 us per sequence, one sequence after another).
+constexpr int kSampleCluster = 8;
+struct SampleArgs {
+    long long *token, *out_tokens;
+    int *pos;
+    const float *logits;
+    int vocab;
+    float inv_temperature;
+    int top_k;
+    unsigned long long seed;
+    int max_tokens;
+    unsigned *status;
+};
+__device__ __forceinline__ void argmax_step(float &best, int &bi, float ov, int oi) {
+    if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+}
+__global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SampleArgs a) {
     __shared__ float s_val[32];
     __shared__ int s_idx[32];
-    __shared__ float top_val[kMaxTopK];
+    __shared__ float top_val[kMaxTopK];      // this CTA's candidates, read by CTA 0 of the cluster
     __shared__ int top_idx[kMaxTopK];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // up to 32 logits per thread stay in registers for all rounds (vocabularies up to 32768); larger ones are re-read
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, seq = blockIdx.y, top_k = a.top_k;
+    uint32_t rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const float *logits = a.logits + (size_t)seq * a.vocab;
+    const int slice = (a.vocab + kSampleCluster - 1) / kSampleCluster, lo = (int)rank * slice, hi = min(a.vocab, lo + slice);
+    // up to 32 logits per thread stay in registers for all rounds (vocabularies up to 262144); larger ones are re-read
     constexpr int kHeld = 32;
-    const bool held = vocab <= kHeld * kSampleThreads;
+    const bool held = slice <= kHeld * kSampleThreads;
     float mine[kHeld];
     if (held) {
 #pragma unroll
         for (int j = 0; j < kHeld; j++) {
-            const int i = threadIdx.x + j * kSampleThreads;
-            mine[j] = i < vocab ? __ldcg(logits + i) : -INFINITY;
+            const int i = lo + threadIdx.x + j * kSampleThreads;
+            mine[j] = i < hi ? __ldcg(logits + i) : -INFINITY;
         }
     }
     for (int round = 0; round < top_k; round++) {
@@ -162,32 +180,24 @@ __global__ void __launch_bounds__(kSampleThreads)
 #pragma unroll
             for (int j = 0; j < kHeld; j++) {
                 const float v = mine[j];
-                if (v > best) { best = v; bi = threadIdx.x + j * kSampleThreads; }    // ascending index: ties keep the lower
+                if (v > best) { best = v; bi = lo + threadIdx.x + j * kSampleThreads; }    // ascending index: ties keep the lower
             }
         } else {
-            for (int i = threadIdx.x; i < vocab; i += kSampleThreads) {
+            for (int i = lo + threadIdx.x; i < hi; i += kSampleThreads) {
                 const float v = __ldcg(logits + i);
                 bool taken = false;
                 for (int q = 0; q < round; q++) taken |= (top_idx[q] == i);
-                if (!taken && (v > best || (v == best && i < bi))) { best = v; bi = i; }
+                if (!taken) argmax_step(best, bi, v, i);
             }
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(kFullMask, best, o);
-            const int oi = __shfl_xor_sync(kFullMask, bi, o);
-            if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-        }
+        for (int o = 16; o > 0; o >>= 1) argmax_step(best, bi, __shfl_xor_sync(kFullMask, best, o), __shfl_xor_sync(kFullMask, bi, o));
         if (lane == 0) { s_val[warp] = best; s_idx[warp] = bi; }
         __syncthreads();
         if (warp == 0) {
             best = s_val[lane]; bi = s_idx[lane];
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ov = __shfl_xor_sync(kFullMask, best, o);
-                const int oi = __shfl_xor_sync(kFullMask, bi, o);
-                if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-            }
+            for (int o = 16; o > 0; o >>= 1) argmax_step(best, bi, __shfl_xor_sync(kFullMask, best, o), __shfl_xor_sync(kFullMask, bi, o));
             if (lane == 0) { top_val[round] = best; top_idx[round] = bi; }
         }
         __syncthreads();
@@ -195,27 +205,70 @@ __global__ void __launch_bounds__(kSampleThreads)
             const int win = top_idx[round];
 #pragma unroll
             for (int j = 0; j < kHeld; j++)
-                if (win == threadIdx.x + j * kSampleThreads) mine[j] = -INFINITY;     // (a -inf logit can be drawn twice)
+                if (win == lo + threadIdx.x + j * kSampleThreads) mine[j] = -INFINITY;     // (a -inf logit can be drawn twice)
         }
     }
-    if (threadIdx.x == 0) {
-        const int p = *pos;
-        float prob[kMaxTopK], sum = 0.f;
-        for (int q = 0; q < top_k; q++) { prob[q] = __expf((top_val[q] - top_val[0]) * inv_temperature); sum += prob[q]; }
-        const unsigned long long bits = splitmix64(seed ^ splitmix64((unsigned long long)p));
-        const float u = (float)(bits >> 40) * (1.0f / 16777216.0f) * sum;      // uniform in [0, sum)
-        int pick = top_k - 1;
-        float cum = 0.f;
-        for (int q = 0; q < top_k; q++) {
-            cum += prob[q];
-            if (u < cum) { pick = q; break; }
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    if (rank == 0 && warp == 0) {
+        // the eight lists (at most 128 candidates, four per lane): top_k rounds over one warp
+        float cv[4];
+        int ci[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            const int c = lane + 32 * e, r = c / top_k, q = c - r * top_k;
+            cv[e] = -INFINITY;
+            ci[e] = 0x7FFFFFFF;
+            if (r < kSampleCluster) {
+                uint32_t av, ai;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(av) : "r"((uint32_t)__cvta_generic_to_shared(top_val + q)), "r"(r));
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ai) : "r"((uint32_t)__cvta_generic_to_shared(top_idx + q)), "r"(r));
+                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(cv[e]) : "r"(av) : "memory");
+                asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(ci[e]) : "r"(ai) : "memory");
+            }
         }
-        const long long t = top_idx[pick];
-        *token = t;
-        if (p >= 0 && p + 1 < max_tokens) out_tokens[p + 1] = t;      // the token log is full: keep sampling, report
-        else if (status) atomicOr(status, 4u);
-        *pos = p + 1;
+        float prob[kMaxTopK], top0 = 0.f, sum = 0.f;
+        int idx[kMaxTopK];
+#pragma unroll
+        for (int q = 0; q < kMaxTopK; q++) {
+            if (q < top_k) {
+                float best = -INFINITY;
+                int bi = 0x7FFFFFFF;
+#pragma unroll
+                for (int e = 0; e < 4; e++) argmax_step(best, bi, cv[e], ci[e]);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) argmax_step(best, bi, __shfl_xor_sync(kFullMask, best, o), __shfl_xor_sync(kFullMask, bi, o));
+#pragma unroll
+                for (int e = 0; e < 4; e++)
+                    if (ci[e] == bi) { cv[e] = -INFINITY; ci[e] = 0x7FFFFFFF; }
+                if (q == 0) top0 = best;
+                prob[q] = __expf((best - top0) * a.inv_temperature);
+                idx[q] = bi;
+                sum += prob[q];
+            }
+        }
+        if (lane == 0) {
+            int *pos = a.pos + seq;
+            const int p = *pos;
+            const unsigned long long bits = splitmix64((a.seed + seq) ^ splitmix64((unsigned long long)p));
+            const float u = (float)(bits >> 40) * (1.0f / 16777216.0f) * sum;      // uniform in [0, sum)
+            int t = 0;
+            float cum = 0.f;
+            bool drawn = false;
+#pragma unroll
+            for (int q = 0; q < kMaxTopK; q++) {
+                if (q < top_k && !drawn) {
+                    cum += prob[q];
+                    t = idx[q];
+                    drawn = u < cum;
+                }
+            }
+            a.token[seq] = t;
+            if (p >= 0 && p + 1 < a.max_tokens) a.out_tokens[(size_t)seq * a.max_tokens + p + 1] = t;      // the token log is full: keep sampling, report
+            else if (a.status) atomicOr(a.status, 4u);
+            *pos = p + 1;
+        }
     }
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");      // the lists are read
 }
 
 template <typename... Args>
@@ -272,12 +325,31 @@ extern "C" int qtip_lm_head(float *logits, const void *res, const void *delta, c
                       static_cast<const __half *>(norm_weight), static_cast<const __half *>(weight), hidden, vocab, eps);
 }
 
+extern "C" int qtip_sample_top_k_batch(long long *token, long long *out_tokens, int *pos, const float *logits, int vocab, int batch,
+                                       float temperature, int top_k, unsigned long long seed, int max_tokens, unsigned *status,
+                                       void *stream) {
+    if (!token || !out_tokens || !pos || !logits || max_tokens <= 0) return QTIP_ERR_BAD_ARG;
+    if (vocab <= 0 || batch < 1 || batch > 65535 || top_k < 1 || top_k > kMaxTopK || top_k > vocab) return QTIP_ERR_BAD_SHAPE;
+    const SampleArgs a = {token, out_tokens, pos, logits, vocab, 1.0f / fmaxf(temperature, 1e-5f), top_k, seed, max_tokens, status};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kSampleCluster, batch);
+    cfg.blockDim = dim3(kSampleThreads);
+    cfg.stream = static_cast<cudaStream_t>(stream);
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = kSampleCluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, sample_kernel, a));
+    return check_launch();
+}
+
 extern "C" int qtip_sample_top_k(long long *token, long long *out_tokens, int *pos, const float *logits, int vocab,
                                  float temperature, int top_k, unsigned long long seed, int max_tokens, unsigned *status,
                                  void *stream) {
-    if (!token || !out_tokens || !pos || !logits || max_tokens <= 0) return QTIP_ERR_BAD_ARG;
-    if (vocab <= 0 || top_k < 1 || top_k > kMaxTopK || top_k > vocab) return QTIP_ERR_BAD_SHAPE;
-    const float inv_t = 1.0f / fmaxf(temperature, 1e-5f);
-    return launch_pdl(sample_kernel, dim3(1), dim3(kSampleThreads), 0, static_cast<cudaStream_t>(stream), token, out_tokens, pos,
-                      logits, vocab, inv_t, top_k, seed, max_tokens, status);
+    return qtip_sample_top_k_batch(token, out_tokens, pos, logits, vocab, 1, temperature, top_k, seed, max_tokens, status, stream);
 }

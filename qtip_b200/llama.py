@@ -403,7 +403,7 @@ class QtipLlama:
     def enable_batch(self, B):
         """Buffers for decoding B (<= 8) independent sequences per step (step_batch).  The batch rides in the matvec
         launches (the packed matrices are streamed once for all B rows); the transforms run as row-batched launches of
-        the transform kernel, rotary embedding / attention / sampling per sequence.  Works for every shape and for
+        the transform kernel, rotary embedding, attention and sampling as one launch for all sequences.  Works for every shape and for
         tensor parallelism (NCCL all-reduce after o_proj and down_proj)."""
         assert 1 <= B <= ops.MAX_MATVEC_BATCH and not self.fuse_qkv
         s, dev, H, KV, MLP = self.shape, self.device, self.H, self.KV, self.MLP
@@ -453,12 +453,11 @@ class QtipLlama:
                            kf_out=self.kf_hl, out=self.b_q)
             self._b_linear(L["k"], rb, norm=L["ln1"], kf_in=self.kf_h, kf_out=self.kf_kv, out=self.b_k)
             self._b_linear(L["v"], rb, norm=L["ln1"], kf_in=self.kf_h, kf_out=self.kf_kv, out=self.b_v)
-            for b in range(B):
-                ck, cv, pos = self.b_cache_k[b, li], self.b_cache_v[b, li], self.b_pos[b:b + 1]
-                ops.rope_kv_append(self.b_q[b], self.b_k[b], self.b_v[b], ck, cv, pos, self.n_heads, self.n_kv_heads,
-                                   s.head_dim, s.rope_theta, status=self.status)
-                ops.attn_decode(self.b_attn[b], self.b_q[b], ck, cv, pos, self.n_heads, self.n_kv_heads, s.head_dim,
-                                status=self.status)
+            ck, cv = self.b_cache_k[:, li], self.b_cache_v[:, li]
+            ops.rope_kv_append_batch(self.b_q, self.b_k, self.b_v, ck, cv, self.b_pos, self.n_heads, self.n_kv_heads, s.head_dim,
+                                     s.rope_theta, status=self.status)
+            ops.attn_decode_batch(self.b_attn, self.b_q, ck, cv, self.b_pos, self.n_heads, self.n_kv_heads, s.head_dim,
+                                  status=self.status)
             self._b_linear(L["o"], self.b_attn, kf_in=self.kf_hl, kf_out=self.kf_h, out=self.b_delta, all_reduce=True)
             # res_a = res_b + delta ; h = RMSNorm(res_a) ; gate, up ; down(silu(gate) * up)
             self._b_linear(L["gate"], self.b_delta, residual=rb, residual_out=ra, norm=L["ln2"], kf_in=self.kf_h,
@@ -470,9 +469,8 @@ class QtipLlama:
         x32 = (ra + self.b_delta).float()
         hn = (x32 * torch.rsqrt(x32.pow(2).mean(-1, keepdim=True) + s.rms_eps)).half() * self.ln_f
         self.b_logits.copy_(torch.matmul(hn, self.lm_head.T))
-        for b in range(B):
-            ops.sample_top_k(self.b_token[b:b + 1], self.b_out_tokens[b], self.b_pos[b:b + 1], self.b_logits[b:b + 1],
-                             temperature=0.6, top_k=5, seed=self.sample_seed + b, status=self.status)
+        ops.sample_top_k_batch(self.b_token, self.b_out_tokens, self.b_pos, self.b_logits, temperature=0.6, top_k=5,
+                               seed=self.sample_seed, status=self.status)
 
     def capture_batch(self):
         tok, pos = self.b_token.clone(), self.b_pos.clone()

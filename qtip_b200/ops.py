@@ -415,6 +415,41 @@ def sample_top_k(token, out_tokens, pos, logits, temperature=0.6, top_k=5, seed=
     launch_count += 1
 
 
+def sample_top_k_batch(token, out_tokens, pos, logits, temperature=0.6, top_k=5, seed=0, status=None):
+    """sample_top_k for the rows of logits (B, vocab): token, pos (B), out_tokens (B, max_tokens), one launch; sequence b draws
+    with seed + b."""
+    _check_device(token, out_tokens, pos, logits, status)
+    _lib.check(_lib.load().qtip_sample_top_k_batch(token.data_ptr(), out_tokens.data_ptr(), pos.data_ptr(), logits.data_ptr(),
+                                                   logits.shape[1], logits.shape[0], float(temperature), int(top_k), int(seed),
+                                                   out_tokens.shape[1], _status_ptr(status), _stream()),
+               "qtip_sample_top_k_batch")
+    global launch_count
+    launch_count += 1
+
+
+def rope_kv_append_batch(q, k, v, cache_k, cache_v, pos, n_heads, n_kv_heads, head_dim, theta=10000.0, status=None):
+    """rope_kv_append for B sequences: q, k, v (B, width), pos (B), caches (B, max_positions, n_kv_heads*head_dim) with any
+    stride between sequences."""
+    _check_device(q, k, v, cache_k, cache_v, pos, status)
+    st = _lib.load().qtip_rope_kv_append_batch(q.data_ptr(), k.data_ptr(), v.data_ptr(), cache_k.data_ptr(), cache_v.data_ptr(),
+                                               pos.data_ptr(), n_heads, n_kv_heads, head_dim, float(theta), cache_k.shape[1],
+                                               q.shape[0], cache_k.stride(0), _status_ptr(status), _stream())
+    _lib.check(st, "qtip_rope_kv_append_batch")
+    global launch_count
+    launch_count += 1
+
+
+def attn_decode_batch(out, q, cache_k, cache_v, pos, n_heads, n_kv_heads, head_dim, status=None):
+    _check_device(out, q, cache_k, cache_v, pos, status)
+    st = _lib.load().qtip_attn_decode_batch(out.data_ptr(), q.data_ptr(), cache_k.data_ptr(), cache_v.data_ptr(), pos.data_ptr(),
+                                            n_heads, n_kv_heads, head_dim, cache_k.shape[1], q.shape[0], cache_k.stride(0),
+                                            _status_ptr(status), _stream())
+    _lib.check(st, "qtip_attn_decode_batch")
+    global launch_count
+    launch_count += 1
+    return out
+
+
 def rope_kv_append(q, k, v, cache_k, cache_v, pos, n_heads, n_kv_heads, head_dim, theta=10000.0, status=None):
     """The caches are (max_positions, n_kv_heads*head_dim); a position outside them makes the kernel skip its work
     and set bit 1 of `status` (same for the three functions below)."""

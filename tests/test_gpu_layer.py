@@ -528,3 +528,49 @@ def test_native_layer_call_input_forms(dtype, shape):
         assert rel_l2(y.reshape(-1, m).float().cpu().numpy(), want) < (4e-3 if dtype == torch.bfloat16 else 1e-3)
     with pytest.raises(RuntimeError):
         q(x.cpu())
+
+
+@pytest.mark.parametrize("heads", [(8, 8), (16, 2)])
+def test_batched_decode_launches_match_single_sequences(heads):
+    """rope / attention / sampler for B sequences in one launch == one launch per sequence, bit for bit."""
+    H, KV = heads
+    B, P, hd, vocab = 3, 700, 128, 5003
+    g = torch.Generator(device=DEV).manual_seed(H)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV).half()  # noqa: E731
+    q, k, v = r(B, H * hd), r(B, KV * hd), r(B, KV * hd)
+    ck, cv = r(B, 2, P, KV * hd), r(B, 2, P, KV * hd)
+    pos = torch.tensor([0, 37, 650], dtype=torch.int32, device=DEV)
+    q1, ck1, cv1 = q.clone(), ck.clone(), cv.clone()
+    out, out1 = torch.zeros_like(q), torch.zeros_like(q)
+    ops.rope_kv_append_batch(q, k, v, ck[:, 1], cv[:, 1], pos, H, KV, hd)
+    ops.attn_decode_batch(out, q, ck[:, 1], cv[:, 1], pos, H, KV, hd)
+    for b in range(B):
+        ops.rope_kv_append(q1[b], k[b], v[b], ck1[b, 1], cv1[b, 1], pos[b:b + 1], H, KV, hd)
+        ops.attn_decode(out1[b], q1[b], ck1[b, 1], cv1[b, 1], pos[b:b + 1], H, KV, hd)
+    assert torch.equal(q, q1) and torch.equal(ck, ck1) and torch.equal(cv, cv1) and torch.equal(out, out1)
+    logits = torch.randn(B, vocab, generator=g, device=DEV)
+    tok, tok1 = torch.zeros(B, dtype=torch.int64, device=DEV), torch.zeros(B, dtype=torch.int64, device=DEV)
+    log, log1 = torch.zeros(B, 700, dtype=torch.int64, device=DEV), torch.zeros(B, 700, dtype=torch.int64, device=DEV)
+    p1 = pos.clone()
+    ops.sample_top_k_batch(tok, log, pos, logits, seed=7)
+    for b in range(B):
+        ops.sample_top_k(tok1[b:b + 1], log1[b], p1[b:b + 1], logits[b:b + 1], seed=7 + b)
+    assert torch.equal(tok, tok1) and torch.equal(log, log1) and torch.equal(pos, p1)
+    top = logits.topk(5).indices
+    assert all(int(tok[b]) in top[b].tolist() for b in range(B))
+
+
+@pytest.mark.parametrize("vocab,top_k", [(5, 5), (9, 1), (1000, 16), (300001, 7)])
+def test_sampler_vocabulary_slices(vocab, top_k):
+    """Vocabularies shorter than a slice per CTA, and longer than the registers hold; near-zero temperature = arg-max, first of ties."""
+    g = torch.Generator(device=DEV).manual_seed(vocab)
+    logits = torch.randn(1, vocab, generator=g, device=DEV)
+    best = int(logits.argmax())
+    logits[0, vocab - 1] = logits[0, best]
+    tok, log = torch.zeros(1, dtype=torch.int64, device=DEV), torch.zeros(64, dtype=torch.int64, device=DEV)
+    pos = torch.zeros(1, dtype=torch.int32, device=DEV)
+    seen = set()
+    for _ in range(40):
+        ops.sample_top_k(tok, log, pos, logits, temperature=1e-3, top_k=top_k, seed=3)
+        seen.add(int(tok))
+    assert seen <= {best, vocab - 1} and (top_k > 1 or seen == {best}) and int(pos) == 40
