@@ -281,8 +281,8 @@ __global__ void __launch_bounds__(kAttnThreads)
 // With few heads a cluster of SPLIT CTAs shares a head: each repeats the (short) front part and owns the positions t with
 // t % 32 in its range of residues.  Scores are exchanged through distributed shared memory, so that every CTA forms the same
 // maximum, probabilities and denominator; CTA 0 adds the 32 residues' sums of V rows in order.  Every sum has the order it has
-// with one CTA per head, so the result does not depend on the split.  Measured in the 7B-shaped step at 500 positions: 19.6 ->
-// PLACEHOLDER us per layer.
+// with one CTA per head, so the result does not depend on the split.  The first batch of K rows is requested before the front part.
+// Measured, 32 heads, 500 positions: 11.5 us (one CTA per head, K after the front part) -> 8.8.
 struct AttnFusedArgs {
     const float *y_q, *y_k, *y_v, *sv_q, *sv_k, *sv_v;
     float scale_q, scale_kv;
@@ -310,6 +310,45 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const A
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int pos = *a.pos;
     if (!position_ok(pos, a.max_pos, a.status)) return;
+
+    const int ctx = pos + 1;
+    const size_t row = (size_t)a.n_kv * hd;
+    // group grp of 16 lanes takes residue rank*R + grp % R of the positions, every SPLIT-th of them
+    const __half *kb = a.cache_k + (size_t)kvh * hd + sub * 8;
+    const int t_first = rank * R + grp % R + (grp / R) * G;
+    uint4 kr[U];
+    auto load_k = [&](int c0, int tb, int cn) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int t = tb + t_first + u * G * SPLIT;
+            kr[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (t < cn && c0 + t < pos) kr[u] = __ldg(reinterpret_cast<const uint4 *>(kb + (size_t)(c0 + t) * row));
+        }
+    };
+    // sum of V rows: residue rank*R + vr of the positions, dimensions vd .. vd + D - 1
+    const int vr = tid / (16 * SPLIT), vd = (tid % (16 * SPLIT)) * D, v_first = rank * R + vr;
+    const __half *vb = a.cache_v + (size_t)kvh * hd + vd;
+    uint32_t vraw[U][D / 2];
+    auto load_v = [&](int c0, int tb, int cn) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int t = tb + v_first + u * G;
+#pragma unroll
+            for (int i = 0; i < D / 2; i++) vraw[u][i] = 0u;
+            if (t < cn && c0 + t < pos) {
+                const __half *src = vb + (size_t)(c0 + t) * row;
+                if constexpr (D == 8) {
+                    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(src));
+                    vraw[u][0] = q.x; vraw[u][1] = q.y; vraw[u][2] = q.z; vraw[u][3] = q.w;
+                } else if constexpr (D == 4) {
+                    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(src));
+                    vraw[u][0] = q.x; vraw[u][1] = q.y;
+                } else vraw[u][0] = __ldg(reinterpret_cast<const uint32_t *>(src));
+            }
+        }
+    };
+    // the first batch of cache rows does not depend on q: in flight during the front part
+    load_k(0, 0, min(kAttnChunk, ctx));
 
     // ---- signed sums over heads: thread (quarter, d) adds a quarter of the heads (all three loads batches in flight)
     {
@@ -376,25 +415,9 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const A
     __syncthreads();
 
     // ---- attention over rows 0..pos (row pos from shared memory)
-    const int ctx = pos + 1;
-    const size_t row = (size_t)a.n_kv * hd;
     float qv[8];
 #pragma unroll
     for (int i = 0; i < 8; i++) qv[i] = cur[0][sub * 8 + i];
-    const __half *kb = a.cache_k + (size_t)kvh * hd + sub * 8;
-    // sum of V rows: residue rank*R + vr of the positions, dimensions vd .. vd + D - 1
-    const int vr = tid / (16 * SPLIT), vd = (tid % (16 * SPLIT)) * D;
-    const __half *vb = a.cache_v + (size_t)kvh * hd + vd;
-    auto load_v = [&](int t_global, uint32_t (&raw)[D / 2]) {
-        const __half *src = vb + (size_t)t_global * row;
-        if constexpr (D == 8) {
-            const uint4 q = __ldg(reinterpret_cast<const uint4 *>(src));
-            raw[0] = q.x; raw[1] = q.y; raw[2] = q.z; raw[3] = q.w;
-        } else if constexpr (D == 4) {
-            const uint2 q = __ldg(reinterpret_cast<const uint2 *>(src));
-            raw[0] = q.x; raw[1] = q.y;
-        } else raw[0] = __ldg(reinterpret_cast<const uint32_t *>(src));
-    };
     uint32_t peer_sc[SPLIT];                           // sc of every CTA of the cluster
 #pragma unroll
     for (int r = 0; r < SPLIT; r++) {
@@ -405,16 +428,8 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const A
     float m_run = -INFINITY, d_run = 0.f, acc[D] = {};
     for (int c0 = 0; c0 < ctx; c0 += kAttnChunk) {
         const int cn = min(kAttnChunk, ctx - c0);
-        // group grp of 16 lanes takes residue rank*R + grp % R, every SPLIT-th of its positions
-        const int t_first = rank * R + grp % R + (grp / R) * G;
         for (int tb = 0; tb < cn; tb += U * G * SPLIT) {
-            uint4 kr[U];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int t = tb + t_first + u * G * SPLIT;
-                kr[u] = make_uint4(0u, 0u, 0u, 0u);
-                if (t < cn && c0 + t < pos) kr[u] = __ldg(reinterpret_cast<const uint4 *>(kb + (size_t)(c0 + t) * row));
-            }
+            if (c0 > 0 || tb > 0) load_k(c0, tb, cn);
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const int t = tb + t_first + u * G * SPLIT;
@@ -434,15 +449,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const A
             }
         }
         // first batch of V rows: in flight during the exchange below
-        uint32_t vraw[U][D / 2];
-        const int v_first = rank * R + vr;
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int t = v_first + u * G;
-#pragma unroll
-            for (int i = 0; i < D / 2; i++) vraw[u][i] = 0u;
-            if (t < cn && c0 + t < pos) load_v(c0 + t, vraw[u]);
-        }
+        load_v(c0, 0, cn);
         if constexpr (SPLIT == 1) __syncthreads();
         else asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
         // every CTA holds all scores of the chunk
@@ -480,11 +487,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const A
             for (int u = 0; u < U; u++)
 #pragma unroll
                 for (int i = 0; i < D / 2; i++) curv[u][i] = vraw[u][i];
-#pragma unroll
-            for (int u = 0; u < U; u++) {
-                const int t = tb + U * G + v_first + u * G;
-                if (t < cn && c0 + t < pos) load_v(c0 + t, vraw[u]);
-            }
+            load_v(c0, tb + U * G, cn);
 #pragma unroll
             for (int u = 0; u < U; u++) {
                 const int t = tb + v_first + u * G;
@@ -639,8 +642,10 @@ extern "C" int qtip_attn_decode_fused(void *out, const float *y_q, const float *
     a.pos = pos; a.n_heads = n_heads; a.n_kv = n_kv_heads; a.log2_theta = log2f(theta);
     a.softmax_scale = 1.0f / sqrtf((float)head_dim);
     a.max_pos = max_positions; a.status = status;
-    // as many CTAs per head as the chip has room for, at most four (the front part is repeated by each)
-    const int split = n_heads * 4 <= sm_count() ? 4 : n_heads * 2 <= sm_count() ? 2 : 1;
+    // Four CTAs per head where the chip has room (two for up to 64 heads); their barriers do not pay on short contexts (32 heads,
+    // microseconds with 1 / 2 / 4 CTAs: 128 positions 6.7 / 7.5 / 7.5, 500 10.4 / 9.1 / 8.8, 1000 17.6 / 15.0 / 11.5), for which the
+    // cache's capacity stands.
+    const int split = max_positions <= 256 ? 1 : n_heads * 4 <= sm_count() ? 4 : n_heads * 2 <= sm_count() ? 2 : 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_heads * split);
     cfg.blockDim = dim3(kAttnThreads);

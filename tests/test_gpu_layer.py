@@ -574,3 +574,31 @@ def test_sampler_vocabulary_slices(vocab, top_k):
         ops.sample_top_k(tok, log, pos, logits, temperature=1e-3, top_k=top_k, seed=3)
         seen.add(int(tok))
     assert seen <= {best, vocab - 1} and (top_k > 1 or seen == {best}) and int(pos) == 40
+
+
+@pytest.mark.parametrize("heads", [(32, 8), (64, 64), (128, 8)])
+@pytest.mark.parametrize("pos_v", [0, 5, 1023, 2047, 2048, 2600])
+def test_attn_decode_fused_splits_agree(heads, pos_v):
+    """Four, two and one CTA per head (64 and 128 heads; a cache of up to 256 positions forces one): the sums keep their order, so a
+    short cache and a long one give the same bits; several chunks of positions against the separate launches."""
+    n_heads, n_kv = heads
+    hd, maxpos = 128, 2700
+    H, KV = n_heads * hd, n_kv * hd
+    g = torch.Generator(device=DEV).manual_seed(n_heads + pos_v)
+    y = [torch.randn(w, generator=g, device=DEV) for w in (H, KV, KV)]
+    pos = torch.tensor([pos_v], dtype=torch.int32, device=DEV)
+    ck, cv = ((0.5 * torch.randn(maxpos, KV, generator=g, device=DEV)).half() for _ in range(2))
+
+    def fused(ck, cv):
+        out = torch.zeros(n_heads, hd, dtype=torch.float16, device=DEV)
+        ops.attn_decode_fused(out, y[0], y[1], y[2], None, None, None, H**-0.5, KV**-0.5, ck, cv, pos, n_heads, n_kv, hd)
+        return out
+    ck1, cv1 = ck.clone(), cv.clone()
+    got = fused(ck1, cv1)
+    if pos_v < 256:
+        assert torch.equal(got, fused(ck[:256].clone(), cv[:256].clone()))
+    q, k, v = [ops.rht(t.view(1, -1), scale=t.numel()**-0.5, out_dtype=torch.float16).view(-1) for t in y]
+    ops.rope_kv_append(q, k, v, ck, cv, pos, n_heads, n_kv, hd)
+    want = torch.zeros_like(got)
+    ops.attn_decode(want, q, ck, cv, pos, n_heads, n_kv, hd)
+    assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) < 2e-3
