@@ -12,11 +12,11 @@
 //   * one thread issues four tcgen05.mma (K = 16 each) per stage and commits them to the stage's
 //     "empty" barrier; a last commit signals the epilogue.
 //   * warps 0-3 read the accumulator with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 = rows) and
-//     write out (coalesced along rows); with a 2-way column split the two CTAs of a row range add
-//     into a zeroed output (two addends: order-independent, so still deterministic).
+//     write out (coalesced along rows); when the row ranges leave SMs idle the columns are split over the
+//     2, 4 or 8 CTAs of a cluster, which leave their parts in shared memory and add them in order.
 // The compute codes (3INST / 1MAD, V = 1, plain layout) use the same kernel with another producer: a lane decodes
-// eight consecutive states of a tile row (44 stream bits) and stores the eight weights as ONE 16-byte chunk of the
-// swizzled A tile; no table is built.  That path is bound by the per-weight arithmetic, not by the tensor pipe.
+// eight consecutive states of a tile row (its own K bytes and the next lane's) and stores the eight weights as ONE 16-byte chunk
+// of the swizzled A tile.  That path is bound by the per-weight arithmetic, not by the tensor pipe.
 // This replaces decode-to-HBM + dense GEMM of BitshiftLinearKernelAG upstream
 // (lib/codebook/bitshift.py:476-489), which writes and re-reads 16x the packed bytes at 2 bits.
 //
@@ -111,17 +111,55 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// 48 stream bits of a plain-layout tile starting at bit pos (circular over the tile's 16K words), first bit at bit 47
-__device__ __forceinline__ uint64_t plain_bits48(const uint16_t *__restrict__ words, int nwords, int pos) {
-    int w = pos >> 4;
-    uint64_t v = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        int wi = w + i;
-        if (wi >= nwords) wi -= nwords;
-        v = (v << 16) | __ldg(words + wi);
+// Plain layout (V = 1 codes): a 16x16 tile is 16K 16-bit words, first stream bit = top bit of word 0, circular.  Lane l decodes
+// states 8l .. 8l+7, whose windows start K bits apart from bit 8Kl on: its own K bytes and 12..15 bits that follow.  A lane loads
+// what starts with its own bytes as whole 16-bit words (a K = 3 lane may start in the middle of one) ...
+template <int K>
+__device__ __forceinline__ uint32_t plain_lane_load(const uint16_t *__restrict__ tile, int lane) {
+    if constexpr (K == 2) return __ldg(tile + lane);
+    else if constexpr (K == 3) return __ldg(tile + (3 * lane) / 2) << 16 | __ldg(tile + (3 * lane) / 2 + 1);      // words of bytes 3l .. 3l+3
+    else {
+        const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(tile) + lane);                               // two words, little-endian pair
+        return v << 16 | v >> 16;
     }
-    return (v << (pos & 15)) >> 16;
+}
+// ... and gets the rest from the next lane: 48 bits with the lane's first bit at bit 47
+template <int K>
+__device__ __forceinline__ uint64_t plain_lane_bits(uint32_t own, int lane) {
+    const uint32_t next = __shfl_sync(kFullMask, own, lane + 1);      // lane 31 wraps to lane 0: tail-biting
+    if constexpr (K == 2) return ((uint64_t)own << 32) | (uint64_t)next << 16;
+    else if constexpr (K == 3) {
+        // bytes 3l .. 3l+2, then the next lane's three (both without what precedes them in their word)
+        const uint32_t a = (lane & 1) ? own & 0xFFFFFFu : own >> 8, b = (lane & 1) ? next >> 8 : next & 0xFFFFFFu;
+        return ((uint64_t)a << 24) | b;
+    } else return ((uint64_t)own << 16) | (next >> 16);
+}
+
+constexpr int kMaxSplit = 8;
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float cluster_load(uint32_t addr, int rank) {
+    uint32_t p;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(p) : "memory");
+    return v;
+}
+
+// Two weights of the compute codes, packed.  3INST: the two fp16 terms of both states are gathered into two registers and added as
+// pairs.  1MAD: byte sums of the LCG values by dot product, weights from the lane's copy of the table.
+__device__ __forceinline__ uint32_t pair_3inst(uint32_t s0, uint32_t s1) {
+    const uint32_t r0 = ((s0 * 89226354u + 64248484u) & 0x8FFF8FFFu) ^ 0x3B603B60u, r1 = ((s1 * 89226354u + 64248484u) & 0x8FFF8FFFu) ^ 0x3B603B60u;
+    const uint32_t lo = __byte_perm(r0, r1, 0x5410), hi = __byte_perm(r0, r1, 0x7632);
+    const __half2 w = __hadd2(*reinterpret_cast<const __half2 *>(&lo), *reinterpret_cast<const __half2 *>(&hi));
+    return *reinterpret_cast<const uint32_t *>(&w);
+}
+__device__ __forceinline__ uint32_t pair_1mad(uint32_t s0, uint32_t s1, uint32_t lut_lane) {
+    uint32_t w0, w1;
+    asm("ld.shared.u32 %0, [%1];" : "=r"(w0) : "r"(__dp4a(s0 * 34038481u + 76625530u, 0x01010101u, 0u) * 128u + lut_lane));
+    asm("ld.shared.u32 %0, [%1];" : "=r"(w1) : "r"(__dp4a(s1 * 34038481u + 76625530u, 0x01010101u, 0u) * 128u + lut_lane));
+    return __byte_perm(w0, w1, 0x5410);
 }
 
 // STAGES: ring depth, 4 for batches up to 64 (B tile <= 8 KiB), 3 above (16 KiB B tiles); a compile-time value so that
@@ -166,24 +204,31 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     // lane-private copies of the table: entry e = sign << 9 | index, copy l at byte e*128 + l*4; the sign bit of
     // the hash flips the first weight of the pair, so it is folded into the table (no per-state sign op)
-    __half *mad_tab = reinterpret_cast<__half *>(lut);     // 1MAD: byte sum -> weight (the table area is otherwise unused)
-    if constexpr (CODE == QTIP_CODE_1MAD) build_1mad_table(mad_tab);
+    // 1MAD: the weight of every byte sum (decode_1mad's own arithmetic) in the same form, 1021 entries used
+    if constexpr (CODE == QTIP_CODE_1MAD) {
+        for (int i = threadIdx.x; i < 1024 * 8; i += kGemmThreads) {
+            const uint32_t e = __half_as_ushort(__float2half_rn(__fdiv_rn((float)((i >> 3) - 510), 147.800537109375f)));
+            reinterpret_cast<uint4 *>(lut)[i] = make_uint4(e, e, e, e);
+        }
+    }
     if constexpr (kHyb) {
         for (int i = threadIdx.x; i < 1024 * 8; i += kGemmThreads) {
             const uint32_t e = __ldg(tlut + ((i >> 3) & 511)) ^ ((uint32_t)(i >> 12) << 15);
             reinterpret_cast<uint4 *>(lut)[i] = make_uint4(e, e, e, e);
         }
     }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_d = ctl->tmem_base;
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // everything above touches weights only
 
     const int nb = n >> 5;                                  // 32-column blocks per row block
     const int r0 = blockIdx.x * kRows;                      // first output row of this CTA
-    const int cols_per_split = n / splitk;
-    const int c0 = blockIdx.y * cols_per_split;             // first input column
-    const int nsteps = cols_per_split / kStageCols;
+    const int all_steps = n / kStageCols;                   // split over the CTAs of the cluster, not necessarily evenly
+    const int step0 = all_steps * (int)blockIdx.y / splitk, nsteps = all_steps * ((int)blockIdx.y + 1) / splitk - step0;
+    const int c0 = step0 * kStageCols;                      // first input column
 
     if (warp < kDecodeWarps) {
         // ---------------------------------- decode warps ------------------------------------------------
@@ -215,8 +260,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // lane decodes row pr of each of the warp's four tiles, columns 8*ph .. 8*ph+7
         const uint16_t *pcodes = reinterpret_cast<const uint16_t *>(codes);
         const int tn = n >> 4, pr = lane >> 1, ph = lane & 1;
+        // this warp's four tiles (ks, ms) of a step: 16K words each, tile rows 2rb, 2rb + 1, tile columns 2cb, 2cb + 1
+        const uint16_t *ptile = pcodes + ((size_t)(r0 / 16 + 2 * rb) * tn + (size_t)(c0 / 16 + 2 * cb)) * (16 * K);
+        uint32_t pown_next[4] = {};
+        auto load_plain = [&](int step) {
+#pragma unroll
+            for (int tt = 0; tt < 4; tt++)
+                pown_next[tt] = plain_lane_load<K>(ptile + ((size_t)(tt & 1) * tn + (tt >> 1) + (size_t)step * (kStageCols / 16)) * (16 * K), lane);
+        };
         if (group < nsteps) {
             if constexpr (kHyb) own_next = load_lane_codes<K>(src + (size_t)group * 2 * kBlockBytes);
+            else load_plain(group);
             if (has0) xv0_next = load_x(group, tid8);
             if (has1) xv1_next = load_x(group, tid8 + 256);
         }
@@ -239,15 +293,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             }
             if constexpr (kHyb)
                 if (step + 2 * kGroups < nsteps) own_next2 = load_lane_codes<K>(src + (size_t)(step + 2 * kGroups) * 2 * kBlockBytes);
-            // V = 1: the 44 bits this lane needs of each of its four tiles are requested before the wait for the stage
-            uint64_t pbits[4];
+            uint32_t pown[4];
             if constexpr (!kHyb) {
 #pragma unroll
-                for (int tt = 0; tt < 4; tt++) {
-                    const int ks = tt >> 1, ms = tt & 1;
-                    const size_t tile = (size_t)(r0 / 16 + 2 * rb + ms) * tn + (size_t)((c0 + step * kStageCols) / 16 + 2 * cb + ks);
-                    pbits[tt] = plain_bits48(pcodes + tile * (16 * K), 16 * K, (pr * 16 + ph * 8) * K);
-                }
+                for (int tt = 0; tt < 4; tt++) pown[tt] = pown_next[tt];
+                if (step + kGroups < nsteps) load_plain(step + kGroups);
             }
             if (round > 0) mbar_wait(smem_addr(&ctl->empty[s]), (round - 1) & 1, abort_flag, status, 1u);
             LaneCodes<K> nxt = {};
@@ -299,15 +349,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
                 for (int tt = 0; tt < 4; tt++) {
                     const int ks = tt >> 1, ms = tt & 1;
+                    const uint64_t bits = plain_lane_bits<K>(pown[tt], lane);
                     uint32_t wv[4];
 #pragma unroll
                     for (int j = 0; j < 4; j++) {          // eight states, K bits apart, two weights per word
-                        const uint32_t s0 = (uint32_t)(pbits[tt] >> (32 - 2 * j * K)) & 0xFFFFu;
-                        const uint32_t s1 = (uint32_t)(pbits[tt] >> (32 - (2 * j + 1) * K)) & 0xFFFFu;
-                        const __half lo = CODE == QTIP_CODE_3INST ? decode_3inst(s0) : decode_1mad_tab(s0, mad_tab);
-                        const __half hi = CODE == QTIP_CODE_3INST ? decode_3inst(s1) : decode_1mad_tab(s1, mad_tab);
-                        const __half2 p2 = __halves2half2(lo, hi);
-                        wv[j] = *reinterpret_cast<const uint32_t *>(&p2);
+                        const uint32_t s0 = (uint32_t)(bits >> (32 - 2 * j * K)) & 0xFFFFu;
+                        const uint32_t s1 = (uint32_t)(bits >> (32 - (2 * j + 1) * K)) & 0xFFFFu;
+                        wv[j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1) : pair_1mad(s0, s1, lut_lane);
                     }
                     // row 32rb + 16ms + pr of the stage, 16-byte chunk 4cb + 2ks + ph of its 128-byte row
                     const uint32_t row = (uint32_t)(32 * rb + 16 * ms + pr), chunk = (uint32_t)(4 * cb + 2 * ks + ph);
@@ -348,6 +396,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         mbar_wait(smem_addr(&ctl->done), 0u, abort_flag, status, 3u);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int row = r0 + warp * 32 + lane;
+        float *part = reinterpret_cast<float *>(smem);      // [bs][128]: the ring is no longer needed (every MMA has completed)
         for (int col = 0; col < npad; col += 8) {
             uint32_t r[8];
             const uint32_t taddr = tmem_d + ((uint32_t)(warp * 32) << 16) + (uint32_t)col;
@@ -362,7 +411,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 if (bcol < bs) {
                     const float v = __uint_as_float(r[j]);
                     if (splitk == 1) out[(size_t)bcol * m + row] = v;
-                    else atomicAdd(out + (size_t)bcol * m + row, v);
+                    else part[bcol * kRows + warp * 32 + lane] = v;
                 }
             }
         }
@@ -376,6 +425,24 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(tmem_cols) : "memory");
+    }
+    // column splits: the cluster's CTAs add their parts in order, each its share of the outputs
+    if (splitk > 1) {
+        cluster_barrier();
+        const int total = bs * kRows;
+        const uint32_t part = smem_addr(smem);
+        for (int i = (int)blockIdx.y * kGemmThreads + (int)threadIdx.x; i < total; i += splitk * kGemmThreads) {
+            float v[kMaxSplit];
+#pragma unroll
+            for (int r = 0; r < kMaxSplit; r++)
+                if (r < splitk) v[r] = cluster_load(part + i * 4u, r);
+            float t = v[0];
+#pragma unroll
+            for (int r = 1; r < kMaxSplit; r++)
+                if (r < splitk) t += v[r];
+            out[(size_t)(i / kRows) * m + r0 + (i & (kRows - 1))] = t;
+        }
+        cluster_barrier();                                   // the parts are read
     }
 }
 
@@ -396,9 +463,21 @@ int launch_gemm_stages(float *out, const uint8_t *codes, const __half *x, const 
             attr_set[dev] = true;
         }
     }
-    if (splitk > 1) QTIP_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)bs * m * sizeof(float), s));
-    decompress_gemm_kernel<K, CODE, STAGES><<<dim3(m / kRows, splitk), kGemmThreads, smem, s>>>(out, codes, x, tlut, m, n, bs,
-                                                                                                npad, splitk, status);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(m / kRows, splitk);
+    cfg.blockDim = dim3(kGemmThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = 1;
+    attr[1].val.clusterDim.y = splitk;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = splitk > 1 ? 2 : 1;
+    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decompress_gemm_kernel<K, CODE, STAGES>, out, codes, x, tlut, m, n, bs, npad, splitk, status));
     return check_launch();
 }
 
@@ -408,6 +487,13 @@ int launch_gemm(float *out, const uint8_t *codes, const __half *x, const uint32_
                 int splitk, unsigned *status, cudaStream_t s) {
     if (npad > 64) return launch_gemm_stages<K, CODE, 3>(out, codes, x, tlut, m, n, bs, npad, splitk, status, s);
     return launch_gemm_stages<K, CODE, kStages>(out, codes, x, tlut, m, n, bs, npad, splitk, status, s);
+}
+
+// CTAs per row range: as many as still fit the chip at once, in a cluster (at most the portable eight), each with a few steps
+int column_splits(int m, int n) {
+    int s = 1;
+    while (s < kMaxSplit && (m / kRows) * s * 2 <= sm_count() && n / kStageCols >= 8 * s) s *= 2;
+    return s;
 }
 
 template <int CODE>
@@ -431,8 +517,7 @@ extern "C" int qtip_decompress_gemm(float *out, const void *codes, const void *x
     if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, 4) || !aligned(tlut, 4) || !aligned(status, 4))
         return QTIP_ERR_ALIGNMENT;
     const int npad = (bs + 15) & ~15;
-    // two CTAs per row range while that still leaves SMs idle and the column range divides
-    const int splitk = ((m / kRows) * 2 <= sm_count() && (n % (2 * kStageCols)) == 0) ? 2 : 1;
+    const int splitk = column_splits(m, n);
     auto *c = static_cast<const uint8_t *>(codes);
     auto *xh = static_cast<const __half *>(x);
     auto *t = static_cast<const uint32_t *>(tlut);
@@ -448,7 +533,7 @@ extern "C" int qtip_decompress_gemm_plain(float *out, const void *codes, const v
     if ((long)(m >> 5) * (n >> 5) >= (1L << 30)) return QTIP_ERR_BAD_SHAPE;
     if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, 4) || !aligned(status, 4)) return QTIP_ERR_ALIGNMENT;
     const int npad = (bs + 15) & ~15;
-    const int splitk = ((m / kRows) * 2 <= sm_count() && (n % (2 * kStageCols)) == 0) ? 2 : 1;
+    const int splitk = column_splits(m, n);
     auto *c = static_cast<const uint8_t *>(codes);
     auto *xh = static_cast<const __half *>(x);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
