@@ -623,10 +623,13 @@ __global__ void __launch_bounds__(VitCfg<CODE, KV>::kThreads, VitCfg<CODE, KV>::
     }
 }
 
+// CTAs of a launch; each has a workspace of its own.  HYB K=2 stores 16 KiB at every second step, twice the 4096 bytes per step
+// and sequence that the workspace contract states, so there a CTA takes at least two sequences.
 template <int CODE, int KV>
 long vit_grid(long N) {
-    const long cap = (long)sm_count() * VitCfg<CODE, KV>::kPerSm;
-    return N < cap ? N : cap;
+    constexpr int kAtLeast = VitCfg<CODE, KV>::kHyb && KV == 4 ? 2 : 1;
+    const long cap = (long)sm_count() * VitCfg<CODE, KV>::kPerSm, want = (N + kAtLeast - 1) / kAtLeast;
+    return want < cap ? want : cap;
 }
 
 template <int CODE, int KV>
