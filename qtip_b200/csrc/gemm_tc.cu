@@ -3,25 +3,27 @@
 //   out (bs, m) fp32 = X (bs, n) fp16 @ decode(codes)^T        HYB code, kernel layout
 //
 // One CTA owns 128 output rows (four 32-row blocks) and a contiguous range of input columns.  The
-// weights are the A operand: D[128 x N] += A[128 x 16] * B[16 x N] with D in tensor memory, A and B
-// in shared memory, K-major, 128-byte swizzle; N = batch rounded up to 16.
-//   * 24 decode warps turn packed codes into fp16 and store them straight into the swizzled A tile
-//     of a ring stage (128 rows x 64 columns = 8 tile blocks, one per warp; three stages are
-//     filled concurrently).  The stores of a warp hit 32 distinct banks.  The same warps copy the 64-column
-//     slice of X into the B tile of the stage.
+// weights are the A operand: D[128 x N] += A[128 x 16] * B[16 x N] with D AND A in tensor memory, B in
+// shared memory, K-major, 128-byte swizzle; N = batch rounded up to 16.
+//   * 24 decode warps turn packed codes into fp16 and store them with tcgen05.st into the A part of a ring stage (128 rows x
+//     64 columns = 8 tile blocks, one per warp; three stages are filled concurrently).  A kernel-layout tile block in its lanes IS
+//     the 16x128b store shape, so the weights never pass through shared memory, whose wavefronts the table lookups need.
+//     The same warps copy the 64-column slice of X into the B tile of the stage.
 //   * one thread issues four tcgen05.mma (K = 16 each) per stage and commits them to the stage's
 //     "empty" barrier; a last commit signals the epilogue.
 //   * warps 0-3 read the accumulator with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 = rows) and
 //     write out (coalesced along rows); when the row ranges leave SMs idle the columns are split over the
 //     2, 4 or 8 CTAs of a cluster, which leave their parts in shared memory and add them in order.
-// The compute codes (3INST / 1MAD, V = 1, plain layout) use the same kernel with another producer: a lane decodes
-// eight consecutive states of a tile row (its own K bytes and the next lane's) and stores the eight weights as ONE 16-byte chunk
-// of the swizzled A tile.  That path is bound by the per-weight arithmetic, not by the tensor pipe.
+// The compute codes (3INST / 1MAD, V = 1, plain layout) use the same kernel with another producer: a lane decodes one row of a
+// tile (its own 2K bytes and the start of the next row), lanes 2r and 2r + 1 row r of two tiles, and stores a row per
+// tensor-memory lane; the accumulator's lanes are mapped back to rows when they are read.
+// Bound: instruction issue of the decode warps (~155 instructions per warp and stage HYB, ~270 3INST; the tensor pipe is busy
+// 10 % of the time, and leaving out three of the four MMAs, the loads or half of the ring's depth changes nothing).  Hence the loop unrolled
+// by two with fixed stages and buffers, and x through asynchronous copies issued a step ahead.  Measured, K = 2, A through shared
+// memory and x through registers -> now:  HYB 8192 x 8192, 27 rows 28.7 -> 20.2 us; 8192 x 28672, 120 rows 123.5 -> 72.1 us;
+// 3INST 8192 x 8192, 27 rows 36.9 -> 33.5 us, 120 rows of 28672 155.7 -> 115.6 us; 1MAD 37.5 -> 30.0 us, 163.7 -> 104.8 us.
 // This replaces decode-to-HBM + dense GEMM of BitshiftLinearKernelAG upstream
 // (lib/codebook/bitshift.py:476-489), which writes and re-reads 16x the packed bytes at 2 bits.
-//
-// Only the decode is expensive (one table lookup + one shared-memory store per state); the MMA work
-// is negligible below batch 256, so the kernel runs at roughly the speed of the batch-1 matvec.
 //
 // Every mbarrier wait is bounded: after kSpinLimit polls the waiter records an error code in
 // `status`, raises a CTA-wide abort flag that makes every later wait fall through, and the kernel
@@ -36,10 +38,10 @@ namespace {
 constexpr int kGroups = 3;                               // groups of 8 decode warps; a group fills one stage
 constexpr int kDecodeWarps = 8 * kGroups;
 constexpr int kGemmThreads = (kDecodeWarps + 1) * 32;   // + one control warp (TMEM allocation, MMA issue)
-constexpr int kStages = 4;                              // ring stages for batches up to 64; 3 for 65..128 (shared memory)
+constexpr int kStages = 2 * kGroups;                    // ring stages: every group may be one step ahead of the MMA
 constexpr int kRows = 128;                               // output rows per CTA
 constexpr int kStageCols = 64;                           // input columns per stage (128 bytes of fp16 per row)
-constexpr int kAStageBytes = kRows * kStageCols * 2;     // 16 KiB
+constexpr int kAStageCols = kStageCols / 2;              // 32-bit tensor-memory columns of an A stage: two weights each
 constexpr int kLut512Bytes = 1024 * 32 * 4;              // (512 entries + sign-flipped twins) x 32 lane-private copies
 constexpr int kMaxN = 128;
 constexpr unsigned kSpinLimit = 1u << 22;
@@ -99,40 +101,68 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
     return d;
 }
 
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// 16 rows x 16 words of tensor memory; lane (a, b) holds words 4j + b of rows a (v[2j]) and a + 8 (v[2j + 1])
+__device__ __forceinline__ void tmem_st_16x128b_x4(uint32_t addr, const uint32_t *v) {
+    asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+// 32 rows x 16 words, a row per lane
+__device__ __forceinline__ void tmem_st_32x32b_x16(uint32_t addr, const uint32_t *v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+                 "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                 : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// Plain layout (V = 1 codes): a 16x16 tile is 16K 16-bit words, first stream bit = top bit of word 0, circular.  Lane l decodes
-// states 8l .. 8l+7, whose windows start K bits apart from bit 8Kl on: its own K bytes and 12..15 bits that follow.  A lane loads
-// what starts with its own bytes as whole 16-bit words (a K = 3 lane may start in the middle of one) ...
+// Plain layout (V = 1 codes): a 16x16 tile is 16K 16-bit words, first stream bit = top bit of word 0, circular.  Row r of a tile is
+// K words; its 16 states' windows start K bits apart at word K*r and end 12..15 bits into the next row.
+// a: the row's first two words, b: the words after them, first in the top half
 template <int K>
-__device__ __forceinline__ uint32_t plain_lane_load(const uint16_t *__restrict__ tile, int lane) {
-    if constexpr (K == 2) return __ldg(tile + lane);
-    else if constexpr (K == 3) return __ldg(tile + (3 * lane) / 2) << 16 | __ldg(tile + (3 * lane) / 2 + 1);      // words of bytes 3l .. 3l+3
-    else {
-        const uint32_t v = __ldg(reinterpret_cast<const uint32_t *>(tile) + lane);                               // two words, little-endian pair
-        return v << 16 | v >> 16;
-    }
-}
-// ... and gets the rest from the next lane: 48 bits with the lane's first bit at bit 47
+struct PlainRow {
+    uint32_t a, b;
+};
 template <int K>
-__device__ __forceinline__ uint64_t plain_lane_bits(uint32_t own, int lane) {
-    const uint32_t next = __shfl_sync(kFullMask, own, lane + 1);      // lane 31 wraps to lane 0: tail-biting
-    if constexpr (K == 2) return ((uint64_t)own << 32) | (uint64_t)next << 16;
+__device__ __forceinline__ PlainRow<K> load_plain_row(const uint16_t *__restrict__ row) {
+    PlainRow<K> r = {};
+    if constexpr (K == 2) r.a = __byte_perm(__ldg(reinterpret_cast<const uint32_t *>(row)), 0, 0x1032);
     else if constexpr (K == 3) {
-        // bytes 3l .. 3l+2, then the next lane's three (both without what precedes them in their word)
-        const uint32_t a = (lane & 1) ? own & 0xFFFFFFu : own >> 8, b = (lane & 1) ? next >> 8 : next & 0xFFFFFFu;
-        return ((uint64_t)a << 24) | b;
-    } else return ((uint64_t)own << 16) | (next >> 16);
+        r.a = (uint32_t)__ldg(row) << 16 | __ldg(row + 1);
+        r.b = (uint32_t)__ldg(row + 2) << 16;
+    } else {
+        const uint2 v = __ldg(reinterpret_cast<const uint2 *>(row));
+        r.a = __byte_perm(v.x, 0, 0x1032);
+        r.b = __byte_perm(v.y, 0, 0x1032);
+    }
+    return r;
+}
+// state i of a row; next: the following row's first two words
+template <int K>
+__device__ __forceinline__ uint32_t plain_state(const PlainRow<K> &r, uint32_t next, int i) {
+    uint32_t hi = r.a, lo = r.b;
+    if constexpr (K == 2) lo = next;
+    if constexpr (K == 3) lo = r.b | next >> 16;
+    if (K * i >= 32) {          // i is a compile-time constant after unrolling
+        hi = lo;
+        lo = next;
+    }
+    return __funnelshift_l(lo, hi, K * i & 31) >> 16;
 }
 
 constexpr int kMaxSplit = 8;
@@ -162,14 +192,12 @@ __device__ __forceinline__ uint32_t pair_1mad(uint32_t s0, uint32_t s1, uint32_t
     return __byte_perm(w0, w1, 0x5410);
 }
 
-// STAGES: ring depth, 4 for batches up to 64 (B tile <= 8 KiB), 3 above (16 KiB B tiles); a compile-time value so that
-// the ring arithmetic of the common case stays free of run-time divisions
-template <int K, int CODE, int STAGES>
+// SMALL: batches up to 64, whose slice of x is at most two copies per thread and whose accumulator leaves half of tensor memory free
+template <int K, int CODE, bool SMALL>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     decompress_gemm_kernel(float *__restrict__ out, const uint8_t *__restrict__ codes, const __half *__restrict__ x,
                            const uint32_t *__restrict__ tlut, int m, int n, int bs, int npad, int splitk,
                            unsigned *__restrict__ status) {
-    constexpr int stages = STAGES;
     constexpr int kBlockBytes = 128 * K;
     constexpr bool kHyb = CODE == QTIP_CODE_HYB;
     extern __shared__ uint8_t smem_raw[];
@@ -177,17 +205,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const uint32_t base = (raw + 1023u) & ~1023u;                 // swizzled tiles need 1024-byte alignment
     uint8_t *smem = smem_raw + (base - raw);
     const int b_stage_bytes = npad * 128;
-    // layout: A stages | B stages | LUT | control
-    const uint32_t a_base = base, b_base = base + stages * kAStageBytes;
-    uint32_t *lut = reinterpret_cast<uint32_t *>(smem + stages * (kAStageBytes + b_stage_bytes));
-    GemmCtrl *ctl = reinterpret_cast<GemmCtrl *>(smem + stages * (kAStageBytes + b_stage_bytes) + kLut512Bytes);
+    // layout: B stages | LUT | control
+    const uint32_t b_base = base;
+    uint32_t *lut = reinterpret_cast<uint32_t *>(smem + kStages * b_stage_bytes);
+    GemmCtrl *ctl = reinterpret_cast<GemmCtrl *>(smem + kStages * b_stage_bytes + kLut512Bytes);
     volatile int *abort_flag = &ctl->abort_flag;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tmem_cols = npad <= 32 ? 32 : (npad <= 64 ? 64 : 128);
+    // tensor memory: kStages A stages, then the accumulator's npad columns
+    constexpr int kTmemD = kStages * kAStageCols, kTmemCols = SMALL ? 256 : 512;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < stages; s++) {
+        for (int s = 0; s < kStages; s++) {
             mbar_init(smem_addr(&ctl->full[s]), 8);     // eight decode warps fill a stage
             mbar_init(smem_addr(&ctl->empty[s]), 1);    // one tcgen05.commit frees it
         }
@@ -196,9 +225,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kDecodeWarps) {
-        // tensor memory for the accumulator: 128 lanes x tmem_cols 32-bit columns
+        // 128 lanes x kTmemCols 32-bit columns
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&ctl->tmem_base)),
-                     "r"(tmem_cols)
+                     "r"(kTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -221,7 +250,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_d = ctl->tmem_base;
+    const uint32_t tmem = ctl->tmem_base, tmem_d = tmem + kTmemD;
     asm volatile("griddepcontrol.wait;" ::: "memory");      // everything above touches weights only
 
     const int nb = n >> 5;                                  // 32-column blocks per row block
@@ -234,143 +263,108 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // ---------------------------------- decode warps ------------------------------------------------
         const int group = warp >> 3;                        // this group fills steps group, group + kGroups, ...
         const int w8 = warp & 7, rb = w8 & 3, cb = w8 >> 2; // row block (of 4) and column block (of 2) of the stage
-        const int a = lane >> 2, b = lane & 3;
         const uint32_t lut_lane = smem_addr(lut) + lane * 4;
-        const uint8_t *src = codes + ((size_t)(r0 / 32 + rb) * nb + (c0 / 32 + cb)) * kBlockBytes + lane * (4 * K);
-        // byte offset inside an A stage of this lane's element (ms, d, ks, c): row 32rb+16ms+8d+a, column 32cb+16ks+8c+2b
-        const uint32_t row_off = (uint32_t)(4 * rb) * 1024u + (uint32_t)a * 128u + (uint32_t)b * 4u;
-        const int tid8 = w8 * 32 + lane;                    // 0..255 within the stage's eight warps
+        // this warp's 32 rows and 16 words of an A stage (a warp reaches the 32 lanes of its index modulo four)
+        const uint32_t tmem_warp = tmem + ((uint32_t)(32 * rb) << 16) + 16u * cb;
         // The 64-column slice of x goes into the B tile of the stage: chunk ch of the tile = batch row ch >> 3, columns
-        // 8*(ch & 7) .. +7, rows beyond bs zero.  Batches up to 64 (at most two 16-byte chunks per thread): the chunks of
-        // the warp's NEXT step are requested into registers before the current step is decoded, so their latency hides
-        // behind a step of work.  Larger batches: asynchronous copies straight into the tile (no registers), awaited
-        // before the stage is handed over.
-        const int chunks = npad * 8;
-        constexpr bool small = STAGES == kStages;
-        const bool has0 = small && tid8 < chunks, has1 = small && tid8 + 256 < chunks;
-        auto load_x = [&](int step, int ch) -> uint4 {
-            const int brow = ch >> 3, c = ch & 7;
-            if (brow >= bs) return make_uint4(0u, 0u, 0u, 0u);
-            return *reinterpret_cast<const uint4 *>(x + (size_t)brow * n + c0 + step * kStageCols + c * 8);
-        };
-        uint4 xv0_next = make_uint4(0u, 0u, 0u, 0u), xv1_next = xv0_next;
-        // codes: two steps of this warp ahead (the warp's steps are kGroups apart)
-        LaneCodes<K> own_next = {}, own_next2 = {};
-        // plain layout (V = 1 codes): tile (tile row, tile column) = 16K words at ((row/16)*(n/16) + col/16)*16K; this
-        // lane decodes row pr of each of the warp's four tiles, columns 8*ph .. 8*ph+7
-        const uint16_t *pcodes = reinterpret_cast<const uint16_t *>(codes);
-        const int tn = n >> 4, pr = lane >> 1, ph = lane & 1;
-        // this warp's four tiles (ks, ms) of a step: 16K words each, tile rows 2rb, 2rb + 1, tile columns 2cb, 2cb + 1
-        const uint16_t *ptile = pcodes + ((size_t)(r0 / 16 + 2 * rb) * tn + (size_t)(c0 / 16 + 2 * cb)) * (16 * K);
-        uint32_t pown_next[4] = {};
-        auto load_plain = [&](int step) {
+        // 8*(ch & 7) .. +7, rows beyond bs zero, 16-byte chunks swizzled by row % 8.  Thread tid8 of the stage's eight warps copies chunks
+        // tid8 + 256 i.  The copies of the warp's NEXT step are issued after the current step is decoded and awaited a step later.
+        const int tid8 = w8 * 32 + lane, brow = tid8 >> 3;
+        const __half *xsrc = x + (size_t)brow * n + c0 + group * kStageCols + (tid8 & 7) * 8;
+        const uint32_t xdst = b_base + (uint32_t)(brow * 128 + (((tid8 & 7) ^ (brow & 7)) << 4));
+        auto copy_x = [&](int s) {
 #pragma unroll
-            for (int tt = 0; tt < 4; tt++)
-                pown_next[tt] = plain_lane_load<K>(ptile + ((size_t)(tt & 1) * tn + (tt >> 1) + (size_t)step * (kStageCols / 16)) * (16 * K), lane);
+            for (int i = 0; i < (SMALL ? 2 : 4); i++)
+                if (brow + 32 * i < npad) {
+                    const bool live = brow + 32 * i < bs;
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(xdst + (uint32_t)(s * b_stage_bytes + 4096 * i)),
+                                 "l"(live ? xsrc + (size_t)(32 * i) * n : x), "r"(live ? 16 : 0)
+                                 : "memory");
+                }
+            xsrc += kGroups * kStageCols;
+        };
+        // codes: two steps of this warp ahead (the warp's steps are kGroups apart), in two buffers that the two steps of the loop take in turn
+        const uint8_t *src = codes + ((size_t)(r0 / 32 + rb) * nb + (c0 / 32 + cb + 2 * group)) * kBlockBytes + lane * (4 * K);
+        LaneCodes<K> own[2] = {};
+        // plain layout (V = 1 codes): tile (tile row, tile column) = 16K words at ((row/16)*(n/16) + col/16)*16K; this
+        // lane decodes row lane >> 1 of tile row 2rb + (lane & 1), in the step's tile columns 2cb and 2cb + 1
+        const uint16_t *prow = reinterpret_cast<const uint16_t *>(codes) +
+                               ((size_t)(r0 / 16 + 2 * rb + (lane & 1)) * (n >> 4) + (size_t)(c0 / 16 + 2 * cb + 4 * group)) * (16 * K) +
+                               (lane >> 1) * K;
+        PlainRow<K> prows[2][2] = {};
+        auto load_codes = [&](int buf) {
+            if constexpr (kHyb) {
+                own[buf] = load_lane_codes<K>(src);
+                src += kGroups * 2 * kBlockBytes;
+            } else {
+#pragma unroll
+                for (int ks = 0; ks < 2; ks++) prows[buf][ks] = load_plain_row<K>(prow + ks * (16 * K));
+                prow += kGroups * (kStageCols / 16) * (16 * K);
+            }
         };
         if (group < nsteps) {
-            if constexpr (kHyb) own_next = load_lane_codes<K>(src + (size_t)group * 2 * kBlockBytes);
-            else load_plain(group);
-            if (has0) xv0_next = load_x(group, tid8);
-            if (has1) xv1_next = load_x(group, tid8 + 256);
+            load_codes(0);
+            copy_x(group);
         }
-        if constexpr (kHyb)
-            if (group + kGroups < nsteps) own_next2 = load_lane_codes<K>(src + (size_t)(group + kGroups) * 2 * kBlockBytes);
-        // HYB: byte offsets of this lane's four 16-byte chunks (ks, c) inside a 128-byte row of the A tile, swizzled by
-        // the row (row % 8 == a for every row this lane writes); rows (ms, d) are 1024-byte groups apart
-        uint32_t chunk_off[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) chunk_off[j] = (((uint32_t)(4 * cb + j)) ^ (uint32_t)a) << 4;
-        // ring position of this warp's step, kept incrementally (stages is a run-time value: no division in the loop)
-        int s = group % stages, round = group / stages;
-        for (int step = group; step < nsteps; step += kGroups) {
-            const LaneCodes<K> own = own_next;
-            const uint4 xv0 = xv0_next, xv1 = xv1_next;
-            own_next = own_next2;
-            if (step + kGroups < nsteps) {
-                if (has0) xv0_next = load_x(step + kGroups, tid8);
-                if (has1) xv1_next = load_x(step + kGroups, tid8 + 256);
-            }
-            if constexpr (kHyb)
-                if (step + 2 * kGroups < nsteps) own_next2 = load_lane_codes<K>(src + (size_t)(step + 2 * kGroups) * 2 * kBlockBytes);
-            uint32_t pown[4];
-            if constexpr (!kHyb) {
-#pragma unroll
-                for (int tt = 0; tt < 4; tt++) pown[tt] = pown_next[tt];
-                if (step + kGroups < nsteps) load_plain(step + kGroups);
-            }
-            if (round > 0) mbar_wait(smem_addr(&ctl->empty[s]), (round - 1) & 1, abort_flag, status, 1u);
-            LaneCodes<K> nxt = {};
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (group + kGroups < nsteps) load_codes(1);
+        // one step; buf and the stage group + kGroups * buf alternate
+        auto decode_step = [&](int step, int buf, int round) {
+            const int s = group + kGroups * buf, snext = group + kGroups * (buf ^ 1);
+            // the weights are decoded into registers first, so only the stores wait for the stage
+            uint32_t wv[16];
             if constexpr (kHyb) {
+                LaneCodes<K> nxt = {};
 #pragma unroll
-                for (int i = 0; i < K; i++) nxt.w[i] = __shfl_sync(kFullMask, own.w[i], lane + 1);
-            }
-            // B tile: rows = batch (zero beyond bs), 64 columns of x, 16-byte chunks swizzled by row % 8; the copies run
-            // while this warp decodes and are awaited before the stage is handed to the MMA
-            const uint32_t bst = b_base + s * b_stage_bytes;
-            if (has0) {
-                const int brow = tid8 >> 3, c = tid8 & 7;
-                const uint32_t dst = bst + brow * 128 + ((c ^ (brow & 7)) << 4);
-                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(xv0.x), "r"(xv0.y), "r"(xv0.z), "r"(xv0.w) : "memory");
-            }
-            if (has1) {
-                const int brow = (tid8 + 256) >> 3, c = tid8 & 7;
-                const uint32_t dst = bst + brow * 128 + ((c ^ (brow & 7)) << 4);
-                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(xv1.x), "r"(xv1.y), "r"(xv1.z), "r"(xv1.w) : "memory");
-            }
-            if constexpr (!small) {
-                for (int ch = tid8; ch < chunks; ch += 256) {
-                    const int brow = ch >> 3, c = ch & 7;
-                    const uint32_t dst = bst + brow * 128 + ((c ^ (brow & 7)) << 4);
-                    const bool live = brow < bs;
-                    const __half *srcx = live ? x + (size_t)brow * n + c0 + step * kStageCols + c * 8 : x;
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(srcx), "r"(live ? 16 : 0) : "memory");
-                }
-            }
-            if constexpr (kHyb) {
-                const uint32_t ast = a_base + s * kAStageBytes + row_off;
-                uint32_t dst4[4];                       // chunk (ks, c) of this lane's row with ms = 0, d = 0
-#pragma unroll
-                for (int j = 0; j < 4; j++) dst4[j] = ast + chunk_off[j];
+                for (int i = 0; i < K; i++) nxt.w[i] = __shfl_sync(kFullMask, own[buf].w[i], lane + 1);
 #pragma unroll
                 for (int tt = 0; tt < 4; tt++) {
                     const int ks = tt >> 1, ms = tt & 1;
                     uint32_t st[4];
-                    tile_states<K>(own, nxt, tt, st);
+                    tile_states<K>(own[buf], nxt, tt, st);
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const int c = q >> 1, d = q & 1;
-                        const uint32_t w = hyb_lookup(st[q], lut_lane);
-                        // the row offset is a compile-time constant after unrolling: register + immediate addressing
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst4[2 * ks + c] + (uint32_t)(2 * ms + d) * 1024u), "r"(w) : "memory");
-                    }
+                    for (int q = 0; q < 4; q++)       // q = 2c + d: column half, row half of the 16x16 tile
+                        wv[8 * ms + 4 * ks + q] = hyb_lookup(st[q], lut_lane);
                 }
             } else {
 #pragma unroll
-                for (int tt = 0; tt < 4; tt++) {
-                    const int ks = tt >> 1, ms = tt & 1;
-                    const uint64_t bits = plain_lane_bits<K>(pown[tt], lane);
-                    uint32_t wv[4];
+                for (int ks = 0; ks < 2; ks++) {
+                    const uint32_t next = __shfl_sync(kFullMask, prows[buf][ks].a, lane + 2);      // row 15 -> row 0: tail-biting
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {          // eight states, K bits apart, two weights per word
-                        const uint32_t s0 = (uint32_t)(bits >> (32 - 2 * j * K)) & 0xFFFFu;
-                        const uint32_t s1 = (uint32_t)(bits >> (32 - (2 * j + 1) * K)) & 0xFFFFu;
-                        wv[j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1) : pair_1mad(s0, s1, lut_lane);
+                    for (int j = 0; j < 8; j++) {
+                        const uint32_t s0 = plain_state<K>(prows[buf][ks], next, 2 * j), s1 = plain_state<K>(prows[buf][ks], next, 2 * j + 1);
+                        wv[8 * ks + j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1) : pair_1mad(s0, s1, lut_lane);
                     }
-                    // row 32rb + 16ms + pr of the stage, 16-byte chunk 4cb + 2ks + ph of its 128-byte row
-                    const uint32_t row = (uint32_t)(32 * rb + 16 * ms + pr), chunk = (uint32_t)(4 * cb + 2 * ks + ph);
-                    const uint32_t dst = a_base + s * kAStageBytes + (row >> 3) * 1024u + (row & 7u) * 128u + ((chunk ^ (row & 7u)) << 4);
-                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(wv[0]), "r"(wv[1]), "r"(wv[2]), "r"(wv[3]) : "memory");
                 }
             }
-            if constexpr (!small) asm volatile("cp.async.wait_all;" ::: "memory");
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic-proxy stores -> visible to the MMA
+#pragma unroll
+            for (int i = 0; i < 16; i++) asm volatile("" : "+r"(wv[i]));
+            if (step + 2 * kGroups < nsteps) load_codes(buf);
+            if (step + kGroups < nsteps) {
+                // the next step's stage: its last use was kStages - kGroups steps ago (round 0 of the second half: never)
+                if (buf || round > 0) mbar_wait(smem_addr(&ctl->empty[snext]), (buf ? round : round - 1) & 1, abort_flag, status, 1u);
+                copy_x(snext);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            __syncwarp();
+            const uint32_t ast = tmem_warp + (uint32_t)(s * kAStageCols);
+            if constexpr (kHyb) {
+                tmem_st_16x128b_x4(ast, wv);
+                tmem_st_16x128b_x4(ast + (16u << 16), wv + 8);
+            } else tmem_st_32x32b_x16(ast, wv);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");            // this step's slice of x
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // -> visible to the MMA
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_addr(&ctl->full[s]));
-            s += kGroups;
-            if (s >= stages) { s -= stages; round++; }      // kGroups <= stages: at most one wrap
+        };
+        for (int step = group, round = 0; step < nsteps; step += kStages, round++) {
+            decode_step(step, 0, round);
+            if (step + kGroups < nsteps) decode_step(step + kGroups, 1, round);
         }
-    } else if (lane == 0) {
+    } else if (elect_one()) {
         // ------------------------------------ MMA issue ---------------------------------------------------
         // instruction descriptor: D fp32, A/B fp16, both K-major, N = npad, M = 128
         const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
@@ -380,13 +374,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             // covers everything issued so far
             if (!mbar_wait(smem_addr(&ctl->full[s]), round & 1, abort_flag, status, 2u)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t adesc = umma_desc(a_base + s * kAStageBytes);
             const uint64_t bdesc = umma_desc(b_base + s * b_stage_bytes);
 #pragma unroll
             for (int kk = 0; kk < 4; kk++)   // 16 columns = 32 bytes further inside the 128-byte swizzled row
-                umma_f16(tmem_d, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), idesc, (step | kk) != 0);
+                umma_f16(tmem_d, tmem + (uint32_t)(s * kAStageCols + kk * 8), bdesc + (uint64_t)(kk * 2), idesc, (step | kk) != 0);
             umma_commit(smem_addr(&ctl->empty[s]));
-            if (++s == stages) { s = 0; round++; }
+            if (++s == kStages) { s = 0; round++; }
         }
         umma_commit(smem_addr(&ctl->done));
     }
@@ -395,7 +388,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // ------------------------------------- epilogue ----------------------------------------------------
         mbar_wait(smem_addr(&ctl->done), 0u, abort_flag, status, 3u);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int row = r0 + warp * 32 + lane;
+        // tensor-memory lane -> row of the CTA: V = 1 codes keep row r of two tiles in lanes 2r and 2r + 1
+        const int row = warp * 32 + (kHyb ? lane : 16 * (lane & 1) + (lane >> 1));
         float *part = reinterpret_cast<float *>(smem);      // [bs][128]: the ring is no longer needed (every MMA has completed)
         for (int col = 0; col < npad; col += 8) {
             uint32_t r[8];
@@ -410,8 +404,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                 const int bcol = col + j;
                 if (bcol < bs) {
                     const float v = __uint_as_float(r[j]);
-                    if (splitk == 1) out[(size_t)bcol * m + row] = v;
-                    else part[bcol * kRows + warp * 32 + lane] = v;
+                    if (splitk == 1) out[(size_t)bcol * m + r0 + row] = v;
+                    else part[bcol * kRows + row] = v;
                 }
             }
         }
@@ -424,7 +418,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (lane == 0) mbar_wait_bounded(smem_addr(&ctl->done), 0u);
         __syncwarp();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(tmem_cols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     }
     // column splits: the cluster's CTAs add their parts in order, each its share of the outputs
     if (splitk > 1) {
@@ -446,10 +440,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
 }
 
-template <int K, int CODE, int STAGES>
-int launch_gemm_stages(float *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, int npad,
+template <int K, int CODE, bool SMALL>
+int launch_gemm_size(float *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, int npad,
                        int splitk, unsigned *status, cudaStream_t s) {
-    const int smem = 1024 + STAGES * (kAStageBytes + npad * 128) + kLut512Bytes + 256;
+    const int smem = 1024 + kStages * npad * 128 + kLut512Bytes + 256;
     static bool attr_set[64] = {};
     static std::mutex attr_mutex;
     int dev = 0;
@@ -458,7 +452,7 @@ int launch_gemm_stages(float *out, const uint8_t *codes, const __half *x, const 
     {
         std::lock_guard<std::mutex> lock(attr_mutex);
         if (!attr_set[dev]) {
-            QTIP_CUDA_TRY(cudaFuncSetAttribute(decompress_gemm_kernel<K, CODE, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            QTIP_CUDA_TRY(cudaFuncSetAttribute(decompress_gemm_kernel<K, CODE, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                227 * 1024));
             attr_set[dev] = true;
         }
@@ -477,16 +471,15 @@ int launch_gemm_stages(float *out, const uint8_t *codes, const __half *x, const 
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = splitk > 1 ? 2 : 1;
-    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decompress_gemm_kernel<K, CODE, STAGES>, out, codes, x, tlut, m, n, bs, npad, splitk, status));
+    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decompress_gemm_kernel<K, CODE, SMALL>, out, codes, x, tlut, m, n, bs, npad, splitk, status));
     return check_launch();
 }
 
-// four ring stages while the B tiles are small; batches above 64 (16 KiB per B tile) leave room for three
 template <int K, int CODE>
 int launch_gemm(float *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, int npad,
                 int splitk, unsigned *status, cudaStream_t s) {
-    if (npad > 64) return launch_gemm_stages<K, CODE, 3>(out, codes, x, tlut, m, n, bs, npad, splitk, status, s);
-    return launch_gemm_stages<K, CODE, kStages>(out, codes, x, tlut, m, n, bs, npad, splitk, status, s);
+    if (npad > 64) return launch_gemm_size<K, CODE, false>(out, codes, x, tlut, m, n, bs, npad, splitk, status, s);
+    return launch_gemm_size<K, CODE, true>(out, codes, x, tlut, m, n, bs, npad, splitk, status, s);
 }
 
 // CTAs per row range: as many as still fit the chip at once, in a cluster (at most the portable eight), each with a few steps

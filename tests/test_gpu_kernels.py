@@ -445,6 +445,23 @@ def test_decompress_gemm_vs_oracle(K, m, n, bs):
     assert rel_l2(y.cpu().numpy(), want) < 1e-5
 
 
+@pytest.mark.parametrize("K", [2, 3, 4])
+@pytest.mark.parametrize("code", [O.CODE_HYB, O.CODE_3INST, O.CODE_1MAD])
+@pytest.mark.parametrize("m,n,bs", [(128, 192, 1), (128, 256, 49), (384, 320, 64), (128, 832, 65), (256, 1216, 128)])
+def test_decompress_gemm_ring_edges(K, code, m, n, bs):
+    """Step counts around the groups and the depth of the stage ring, batches around the 32-row copies of x."""
+    lay = synth.make_layer(m, n, K, seed=3600 + K, bs=bs, **({} if code == O.CODE_HYB else {"code": "none"}))
+    codes, x = dev(lay["codes"]), dev(lay["x"])
+    if code == O.CODE_HYB:
+        tl = dev(lay["tlut"])
+        y, W = ops.decompress_gemm(codes, x, tl, K, m, n), ops.decode_hyb(codes, tl, K, m, n)
+    else:
+        y, W = ops.decompress_gemm_plain(codes, x, code, K, m, n), ops.decode_plain(codes, code, K, m, n)
+    want = C.matvec_dense(W.cpu().numpy(), lay["x"])
+    assert ops.gemm_status(DEV) == 0
+    assert rel_l2(y.cpu().numpy(), want) < 1e-5
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("ctx", [1, 7, 200, 257, 2048, 2049, 5000])
 @pytest.mark.parametrize("heads", [(8, 8), (16, 2)])
