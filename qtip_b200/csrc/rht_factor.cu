@@ -12,10 +12,12 @@
 //                       these parts, many rows take whole-row CTAs that read their input once and walk over the rows.
 //   rht_cluster_kernel  a thread-block cluster per row, for few long rows.
 //
-// Measured, microseconds per launch (fp16 -> fp16; before: 4 to 8 result rows per CTA, each CTA re-reading the row, fp32
+// Measured, microseconds per launch (fp16 -> fp16, general path; before: 4 to 8 result rows per CTA, each CTA re-reading the row, fp32
 // multiply-adds):  11008 x 1000 rows 1021 -> 62, x 120 124 -> 13, x 8 13.6 -> 5.9, x 1 6.6 -> 5.6;  28672 x 1000 454 -> 99,
 // x 27 18.7 -> 7.3, x 1 9.3 -> 5.4;  53248 x 8 15.6 -> 8.4.  Many rows are bound by the operand reads from shared memory
 // (two wavefronts per mma) and the mma.sync rate together; few rows by the chain load, barrier, product, exchange, store.
+// fp16 rows without statistics and conversions (HALVES): 11008 x 1000 rows 55 -> 45, x 120 10.3 -> 9.3, x 1 6.4 -> 4.6;
+// 28672 x 1000 with signs 98 -> 67; 14336 x 1000 43 -> 30.
 #include <algorithm>
 
 #include "rht.cuh"
@@ -278,8 +280,9 @@ __device__ __forceinline__ void row_finish(const RhtArgs &a, const float *obuf, 
 }
 
 // NTL: n-tiles (8 columns) of a warp task, at most min(2^p, 64) / 8;  TPW: tasks per warp;  HOLD: row-vector pairs a thread
-// keeps in registers between the statistics and the conversion; 0: rows too long for that are read again.
-template <int NTL, int TPW, int HOLD>
+// keeps in registers between the statistics and the conversion; 0: rows too long for that are read again.  HALVES: fp16 rows with at
+// most fp16 signs before the transform.
+template <int NTL, int TPW, int HOLD, bool HALVES>
 __global__ void __launch_bounds__(kRowMaxThreads) rht_row_kernel(const RhtArgs a, const RowShape S, const long rows) {
     extern __shared__ __align__(16) float sm[];
     const int len = 1 << a.p, kfac = a.kfac, n = a.n;
@@ -304,82 +307,128 @@ __global__ void __launch_bounds__(kRowMaxThreads) rht_row_kernel(const RhtArgs a
     for (long row = blockIdx.y; row < rows; row += gridDim.y) {
         const size_t sign_off = (size_t)(row % a.sign_rep) * n, in_off = (size_t)row * a.in_row_stride;
         const bool write_res = a.residual_out && blockIdx.x == 0 && (a.in_row_stride != 0 || row == 0);
-        float rnorm = 0.f, ss = 0.f;
-        float v[HOLD > 0 ? HOLD : 1][2][8];
-        RowStats st;
-        auto sum_squares = [&](size_t e, const float (&x)[8]) {
-            if (write_res) store8_f16(a.residual_out, in_off + e, x);
-#pragma unroll
-            for (int c = 0; c < 8; c++) ss += x[c] * x[c];
-        };
-        if constexpr (HOLD > 0) {
-            // every load of the row is requested before the first value is used
+        auto dst = [&](int q) { return b0p + (q >> j8_log) * stride + 8 * (q & ((1 << j8_log) - 1)); };
+        float inv = 1.f;
+        bool remainder = false, packed = false;
+        if constexpr (HALVES) {
+            // an fp16 row, its signs applied to the sign bits, is the operand as it is: no statistics, no conversions.  Decided by the
+            // row's signs; one that is not +-1 sends the row through the general path.
+            uint4 w[HOLD][2];
+            bool other = false;
 #pragma unroll
             for (int u = 0; u < HOLD; u++)
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int q = threadIdx.x + u * blockDim.x;
-                    if (q < npairs) load_row_vec(a, in_off, at(q, h), v[u][h]);
-                    else
-#pragma unroll
-                        for (int c = 0; c < 8; c++) v[u][h][c] = 0.f;
+                    if (q < npairs) w[u][h] = *reinterpret_cast<const uint4 *>(static_cast<const __half *>(a.in) + in_off + at(q, h));
                 }
-            if (a.norm_weight || write_res) {
+            if (a.sign_in) {
 #pragma unroll
                 for (int u = 0; u < HOLD; u++)
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         const int q = threadIdx.x + u * blockDim.x;
-                        if (q < npairs) sum_squares(at(q, h), v[u][h]);
+                        if (q < npairs) {
+                            const uint4 s = *reinterpret_cast<const uint4 *>(static_cast<const __half *>(a.sign_in) + sign_off + at(q, h));
+                            other |= (((s.x ^ 0x3C003C00u) | (s.y ^ 0x3C003C00u) | (s.z ^ 0x3C003C00u) | (s.w ^ 0x3C003C00u)) & 0x7FFF7FFFu) != 0u;
+                            w[u][h].x ^= s.x & 0x80008000u; w[u][h].y ^= s.y & 0x80008000u;
+                            w[u][h].z ^= s.z & 0x80008000u; w[u][h].w ^= s.w & 0x80008000u;
+                        }
                     }
             }
-            if (a.norm_weight) rnorm = rsqrtf(block_sum(ss, scratch) / (float)n + a.eps);
+            packed = !__syncthreads_or(other);                   // also frees the result buffer of the row before
+            if (packed) {
 #pragma unroll
-            for (int u = 0; u < HOLD; u++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
+                for (int u = 0; u < HOLD; u++) {
                     const int q = threadIdx.x + u * blockDim.x;
-                    if (q < npairs) finish_row_vec(a, in_off, sign_off, at(q, h), rnorm, v[u][h]);
-                    st.add(v[u][h]);
+                    if (q < npairs) {
+                        const uint4 x = w[u][0], y = w[u][1];
+                        reinterpret_cast<uint4 *>(dst(q))[0] = make_uint4(__byte_perm(x.x, y.x, 0x5410), __byte_perm(x.x, y.x, 0x7632),
+                                                                          __byte_perm(x.y, y.y, 0x5410), __byte_perm(x.y, y.y, 0x7632));
+                        reinterpret_cast<uint4 *>(dst(q))[1] = make_uint4(__byte_perm(x.z, y.z, 0x5410), __byte_perm(x.z, y.z, 0x7632),
+                                                                          __byte_perm(x.w, y.w, 0x5410), __byte_perm(x.w, y.w, 0x7632));
+                    }
                 }
-        } else {
-            if (a.norm_weight || write_res) {
+            }
+        }
+        if (!packed) {
+            float rnorm = 0.f, ss = 0.f;
+            float v[HOLD > 0 ? HOLD : 1][2][8];
+            RowStats st;
+            auto sum_squares = [&](size_t e, const float (&x)[8]) {
+                if (write_res) store8_f16(a.residual_out, in_off + e, x);
+#pragma unroll
+                for (int c = 0; c < 8; c++) ss += x[c] * x[c];
+            };
+            if constexpr (HOLD > 0) {
+                // every load of the row is requested before the first value is used
+#pragma unroll
+                for (int u = 0; u < HOLD; u++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int q = threadIdx.x + u * blockDim.x;
+                        if (q < npairs) load_row_vec(a, in_off, at(q, h), v[u][h]);
+                        else
+#pragma unroll
+                            for (int c = 0; c < 8; c++) v[u][h][c] = 0.f;
+                    }
+                if (a.norm_weight || write_res) {
+#pragma unroll
+                    for (int u = 0; u < HOLD; u++)
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const int q = threadIdx.x + u * blockDim.x;
+                            if (q < npairs) sum_squares(at(q, h), v[u][h]);
+                        }
+                }
+                if (a.norm_weight) rnorm = rsqrtf(block_sum(ss, scratch) / (float)n + a.eps);
+#pragma unroll
+                for (int u = 0; u < HOLD; u++)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int q = threadIdx.x + u * blockDim.x;
+                        if (q < npairs) finish_row_vec(a, in_off, sign_off, at(q, h), rnorm, v[u][h]);
+                        st.add(v[u][h]);
+                    }
+            } else {
+                if (a.norm_weight || write_res) {
+                    for (int q = threadIdx.x; q < npairs; q += blockDim.x)
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            load_row_vec(a, in_off, at(q, h), v[0][h]);
+                            sum_squares(at(q, h), v[0][h]);
+                        }
+                }
+                if (a.norm_weight) rnorm = rsqrtf(block_sum(ss, scratch) / (float)n + a.eps);
                 for (int q = threadIdx.x; q < npairs; q += blockDim.x)
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
                         load_row_vec(a, in_off, at(q, h), v[0][h]);
-                        sum_squares(at(q, h), v[0][h]);
+                        finish_row_vec(a, in_off, sign_off, at(q, h), rnorm, v[0][h]);
+                        st.add(v[0][h]);
                     }
             }
-            if (a.norm_weight) rnorm = rsqrtf(block_sum(ss, scratch) / (float)n + a.eps);
-            for (int q = threadIdx.x; q < npairs; q += blockDim.x)
+            st.over_cta(reinterpret_cast<uint32_t *>(scratch));      // its first barrier also frees the result buffer of the row before
+            const int ex = st.scale_exponent();
+            const float up = __uint_as_float((uint32_t)(127 + ex) << 23);
+            inv = __uint_as_float((uint32_t)(127 - ex) << 23);
+            remainder = st.inexact != 0u;
+            if constexpr (HOLD > 0) {
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    load_row_vec(a, in_off, at(q, h), v[0][h]);
-                    finish_row_vec(a, in_off, sign_off, at(q, h), rnorm, v[0][h]);
-                    st.add(v[0][h]);
+                for (int u = 0; u < HOLD; u++) {
+                    const int q = threadIdx.x + u * blockDim.x;
+                    if (q < npairs) put_pairs(dst(q), plane, remainder, up, v[u][0], v[u][1]);
                 }
-        }
-        st.over_cta(reinterpret_cast<uint32_t *>(scratch));      // its first barrier also frees the result buffer of the row before
-        const int ex = st.scale_exponent();
-        const float up = __uint_as_float((uint32_t)(127 + ex) << 23), inv = __uint_as_float((uint32_t)(127 - ex) << 23);
-        const bool remainder = st.inexact != 0u;
-        auto dst = [&](int q) { return b0p + (q >> j8_log) * stride + 8 * (q & ((1 << j8_log) - 1)); };
-        if constexpr (HOLD > 0) {
+            } else {
+                for (int q = threadIdx.x; q < npairs; q += blockDim.x) {
+                    float x[2][8];
 #pragma unroll
-            for (int u = 0; u < HOLD; u++) {
-                const int q = threadIdx.x + u * blockDim.x;
-                if (q < npairs) put_pairs(dst(q), plane, remainder, up, v[u][0], v[u][1]);
-            }
-        } else {
-            for (int q = threadIdx.x; q < npairs; q += blockDim.x) {
-                float x[2][8];
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    load_row_vec(a, in_off, at(q, h), x[h]);
-                    finish_row_vec(a, in_off, sign_off, at(q, h), rnorm, x[h]);
+                    for (int h = 0; h < 2; h++) {
+                        load_row_vec(a, in_off, at(q, h), x[h]);
+                        finish_row_vec(a, in_off, sign_off, at(q, h), rnorm, x[h]);
+                    }
+                    put_pairs(dst(q), plane, remainder, up, x[0], x[1]);
                 }
-                put_pairs(dst(q), plane, remainder, up, x[0], x[1]);
             }
         }
         for (int i = threadIdx.x; i < stride; i += blockDim.x) { b0p[k2n * stride + i] = 0u; b0p[plane + k2n * stride + i] = 0u; }
@@ -594,8 +643,14 @@ int launch_opted_in(void (*kernel)(Params...), bool (&attr_set)[64], dim3 grid, 
 
 template <int NTL, int TPW, int HOLD>
 int launch_rows_variant(const RhtArgs &a, const RowShape &S, long rows, int threads, int grid_y, size_t smem, cudaStream_t s) {
-    static bool attr_set[64] = {};
-    return launch_opted_in(rht_row_kernel<NTL, TPW, HOLD>, attr_set, dim3(S.parts, grid_y), threads, smem, 1, s, a, S, rows);
+    static bool attr_set[64] = {}, attr_set_halves[64] = {};
+    // an own variant: the general path alone is 2 to 5 % faster than beside the packed one
+    const bool halves = a.in_dtype == QTIP_F16 && !a.residual && !a.residual_out && !a.norm_weight && !a.gate &&
+                        (!a.sign_in || a.sign_in_dtype == QTIP_F16);
+    if constexpr (HOLD > 0)
+        if (halves)
+            return launch_opted_in(rht_row_kernel<NTL, TPW, HOLD, true>, attr_set_halves, dim3(S.parts, grid_y), threads, smem, 1, s, a, S, rows);
+    return launch_opted_in(rht_row_kernel<NTL, TPW, HOLD, false>, attr_set, dim3(S.parts, grid_y), threads, smem, 1, s, a, S, rows);
 }
 template <int NTL>
 int launch_rows_ntl(const RhtArgs &a, const RowShape &S, long rows, int threads, int grid_y, int tpw, int hold, size_t smem, cudaStream_t s) {

@@ -328,10 +328,10 @@ def test_rht_vs_oracle(n):
 
 @pytest.mark.parametrize("n", [96, 1376, 2240, 2496, 3328, 5120, 11008, 13824, 14336, 22016, 24576, 28672, 53248])
 @pytest.mark.parametrize("rows", [1, 3, 28, 75, 151])
-@pytest.mark.parametrize("kind", ["fp16", "fp32", "wide"])
+@pytest.mark.parametrize("kind", ["fp16", "fp16-scales", "fp32", "wide"])
 def test_rht_factor_rows(n, rows, kind):
     """Factor widths over every split of the work (rows of the view of 8..2048 columns, parts of a row, clusters, whole rows),
-    both directions: fp16 activations with signs (exact operands), fp32 values, and fp32 rows whose magnitudes differ by
+    both directions: fp16 activations with signs (exact operands), or with a scale among the signs, fp32 values, and fp32 rows whose magnitudes differ by
     many orders (scaled heads and remainders)."""
     g = torch.Generator(device=DEV).manual_seed(n + rows)
     k = ops.had_factor(n)
@@ -340,8 +340,10 @@ def test_rht_factor_rows(n, rows, kind):
     x = torch.randn(rows, n, generator=g, device=DEV)
     if kind == "wide":
         x = x * 10.0 ** torch.linspace(-30, 30, rows, device=DEV)[:, None] * 10.0 ** torch.linspace(-4, 0, n, device=DEV)
-    x = x.half() if kind == "fp16" else x
+    x = x.half() if "fp16" in kind else x
     su = (torch.randn(n, generator=g, device=DEV).sign() + 1e-5).sign().half()
+    if kind == "fp16-scales":
+        su[n // 3] = 1.3
     sv = torch.randn(n, generator=g, device=DEV)
     hh = torch.ones(1, 1, dtype=torch.float64, device=DEV)
     while hh.shape[0] < n // k:
