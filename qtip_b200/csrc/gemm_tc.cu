@@ -21,7 +21,8 @@
 // 10 % of the time, and leaving out three of the four MMAs, the loads or half of the ring's depth changes nothing).  Hence the loop unrolled
 // by two with fixed stages and buffers, and x through asynchronous copies issued a step ahead.  Measured, K = 2, A through shared
 // memory and x through registers -> now:  HYB 8192 x 8192, 27 rows 28.7 -> 20.2 us; 8192 x 28672, 120 rows 123.5 -> 72.1 us;
-// 3INST 8192 x 8192, 27 rows 36.9 -> 33.5 us, 120 rows of 28672 155.7 -> 115.6 us; 1MAD 37.5 -> 30.0 us, 163.7 -> 104.8 us.
+// 3INST 8192 x 8192, 27 rows 36.9 -> 31.3 us, 120 rows of 28672 155.7 -> 108.8 us; 1MAD 37.5 -> 29.4 us, 163.7 -> 102.7 us (of
+// which windows as byte permutes: 3INST 33.5 -> 31.3, 115.9 -> 108.8).
 // This replaces decode-to-HBM + dense GEMM of BitshiftLinearKernelAG upstream
 // (lib/codebook/bitshift.py:476-489), which writes and re-reads 16x the packed bytes at 2 bits.
 //
@@ -162,7 +163,14 @@ __device__ __forceinline__ uint32_t plain_state(const PlainRow<K> &r, uint32_t n
         hi = lo;
         lo = next;
     }
-    return __funnelshift_l(lo, hi, K * i & 31) >> 16;
+    // a window that starts in one of the upper three bytes is two bytes of the stream shifted by less than one: a permute, and the
+    // shift is shared by the states of the same residue (K = 2, 4: 23 and 18 instructions a row instead of 32)
+    const int bit = K * i & 31, byte = bit >> 3, rest = bit & 7;
+    if (K != 3 && byte < 3) {
+        const uint32_t shifted = rest ? __funnelshift_l(lo, hi, rest) : hi;
+        return __byte_perm(shifted, 0, byte == 0 ? 0x4432 : byte == 1 ? 0x4421 : 0x4410);
+    }
+    return __funnelshift_l(lo, hi, bit) >> 16;
 }
 
 constexpr int kMaxSplit = 8;
