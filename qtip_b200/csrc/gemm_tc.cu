@@ -21,7 +21,7 @@
 // 10 % of the time, and leaving out three of the four MMAs, the loads or half of the ring's depth changes nothing).  Hence the loop unrolled
 // by two with fixed stages and buffers, and x through asynchronous copies issued a step ahead.  Measured, K = 2, A through shared
 // memory and x through registers -> now:  HYB 8192 x 8192, 27 rows 28.7 -> 20.2 us; 8192 x 28672, 120 rows 123.5 -> 72.1 us;
-// 3INST 8192 x 8192, 27 rows 36.9 -> 31.3 us, 120 rows of 28672 155.7 -> 108.8 us; 1MAD 37.5 -> 29.4 us, 163.7 -> 102.7 us (of
+// 3INST 8192 x 8192, 27 rows 36.9 -> 29.4 us, 120 rows of 28672 155.7 -> 103.7 us; 1MAD 37.5 -> 29.4 us, 163.7 -> 102.7 us (of
 // which windows as byte permutes: 3INST 33.5 -> 31.3, 115.9 -> 108.8).
 // This replaces decode-to-HBM + dense GEMM of BitshiftLinearKernelAG upstream
 // (lib/codebook/bitshift.py:476-489), which writes and re-reads 16x the packed bytes at 2 bits.
@@ -185,13 +185,14 @@ __device__ __forceinline__ float cluster_load(uint32_t addr, int rank) {
     return v;
 }
 
-// Two weights of the compute codes, packed.  3INST: the two fp16 terms of both states are gathered into two registers and added as
-// pairs.  1MAD: byte sums of the LCG values by dot product, weights from the lane's copy of the table.
+// Two weights of the compute codes, packed.  3INST: each state's two fp16 terms are added by a half2 instruction that takes them
+// from one register (the multiply pipe has room; gathering both states' terms for one addition costs a permute more, 31.3 against
+// 29.4 us at 8192 x 8192, 27 rows).  1MAD: byte sums of the LCG values by dot product, weights from the lane's copy of the table.
 __device__ __forceinline__ uint32_t pair_3inst(uint32_t s0, uint32_t s1) {
     const uint32_t r0 = ((s0 * 89226354u + 64248484u) & 0x8FFF8FFFu) ^ 0x3B603B60u, r1 = ((s1 * 89226354u + 64248484u) & 0x8FFF8FFFu) ^ 0x3B603B60u;
-    const uint32_t lo = __byte_perm(r0, r1, 0x5410), hi = __byte_perm(r0, r1, 0x7632);
-    const __half2 w = __hadd2(*reinterpret_cast<const __half2 *>(&lo), *reinterpret_cast<const __half2 *>(&hi));
-    return *reinterpret_cast<const uint32_t *>(&w);
+    const __half2 h0 = *reinterpret_cast<const __half2 *>(&r0), h1 = *reinterpret_cast<const __half2 *>(&r1);
+    const __half2 w0 = __hadd2(__low2half2(h0), __high2half2(h0)), w1 = __hadd2(__low2half2(h1), __high2half2(h1));
+    return __byte_perm(*reinterpret_cast<const uint32_t *>(&w0), *reinterpret_cast<const uint32_t *>(&w1), 0x5410);
 }
 __device__ __forceinline__ uint32_t pair_1mad(uint32_t s0, uint32_t s1, uint32_t lut_lane) {
     uint32_t w0, w1;
