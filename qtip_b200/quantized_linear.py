@@ -63,11 +63,10 @@ class QuantizedLinear(nn.Module):
             elif self.mode != 'eval':
                 raise NotImplementedError(f"mode {self.mode!r} is not built")
             self.built_codebook_class = True
-        b = self._buffers      # straight from the dict: nn.Module's attribute lookup is most of a microsecond per buffer
-        result = self._modules['codebook_class'](input, b['trellis'], b['SU'], b['SV'], b['had_left'], b['had_right'],
-                                                 self.K_left, self.K_right, self.rcp, self.tp, mode=self.mode)
-        if b.get('bias') is not None:
-            return result + b['bias']
+        result = self.codebook_class(input, self.trellis, self.SU, self.SV, self.had_left, self.had_right,
+                                     self.K_left, self.K_right, self.rcp, self.tp, mode=self.mode)
+        if self.bias is not None:
+            return result + self.bias
         return result
 
     no_ckpt_forward = forward

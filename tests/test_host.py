@@ -88,6 +88,52 @@ def test_quantized_linear_state_dict_keys():
     assert q3.tlut is None and not q3.has_kernel
 
 
+def _stub_layer(monkeypatch, bias=False):
+    """A layer whose native call is replaced by one that records its arguments and returns zeros."""
+    import types
+    from qtip_b200 import bitshift
+    seen = {}
+
+    def linear_forward(x, trellis, tlut, SU, SV, *rest):
+        seen.update(trellis=trellis, SU=SU, SV=SV)
+        return torch.zeros(*x.shape[:-1], SV.numel(), dtype=x.dtype), 3
+    monkeypatch.setattr(bitshift._lib, "host", lambda: types.SimpleNamespace(linear_forward=linear_forward))
+    monkeypatch.setattr(bitshift.ops, "launch_count", 0)
+    return QuantizedLinear(64, 32, 16, 16, 16, 2, 2, 9, 'quantlut_sym', bias=bias), seen
+
+
+@pytest.mark.parametrize("how", ["buffer", "parameter", "plain", "parameter_on_biasless", "plain_on_biasless", "none"])
+def test_forward_adds_bias_however_it_is_held(monkeypatch, how):
+    q, _ = _stub_layer(monkeypatch, bias=how in ("buffer", "parameter", "plain"))
+    want = torch.arange(32).float()
+    if how == "buffer":
+        q.bias.copy_(want)
+    elif how != "none":
+        if not how.endswith("biasless"):
+            del q.bias
+        q.bias = torch.nn.Parameter(want.clone(), requires_grad=False) if how.startswith("parameter") else want.clone()
+    y = q(torch.ones(3, 64, dtype=torch.float16))
+    assert torch.equal(y.float(), (torch.zeros(32) if how == "none" else want).expand(3, 32))
+
+
+@pytest.mark.parametrize("name", ["SU", "SV", "trellis"])
+def test_forward_reads_its_tensors_as_attributes(monkeypatch, name):
+    """Replaced by a parameter, or computed by a parametrization: what the attribute gives is what the kernels get."""
+    q, seen = _stub_layer(monkeypatch)
+    value = getattr(q, name).clone() + 1
+    delattr(q, name)
+    setattr(q, name, torch.nn.Parameter(value, requires_grad=False))
+    q(torch.ones(1, 64, dtype=torch.float16))
+    assert torch.equal(seen[name], value)
+
+    class PlusTwo(torch.nn.Module):
+        def forward(self, t):
+            return t + 2
+    torch.nn.utils.parametrize.register_parametrization(q, name, PlusTwo())
+    q(torch.ones(1, 64, dtype=torch.float16))
+    assert torch.equal(seen[name], value + 2)
+
+
 def test_unpack_quip_scale_folding():
     """lib/utils/data_utils.py:281-307 upstream: where the weight scale goes for rcp 0 / 1 / 2."""
     from qtip_b200.checkpoint import unpack_quip
