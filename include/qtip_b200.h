@@ -95,6 +95,11 @@ int qtip_pack_trellis(void *words, const int *states, long tiles, int K, int V, 
 size_t qtip_viterbi_workspace_bytes(int code, int K, int T, long N);
 int qtip_viterbi_quantize(int *states, float *final_cost, const void *X, long N, int T, int code, int K, const float *tlut,
                           void *workspace, size_t workspace_bytes, void *stream);
+/* The same with the limit of the kernel's waits for its own copies (polls per wait; qtip_viterbi_quantize: 2^20, far above
+ * anything a copy takes; 0: none succeeds).  After a wait that ran out - in either function - the sequences the CTA had left carry
+ * negative states, no two neighbours of which overlap (qtip_pack_trellis counts them), and a cost that is not a number. */
+int qtip_viterbi_quantize_polls(int *states, float *final_cost, const void *X, long N, int T, int code, int K, const float *tlut,
+                                void *workspace, size_t workspace_bytes, unsigned row_polls, void *stream);
 
 /* The byte shuffle from the plain layout to the kernel layout for L = 16, V = 2, 16x16 tiles
  * (lib/algo/finetune.py:196-201) and its inverse (lib/utils/kernel_decompress.py:19-24).  Both buffers hold

@@ -36,7 +36,9 @@
 // Measured on 4096 sequences of 256 values, milliseconds, before (index kept per candidate, byte back-pointers, 1024 threads
 // per sequence) -> now:  HYB K=2 50.8 -> 7.0, 3INST K=2 98 -> 42, 1MAD K=2 97 -> 49.  HYB spends 1500 shared-memory
 // wavefronts per step and sequence in 1700 cycles; the compute codes keep the fp32 / integer multiply pipe 80 % busy.
-// Waits: CTA barriers, the bulk-store groups of thread 0, and the bounded waits of the back-trace.
+// Waits: CTA barriers, the bulk-store groups of thread 0, and the bounded waits of the back-trace (see there).
+#include <climits>
+
 #include "common.cuh"
 
 namespace qtip {
@@ -44,7 +46,8 @@ namespace {
 
 constexpr int kMaxT = 1024;
 constexpr uint32_t kMaxSlots = 8;             // rows in flight during the back-trace
-constexpr uint32_t kRowSpinLimit = 1u << 20;
+constexpr uint32_t kRowPolls = 1u << 20;      // polls of a wait for a row, and of each wait for what is in flight after one ran out
+constexpr uint32_t kGivenUp = 0xFFFFFFFFu;    // no state and no overlap
 
 // Threads per sequence, resident sequences per SM and steps between stored rows, per code and KV.
 template <int CODE, int KV>
@@ -169,13 +172,6 @@ __device__ __forceinline__ float best_at(const float *row, uint32_t q) {     // 
     if constexpr (C::kHalves == 2) b = fminf(b, row[C::G + pos<CODE, KV>(q)]);
     return b;
 }
-template <int CODE, int KV>
-__device__ __forceinline__ float best_row(const float *row, uint32_t q) {    // the same from global memory, past L1
-    using C = VitCfg<CODE, KV>;
-    float b = __ldcg(row + pos<CODE, KV>(q));
-    if constexpr (C::kHalves == 2) b = fminf(b, __ldcg(row + C::G + pos<CODE, KV>(q)));
-    return b;
-}
 
 // Everything a pass needs that does not change within a launch.
 struct PassCtx {
@@ -186,6 +182,7 @@ struct PassCtx {
     float *rows;           // this CTA's slab: rows of best_i, i = 0, stride, 2 stride ...
     int T;
     float minus_zero;      // -0.0f as a run-time value (see v1_errors)
+    uint32_t row_polls;
 };
 
 __device__ __forceinline__ void bulk_store(void *dst, uint32_t src, uint32_t bytes) {
@@ -509,7 +506,10 @@ __device__ __forceinline__ uint32_t trace_tree_of_depth(int depth, const PassCtx
 // Back-trace by one warp: from state st at step i_from to the state at step i_stop (returned); states of the steps in
 // between (i_stop included) go to out[step] if out is given.  The stored rows are streamed back through the shared memory
 // that the forward pass no longer needs (kSlots rows in flight): a chain of dependent reads from global memory took
-// 2.4 us per tree, 0.23 ms of a sequence's 0.6.
+// 2.4 us per tree, 0.23 ms of a sequence's 0.6.  (cp.async groups, which need no polling, take the shared-memory pipe that the
+// forward passes of the other CTAs are bound by: 4096 HYB sequences 7.07 -> 7.19 ms with one warp copying, 7.30 with all.)
+// The waits are bounded: when one runs out nothing of the row is used, the rows still in flight are waited for, and kGivenUp is
+// returned.
 template <int CODE, int KV>
 __device__ __forceinline__ uint32_t backtrace(Smem *sh, const PassCtx &P, uint32_t st, int i_from, int i_stop, int xoff, int *out) {
     using C = VitCfg<CODE, KV>;
@@ -532,15 +532,21 @@ __device__ __forceinline__ uint32_t backtrace(Smem *sh, const PassCtx &P, uint32
     int i = i_from;
     for (int r = r_first; r >= r_last; r--) {
         const uint32_t s = (uint32_t)(r_first - r) % C::kSlots, parity = ((uint32_t)(r_first - r) / C::kSlots) & 1u;
-        bool ready = false;            // bounded wait; a row that has not come is read where it lies
-        for (uint32_t spin = 0; spin < kRowSpinLimit && !ready; spin++) ready = mbar_try_wait(bars + 8 * s, parity);
-        ready = __all_sync(kFullMask, ready);
-        const float *slot = P.buf0 + s * C::kRowFloats, *global = P.rows + (size_t)r * C::kRowFloats;
-        auto row = [&](uint32_t q) { return ready ? best_at<CODE, KV>(slot, q) : best_row<CODE, KV>(global, q); };
+        bool ready = false;
+        for (uint32_t spin = 0; spin < P.row_polls && !ready; spin++) ready = mbar_try_wait(bars + 8 * s, parity);
+        if (!__all_sync(kFullMask, ready)) {
+            for (int q = r; q >= r_last && q > r - (int)C::kSlots; q--) {
+                const uint32_t at = (uint32_t)(r_first - q) % C::kSlots, phase = ((uint32_t)(r_first - q) / C::kSlots) & 1u;
+                for (uint32_t spin = 0; spin < kRowPolls && !mbar_try_wait(bars + 8 * at, phase); spin++) {}
+            }
+            return kGivenUp;
+        }
+        const float *slot = P.buf0 + s * C::kRowFloats;
+        auto row = [&](uint32_t q) { return best_at<CODE, KV>(slot, q); };
         const int depth = i - r * C::kStride;
         const uint32_t c = trace_tree_of_depth<CODE, KV, C::kStride>(depth, P, st, i, xoff, row);
         __syncwarp();                  // every lane has read the slot
-        if (lane == 0 && ready && r - (int)C::kSlots >= r_last) fetch(r - (int)C::kSlots);
+        if (lane == 0 && r - (int)C::kSlots >= r_last) fetch(r - (int)C::kSlots);
         const int steps = min(depth, i - i_stop);
         for (int t = 1; t <= steps; t++)
             if (out && lane == 0) out[i - t] = (int)path_state<KV>(st, c, depth, t);
@@ -564,7 +570,7 @@ inline int vit_smem_bytes(int T) {
 template <int CODE, int KV>
 __global__ void __launch_bounds__(VitCfg<CODE, KV>::kThreads, VitCfg<CODE, KV>::kPerSm)
     viterbi_kernel(int *__restrict__ states, float *__restrict__ final_cost, const __half *__restrict__ X, long N, int T,
-                   const float2 *__restrict__ tlut, float *__restrict__ workspace, float minus_zero) {
+                   const float2 *__restrict__ tlut, float *__restrict__ workspace, float minus_zero, uint32_t row_polls) {
     using C = VitCfg<CODE, KV>;
     constexpr int V = C::kV;
     extern __shared__ __align__(128) uint8_t smem_raw[];
@@ -578,7 +584,7 @@ __global__ void __launch_bounds__(VitCfg<CODE, KV>::kThreads, VitCfg<CODE, KV>::
     P.etab = smem_u32(at); at += C::kHyb ? 2 * 8192 : 0;
     float *table = reinterpret_cast<float *>(at); at += vit_table_bytes<CODE, KV>();
     float *x = reinterpret_cast<float *>(at);
-    P.x = x; P.tl = smem_u32(table); P.T = T; P.minus_zero = minus_zero;
+    P.x = x; P.tl = smem_u32(table); P.T = T; P.minus_zero = minus_zero; P.row_polls = row_polls;
     P.rows = workspace + (size_t)blockIdx.x * ((S + C::kStride - 1) / C::kStride) * C::kRowFloats;
 
     float2 lut[4] = {};
@@ -598,7 +604,6 @@ __global__ void __launch_bounds__(VitCfg<CODE, KV>::kThreads, VitCfg<CODE, KV>::
     if constexpr (CODE == QTIP_CODE_1MAD)
         for (int i = tid; i < 1024; i += C::kThreads) table[i] = __fdiv_rn((float)(i - 510), 147.800537109375f);
     for (long b = blockIdx.x; b < N; b += gridDim.x) {
-        __syncthreads();
         for (int t = tid; t < T; t += C::kThreads) x[t] = __half2float(X[b * T + t]);
         __syncthreads();
         // first pass: the sequence rolled by T/(2V)*V (rolled[t] = x[t - roll]), free ends; the state at step T/(2V) of the
@@ -608,17 +613,30 @@ __global__ void __launch_bounds__(VitCfg<CODE, KV>::kThreads, VitCfg<CODE, KV>::
         if (tid < 32) {
             const uint32_t st = backtrace<CODE, KV>(sh, P, sh->arg, S - 1, half, xoff, nullptr);
             __syncwarp();
-            if (tid == 0) sh->arg = st >> KV;
+            if (tid == 0) sh->arg = st == kGivenUp ? kGivenUp : st >> KV;
         }
         __syncthreads();
         const uint32_t overlap = sh->arg;
         __syncthreads();
-        viterbi_forward<CODE, KV>(sh, P, ts, lut, 0, true, overlap, 0, final_cost ? final_cost + b : nullptr);
-        if (tid < 32) {
-            int *out = states + b * S;
-            const uint32_t st = sh->arg;
-            if (tid == 0) out[S - 1] = (int)st;
-            backtrace<CODE, KV>(sh, P, st, S - 1, 0, 0, out);
+        if (overlap != kGivenUp) {
+            viterbi_forward<CODE, KV>(sh, P, ts, lut, 0, true, overlap, 0, final_cost ? final_cost + b : nullptr);
+            if (tid < 32) {
+                int *out = states + b * S;
+                const uint32_t st = sh->arg;
+                if (tid == 0) out[S - 1] = (int)st;
+                const uint32_t first = backtrace<CODE, KV>(sh, P, st, S - 1, 0, 0, out);
+                __syncwarp();
+                if (tid == 0) sh->arg = first;
+            }
+            __syncthreads();
+        }
+        if (sh->arg == kGivenUp) {
+            // this sequence and the CTA's remaining ones: negative states of which no two neighbours overlap, cost not a number
+            for (; b < N; b += gridDim.x) {
+                for (int i = tid; i < S; i += C::kThreads) states[b * S + i] = i & 1 ? INT_MIN : -1;
+                if (tid == 0 && final_cost) final_cost[b] = __uint_as_float(0x7FC00000u);
+            }
+            return;
         }
     }
 }
@@ -640,10 +658,11 @@ size_t vit_workspace(int T, long N) {
 }
 
 template <int CODE, int KV>
-int launch_viterbi(int *states, float *final_cost, const __half *X, long N, int T, const float2 *tlut, float *ws, cudaStream_t s) {
+int launch_viterbi(int *states, float *final_cost, const __half *X, long N, int T, const float2 *tlut, float *ws, unsigned row_polls,
+                   cudaStream_t s) {
     QTIP_CUDA_TRY(cudaFuncSetAttribute(viterbi_kernel<CODE, KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     viterbi_kernel<CODE, KV><<<(unsigned)vit_grid<CODE, KV>(N), VitCfg<CODE, KV>::kThreads, vit_smem_bytes<CODE, KV>(T), s>>>(
-        states, final_cost, X, N, T, tlut, ws, -0.0f);
+        states, final_cost, X, N, T, tlut, ws, -0.0f, row_polls);
     return check_launch();
 }
 
@@ -679,9 +698,10 @@ struct LaunchCall {
     int T;
     const float2 *tlut;
     float *ws;
+    unsigned row_polls;
     cudaStream_t s;
     template <int CODE, int KV>
-    int operator()() const { return launch_viterbi<CODE, KV>(states, final_cost, X, N, T, tlut, ws, s); }
+    int operator()() const { return launch_viterbi<CODE, KV>(states, final_cost, X, N, T, tlut, ws, row_polls, s); }
 };
 
 }  // namespace
@@ -694,8 +714,8 @@ extern "C" size_t qtip_viterbi_workspace_bytes(int code, int K, int T, long N) {
     return vit_dispatch(code, K, WorkspaceCall{T, N});
 }
 
-extern "C" int qtip_viterbi_quantize(int *states, float *final_cost, const void *X, long N, int T, int code, int K,
-                                     const float *tlut, void *workspace, size_t workspace_bytes, void *stream) {
+extern "C" int qtip_viterbi_quantize_polls(int *states, float *final_cost, const void *X, long N, int T, int code, int K,
+                                           const float *tlut, void *workspace, size_t workspace_bytes, unsigned row_polls, void *stream) {
     if (!states || !X || N <= 0 || K < 2 || K > 4) return QTIP_ERR_BAD_ARG;
     if (code != QTIP_CODE_HYB && code != QTIP_CODE_3INST && code != QTIP_CODE_1MAD) return QTIP_ERR_BAD_ARG;
     if (code == QTIP_CODE_HYB && !tlut) return QTIP_ERR_BAD_ARG;
@@ -708,5 +728,10 @@ extern "C" int qtip_viterbi_quantize(int *states, float *final_cost, const void 
     if (!workspace || workspace_bytes < qtip_viterbi_workspace_bytes(code, K, T, N)) return QTIP_ERR_WORKSPACE;
     return vit_dispatch(code, K, LaunchCall{states, final_cost, static_cast<const __half *>(X), N, T,
                                             reinterpret_cast<const float2 *>(tlut), static_cast<float *>(workspace),
-                                            static_cast<cudaStream_t>(stream)});
+                                            row_polls, static_cast<cudaStream_t>(stream)});
+}
+
+extern "C" int qtip_viterbi_quantize(int *states, float *final_cost, const void *X, long N, int T, int code, int K,
+                                     const float *tlut, void *workspace, size_t workspace_bytes, void *stream) {
+    return qtip_viterbi_quantize_polls(states, final_cost, X, N, T, code, K, tlut, workspace, workspace_bytes, kRowPolls, stream);
 }

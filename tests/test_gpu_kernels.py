@@ -92,6 +92,34 @@ def test_viterbi_quantize_vs_oracle(mode, K, V, N):
     assert np.array_equal(cost.cpu().numpy().view(np.uint32), want_cost.view(np.uint32))
 
 
+@pytest.mark.parametrize("mode,K,V", VITERBI_CASES)
+@pytest.mark.parametrize("T,N", [(16, 1), (256, 1500)])
+def test_viterbi_wait_that_runs_out(mode, K, V, T, N):
+    """No poll allowed: every wait for a stored row is given up.  The kernel ends, every sequence (also those a CTA had not begun)
+    is marked by negative states that pack_trellis refuses and a cost that is no number, and the next call is right."""
+    from qtip_b200 import _lib
+    code = ops.CODE_IDS[mode]
+    g = torch.Generator(device=DEV).manual_seed(T + K)
+    X = torch.randn(N, T, generator=g, device=DEV).half()
+    tlut = torch.randn(512, 2, generator=g, device=DEV)
+    want, want_cost = ops.viterbi_quantize(X, mode, K, tlut=tlut, return_cost=True)
+    lib = _lib.load()
+    need = lib.qtip_viterbi_workspace_bytes(code, K, T, N)
+    ws = torch.empty(need, dtype=torch.uint8, device=DEV)
+    states, cost = torch.empty_like(want), torch.zeros(N, device=DEV)
+
+    def call(polls):
+        _lib.check(lib.qtip_viterbi_quantize_polls(states.data_ptr(), cost.data_ptr(), X.data_ptr(), N, T, code, K, tlut.data_ptr(),
+                                                   ws.data_ptr(), need, polls, torch.cuda.current_stream().cuda_stream), "viterbi")
+    call(0)
+    assert bool((states < 0).all()) and bool(torch.isnan(cost).all())
+    if T == 256:
+        with pytest.raises(RuntimeError, match="do not overlap"):
+            ops.pack_trellis(states, K, V)
+    call(1 << 20)
+    assert torch.equal(states, want) and torch.equal(cost, want_cost)
+
+
 @pytest.mark.parametrize("mode,K,T,N", [("quantlut_sym", 2, 8, 3), ("quantlut_sym", 4, 16, 1), ("3inst", 2, 8, 2), ("1mad", 3, 64, 1),
                                         ("quantlut_sym", 3, 1024, 2)])
 def test_viterbi_quantize_short_and_long_sequences(mode, K, T, N):
