@@ -95,7 +95,7 @@ class BitshiftLinear(nn.Module):
         if mode == 'eval':
             # x * SU -> Hadamard^T (per chunk when row-parallel) -> / 32 -> fp16; decode + product; Hadamard (per chunk when
             # column-parallel) -> * SV * 32: one native call (csrc/host.cpp), whose cost the host does not notice
-            cb, dev = self.cb, input.device
+            cb, dev = self._modules.get('cb') or self.cb, input.device
             out, launches = _lib.host().linear_forward(input, trellis, cb.tlut, SU, SV, self._hadk_bits(0, had_left, dev), K_left or 1,
                                                        self._hadk_bits(1, had_right, dev), K_right or 1, cb.code, cb.K, self.has_kernel,
                                                        rcp, int(tp_rank), self.workspace)

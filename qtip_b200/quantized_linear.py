@@ -63,8 +63,16 @@ class QuantizedLinear(nn.Module):
             elif self.mode != 'eval':
                 raise NotImplementedError(f"mode {self.mode!r} is not built")
             self.built_codebook_class = True
-        result = self.codebook_class(input, self.trellis, self.SU, self.SV, self.had_left, self.had_right,
-                                     self.K_left, self.K_right, self.rcp, self.tp, mode=self.mode)
+        # Registered names come straight from the module's dicts; with any of them held otherwise (a parameter, a plain
+        # tensor, the property of a parametrization) all are read as attributes.  nn.Module's attribute lookup of these names
+        # is 1.3 of the 16.6 us of a 1024 x 4096 call at one row.
+        try:
+            b, linear = self._buffers, self._modules['codebook_class']
+            tensors = b['trellis'], b['SU'], b['SV'], b['had_left'], b['had_right']
+        except KeyError:
+            linear = self.codebook_class
+            tensors = self.trellis, self.SU, self.SV, self.had_left, self.had_right
+        result = linear(input, *tensors, self.K_left, self.K_right, self.rcp, self.tp, mode=self.mode)
         if self.bias is not None:
             return result + self.bias
         return result
