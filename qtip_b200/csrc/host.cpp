@@ -21,6 +21,7 @@
 #include <cmath>
 #include <algorithm>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <utility>
@@ -53,30 +54,50 @@ int dtype_id(const at::Tensor &t) {
 // Per-device / per-stream scratch that outlives a call.  One matvec workspace per (device, stream): calls on one stream
 // are ordered, so they can share it; torch hands out a bounded set of streams.  It is zeroed once and the kernels leave
 // it zeroed.  Never destroyed at exit (the CUDA context may be gone by then).
+//
+// g_mutex is taken with and without the GIL, so nothing that may call into Python (and wait for the GIL) happens under it:
+// no allocation or release of a tensor (memory history, allocator hooks) and no copy of a tensor handle (its Python object).
+// The maps hold shared pointers; those are what is read and exchanged under the lock.
+using TensorPtr = std::shared_ptr<const at::Tensor>;
 std::mutex g_mutex;
-std::map<std::pair<int, void *>, at::Tensor> &workspaces() {
-    static auto *m = new std::map<std::pair<int, void *>, at::Tensor>();
+std::map<std::pair<int, void *>, TensorPtr> &workspaces() {
+    static auto *m = new std::map<std::pair<int, void *>, TensorPtr>();
     return *m;
 }
-std::map<int, at::Tensor> &status_words() {
-    static auto *m = new std::map<int, at::Tensor>();
+std::map<int, TensorPtr> &status_words() {
+    static auto *m = new std::map<int, TensorPtr>();
     return *m;
+}
+
+// The entry of `key`, made by `make` when it is missing or `ok` refuses it.  Of two threads that make one at the same time
+// the first to store it wins; what the other made, or what was replaced, is released outside the lock.
+template <class Map, class Key, class Ok, class Make>
+TensorPtr find_or_make(Map &map, const Key &key, Ok ok, Make make) {
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        const auto it = map.find(key);
+        if (it != map.end() && ok(*it->second)) return it->second;
+    }
+    TensorPtr made = std::make_shared<const at::Tensor>(make()), got;
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        TensorPtr &slot = map[key];
+        if (!slot || !ok(*slot)) slot.swap(made);
+        got = slot;
+    }
+    return got;
 }
 
 at::Tensor matvec_workspace(int dev, int64_t m, int64_t n, int64_t bs, void *stream) {
     const size_t need = qtip_matvec_workspace_bytes((int)m, (int)n, (int)bs);
-    std::lock_guard<std::mutex> lock(g_mutex);
-    at::Tensor &ws = workspaces()[{dev, stream}];
-    if (!ws.defined() || (size_t)ws.numel() < need)
-        ws = at::zeros({(int64_t)std::max<size_t>(need, 1u << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
-    return ws;
+    return *find_or_make(workspaces(), std::make_pair(dev, stream), [&](const at::Tensor &t) { return (size_t)t.numel() >= need; }, [&] {
+        return at::zeros({(int64_t)std::max<size_t>(need, 1u << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+    });
 }
 
 at::Tensor gemm_status(int dev) {
-    std::lock_guard<std::mutex> lock(g_mutex);
-    at::Tensor &t = status_words()[dev];
-    if (!t.defined()) t = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev));
-    return t;
+    return *find_or_make(status_words(), dev, [](const at::Tensor &) { return true; },
+                         [&] { return at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev)); });
 }
 
 struct Layer {

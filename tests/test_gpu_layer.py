@@ -602,3 +602,56 @@ def test_attn_decode_fused_splits_agree(heads, pos_v):
     want = torch.zeros_like(got)
     ops.attn_decode(want, q, ck, cv, pos, n_heads, n_kv, hd)
     assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) < 2e-3
+
+
+_THREADS = """
+import threading, torch
+from qtip_b200 import ops, synth
+from qtip_b200.quantized_linear import QuantizedLinear
+dev = torch.device("cuda", 0)
+lins = []
+for m in (32, 4096, 8192):           # one row each: the workspace grows twice on every stream
+    lay = synth.make_layer(m, 1024, 2, 7, bs=1, code="hyb", device=dev)
+    with torch.device(dev):
+        lin = QuantizedLinear(1024, m, 16, 16, 16, 2, 2, 9, "quantlut_sym")
+    lin.trellis.copy_(lay["codes"].view(torch.int16))
+    lin.tlut.data.copy_(lay["tlut"])
+    lins.append((lin, lay["x"], lin(lay["x"])))
+torch.cuda.synchronize()
+# every allocation and release now records Python frames, which needs the GIL
+torch.cuda.memory._record_memory_history(context="all", stacks="python")
+bad = []
+
+def layers(stream):
+    with torch.cuda.stream(stream), torch.no_grad():
+        for lin, x, want in lins:
+            y = lin(x)
+            stream.synchronize()
+            if not torch.equal(y, want):
+                bad.append(lin.out_features)
+
+def lookups(stream):
+    with torch.cuda.stream(stream):
+        for m in (32, 16384, 65536):
+            ops.matvec_workspace(m, 1024, 1, dev)
+            ops.gemm_status(dev)
+
+streams = [torch.cuda.Stream() for _ in range(32)]
+threads = [threading.Thread(target=f, args=(s,)) for s in streams for f in (layers, lookups)]
+for t in threads:
+    t.start()
+for t in threads:
+    t.join()
+assert not bad, bad
+print("threads ok")
+"""
+
+
+def test_native_layer_call_from_threads_while_allocations_call_into_python():
+    """The layer call allocates and looks its scratch up without the GIL, the Python lookups hold it: with an allocator that calls
+    into Python neither may wait for the other (a lock held over an allocation deadlocked here).  In a child, under a time limit."""
+    import subprocess
+    import sys
+    from conftest import ROOT
+    r = subprocess.run([sys.executable, "-c", _THREADS], capture_output=True, text=True, cwd=ROOT, timeout=300)
+    assert r.returncode == 0 and "threads ok" in r.stdout, r.stderr[-2000:]
