@@ -54,6 +54,9 @@ int dtype_id(const at::Tensor &t) {
 // Per-device / per-stream scratch that outlives a call.  One matvec workspace per (device, stream): calls on one stream
 // are ordered, so they can share it; torch hands out a bounded set of streams.  It is zeroed once and the kernels leave
 // it zeroed.  Never destroyed at exit (the CUDA context may be gone by then).
+// A CUDA graph keeps the addresses it was captured with: a workspace that has to grow is replaced by one of at least twice its
+// size and kept (all replaced ones of a stream are smaller together than the one in use), and a capture that finds none gets one
+// of its own from the graph's memory, zeroed by the graph (a zeroing recorded into a graph is no zeroing of what others use).
 //
 // g_mutex is taken with and without the GIL, so nothing that may call into Python (and wait for the GIL) happens under it:
 // no allocation or release of a tensor (memory history, allocator hooks) and no copy of a tensor handle (its Python object).
@@ -64,25 +67,38 @@ std::map<std::pair<int, void *>, TensorPtr> &workspaces() {
     static auto *m = new std::map<std::pair<int, void *>, TensorPtr>();
     return *m;
 }
+std::vector<TensorPtr> &replaced() {
+    static auto *v = new std::vector<TensorPtr>();
+    return *v;
+}
 std::map<int, TensorPtr> &status_words() {
     static auto *m = new std::map<int, TensorPtr>();
     return *m;
 }
 
 // The entry of `key`, made by `make` when it is missing or `ok` refuses it.  Of two threads that make one at the same time
-// the first to store it wins; what the other made, or what was replaced, is released outside the lock.
+// the first to store it wins; what the other made is released outside the lock.
 template <class Map, class Key, class Ok, class Make>
 TensorPtr find_or_make(Map &map, const Key &key, Ok ok, Make make) {
+    size_t had = 0;      // bytes of the entry that is too small
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         const auto it = map.find(key);
-        if (it != map.end() && ok(*it->second)) return it->second;
+        if (it != map.end()) {
+            if (ok(*it->second)) return it->second;
+            had = it->second->nbytes();
+        }
     }
-    TensorPtr made = std::make_shared<const at::Tensor>(make()), got;
+    bool keep = true;
+    TensorPtr made = std::make_shared<const at::Tensor>(make(had, keep)), got;
+    if (!keep) return made;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
         TensorPtr &slot = map[key];
-        if (!slot || !ok(*slot)) slot.swap(made);
+        if (!slot || !ok(*slot)) {
+            if (slot) replaced().push_back(std::move(slot));
+            slot = std::move(made);
+        }
         got = slot;
     }
     return got;
@@ -90,14 +106,19 @@ TensorPtr find_or_make(Map &map, const Key &key, Ok ok, Make make) {
 
 at::Tensor matvec_workspace(int dev, int64_t m, int64_t n, int64_t bs, void *stream) {
     const size_t need = qtip_matvec_workspace_bytes((int)m, (int)n, (int)bs);
-    return *find_or_make(workspaces(), std::make_pair(dev, stream), [&](const at::Tensor &t) { return (size_t)t.numel() >= need; }, [&] {
-        return at::zeros({(int64_t)std::max<size_t>(need, 1u << 20)}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+    return *find_or_make(workspaces(), std::make_pair(dev, stream), [&](const at::Tensor &t) { return (size_t)t.numel() >= need; },
+                         [&](size_t had, bool &keep) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &capture) != cudaSuccess) throw Failure{"cudaStreamIsCapturing failed"};
+        keep = capture == cudaStreamCaptureStatusNone;
+        const size_t bytes = keep ? std::max<size_t>({need, 2 * had, (size_t)1 << 20}) : need;
+        return at::zeros({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
     });
 }
 
 at::Tensor gemm_status(int dev) {
     return *find_or_make(status_words(), dev, [](const at::Tensor &) { return true; },
-                         [&] { return at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev)); });
+                         [&](size_t, bool &) { return at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev)); });
 }
 
 struct Layer {

@@ -604,6 +604,64 @@ def test_attn_decode_fused_splits_agree(heads, pos_v):
     assert rel_l2(got.float().cpu().numpy(), want.float().cpu().numpy()) < 2e-3
 
 
+def _hyb_layer(m, n, seed):
+    lay = synth.make_layer(m, n, 2, seed, bs=1, code="hyb", device=torch.device(DEV))
+    with torch.device(DEV):
+        lin = QuantizedLinear(n, m, 16, 16, 16, 2, 2, 9, "quantlut_sym")
+    lin.trellis.copy_(lay["codes"].view(torch.int16))
+    lin.tlut.data.copy_(lay["tlut"])
+    return lin, lay["x"]
+
+
+_HUGE = (1 << 19, 32768, 8)      # the largest workspace there is
+
+
+def _stream_with_small_workspace():
+    for _ in range(64):          # torch hands out a bounded set of streams in turn
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            if ops.matvec_workspace(32, 32, 1, DEV).numel() < ops._lib.load().qtip_matvec_workspace_bytes(*_HUGE):
+                return s
+    raise AssertionError("every stream has the largest workspace")
+
+
+def test_workspace_of_a_captured_layer_outlives_a_larger_one():
+    """A graph keeps the workspace it was captured with; a larger layer on the same stream must not give that memory away."""
+    lin, x = _hyb_layer(256, 8192, 31)           # 256 rows: shared row blocks, tickets and partial sums
+    s, g = _stream_with_small_workspace(), torch.cuda.CUDAGraph()
+    with torch.no_grad():
+        with torch.cuda.stream(s):
+            want = lin(x)
+            s.synchronize()
+            with torch.cuda.graph(g, stream=s):
+                y = lin(x)
+            first = ops.matvec_workspace(256, 8192, 1, DEV)
+            assert 2 * first.numel() <= ops.matvec_workspace(*_HUGE, DEV).numel()
+            address, size = first.data_ptr(), first.numel()
+            del first
+            filler = [torch.full((size,), 255, dtype=torch.uint8, device=DEV) for _ in range(64)]
+            assert all(f.data_ptr() + size <= address or address + size <= f.data_ptr() for f in filler)
+        torch.cuda.synchronize()
+        y.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+    assert torch.equal(y, want) and all(bool((f == 255).all()) for f in filler)
+
+
+def test_workspace_first_needed_inside_a_capture():
+    """The zeroing that a capture records has not happened outside the graph: eager calls get a workspace of their own."""
+    s, g = _stream_with_small_workspace(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(s):
+        lin, x = _hyb_layer(256, 8192, 33)
+        with torch.no_grad():
+            want = lin(x)
+            with torch.cuda.graph(g, stream=s):
+                inside = ops.matvec_workspace(*_HUGE, DEV)
+            outside = ops.matvec_workspace(*_HUGE, DEV)
+            assert inside.data_ptr() != outside.data_ptr() and not bool(outside.any())
+            assert torch.equal(lin(x), want)
+
+
 _THREADS = """
 import threading, torch
 from qtip_b200 import ops, synth
