@@ -852,6 +852,8 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
             bulk_copy(ring_w + C * kBlockBytes, reinterpret_cast<const uint8_t *>(x) + (size_t)first_col * xblk_bytes,
                       (uint32_t)(first_n * xblk_bytes), bar_w);
     }
+    // a scratch over ring slot 1 has been read and written by plain accesses, which the copy below must not overtake
+    if (scratch_offset <= 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     if (ichunk < 2) issue(true);        // second chunk: x may be read now, and the scratch no longer lies over ring slot 1
 
