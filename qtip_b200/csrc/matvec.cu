@@ -671,12 +671,15 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
         i_ptr = codes + ((size_t)(row0 + row * rstep) * nb + i_col) * kBlockBytes;
         if (PIECES) i_total = rows_total * piece_n;
     };
+    // 0: issues the warp's copies.  From 32: a wait ran out, no more waits and no more copies (the results are meaningless); the chunk
+    // waited for (modulo 4) << 6 and how many are on their way << 8.  One register for all of it keeps the loop as short as it is.
+    unsigned role = lane;
     // codes: the packed weights (any time); with x through the ring the x part follows separately for the chunk issued
     // before the activations may be read
     auto issue = [&](bool with_x) {
         if (i_left <= 0) return;
         const int nblk = min(C, i_left);
-        if (lane == 0) {
+        if (role == 0) {
             const uint32_t dst = ring_w + (ichunk & 1u) * slot_stride, bar = bar_w + (ichunk & 1u) * 8;
             mbar_expect(bar, (uint32_t)(nblk * (kBlockBytes + xblk_bytes)));
             bulk_copy(dst, i_ptr, (uint32_t)(nblk * kBlockBytes), bar);
@@ -865,7 +868,6 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
     const uint32_t own_off = lane * (4 * K), nxt_off = ((lane + 1) & 31) * (4 * K);   // lane 31 wraps to lane 0: tail-biting
 
     unsigned cchunk = 0;       // chunks consumed so far: slot cchunk & 1, barrier phase (cchunk >> 1) & 1
-    bool ring_dead = false;    // a wait ran out: stop waiting (the results are meaningless, the kernel terminates)
     for (;;) {
         if (!PIECES && e - p < NW) {      // some warps have no block: what they do not write counts as zero
             for (int i = threadIdx.x; i < (NW + (e - 1) / nb - rbase) * stride; i += kThreads) red[i] = 0.f;
@@ -880,13 +882,13 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
         while (total > 0) {
             const int nblk = min(C, left);
             uint32_t slot = ring_w + (cchunk & 1u) * slot_stride;
-            if (!ring_dead) {
+            if (role < 32) {
                 const uint32_t bar = bar_w + (cchunk & 1u) * 8, parity = (cchunk >> 1) & 1u;
                 unsigned spins = 0;
                 while (!mbar_try_wait(bar, parity)) {
                     if (++spins > kRingSpinLimit) {
-                        ring_dead = true;
                         if (lane == 0) atomicOr(done_counter + 1, 1u);
+                        role = 32u + ((cchunk & 3u) << 6) + ((ichunk - cchunk) << 8);
                         break;
                     }
                 }
@@ -949,6 +951,10 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
         __syncthreads();       // the slots are read before the next round writes them
     }
 
+    if (role >= 32) {          // nothing may land after the CTA has gone: what was on its way, with a limit again
+        for (unsigned c = (role >> 6) & 3u, end = c + (role >> 8); c != end; c++)
+            for (unsigned spins = 0; spins < kRingSpinLimit && !mbar_try_wait(bar_w + (c & 1u) * 8, (c >> 1) & 1u); spins++) {}
+    }
     if (TP && P.sig.seq) {
         // row-parallel partial result: the values are already on their way to every GPU (stamped); the CTA that
         // finishes last advances the sequence counter that the stamps of the next launch are derived from

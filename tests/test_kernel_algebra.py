@@ -90,3 +90,15 @@ def test_head_remainder_split_keeps_fp32_inputs():
     assert np.all(np.abs(rebuilt - x) <= np.maximum(np.abs(x) * 2.0 ** -21, 2.0 ** -25))
     exact = hi.astype(np.float32)                     # values that are fp16 numbers already
     assert np.all((exact - exact.astype(np.float16).astype(np.float32)).astype(np.float16) == 0)
+
+
+def test_matvec_ring_drain_addresses_the_copies_in_flight():
+    """matvec_hyb_kernel (qtip_b200/csrc/matvec.cu): chunk c of a warp uses ring slot c & 1 in barrier phase (c >> 1) & 1.  A wait that
+    runs out packs the chunk waited for (modulo 4) and the number of chunks on their way into one word; the drain at the kernel's end
+    must wait for exactly their slots and phases."""
+    for cchunk in range(40):
+        for in_flight in (1, 2):
+            role = 32 + ((cchunk & 3) << 6) + (in_flight << 8)
+            first = (role >> 6) & 3
+            got = [(c & 1, (c >> 1) & 1) for c in range(first, first + (role >> 8))]
+            assert role >= 32 and got == [(c & 1, (c >> 1) & 1) for c in range(cchunk, cchunk + in_flight)]
