@@ -90,9 +90,15 @@ int qtip_pack_trellis(void *words, const int *states, long tiles, int K, int V, 
  * upstream's implementation returns (same fp32 arithmetic, same tie-breaking), ready for qtip_pack_trellis.
  * final_cost (optional): the walk's total squared error per sequence.  code: QTIP_CODE_HYB (V = 2; tlut = 512 x 2 FP32,
  * the table the quantizer holds in fp32) or QTIP_CODE_3INST / QTIP_CODE_1MAD (V = 1, tlut ignored).  K in {2,3,4};
- * T a multiple of 2V, 4V <= T <= 1024 and T*K >= 16 (a tail-biting walk needs at least 16 stream bits).  workspace: qtip_viterbi_workspace_bytes() bytes of device memory,
- * 16-byte aligned (rows of path costs, about 1 MiB to 4 MiB per sequence in flight; no initialisation needed). */
+ * T a multiple of 2V, 4V <= T <= 1024 and T*K >= 16 (a tail-biting walk needs at least 16 stream bits).  workspace: at least
+ * qtip_viterbi_workspace_bytes() bytes of device memory, 16-byte aligned, no initialisation needed.  It holds rows of path costs for
+ * every sequence in flight: at T = 256 (T in proportion) HYB 1 / 1 / 0.25 MiB for K = 2 / 3 / 4 and up to 4 sequences per SM, compute
+ * codes 4 / 4 / 2 MiB and up to 1 / 2 / 2 per SM - on 148 SMs up to 592 / 592 / 148 and 592 / 1184 / 592 MiB, and four times that at
+ * T = 1024.  A caller short of memory passes fewer sequences per call.  qtip_viterbi_workspace_bytes_full(): with that many bytes
+ * every sequence that fits on the GPU at once is in flight; it exceeds the least workspace for HYB K = 2 and 2 to 1182 sequences, where
+ * the least one makes two sequences share a place (twice the time up to 296 sequences). */
 size_t qtip_viterbi_workspace_bytes(int code, int K, int T, long N);
+size_t qtip_viterbi_workspace_bytes_full(int code, int K, int T, long N);
 int qtip_viterbi_quantize(int *states, float *final_cost, const void *X, long N, int T, int code, int K, const float *tlut,
                           void *workspace, size_t workspace_bytes, void *stream);
 /* The same with the limit of the kernel's waits for its own copies (polls per wait; qtip_viterbi_quantize: 2^20, far above

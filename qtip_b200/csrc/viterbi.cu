@@ -641,27 +641,34 @@ __global__ void __launch_bounds__(VitCfg<CODE, KV>::kThreads, VitCfg<CODE, KV>::
     }
 }
 
-// CTAs of a launch; each has a workspace of its own.  HYB K=2 stores 16 KiB at every second step, twice the 4096 bytes per step
-// and sequence that the workspace contract states, so there a CTA takes at least two sequences.
+// CTAs of a launch: one per sequence, as far as the GPU holds them at once and the workspace has a slab of rows for each.
 template <int CODE, int KV>
 long vit_grid(long N) {
-    constexpr int kAtLeast = VitCfg<CODE, KV>::kHyb && KV == 4 ? 2 : 1;
-    const long cap = (long)sm_count() * VitCfg<CODE, KV>::kPerSm, want = (N + kAtLeast - 1) / kAtLeast;
-    return want < cap ? want : cap;
+    const long cap = (long)sm_count() * VitCfg<CODE, KV>::kPerSm;
+    return N < cap ? N : cap;
 }
-
 template <int CODE, int KV>
-size_t vit_workspace(int T, long N) {
+size_t vit_slab(int T) {
     using C = VitCfg<CODE, KV>;
     const int S = T / C::kV;
-    return (size_t)vit_grid<CODE, KV>(N) * ((S + C::kStride - 1) / C::kStride) * C::kRowFloats * sizeof(float);
+    return (size_t)((S + C::kStride - 1) / C::kStride) * C::kRowFloats * sizeof(float);
+}
+
+// The least workspace a call takes.  HYB K=2 stores 16 KiB at every second step but asks for 4096 bytes per step and sequence, what
+// it has always asked for, so the least workspace of up to 1182 sequences has a slab for every second one (4 sequences of 256 values:
+// 0.87 ms instead of 0.44).
+template <int CODE, int KV>
+size_t vit_workspace(int T, long N) {
+    constexpr int kShare = VitCfg<CODE, KV>::kHyb && KV == 4 ? 2 : 1;
+    return (size_t)vit_grid<CODE, KV>((N + kShare - 1) / kShare) * vit_slab<CODE, KV>(T);
 }
 
 template <int CODE, int KV>
-int launch_viterbi(int *states, float *final_cost, const __half *X, long N, int T, const float2 *tlut, float *ws, unsigned row_polls,
-                   cudaStream_t s) {
+int launch_viterbi(int *states, float *final_cost, const __half *X, long N, int T, const float2 *tlut, float *ws, size_t ws_bytes,
+                   unsigned row_polls, cudaStream_t s) {
     QTIP_CUDA_TRY(cudaFuncSetAttribute(viterbi_kernel<CODE, KV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    viterbi_kernel<CODE, KV><<<(unsigned)vit_grid<CODE, KV>(N), VitCfg<CODE, KV>::kThreads, vit_smem_bytes<CODE, KV>(T), s>>>(
+    const long slabs = (long)(ws_bytes / vit_slab<CODE, KV>(T)), want = vit_grid<CODE, KV>(N);
+    viterbi_kernel<CODE, KV><<<(unsigned)(want < slabs ? want : slabs), VitCfg<CODE, KV>::kThreads, vit_smem_bytes<CODE, KV>(T), s>>>(
         states, final_cost, X, N, T, tlut, ws, -0.0f, row_polls);
     return check_launch();
 }
@@ -690,6 +697,12 @@ struct WorkspaceCall {
     template <int CODE, int KV>
     size_t operator()() const { return vit_workspace<CODE, KV>(T, N); }
 };
+struct FullWorkspaceCall {
+    int T;
+    long N;
+    template <int CODE, int KV>
+    size_t operator()() const { return (size_t)vit_grid<CODE, KV>(N) * vit_slab<CODE, KV>(T); }
+};
 struct LaunchCall {
     int *states;
     float *final_cost;
@@ -698,10 +711,11 @@ struct LaunchCall {
     int T;
     const float2 *tlut;
     float *ws;
+    size_t ws_bytes;
     unsigned row_polls;
     cudaStream_t s;
     template <int CODE, int KV>
-    int operator()() const { return launch_viterbi<CODE, KV>(states, final_cost, X, N, T, tlut, ws, row_polls, s); }
+    int operator()() const { return launch_viterbi<CODE, KV>(states, final_cost, X, N, T, tlut, ws, ws_bytes, row_polls, s); }
 };
 
 }  // namespace
@@ -709,9 +723,16 @@ struct LaunchCall {
 
 using namespace qtip;
 
+static bool vit_sizes_ok(int code, int K, int T, long N) {
+    return K >= 2 && K <= 4 && T > 0 && N > 0 && code >= QTIP_CODE_HYB && code <= QTIP_CODE_1MAD;
+}
+
 extern "C" size_t qtip_viterbi_workspace_bytes(int code, int K, int T, long N) {
-    if (K < 2 || K > 4 || T <= 0 || N <= 0 || code < QTIP_CODE_HYB || code > QTIP_CODE_1MAD) return 0;
-    return vit_dispatch(code, K, WorkspaceCall{T, N});
+    return vit_sizes_ok(code, K, T, N) ? vit_dispatch(code, K, WorkspaceCall{T, N}) : 0;
+}
+
+extern "C" size_t qtip_viterbi_workspace_bytes_full(int code, int K, int T, long N) {
+    return vit_sizes_ok(code, K, T, N) ? vit_dispatch(code, K, FullWorkspaceCall{T, N}) : 0;
 }
 
 extern "C" int qtip_viterbi_quantize_polls(int *states, float *final_cost, const void *X, long N, int T, int code, int K,
@@ -727,7 +748,7 @@ extern "C" int qtip_viterbi_quantize_polls(int *states, float *final_cost, const
         return QTIP_ERR_ALIGNMENT;
     if (!workspace || workspace_bytes < qtip_viterbi_workspace_bytes(code, K, T, N)) return QTIP_ERR_WORKSPACE;
     return vit_dispatch(code, K, LaunchCall{states, final_cost, static_cast<const __half *>(X), N, T,
-                                            reinterpret_cast<const float2 *>(tlut), static_cast<float *>(workspace),
+                                            reinterpret_cast<const float2 *>(tlut), static_cast<float *>(workspace), workspace_bytes,
                                             row_polls, static_cast<cudaStream_t>(stream)});
 }
 

@@ -173,7 +173,7 @@ def viterbi_quantize(X, mode, K, tlut=None, return_cost=False):
         if tl.numel() != 1024:
             raise RuntimeError("tlut must hold 512 x 2 values")
     lib = _lib.load()
-    need = lib.qtip_viterbi_workspace_bytes(code, K, T, N)
+    need = lib.qtip_viterbi_workspace_bytes_full(code, K, T, N)      # a place for every sequence
     ws = torch.empty(max(need, 1), dtype=torch.uint8, device=X.device)
     states = torch.empty(N, T // V, dtype=torch.int32, device=X.device)
     cost = torch.empty(N, dtype=torch.float32, device=X.device)

@@ -108,7 +108,14 @@ def test_argument_validation_without_device():
     assert need == 4 * 128 * 4096
     assert lib.qtip_viterbi_workspace_bytes(_lib.CODE_3INST, 2, 256, 1000) == 148 * 256 * 16384 or \
         lib.qtip_viterbi_workspace_bytes(_lib.CODE_3INST, 2, 256, 1000) % (256 * 16384) == 0
-    assert lib.qtip_viterbi_workspace_bytes(7, 2, 256, 4) == 0
+    assert lib.qtip_viterbi_workspace_bytes(7, 2, 256, 4) == 0 and lib.qtip_viterbi_workspace_bytes_full(7, 2, 256, 4) == 0
+    # a place for every sequence: more than the least only where two sequences share one (HYB K = 2, short batches)
+    for code in (_lib.CODE_HYB, _lib.CODE_3INST, _lib.CODE_1MAD):
+        for K in (2, 3, 4):
+            for N in (1, 4, 64, 592, 1182, 1183, 5000):
+                least, full = lib.qtip_viterbi_workspace_bytes(code, K, 256, N), lib.qtip_viterbi_workspace_bytes_full(code, K, 256, N)
+                shared = code == _lib.CODE_HYB and K == 2 and (N + 1) // 2 < full >> 20
+                assert least < full <= 2 * least if shared else least == full, (code, K, N)
     assert lib.qtip_viterbi_quantize(p, None, p, 4, 256, _lib.CODE_HYB, 2, None, p, need, None) == _lib.ERR_BAD_ARG      # no table
     assert lib.qtip_viterbi_quantize(p, None, p, 4, 256, _lib.CODE_HYB, 5, p, p, need, None) == _lib.ERR_BAD_ARG
     assert lib.qtip_viterbi_quantize(p, None, p, 0, 256, _lib.CODE_3INST, 2, None, p, need, None) == _lib.ERR_BAD_ARG     # no sequences

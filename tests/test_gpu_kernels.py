@@ -92,6 +92,24 @@ def test_viterbi_quantize_vs_oracle(mode, K, V, N):
     assert np.array_equal(cost.cpu().numpy().view(np.uint32), want_cost.view(np.uint32))
 
 
+@pytest.mark.parametrize("N", [2, 5, 301, 1182])
+def test_viterbi_sequences_sharing_a_place(N):
+    """HYB K = 2: the least workspace makes two sequences share a place, anything up to the full one fewer; the same results."""
+    from qtip_b200 import _lib
+    g = torch.Generator(device=DEV).manual_seed(N)
+    X, tlut = torch.randn(N, 64, generator=g, device=DEV).half(), torch.randn(512, 2, generator=g, device=DEV)
+    want, want_cost = ops.viterbi_quantize(X, "quantlut_sym", 2, tlut=tlut, return_cost=True)
+    lib = _lib.load()
+    least, full = (f(_lib.CODE_HYB, 2, 64, N) for f in (lib.qtip_viterbi_workspace_bytes, lib.qtip_viterbi_workspace_bytes_full))
+    assert least < full
+    for size in (least, (least + full) // 2, full, 2 * full):
+        ws = torch.empty(size, dtype=torch.uint8, device=DEV)
+        states, cost = torch.zeros_like(want), torch.zeros_like(want_cost)
+        _lib.check(lib.qtip_viterbi_quantize(states.data_ptr(), cost.data_ptr(), X.data_ptr(), N, 64, _lib.CODE_HYB, 2, tlut.data_ptr(),
+                                             ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream), "viterbi")
+        assert torch.equal(states, want) and torch.equal(cost, want_cost)
+
+
 @pytest.mark.parametrize("mode,K,V", VITERBI_CASES)
 @pytest.mark.parametrize("T,N", [(16, 1), (256, 1500)])
 def test_viterbi_wait_that_runs_out(mode, K, V, T, N):
