@@ -156,6 +156,21 @@ def decode_plain(codes, code, K, m, n, tlut=None, out=None):
     return out
 
 
+def _viterbi_workspace(lib, code, K, T, N, device):
+    """(workspace, sequences per launch): a place for every sequence the GPU holds at once (0.25 to 4 MiB each at T = 256, up to 4.7
+    GB in all at T = 1024), or for half as many, a quarter ... while the memory for that is not there."""
+    per = N
+    while True:
+        need = lib.qtip_viterbi_workspace_bytes_full(code, K, T, per)
+        try:
+            return torch.empty(max(need, 1), dtype=torch.uint8, device=device), per
+        except torch.OutOfMemoryError:
+            while per > 1 and lib.qtip_viterbi_workspace_bytes_full(code, K, T, per) >= need:
+                per = (per + 1) // 2
+            if lib.qtip_viterbi_workspace_bytes_full(code, K, T, per) >= need:
+                raise
+
+
 def viterbi_quantize(X, mode, K, tlut=None, return_cost=False):
     """bitshift_codebook.quantize upstream (lib/codebook/bitshift.py:283-292): X (N, T) -> trellis states (N, T/V) int32 of
     the tail-biting minimum-squared-error walk (X is rounded to fp16 first, as upstream does).  mode: 'quantlut_sym'
@@ -173,16 +188,16 @@ def viterbi_quantize(X, mode, K, tlut=None, return_cost=False):
         if tl.numel() != 1024:
             raise RuntimeError("tlut must hold 512 x 2 values")
     lib = _lib.load()
-    need = lib.qtip_viterbi_workspace_bytes_full(code, K, T, N)      # a place for every sequence
-    ws = torch.empty(max(need, 1), dtype=torch.uint8, device=X.device)
+    ws, per = _viterbi_workspace(lib, code, K, T, N, X.device)
     states = torch.empty(N, T // V, dtype=torch.int32, device=X.device)
     cost = torch.empty(N, dtype=torch.float32, device=X.device)
-    with torch.cuda.device(X.device):
-        st = lib.qtip_viterbi_quantize(states.data_ptr(), cost.data_ptr(), X.data_ptr(), N, T, code, K,
-                                       None if tl is None else tl.data_ptr(), ws.data_ptr(), ws.numel(), _stream())
-    _lib.check(st, "qtip_viterbi_quantize")
     global launch_count
-    launch_count += 1
+    with torch.cuda.device(X.device):
+        for i in range(0, max(N, 1), max(per, 1)):
+            st = lib.qtip_viterbi_quantize(states[i:].data_ptr(), cost[i:].data_ptr(), X[i:].data_ptr(), min(per, N - i), T, code, K,
+                                           None if tl is None else tl.data_ptr(), ws.data_ptr(), ws.numel(), _stream())
+            _lib.check(st, "qtip_viterbi_quantize")
+            launch_count += 1
     return (states, cost) if return_cost else states
 
 

@@ -110,6 +110,30 @@ def test_viterbi_sequences_sharing_a_place(N):
         assert torch.equal(states, want) and torch.equal(cost, want_cost)
 
 
+@pytest.mark.parametrize("mode,K,T,N,limit", [("3inst", 3, 64, 11, 3 << 20), ("quantlut_sym", 2, 36, 700, 1 << 20), ("1mad", 4, 22, 5, 1 << 18)])
+def test_viterbi_quantize_with_little_memory(monkeypatch, mode, K, T, N, limit):
+    """Where the workspace for all sequences cannot be had the call takes fewer at a time; where not even one fits it raises."""
+    g = torch.Generator(device=DEV).manual_seed(N)
+    X, tlut = torch.randn(N, T, generator=g, device=DEV).half(), torch.randn(512, 2, generator=g, device=DEV)
+    want, want_cost = ops.viterbi_quantize(X, mode, K, tlut=tlut, return_cost=True)
+    real, sizes = torch.empty, []
+
+    def empty(*size, **kw):
+        if kw.get("dtype") == torch.uint8:
+            sizes.append(size[0])
+            if size[0] > limit:
+                raise torch.OutOfMemoryError("not in this test")
+        return real(*size, **kw)
+    monkeypatch.setattr(ops.torch, "empty", empty)
+    before = ops.launch_count
+    got, cost = ops.viterbi_quantize(X, mode, K, tlut=tlut, return_cost=True)
+    assert len(sizes) > 1 and sizes == sorted(set(sizes), reverse=True) and ops.launch_count - before > 1
+    assert torch.equal(got, want) and torch.equal(cost, want_cost)
+    limit = 1 << 10
+    with pytest.raises(torch.OutOfMemoryError):
+        ops.viterbi_quantize(X, mode, K, tlut=tlut)
+
+
 @pytest.mark.parametrize("mode,K,V", VITERBI_CASES)
 @pytest.mark.parametrize("T,N", [(16, 1), (256, 1500)])
 def test_viterbi_wait_that_runs_out(mode, K, V, T, N):
