@@ -282,7 +282,11 @@ __global__ void __launch_bounds__(kAttnThreads)
 // t % 32 in its range of residues.  Scores are exchanged through distributed shared memory, so that every CTA forms the same
 // maximum, probabilities and denominator; CTA 0 adds the 32 residues' sums of V rows in order.  Every sum has the order it has
 // with one CTA per head, so the result does not depend on the split.  The first batch of K rows is requested before the front part.
-// Measured, 32 heads, 500 positions: 11.5 us (one CTA per head, K after the front part) -> 8.8.
+// Up to kAloneUpTo positions, which one CTA requests in one batch, the exchange costs more than it saves: CTA 0 works alone and the
+// others leave (by position, not by the cache's capacity: a server allocates the longest conversation it admits).
+// Measured, 32 heads, cache of 4096 positions, microseconds: 500 positions 11.5 (one CTA per head, K after the front part) -> 8.4,
+// 8.1 with the loads of the front part's three sums requested together; 16 / 128 / 255 positions 7.1 / 7.3 / 7.4 with four CTAs ->
+// 5.4 / 5.8 / 6.2 with one.
 struct AttnFusedArgs {
     const float *y_q, *y_k, *y_v, *sv_q, *sv_k, *sv_v;
     float scale_q, scale_kv;
@@ -294,22 +298,51 @@ struct AttnFusedArgs {
     unsigned *status;
 };
 
-template <int SPLIT>
-__global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const AttnFusedArgs a) {
+constexpr int kAloneUpTo = kAttnGroups * kAttnBatch;
+
+// Shared memory of a split kernel: the same place for its CTAs' parts and for a CTA that works alone.
+template <int RESIDUES>
+struct AttnFusedSmem {
+    __align__(16) float accs[RESIDUES][128 + 4];
+    __align__(16) float cur[3][128];
+    float part[3][4][128];
+    float red_max[kAttnThreads / 32], red_sum[kAttnThreads / 32];
+    float sc[kAttnChunk + 1];
+};
+
+__device__ __noinline__ void attn_decode_alone(const AttnFusedArgs &a, int head, int pos);
+
+// One head.  ALONE: called by CTA 0 of a cluster for head `at_head` and position `at_pos`, instead of by all threads of a grid.
+template <int SPLIT, bool ALONE>
+__device__ __forceinline__ void attn_decode_head(const AttnFusedArgs &a, int at_head, int at_pos) {
     constexpr int hd = 128, G = kAttnGroups, U = kAttnBatch;
     constexpr int R = G / SPLIT, D = 8 / SPLIT;     // residues of this CTA; head dimensions of a thread in the sum of V rows
-    __shared__ float sc[kAttnChunk + 1];
-    __shared__ float red_max[kAttnThreads / 32], red_sum[kAttnThreads / 32];
-    __shared__ __align__(16) float accs[R][hd + 4];
-    __shared__ float part[3][4][hd];          // signed head sums of q, k, v: four partial sums each
-    __shared__ __align__(16) float cur[3][hd];   // this position's q (rotated, pre-scaled), k (rotated), v
-    const int head = blockIdx.x / SPLIT, rank = blockIdx.x % SPLIT, rep = a.n_heads / a.n_kv, kvh = head / rep;
+    // one CTA per head, without clusters: static arrays, otherwise the launch's shared memory (the two paths' arrays together are
+    // more than the 48 KiB of static ones)
+    constexpr bool kDynamic = SPLIT > 1 || ALONE;
+    extern __shared__ __align__(16) uint8_t attn_smem[];
+    auto &S = *reinterpret_cast<AttnFusedSmem<R> *>(attn_smem);
+    __shared__ float sc_[kDynamic ? 1 : kAttnChunk + 1], red_max_[kDynamic ? 1 : kAttnThreads / 32], red_sum_[kDynamic ? 1 : kAttnThreads / 32];
+    __shared__ __align__(16) float accs_[kDynamic ? 1 : R][hd + 4], part_[kDynamic ? 1 : 3][4][hd], cur_[kDynamic ? 1 : 3][hd];
+    float *sc = kDynamic ? S.sc : sc_, *red_max = kDynamic ? S.red_max : red_max_, *red_sum = kDynamic ? S.red_sum : red_sum_;
+    float(*accs)[hd + 4] = kDynamic ? S.accs : accs_;
+    float(*part)[4][hd] = kDynamic ? S.part : part_;     // signed head sums of q, k, v: four partial sums each
+    float(*cur)[hd] = kDynamic ? S.cur : cur_;           // this position's q (rotated, pre-scaled), k (rotated), v
+    const int head = ALONE ? at_head : blockIdx.x / SPLIT, rank = blockIdx.x % SPLIT, rep = a.n_heads / a.n_kv, kvh = head / rep;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, grp = tid >> 4, sub = tid & 15;
-    if constexpr (SPLIT > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");      // awaited before the first remote store
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int pos = *a.pos;
-    if (!position_ok(pos, a.max_pos, a.status)) return;
+    int pos = at_pos;
+    if constexpr (!ALONE) {
+        if constexpr (SPLIT > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");      // awaited before the first remote store
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        pos = *a.pos;
+        if (!position_ok(pos, a.max_pos, a.status)) return;
+        if (SPLIT > 1 && pos < kAloneUpTo) {       // (the same for the whole cluster)
+            if constexpr (SPLIT > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+            if (rank == 0) attn_decode_alone(a, head, pos);
+            return;
+        }
+    }
 
     const int ctx = pos + 1;
     const size_t row = (size_t)a.n_kv * hd;
@@ -353,19 +386,27 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const A
     // ---- signed sums over heads: thread (quarter, d) adds a quarter of the heads (all three loads batches in flight)
     {
         const int d = tid & (hd - 1), quarter = tid >> 7;
-        float s3[3];
+        // eight heads at a time, so that the loads of the three sums are in flight together
+        float s3[3] = {};
+        const int per_q = (a.n_heads + 3) >> 2, per_kv = (a.n_kv + 3) >> 2;
+        for (int c = 0; c < per_q; c += 8) {
+            float v[3][8];
 #pragma unroll
-        for (int w = 0; w < 3; w++) {
-            const float *y = w == 0 ? a.y_q : w == 1 ? a.y_k : a.y_v;
-            const int nh = w == 0 ? a.n_heads : a.n_kv, h = w == 0 ? head : kvh;
-            const int per = (nh + 3) >> 2, h0 = quarter * per, h1 = min(nh, h0 + per);
-            float s = 0.f;
-#pragma unroll 8
-            for (int h2 = h0; h2 < h1; h2++) {
-                const float v = __ldcg(y + (size_t)h2 * hd + d);
-                s += (__popc(h & h2) & 1) ? -v : v;
+            for (int w = 0; w < 3; w++) {
+                const float *y = w == 0 ? a.y_q : w == 1 ? a.y_k : a.y_v;
+                const int nh = w == 0 ? a.n_heads : a.n_kv, per = w == 0 ? per_q : per_kv;
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int h2 = quarter * per + c + j;
+                    v[w][j] = c + j < per && h2 < nh ? __ldcg(y + (size_t)h2 * hd + d) : 0.f;
+                }
             }
-            s3[w] = s;
+#pragma unroll
+            for (int w = 0; w < 3; w++) {
+                const int per = w == 0 ? per_q : per_kv, h = w == 0 ? head : kvh;
+#pragma unroll
+                for (int j = 0; j < 8; j++) s3[w] += (__popc(h & (quarter * per + c + j)) & 1) ? -v[w][j] : v[w][j];
+            }
         }
 #pragma unroll
         for (int w = 0; w < 3; w++) part[w][quarter][d] = s3[w];
@@ -528,6 +569,16 @@ __global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const A
     if constexpr (SPLIT > 1) asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");      // the parts are read
 }
 
+// Not inlined: the split kernels then keep their registers (inlined, 40 bytes of spills: 500 positions 8.4 -> 8.8 us).  The arguments
+// are copied: by reference every field would be read again after a store to the cache (7.2 instead of 6.8 us at 16 positions).
+__device__ __noinline__ void attn_decode_alone(const AttnFusedArgs &a, int head, int pos) {
+    const AttnFusedArgs args = a;
+    attn_decode_head<1, true>(args, head, pos);
+}
+
+template <int SPLIT>
+__global__ void __launch_bounds__(kAttnThreads) attn_decode_fused_kernel(const AttnFusedArgs a) { attn_decode_head<SPLIT, false>(a, 0, 0); }
+
 template <typename... Args>
 int launch_pdl(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -642,13 +693,12 @@ extern "C" int qtip_attn_decode_fused(void *out, const float *y_q, const float *
     a.pos = pos; a.n_heads = n_heads; a.n_kv = n_kv_heads; a.log2_theta = log2f(theta);
     a.softmax_scale = 1.0f / sqrtf((float)head_dim);
     a.max_pos = max_positions; a.status = status;
-    // Four CTAs per head where the chip has room (two for up to 64 heads); their barriers do not pay on short contexts (32 heads,
-    // microseconds with 1 / 2 / 4 CTAs: 128 positions 6.7 / 7.5 / 7.5, 500 10.4 / 9.1 / 8.8, 1000 17.6 / 15.0 / 11.5), for which the
-    // cache's capacity stands.
-    const int split = max_positions <= 256 ? 1 : n_heads * 4 <= sm_count() ? 4 : n_heads * 2 <= sm_count() ? 2 : 1;
+    // Four CTAs per head where the chip has room (two for up to 64 heads), unless no position of the cache needs them.
+    const int split = max_positions <= kAloneUpTo ? 1 : n_heads * 4 <= sm_count() ? 4 : n_heads * 2 <= sm_count() ? 2 : 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n_heads * split);
     cfg.blockDim = dim3(kAttnThreads);
+    cfg.dynamicSmemBytes = split > 1 ? sizeof(AttnFusedSmem<kAttnGroups>) : 0;      // CTA 0 of a cluster may work alone
     cfg.stream = static_cast<cudaStream_t>(stream);
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

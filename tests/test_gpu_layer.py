@@ -576,11 +576,12 @@ def test_sampler_vocabulary_slices(vocab, top_k):
     assert seen <= {best, vocab - 1} and (top_k > 1 or seen == {best}) and int(pos) == 40
 
 
-@pytest.mark.parametrize("heads", [(32, 8), (64, 64), (128, 8)])
-@pytest.mark.parametrize("pos_v", [0, 5, 1023, 2047, 2048, 2600])
+@pytest.mark.parametrize("heads", [(1, 1), (32, 8), (32, 32), (64, 64), (128, 8)])
+@pytest.mark.parametrize("pos_v", [0, 5, 254, 255, 256, 257, 1023, 2047, 2048, 2600])
 def test_attn_decode_fused_splits_agree(heads, pos_v):
-    """Four, two and one CTA per head (64 and 128 heads; a cache of up to 256 positions forces one): the sums keep their order, so a
-    short cache and a long one give the same bits; several chunks of positions against the separate launches."""
+    """Four, two and one CTA per head (64 and 128 heads; up to 256 positions one of the four works alone, a cache of that capacity
+    forces one): the sums keep their order, so a short cache and a long one give the same bits; several chunks of positions against the
+    separate launches."""
     n_heads, n_kv = heads
     hd, maxpos = 128, 2700
     H, KV = n_heads * hd, n_kv * hd
