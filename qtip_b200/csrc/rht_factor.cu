@@ -652,20 +652,26 @@ int launch_rows_variant(const RhtArgs &a, const RowShape &S, long rows, int thre
             return launch_opted_in(rht_row_kernel<NTL, TPW, HOLD, true>, attr_set_halves, dim3(S.parts, grid_y), threads, smem, 1, s, a, S, rows);
     return launch_opted_in(rht_row_kernel<NTL, TPW, HOLD, false>, attr_set, dim3(S.parts, grid_y), threads, smem, 1, s, a, S, rows);
 }
+// The variants that the supported widths reach, at any number of rows and SMs (by enumeration of the rules in launch_rht_rows): with
+// eight n-tiles one or two tasks per warp and rows of up to 27648 values in registers, longer ones read again; with fewer n-tiles
+// short rows and more tasks, or (4 and 2) rows of 17920 to 27648 values and one task.  Anything else: kNoVariant.
+constexpr int kNoVariant = -1;
 template <int NTL>
 int launch_rows_ntl(const RhtArgs &a, const RowShape &S, long rows, int threads, int grid_y, int tpw, int hold, size_t smem, cudaStream_t s) {
     if constexpr (NTL == 8) {
         if (hold == 0) return tpw <= 1 ? launch_rows_variant<8, 1, 0>(a, S, rows, threads, grid_y, smem, s)
                                        : launch_rows_variant<8, 2, 0>(a, S, rows, threads, grid_y, smem, s);
+        if (tpw == 2) return launch_rows_variant<8, 2, 4>(a, S, rows, threads, grid_y, smem, s);
     }
-    if constexpr (NTL <= 2) {
-        if (tpw > 2) return hold <= 2 ? launch_rows_variant<NTL, 4, 2>(a, S, rows, threads, grid_y, smem, s)
-                                      : launch_rows_variant<NTL, 4, 4>(a, S, rows, threads, grid_y, smem, s);
-    }
-    if (tpw == 2) return hold <= 2 ? launch_rows_variant<NTL, 2, 2>(a, S, rows, threads, grid_y, smem, s)
-                                   : launch_rows_variant<NTL, 2, 4>(a, S, rows, threads, grid_y, smem, s);
-    return hold <= 2 ? launch_rows_variant<NTL, 1, 2>(a, S, rows, threads, grid_y, smem, s)
-                     : launch_rows_variant<NTL, 1, 4>(a, S, rows, threads, grid_y, smem, s);
+    if (hold <= 2) {
+        if constexpr (NTL <= 2)
+            if (tpw > 2) return launch_rows_variant<NTL, 4, 2>(a, S, rows, threads, grid_y, smem, s);
+        if constexpr (NTL <= 4)
+            if (tpw == 2) return launch_rows_variant<NTL, 2, 2>(a, S, rows, threads, grid_y, smem, s);
+        if (tpw <= 1) return launch_rows_variant<NTL, 1, 2>(a, S, rows, threads, grid_y, smem, s);
+    } else if constexpr (NTL >= 2)
+        if (tpw <= 1) return launch_rows_variant<NTL, 1, 4>(a, S, rows, threads, grid_y, smem, s);
+    return kNoVariant;
 }
 
 template <int NTL, int TPW, int HOLD>
@@ -674,10 +680,16 @@ int launch_cluster_variant(const RhtArgs &a, const ClusterShape &S, long rows, s
     return launch_opted_in(rht_cluster_kernel<NTL, TPW, HOLD>, attr_set, dim3(1u << S.csize_log, (unsigned)rows), kClusterThreads, smem,
                            1 << S.csize_log, s, a, S);
 }
+// Reached by the supported widths: one task per warp, except in rows of 17920 to 22016 values (two n-tiles) and 35840 to 44032 (four).
 template <int NTL>
 int launch_cluster_ntl(const RhtArgs &a, const ClusterShape &S, long rows, int tpw, int hold, size_t smem, cudaStream_t s) {
-    if (tpw == 1) return hold == 1 ? launch_cluster_variant<NTL, 1, 1>(a, S, rows, smem, s) : launch_cluster_variant<NTL, 1, 2>(a, S, rows, smem, s);
-    return hold == 1 ? launch_cluster_variant<NTL, 2, 1>(a, S, rows, smem, s) : launch_cluster_variant<NTL, 2, 2>(a, S, rows, smem, s);
+    if (tpw == 1 && hold == 1) return launch_cluster_variant<NTL, 1, 1>(a, S, rows, smem, s);
+    if constexpr (NTL == 8)
+        if (tpw == 1) return launch_cluster_variant<8, 1, 2>(a, S, rows, smem, s);
+    if constexpr (NTL == 4) return launch_cluster_variant<4, 2, 2>(a, S, rows, smem, s);
+    if constexpr (NTL == 2)
+        if (hold == 1) return launch_cluster_variant<2, 2, 1>(a, S, rows, smem, s);
+    return kNoVariant;
 }
 
 }  // namespace
@@ -721,7 +733,7 @@ bool launch_rht_rows(const RhtArgs &a, long rows, cudaStream_t s, int &status) {
         case 2: status = launch_rows_ntl<2>(a, S, rows, threads, grid_y, tpw, h, smem, s); break;
         default: status = launch_rows_ntl<1>(a, S, rows, threads, grid_y, tpw, h, smem, s); break;
     }
-    return true;
+    return status != kNoVariant;
 }
 
 // Few long rows: a cluster of eight CTAs per row.  Below 128 columns a CTA would have too little of a row (the parts of
@@ -748,7 +760,7 @@ bool launch_rht_cluster(const RhtArgs &a, long rows, cudaStream_t s, int &status
         case 4: status = launch_cluster_ntl<4>(a, S, rows, tpw, hold, smem, s); break;
         default: status = launch_cluster_ntl<2>(a, S, rows, tpw, hold, smem, s); break;
     }
-    return true;
+    return status != kNoVariant;
 }
 
 }  // namespace qtip
