@@ -168,13 +168,10 @@ static_assert(sizeof(Shared) <= kCtrlBytes, "control block too large");
 // Cross-warp sum of the per-warp 32 x 8 accumulators of one segment, then the final store or the
 // partial-sum / ticket protocol.  Consumer threads only (NW warps).  Only the first `bs` batch
 // columns are kept: red holds [NW][bs][32] floats.
-// trailing_sync = false is allowed only when the caller alternates between two `red` buffers, so
-// that the next segment's stores cannot overtake this segment's readers.
 template <int NW>
 __device__ __forceinline__ void finish_segment(float (&acc)[2][4], float *red, Shared *sh, float *__restrict__ out,
                                                float *__restrict__ partial, unsigned *__restrict__ counters, long M,
-                                               long nb, long B, long G, int kmax, int m, int bs, bool whole_row,
-                                               bool trailing_sync, const OutCopies &copies, unsigned stamp) {
+                                               long nb, long B, long G, int kmax, int m, int bs, bool whole_row) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int stride = 32 * bs;
@@ -200,11 +197,8 @@ __device__ __forceinline__ void finish_segment(float (&acc)[2][4], float *red, S
         contributors = (int)(cta_of_block((M + 1) * nb - 1, B, G) - c_first) + 1;
     }
     if (contributors == 1) {
-        if (tid < stride) {
-            out[(size_t)b * m + 32 * M + r] = v;
-            for (int q = 0; q < copies.n; q++) store_stamped(copies.dst[q] + (size_t)b * m + 32 * M + r, v, stamp);
-        }
-        if (trailing_sync) asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");
+        if (tid < stride) out[(size_t)b * m + 32 * M + r] = v;
+        asm volatile("bar.sync 1, %0;" ::"n"(NW * 32) : "memory");      // the next segment writes `red` again
         return;
     }
     const int k = (int)(blockIdx.x - c_first);
@@ -223,7 +217,6 @@ __device__ __forceinline__ void finish_segment(float (&acc)[2][4], float *red, S
             float s = 0.f;
             for (int c = 0; c < contributors; c++) s += __ldcg(slot + (size_t)c * 256 + tid);
             out[(size_t)b * m + 32 * M + r] = s;
-            for (int q = 0; q < copies.n; q++) store_stamped(copies.dst[q] + (size_t)b * m + 32 * M + r, s, stamp);
         }
         if (tid == 0) counters[M] = 0;  // leave the workspace ready for the next call
     }
@@ -1096,8 +1089,7 @@ __global__ void __launch_bounds__(kPlainWarps * 32, 2)
                 mma_16816(acc[ms], a, b0, b1);
             }
         }
-        finish_segment<kPlainWarps>(acc, red, sh, out, partial, counters, M, nb, B, G, kmax, m, bs, mode == kModeRows, true,
-                                    OutCopies{}, 0u);
+        finish_segment<kPlainWarps>(acc, red, sh, out, partial, counters, M, nb, B, G, kmax, m, bs, mode == kModeRows);
     }
 }
 

@@ -599,7 +599,3 @@ def decompress_gemm_plain(codes, x, code, K, m, n, out=None):
 
 def gemm_plain_supported(m, n, bs):
     return 1 <= bs <= MAX_GEMM_BATCH and m % 128 == 0 and n % 64 == 0
-
-
-def gemm_supported(m, n, bs):
-    return MAX_MATVEC_BATCH < bs <= MAX_GEMM_BATCH and m % 128 == 0 and n % 64 == 0
