@@ -170,6 +170,86 @@ def test_batched_decode_matches_single_sequence_decode():
     model.check_status()
 
 
+def transform64(x, transpose):
+    """Orthonormal Hadamard transform of the rows of x (float64) over k * 2^p columns; transpose: its transpose."""
+    n = x.shape[-1]
+    hk, k = ops.get_hadK(n)
+    v = x.reshape(-1, k, n // k)
+    h = 1
+    while h < n // k:
+        v = v.reshape(x.shape[0], k, -1, 2, h)
+        v = torch.stack([v[:, :, :, 0] + v[:, :, :, 1], v[:, :, :, 0] - v[:, :, :, 1]], dim=3)
+        h *= 2
+    v = v.reshape(-1, k, n // k)
+    if k > 1:
+        hk = hk.double().to(x.device)
+        v = (hk.T if transpose else hk) @ v
+    return v.reshape(x.shape) / math.sqrt(n)
+
+
+def reference_batch_logits(model, tokens):
+    """step_batch in float64 between the fp16 tensors of the model: tokens (T, B), logits after the last step.  Every sum (transforms,
+    products, norms, attention) in 64 bits from dense decoded weights; nothing of the kernels under test but the decoder."""
+    s, B = model.shape, tokens.shape[1]
+
+    def norm(v, w):
+        return (w * (v.double() * torch.rsqrt(v.double().pow(2).mean(-1, keepdim=True) + s.rms_eps)).half()).double()
+
+    def lin(l, v):
+        xs = (transform64(v * l.SU.double(), True) / 32).half()
+        W = ops.decode_hyb(l.codes, l.tlut, l.K, l.m, l.n)
+        y = torch.cat([xs.double() @ W[i:i + 8192].double().T for i in range(0, l.m, 8192)], dim=1)
+        return (transform64(y, False) * l.SV32.double()).half()
+
+    half, rep = s.head_dim // 2, s.n_heads // s.n_kv_heads
+    inv = s.rope_theta ** (-torch.arange(half, device=DEV, dtype=torch.float64) * 2 / s.head_dim)
+
+    def rope(t, pos):
+        t = t.double().view(B, -1, s.head_dim)
+        a, b, cs, sn = t[..., :half], t[..., half:], torch.cos(pos * inv), torch.sin(pos * inv)
+        return torch.cat([a * cs - b * sn, b * cs + a * sn], dim=-1).half().double()
+    first = int(model.b_pos[0])
+    ck = [model.b_cache_k[:, li, :first].double().view(B, first, -1, s.head_dim) for li in range(s.n_layers)]
+    cv = [model.b_cache_v[:, li, :first].double().view(B, first, -1, s.head_dim) for li in range(s.n_layers)]
+    for t, ids in enumerate(tokens):
+        x = model.embed[ids]
+        for li, L in enumerate(model.layers):
+            h = norm(x, L["ln1"])
+            q, k = rope(lin(L["q"], h), first + t), rope(lin(L["k"], h), first + t)
+            ck[li] = torch.cat([ck[li], k[:, None]], dim=1)
+            cv[li] = torch.cat([cv[li], lin(L["v"], h).double().view(B, 1, -1, s.head_dim)], dim=1)
+            K, V = ck[li].repeat_interleave(rep, dim=2), cv[li].repeat_interleave(rep, dim=2)
+            p = torch.softmax(torch.einsum("bhd,bchd->bhc", q, K) / math.sqrt(s.head_dim), dim=-1)
+            att = torch.einsum("bhc,bchd->bhd", p, V).reshape(B, -1).half()
+            x = x + lin(L["o"], att.double())
+            h = norm(x, L["ln2"])
+            g, u = lin(L["gate"], h).double(), lin(L["up"], h)
+            x = x + lin(L["down"], ((g / (1 + torch.exp(-g))).half() * u).double())
+    return norm(x, model.ln_f) @ model.lm_head.double().T
+
+
+@pytest.mark.parametrize("hidden,heads,kv,mlp,B", [(16384, 128, 8, 53248, 8), (8192, 64, 8, 28672, 5), (4096, 32, 8, 14336, 2)])
+def test_batched_decode_at_large_widths_matches_64_bits(hidden, heads, kv, mlp, B):
+    """One layer of the widths that lockstep decoding is measured with (x through the ring, cluster and row transforms, eight rows in
+    the matvec), in the middle of a conversation.  Measured over three seeds each: 0.88e-3 to 1.13e-3 of the norm (what fp16 tensors
+    between the linears and the final fp16 product give); four times the largest is allowed."""
+    shape = LlamaShape(n_layers=1, hidden=hidden, n_heads=heads, n_kv_heads=kv, head_dim=128, mlp=mlp, vocab=2048, K=2)
+    model = QtipLlama(shape, max_positions=64, device=DEV, seed=51)
+    model.enable_batch(B)
+    g = torch.Generator(device=DEV).manual_seed(52)
+    for c in (model.b_cache_k, model.b_cache_v):
+        c[:, :, :20].normal_(generator=g)
+    model.b_pos.fill_(20)
+    tokens = torch.randint(0, shape.vocab, (2, B), generator=g, device=DEV)
+    want = reference_batch_logits(model, tokens)
+    for ids in tokens:
+        model.b_token.copy_(ids)
+        model.step_batch()
+    model.check_status()
+    err = float((model.b_logits.double() - want).norm() / want.norm())
+    assert err < 4.5e-3, err
+
+
 def test_state_dict_round_trip_into_decode_model():
     """A synthetic checkpoint with upstream's keys, shapes and dtypes (lib/linear/quantized_linear.py:41-67) loaded into
     a differently seeded model reproduces the source model's logits bit for bit; wrong shapes and tensor-parallel

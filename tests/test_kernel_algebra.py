@@ -102,3 +102,25 @@ def test_matvec_ring_drain_addresses_the_copies_in_flight():
             first = (role >> 6) & 3
             got = [(c & 1, (c >> 1) & 1) for c in range(first, first + (role >> 8))]
             assert role >= 32 and got == [(c & 1, (c >> 1) & 1) for c in range(cchunk, cchunk + in_flight)]
+
+
+def test_1mad_quotient_by_reciprocal_is_the_quotient():
+    """v1_errors (qtip_b200/csrc/viterbi.cu) divides the byte sums of the 1MAD code by 147.800537109375 with a rounded reciprocal and one
+    exact residual (Markstein 1990): for all 1021 sums the result is the correctly rounded quotient that the code is defined by.  Every
+    operation is evaluated exactly and rounded once."""
+    from fractions import Fraction
+
+    def rn32(x):
+        """Nearest fp32 value of a fraction, ties to the even one."""
+        f = np.float32(float(x))
+        near = sorted({f, np.nextafter(f, np.float32(-np.inf)), np.nextafter(f, np.float32(np.inf))},
+                      key=lambda v: (abs(Fraction(float(v)) - x), int(v.view(np.uint32)) & 1))
+        return Fraction(float(near[0]))
+    c = Fraction(147.800537109375)
+    rc = rn32(1 / c)
+    assert rn32(c) == c
+    for total in range(1021):
+        y = Fraction(total - 510)
+        q = rn32(y * rc)                       # fma(y, rc, -0)
+        q = rn32(rn32(-q * c + y) * rc + q)    # fma(fma(-q, c, y), rc, q)
+        assert q == rn32(y / c), total
