@@ -1103,6 +1103,8 @@ int check_common(const void *out, const void *codes, const void *x, int K, int m
     return QTIP_OK;
 }
 
+constexpr int kMaxRowBlocks = 32;     // row blocks whose sums share the slots at most, without pieces
+
 struct SmemPlan {
     int chunk_blocks, xs_offset, total, max_rows, scratch_offset;
 };
@@ -1158,12 +1160,11 @@ int launch_hyb_variant(const MatvecBatch &batch, int nprob, int m, int n, int bs
 }
 
 // Fit ring, partial-sum slots, x and the scratch of the fused input side into the shared memory left beside the table.
-// cta_rows: row blocks a CTA meets; they share the slots in rounds of max_rows: up to `pieces` with a slot per warp and row
-// block, or (pieces = 0) up to 32 for contiguous runs.  Returns false if not even a one-block ring fits.
+// cta_rows: row blocks a CTA meets; they share the slots in rounds of max_rows <= cap: with pieces a slot per warp and row block,
+// else one per warp and one per row block.  Returns false if not even a one-block ring fits.
 template <int K>
-bool plan_smem(int n, int bs, int cta_rows, int pieces, bool xs, bool fused_in, SmemPlan &plan) {
+bool plan_smem(int n, int bs, int cta_rows, bool pieces, int cap, bool xs, bool fused_in, SmemPlan &plan) {
     constexpr int NW = kConsumerWarps, BB = 128 * K;
-    const int cap = pieces ? pieces : 32;
     plan.max_rows = cta_rows < cap ? cta_rows : cap;
     const int red_bytes = (pieces ? NW * plan.max_rows : NW + plan.max_rows) * 32 * bs * (int)sizeof(float);
     const int x_bytes = xs ? bs * n * 2 : 0, ring_x = xs ? 0 : bs * 64;
@@ -1228,8 +1229,8 @@ int launch_hyb_batch(const MatvecBatch &batch, int nprob, int m, int n, int bs, 
     const bool pieces = (bs == 1 || cta_rows == 1) && p.mode == kModeRows && nb >= kConsumerWarps;
     SmemPlan plan;
     // slots of up to four row blocks at once, fewer where memory is short
-    for (int rows = pieces ? 4 : 1; rows >= 1; rows >>= 1)
-        if (plan_smem<K>(n, bs, cta_rows, pieces ? rows : 0, true, fused_in, plan))
+    for (int rows = pieces ? 4 : kMaxRowBlocks; rows >= 1; rows = pieces ? rows >> 1 : 0)
+        if (plan_smem<K>(n, bs, cta_rows, pieces, rows, true, fused_in, plan))
             return pieces ? launch_hyb_variant<K, kStagedX | kPieces>(batch, nprob, m, n, bs, p, plan, s)
                           : launch_hyb_variant<K, kStagedX>(batch, nprob, m, n, bs, p, plan, s);
     if (fused_in) return QTIP_ERR_BAD_SHAPE;      // the fused input side leaves x in shared memory
@@ -1240,7 +1241,10 @@ int launch_hyb_batch(const MatvecBatch &batch, int nprob, int m, int n, int bs, 
         a.frag[i] = reinterpret_cast<uint32_t *>(batch.p[i].workspace + partials_end(m, n));
         ring.p[i].x = reinterpret_cast<const __half *>(a.frag[i]);
     }
-    if (!plan_smem<K>(n, bs, cta_rows, 0, false, false, plan)) return QTIP_ERR_BAD_SHAPE;
+    // the ring takes all of the memory at K = 4 and 8 rows but for the slots of two row blocks (7 rows: 11; K = 3, 8 rows: 10)
+    int rows = kMaxRowBlocks;
+    while (rows >= 1 && !plan_smem<K>(n, bs, cta_rows, false, rows, false, false, plan)) rows >>= 1;
+    if (rows < 1) return QTIP_ERR_BAD_SHAPE;
     const int st = launch_fragments(a, nprob, n, bs, s);
     if (st != QTIP_OK) return st;
     return launch_hyb_variant<K, 0>(ring, nprob, m, n, bs, p, plan, s);

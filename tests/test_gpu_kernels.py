@@ -612,7 +612,8 @@ def test_embed_and_sampler():
 
 @pytest.mark.parametrize("K", [2, 3, 4])
 @pytest.mark.parametrize("m,n,bs", [(32, 32, 1), (32, 992, 1), (64, 32, 3), (9600, 64, 1), (4736, 1024, 1), (4768, 1056, 1), (9472, 1024, 2),
-                                    (5000 * 32, 32, 1), (64, 65536, 1), (96, 32768, 8), (14208, 4096, 7), (512, 16384, 5)])
+                                    (5000 * 32, 32, 1), (64, 65536, 1), (96, 32768, 8), (14208, 4096, 7), (512, 16384, 5),
+                                    (9504, 4768, 8), (12288, 4096, 8), (28672, 8192, 8)])
 def test_matvec_hyb_partitions(K, m, n, bs):
     """Every way of cutting the work: rows shorter than a warp each, pieces and contiguous runs, several rounds of row blocks,
     shared row blocks, x staged and x through the ring - against the decoded matrix."""
