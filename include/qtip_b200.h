@@ -318,7 +318,7 @@ int qtip_lm_head(float *logits, const void *res, const void *delta, const void *
  * multinomial_sample_one_no_sync): the top_k (<= 16) largest logits, softmax(top / temperature), one draw from a
  * counter-based generator keyed by (seed, *pos).  Writes the token to *token and out_tokens[*pos + 1] (out_tokens
  * holds max_tokens entries) and advances *pos (32-bit, device memory).  The draw is reproducible for a given seed
- * but is not torch's stream. */
+ * but is not torch's stream.  Logits of which none is a number above -inf: token 0, and bit 2 of *status. */
 int qtip_sample_top_k(long long *token, long long *out_tokens, int *pos, const float *logits, int vocab,
                       float temperature, int top_k, unsigned long long seed, int max_tokens, unsigned *status,
                       void *stream);

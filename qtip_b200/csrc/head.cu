@@ -262,6 +262,11 @@ __global__ void __launch_bounds__(kSampleThreads) sample_kernel(const SampleArgs
                     drawn = u < cum;
                 }
             }
+            // logits without a number above -inf name no token: the next step must not index the embedding with what is left
+            if ((unsigned)t >= (unsigned)a.vocab) {
+                t = 0;
+                if (a.status) atomicOr(a.status, 2u);
+            }
             a.token[seq] = t;
             if (p >= 0 && p + 1 < a.max_tokens) a.out_tokens[(size_t)seq * a.max_tokens + p + 1] = t;      // the token log is full: keep sampling, report
             else if (a.status) atomicOr(a.status, 4u);

@@ -576,6 +576,22 @@ def test_sampler_vocabulary_slices(vocab, top_k):
     assert seen <= {best, vocab - 1} and (top_k > 1 or seen == {best}) and int(pos) == 40
 
 
+@pytest.mark.parametrize("vocab", [5, 2048, 128256])
+@pytest.mark.parametrize("value", [float("nan"), float("-inf")])
+def test_sampler_without_a_usable_logit(vocab, value):
+    """A row of NaN or -inf beside an ordinary one: a token of the vocabulary and the status bit, not the sentinel index (which the
+    batched step would index the embedding with)."""
+    logits = torch.randn(2, vocab, device=DEV)
+    logits[0] = value
+    tok = torch.full((2,), -1, dtype=torch.int64, device=DEV)
+    log, pos = torch.zeros(2, 8, dtype=torch.int64, device=DEV), torch.zeros(2, dtype=torch.int32, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.sample_top_k_batch(tok, log, pos, logits, temperature=1e-3, top_k=5, seed=3, status=status)
+    assert 0 <= int(tok[0]) < vocab and int(tok[1]) == int(logits[1].argmax()) and int(status) in (0, 2) and pos.tolist() == [1, 1]
+    if value != value:
+        assert int(tok[0]) == 0 and int(status) == 2
+
+
 @pytest.mark.parametrize("heads", [(1, 1), (32, 8), (32, 32), (64, 64), (128, 8)])
 @pytest.mark.parametrize("pos_v", [0, 5, 254, 255, 256, 257, 1023, 2047, 2048, 2600])
 def test_attn_decode_fused_splits_agree(heads, pos_v):
