@@ -77,9 +77,9 @@ def plain_launches(m, n, K, bs, code, count, device="cuda:0"):
     torch.cuda.synchronize(device)
 
 
-def time_rht(n, rows=1, device="cuda:0", replays=20, launches=32, plain=0, mid=False):
-    """Input-side transform (fp16 in, SwiGLU gate, signs, fp16 out) of `rows` rows of width n; mid=True times
-    qtip_mlp_mid (gate/up output side + SwiGLU + down input side) instead."""
+def time_rht(n, rows=1, device="cuda:0", replays=20, launches=32, plain=0, mid=False, out_side=False):
+    """Input-side transform (fp16 in, SwiGLU gate, signs, fp16 out) of `rows` rows of width n; out_side=True the
+    output side (fp16 in, signs after the transform), mid=True qtip_mlp_mid (gate/up output side + SwiGLU + down input side) instead."""
     import math
     k = ops.had_factor(n)
     bits = None if k == 1 else ops.pack_hadk(ops.get_hadK(n)[0].to(device))
@@ -92,6 +92,8 @@ def time_rht(n, rows=1, device="cuda:0", replays=20, launches=32, plain=0, mid=F
     def launch():
         if mid:
             ops.mlp_mid(out, y_g, y_u, sv, sv, su, n, 1 / math.sqrt(n), 1 / math.sqrt(n))
+        elif out_side:
+            ops.rht_fused(x, rows, n, out, sign_out=sv, hadk_bits=bits, kfac=k, scale=1 / math.sqrt(n))
         else:
             ops.rht_fused(x, rows, n, out, gate=gate, sign_in=su, hadk_bits=bits, kfac=k, transpose=True, scale=1 / math.sqrt(n))
 
@@ -163,7 +165,8 @@ def pipe_rates():
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--mlp-mid", default="", help="comma-separated widths: time qtip_mlp_mid")
-    ap.add_argument("--rht", default="", help="comma-separated widths: time the transform kernel instead of the matvec")
+    ap.add_argument("--rht", default="", help="comma-separated widths: time the transform kernels instead of the matvec, --batch rows")
+    ap.add_argument("--rht-out", action="store_true", help="with --rht: the output side of a linear instead of the input side")
     ap.add_argument("--shapes", default=LLAMA7B)
     ap.add_argument("--bits", default="2,3,4")
     ap.add_argument("--batch", default="1")
@@ -202,9 +205,11 @@ def main():
             return
     if args.rht:
         for n in (int(v) for v in args.rht.split(",")):
-            us = time_rht(n, plain=args.plain_launches)
-            if us is not None:
-                print(f"rht n={n} (factor {ops.had_factor(n)}): {us:7.2f} us per launch (back-to-back launches in one graph)", flush=True)
+            for rows in (int(b) for b in args.batch.split(",")):
+                us = time_rht(n, rows, plain=args.plain_launches, out_side=args.rht_out)
+                if us is not None:
+                    print(f"rht n={n} (factor {ops.had_factor(n)}), {rows} rows: {us:7.2f} us per launch (back-to-back launches in one "
+                          "graph)", flush=True)
         return
     rows = []
     for K in (int(b) for b in args.bits.split(",")):
