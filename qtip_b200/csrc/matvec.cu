@@ -20,6 +20,10 @@
 // fragment order (one 16-byte load per block and lane) when it fits beside the table; longer x is put into that order once per
 // launch in global memory and travels through the ring with the codes.
 //
+// Precision: the error of out against 64 bits grows with the number of additions in one accumulator, so a run is cut into parts of
+// a 32nd of a row: 28672 x 8192 3.5e-7, 53248 x 16384 6.4e-7, 16384 x 53248 1.9e-6 of the norm at any number of rows (uncut runs: 1.8e-6,
+// 6.2e-6, 6.7e-6).  The cut costs 1 to 3 % of the time at 8192 columns, up to 11 % at 4096 columns and 5 to 8 rows, nothing above.
+//
 // The kernel is instruction-issue bound, not HBM bound (about 5 instructions per state are irreducible: shift, multiply-add
 // hash, mask, multiply-add address, shared load).  The decode loop alone, on resident data, takes 28 cycles per block and SM
 // (K = 2), with the ring 31; in the kernel 35.  A launch adds about 4000 cycles before the loop (table, x) and, for shared
@@ -627,6 +631,9 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
     }
     int p = v_begin, e = min(v_end, max_rows * nb), rbase = 0;     // the round's blocks [p, e), its first row block rbase
     const int piece_lo = (int)(((long)warp * nb) >> 5), piece_n = (int)(((long)(warp + 1) * nb) >> 5) - piece_lo;
+    // Blocks added up in one accumulator: a 32nd of a row (whole chunks).  The tensor cores' additions truncate, and over a run of up
+    // to 100 blocks that adds up; the parts are added in the slot, in fp32 with rounding (see the head of this file).
+    const int part_n = PIECES ? piece_n : ((nb + NW - 1) / NW + C - 1) / C * C;
     const int seg_n = PIECES ? piece_n : nb;                       // blocks of a segment (what lies in one row block), but for ends
     // this warp's blocks of a round: first block v (column col of its row block), `left` of the first segment, `total`
     auto run_of = [&](int &v, int &col, int &left, int &total) {
@@ -862,7 +869,7 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
 
     unsigned cchunk = 0;       // chunks consumed so far: slot cchunk & 1, barrier phase (cchunk >> 1) & 1
     for (;;) {
-        if (!PIECES && e - p < NW) {      // some warps have no block: what they do not write counts as zero
+        if (!PIECES) {      // the parts of a sum are added to the slot; what a warp without a block does not write counts as zero
             for (int i = threadIdx.x; i < (NW + (e - 1) / nb - rbase) * stride; i += kThreads) red[i] = 0.f;
             __syncthreads();
         }
@@ -872,8 +879,12 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
         uint32_t xsp = xs_base + (uint32_t)col * xs_step;
         const uint32_t xs_next = PIECES ? xsp : xs_base;           // x at the start of the segments that follow
         float acc[2][4] = {};
-        while (total > 0) {
-            const int nblk = min(C, left);
+        // the part being decoded, and what follows it in its segment and in all
+        int part = PIECES ? left : min(part_n, left);
+        left -= part;
+        total -= part;
+        while (part > 0) {
+            const int nblk = min(C, part);
             uint32_t slot = ring_w + (cchunk & 1u) * slot_stride;
             if (role < 32) {
                 const uint32_t bar = bar_w + (cchunk & 1u) * 8, parity = (cchunk >> 1) & 1u;
@@ -900,24 +911,29 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
                 decode_block<K>(own, nxt, xb, acc, lut_lane);
             }
             xsp = xa;
-            left -= nblk;
-            total -= nblk;
+            part -= nblk;
             __syncwarp();      // every lane has read the slot before it is filled again
             issue(true);
             cchunk++;
-            if (left == 0) {
+            if (part == 0) {
                 // accumulator (ms, i): row = 16*ms + g + 8*(i>>1), batch = 2*t + (i&1); slot word = batch*32 + row
 #pragma unroll
                 for (int ms = 0; ms < 2; ms++)
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
                         const int b = 2 * t + (i & 1);
-                        if (b < bs) slot_out[b * 32 + 16 * ms + g + 8 * (i >> 1)] = acc[ms][i];
+                        float *word = slot_out + b * 32 + 16 * ms + g + 8 * (i >> 1);
+                        if (b < bs) *word = PIECES ? acc[ms][i] : *word + acc[ms][i];
                         acc[ms][i] = 0.f;
                     }
-                slot_out += PIECES ? NW * stride : stride;
-                left = min(seg_n, total);
-                xsp = xs_next;
+                if (PIECES || left == 0) {
+                    slot_out += PIECES ? NW * stride : stride;
+                    left = min(seg_n, total);
+                    xsp = xs_next;
+                }
+                part = PIECES ? left : min(part_n, left);
+                left -= part;
+                total -= part;
             }
         }
         __syncthreads();

@@ -613,7 +613,7 @@ def test_embed_and_sampler():
 @pytest.mark.parametrize("K", [2, 3, 4])
 @pytest.mark.parametrize("m,n,bs", [(32, 32, 1), (32, 992, 1), (64, 32, 3), (9600, 64, 1), (4736, 1024, 1), (4768, 1056, 1), (9472, 1024, 2),
                                     (5000 * 32, 32, 1), (64, 65536, 1), (96, 32768, 8), (14208, 4096, 7), (512, 16384, 5),
-                                    (9504, 4768, 8), (12288, 4096, 8), (28672, 8192, 8)])
+                                    (9504, 4768, 8), (12288, 4096, 8), (28672, 8192, 8), (53248, 8192, 8), (65536, 8192, 7)])
 def test_matvec_hyb_partitions(K, m, n, bs):
     """Every way of cutting the work: rows shorter than a warp each, pieces and contiguous runs, several rounds of row blocks,
     shared row blocks, x staged and x through the ring - against the decoded matrix."""
@@ -623,3 +623,16 @@ def test_matvec_hyb_partitions(K, m, n, bs):
     want = lay["x"].double() @ ops.decode_hyb(codes, lay["tlut"], K, m, n).double().T
     assert float((got.double() - want).norm() / want.norm()) < 2e-6
     assert torch.equal(got, ops.decompress_matvec(codes, lay["x"], lay["tlut"], K, m, n))
+
+
+@pytest.mark.parametrize("K,m,n,bs", [(2, 28672, 8192, 1), (2, 28672, 8192, 5), (3, 53248, 8192, 8), (4, 53248, 4096, 2), (2, 16384, 16384, 8)])
+def test_matvec_hyb_error_of_long_runs(K, m, n, bs):
+    """A warp that decodes a run of many blocks must not add all of them in one tensor-core accumulator, whose additions truncate.
+    Bound: an accumulator takes a 32nd of a row, n / 512 additions of at most 2^-23 of the partial sum and 2^-24 on average, and 32 parts
+    are added with rounding (about 6 units of 2^-24 as a random walk)."""
+    lay = synth.make_layer(m, n, K, seed=m + n + bs, bs=bs, device=DEV)
+    codes = lay["codes"].view(torch.int16)
+    got = ops.decompress_matvec(codes, lay["x"], lay["tlut"], K, m, n).double()
+    W = ops.decode_hyb(codes, lay["tlut"], K, m, n)
+    want = torch.cat([lay["x"].double() @ W[i:i + 8192].double().T for i in range(0, m, 8192)], dim=1)
+    assert float((got - want).norm() / want.norm()) < 2.0**-24 * (n / 512 + 6)
