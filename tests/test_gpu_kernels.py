@@ -636,3 +636,23 @@ def test_matvec_hyb_error_of_long_runs(K, m, n, bs):
     W = ops.decode_hyb(codes, lay["tlut"], K, m, n)
     want = torch.cat([lay["x"].double() @ W[i:i + 8192].double().T for i in range(0, m, 8192)], dim=1)
     assert float((got - want).norm() / want.norm()) < 2.0**-24 * (n / 512 + 6)
+
+
+@pytest.mark.parametrize("n", [1152, 6656, 11008, 17920, 28672, 53248])
+@pytest.mark.parametrize("rows", [1, 300])
+def test_factor_transform_error_of_fp32_rows(n, rows):
+    """fp32 rows are split into two fp16 parts (2^-23 of a value, uniform: 2^-23 / sqrt(3) in the norm); the additions of the factor
+    (truncating, at most 11 of them on the heads) and the stages stay below that again: 1.25 * 2^-23 in all, which the fp32 additions
+    of a plain evaluation take as well."""
+    hk, k = ops.get_hadK(n)
+    x = torch.randn(rows, n, generator=torch.Generator(device=DEV).manual_seed(n), device=DEV)
+    for transpose in (False, True):
+        got = ops.rht(x, hadk_bits=ops.pack_hadk(hk.to(DEV)), kfac=k, transpose=transpose, scale=n**-0.5).double()
+        v, h = x.double().view(rows, k, -1), 1
+        while h < n // k:
+            v = v.reshape(rows, k, -1, 2, h)
+            v = torch.stack([v[:, :, :, 0] + v[:, :, :, 1], v[:, :, :, 0] - v[:, :, :, 1]], dim=3)
+            h *= 2
+        hd = hk.double().to(DEV)
+        want = ((hd.T if transpose else hd) @ v.reshape(rows, k, -1)).view(rows, n) * n**-0.5
+        assert float((got - want).norm() / want.norm()) < 1.25 * 2.0**-23
