@@ -17,8 +17,8 @@
 // The compute codes (3INST / 1MAD, V = 1, plain layout) use the same kernel with another producer: a lane decodes one row of a
 // tile (its own 2K bytes and the start of the next row), lanes 2r and 2r + 1 row r of two tiles, and stores a row per
 // tensor-memory lane; the accumulator's lanes are mapped back to rows when they are read.
-// Bound: instruction issue of the decode warps (~155 instructions per warp and stage HYB, ~270 3INST; the tensor pipe is busy
-// 10 % of the time, and leaving out three of the four MMAs, the loads or half of the ring's depth changes nothing).  Hence the loop unrolled
+// Bound: instruction issue of the decode warps (8192 x 8192, 27 rows: 190 instructions per warp and stage HYB, 295 3INST, issued in
+// 64 and 66 % of the cycles; the tensor pipe is busy 7 to 10 % of the time, and leaving out three of the four MMAs, the loads or half of the ring's depth changes nothing).  Hence the loop unrolled
 // by two with fixed stages and buffers, and x through asynchronous copies issued a step ahead.  Measured, K = 2, A through shared
 // memory and x through registers -> now:  HYB 8192 x 8192, 27 rows 28.7 -> 20.2 us; 8192 x 28672, 120 rows 123.5 -> 72.1 us;
 // 3INST 8192 x 8192, 27 rows 36.9 -> 29.4 us, 120 rows of 28672 155.7 -> 103.7 us; 1MAD 37.5 -> 29.4 us, 163.7 -> 102.7 us (of

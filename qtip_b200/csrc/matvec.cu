@@ -25,10 +25,12 @@
 // 6.2e-6, 6.7e-6).  The cut costs 1 to 3 % of the time at 8192 columns, up to 11 % at 4096 columns and 5 to 8 rows, nothing above.
 //
 // The kernel is instruction-issue bound, not HBM bound (about 5 instructions per state are irreducible: shift, multiply-add
-// hash, mask, multiply-add address, shared load).  The decode loop alone, on resident data, takes 28 cycles per block and SM
-// (K = 2), with the ring 31; in the kernel 35.  A launch adds about 4000 cycles before the loop (table, x) and, for shared
-// row blocks, 4500 after it.  Measured, K = 2, against one CTA barrier and reduction per row block and four blocks unrolled
-// (microseconds): 28672 x 8192 1 row 43.1 -> 38.7, 5 rows 58.1 -> 47.8; 22016 x 4096 18.3 -> 16.2; 4096 x 4096 5.6 -> 5.4.
+// hash, mask, multiply-add address, shared load).  K = 2, 1 row: 137 warp instructions per block with everything that surrounds the
+// loop, 34 issue cycles of the four schedulers, which issue in 61 % (22016 x 4096) to 69 % (28672 x 8192) of the cycles; 8 rows
+// through the ring 210, 82 %.  A launch takes about 4000 cycles before the loop (table, x) and, for shared row blocks, 4500 after it;
+// what is left is 44 cycles per block and SM at both sizes.  (The loop without ring, barriers and sums, on resident data: 28; with
+// the ring 31.)  Measured, K = 2, against one CTA barrier and reduction per row block and four blocks unrolled (microseconds):
+// 28672 x 8192 1 row 43.1 -> 39.4, 5 rows 58.1 -> 48.9; 22016 x 4096 18.3 -> 16.3; 4096 x 4096 5.6 -> 5.4.
 //
 // Reduction.  Slots are summed in warp order at the end of a round.  When a row block is shared by several CTAs each stores
 // its partial sums to the workspace and takes a ticket; the CTA that draws the last ticket adds the partials in CTA order and

@@ -27,8 +27,8 @@
 //     known at compile time and the table repeated once the address is register + immediate.
 // best_i is stored under an XOR permutation of its index (pos()) that makes both the reads (stride 4 or 1 in lanes) and the
 // writes (stride 64) conflict-free.  Four warps per sequence, four sequences per SM.  Bound: shared-memory wavefronts (32768
-// lookups = 1024 wavefronts per step and sequence, plus reads of best) and issue (about 1.6 instructions per candidate),
-// close to each other.
+// lookups = 1024 wavefronts per step and sequence, plus reads of best) and issue (2.0 warp instructions per 32
+// candidates, everything included), close to each other.
 // 3INST / 1MAD forward.  65536 (1021) different values, so each candidate computes its error: LCG by constant increments,
 // two values per packed fp32x2 instruction, minimum of three per instruction; issue bound at about 6.5 instructions per
 // candidate.
@@ -36,6 +36,9 @@
 // Measured on 4096 sequences of 256 values, milliseconds, before (index kept per candidate, byte back-pointers, 1024 threads
 // per sequence) -> now:  HYB K=2 50.8 -> 7.0, 3INST K=2 98 -> 42, 1MAD K=2 97 -> 49.  HYB spends 1500 shared-memory
 // wavefronts per step and sequence in 1700 cycles; the compute codes keep the fp32 / integer multiply pipe 80 % busy.
+// Memory: the stored rows of every sequence in flight, at 256 values 1 / 1 / 0.25 MiB (HYB, K = 2 / 3 / 4) and 4 / 4 / 2 MiB (compute
+// codes); with a full grid on 148 SMs 592 / 592 / 148 and 592 / 1184 / 592 MiB, where byte back-pointers of one sequence per SM took
+// 74 / 18.5 / 4.6 and 592 / 296 / 148.
 // Waits: CTA barriers, the bulk-store groups of thread 0, and the bounded waits of the back-trace (see there).
 #include <climits>
 
