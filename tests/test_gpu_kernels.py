@@ -638,7 +638,7 @@ def test_matvec_hyb_error_of_long_runs(K, m, n, bs):
     assert float((got - want).norm() / want.norm()) < 2.0**-24 * (n / 512 + 6)
 
 
-@pytest.mark.parametrize("n", [1152, 6656, 11008, 17920, 28672, 53248])
+@pytest.mark.parametrize("n", [1152, 6656, 11008, 17920, 28672, 53248, 55296])
 @pytest.mark.parametrize("rows", [1, 300])
 def test_factor_transform_error_of_fp32_rows(n, rows):
     """fp32 rows are split into two fp16 parts (2^-23 of a value, uniform: 2^-23 / sqrt(3) in the norm); the additions of the factor
