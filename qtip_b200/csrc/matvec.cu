@@ -9,9 +9,13 @@
 // The warps of a CTA share its blocks without meeting until the end of a round of several row blocks: each owns either a
 // fixed 32nd of every row block or one contiguous run (see PIECES), and leaves its sums of a row block in a slot of its own.
 //
-// Data path.  A warp pulls its blocks in chunks of up to 1 KiB with one bulk copy (cp.async.bulk, the 1-D form of TMA) per
-// chunk into a two-slot ring of its own in shared memory, completion on an mbarrier of its own; the next chunk is always in
-// flight while one is decoded (up to 64 KiB in flight per SM, no registers held, no load-latency stalls in the loop).  A lane
+// Data path.  A warp pulls its blocks in chunks of up to 1 KiB with asynchronous copies (cp.async, 16 bytes per lane) into a two-slot
+// ring of its own in shared memory, one group of copies per chunk; the next chunk is always in flight while one is decoded (up to
+// 64 KiB in flight per SM, no registers held).  The kernel is bound by instruction issue, so what controls the ring is kept short: the
+// group wait has no polling loop, no lane is elected, and every count is the same in all lanes in a way the compiler can see (warp
+// index and division results through a shuffle), which makes the control scalar and spares the reconvergence code.  A bulk copy per
+// chunk with an mbarrier wait, issued by one lane, took 137 warp instructions per block against 123 at 1 row, 210 against 138 at 8 rows
+// through the ring.  A lane
 // reads its 4K bytes of a block and those of lane+1 (the wrap-around bits of the tail-biting stream) from the ring, so the loop
 // has no shuffles.  A lane decodes its 16 trellis states into four mma.m16n8k16 A fragments in registers - HYB: h = s*(s+1),
 // entry (h>>6)&1023 of a 1024-entry table (the 512-entry LUT and its sign-flipped twin) kept as 32 lane-private copies in
@@ -22,15 +26,15 @@
 //
 // Precision: the error of out against 64 bits grows with the number of additions in one accumulator, so a run is cut into parts of
 // a 32nd of a row: 28672 x 8192 3.5e-7, 53248 x 16384 6.4e-7, 16384 x 53248 1.9e-6 of the norm at any number of rows (uncut runs: 1.8e-6,
-// 6.2e-6, 6.7e-6).  The cut costs 1 to 3 % of the time at 8192 columns, up to 11 % at 4096 columns and 5 to 8 rows, nothing above.
+// 6.2e-6, 6.7e-6).  The parts are added in registers.
 //
 // The kernel is instruction-issue bound, not HBM bound (about 5 instructions per state are irreducible: shift, multiply-add
-// hash, mask, multiply-add address, shared load).  K = 2, 1 row: 137 warp instructions per block with everything that surrounds the
-// loop, 34 issue cycles of the four schedulers, which issue in 61 % (22016 x 4096) to 69 % (28672 x 8192) of the cycles; 8 rows
-// through the ring 210, 82 %.  A launch takes about 4000 cycles before the loop (table, x) and, for shared row blocks, 4500 after it;
-// what is left is 44 cycles per block and SM at both sizes.  (The loop without ring, barriers and sums, on resident data: 28; with
-// the ring 31.)  Measured, K = 2, against one CTA barrier and reduction per row block and four blocks unrolled (microseconds):
-// 28672 x 8192 1 row 43.1 -> 39.4, 5 rows 58.1 -> 48.9; 22016 x 4096 18.3 -> 16.3; 4096 x 4096 5.6 -> 5.4.
+// hash, mask, multiply-add address, shared load).  K = 2, 1 row: 123 warp instructions per block with everything that surrounds the
+// loop, 31 issue cycles of the four schedulers; the loop alone on resident data (100 instructions) runs at 83 % of the issue slots,
+// 30 cycles per block and SM, whichever pipe the address arithmetic is given to (integer or float multiply-add, adds).  A launch
+// takes about 4000 cycles before the loop (table, x) and, for shared row blocks, 4500 after it.  Measured, K = 2 unless stated, the
+// bulk-copy ring -> now (microseconds): 28672 x 8192 1 row 39.6 -> 35.8, K = 4 45.4 -> 39.6; 22016 x 4096 16.4 -> 14.7; 4096 x 4096
+// 5.4 -> 5.0; 8192 x 8192 5 rows 18.3 -> 16.0; 53248 x 16384 8 rows 188.6 -> 130.5, K = 4 204.5 -> 146.8.
 //
 // Reduction.  Slots are summed in warp order at the end of a round.  When a row block is shared by several CTAs each stores
 // its partial sums to the workspace and takes a ticket; the CTA that draws the last ticket adds the partials in CTA order and
@@ -39,9 +43,8 @@
 // Launch overlap.  The kernel is launched with programmatic stream serialization: everything that
 // touches only weights (the first code loads, the table build) runs before griddepcontrol.wait,
 // i.e. while the previous kernel of the stream drains; x, out and the workspace are touched only
-// after it.  Waits: the per-chunk mbarrier wait (bounded; a time-out sets word 1 of the workspace's control
-// area and the kernel runs to its end with meaningless results) and, in the tensor-parallel instantiation
-// (TP), one bounded wait for the other GPUs' result values (see PeerIn below).
+// after it.  Waits: none that polls but, in the tensor-parallel instantiation (TP), one bounded wait for the other GPUs' result
+// values (see PeerIn below).
 //
 // Upstream counterpart: kernel_decompress_matvec, qtip-kernels/src/inference.cu:168-425.
 #include <mutex>
@@ -58,17 +61,14 @@ constexpr int kConsumerWarps = 32;
 // sign flip is needed) x 32 lane-private copies x half2 = 128 KiB.  Entry e, copy l at byte e*128 + l*4:
 // every lane reads its own bank, so a warp's 32 random lookups never conflict.
 constexpr int kLutBytes = 1024 * 32 * 4;
-constexpr int kCtrlBytes = 1024;      // Shared (256 bytes) + two mbarriers per warp
-constexpr int kBarOffset = 256;
-constexpr int kMaxChunkBytes = 1024;  // bytes of packed codes per bulk copy
-constexpr unsigned kRingSpinLimit = 1u << 22;
+constexpr int kCtrlBytes = 256;       // Shared
+constexpr int kMaxChunkBytes = 1024;  // bytes of packed codes per ring slot
 constexpr int kSmemLimit = 227 * 1024;
 constexpr int kMaxBatch = 8;
 
 // ---- workspace layout (all offsets fixed, independent of the problem) -----------------------------
 // [0, 64 KiB)   ticket counters, one uint32 per 32-row block (m <= 524288); zero between calls
 // [64 KiB, +256) word 0: counter of finished CTAs (fused output transform); zero between calls
-//               word 1: sticky flag, set if a wait for a bulk copy ever ran out (never cleared by the kernels)
 // [.., ..)      partial sums: [row block][contributor][8 batch x 32 rows] fp32
 // [.., end)     x of the call in fragment order, when it is too long for shared memory
 constexpr size_t kCounterBytes = 64 * 1024;
@@ -296,29 +296,12 @@ struct MatvecBatch {
 };
 
 // ---- per-warp staging ring ----------------------------------------------------------------------------
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+__device__ __forceinline__ void copy16_async(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bulk copy global -> shared (addresses and size multiples of 16 bytes), completion counted on `bar`; the bytes of all copies
-// of a phase are announced once.
-__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// all groups of this thread but the last one have landed
+__device__ __forceinline__ void copies_wait_but_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 // A lane's 4K bytes of a block in the ring (address = block start + lane * 4K); every access pattern below is
 // conflict-free (8 / 16 bytes per lane contiguous, or words at stride 3).
 template <int K>
@@ -572,7 +555,7 @@ __device__ __forceinline__ void reduce_round(const float *red, Shared *sh, float
 //           through the ring.
 // blockIdx.y selects the problem of the batch (all problems have the same m, n, K, bs).
 // TP: the tensor-parallel fields (PeerIn / Signal) are live; the single-GPU instantiation carries none of that code.
-// C:  blocks per bulk copy; xs_offset: byte offset of the staged x in shared memory (the host fits the ring, the partial-sum
+// C:  blocks per ring slot; xs_offset: byte offset of the staged x in shared memory (the host fits the ring, the partial-sum
 // slots, x and the scratch of the fused input side into 227 KiB and picks C accordingly); max_rows: row blocks whose partial sums
 // fit the slots at once.
 enum { kStagedX = 1, kPieces = 2 };
@@ -588,7 +571,7 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
     constexpr int kBlockBytes = 128 * K;
     constexpr int NW = kConsumerWarps, kThreads = NW * 32;
     extern __shared__ __align__(128) uint8_t smem[];
-    // layout: control block (incl. two mbarriers per warp) | LUT | ring slot 0 [NW][slot] | ring slot 1 [NW][slot] |
+    // layout: control block | LUT | ring slot 0 [NW][slot] | ring slot 1 [NW][slot] |
     //         partial sums [NW + max_rows, or NW * max_rows with pieces][bs][32] fp32 | (padding) | x (bs, n) fp16 permuted
     // The fp32 scratch of the fused input transform lies behind x when everything fits (scratch_offset > 0); otherwise
     // it overlays ring slot 1 and what follows it up to x, and slot 1 is first filled after the transform is done.
@@ -613,7 +596,9 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
 
     const int nb = n >> 5, mb = m >> 5;
     const int G = gridDim.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the warp index through a shuffle: known to be the same in all lanes, so the loop control below is scalar and its branches need
+    // no reconvergence
+    const int warp = __shfl_sync(kFullMask, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
     // Blocks are numbered row block by row block (B = mb*nb < 2^30 is checked by the host).  stream-K: this CTA's blocks are
     // [c*B/G, (c+1)*B/G); rows mode: the row blocks c, c + G, ... as if they were consecutive ("virtual" numbering: block v is
@@ -627,14 +612,16 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
         row0 = blockIdx.x; rstep = G;
         v_begin = 0; v_end = rows_total * nb;
     } else {
-        const int r0 = (int)range_start(blockIdx.x, B, G);
-        row0 = r0 / nb; rstep = 1;
-        v_begin = r0 - row0 * nb; v_end = (int)range_start(blockIdx.x + 1, B, G) - row0 * nb;
+        // (divisions are not scalar arithmetic: their results are made so by a shuffle)
+        const int r0 = __shfl_sync(kFullMask, (int)range_start(blockIdx.x, B, G), 0);
+        const int r1 = __shfl_sync(kFullMask, (int)range_start(blockIdx.x + 1, B, G), 0);
+        row0 = __shfl_sync(kFullMask, r0 / nb, 0); rstep = 1;
+        v_begin = r0 - row0 * nb; v_end = r1 - row0 * nb;
     }
     int p = v_begin, e = min(v_end, max_rows * nb), rbase = 0;     // the round's blocks [p, e), its first row block rbase
     const int piece_lo = (int)(((long)warp * nb) >> 5), piece_n = (int)(((long)(warp + 1) * nb) >> 5) - piece_lo;
     // Blocks added up in one accumulator: a 32nd of a row (whole chunks).  The tensor cores' additions truncate, and over a run of up
-    // to 100 blocks that adds up; the parts are added in the slot, in fp32 with rounding (see the head of this file).
+    // to 100 blocks that adds up; the parts are added in fp32 with rounding (see the head of this file).
     const int part_n = PIECES ? piece_n : ((nb + NW - 1) / NW + C - 1) / C * C;
     const int seg_n = PIECES ? piece_n : nb;                       // blocks of a segment (what lies in one row block), but for ends
     // this warp's blocks of a round: first block v (column col of its row block), `left` of the first segment, `total`
@@ -648,60 +635,68 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
             const int cnt = e - p;
             v = p + (int)(((long)warp * cnt) >> 5);
             total = p + (int)(((long)(warp + 1) * cnt) >> 5) - v;
-            col = v - v / nb * nb;
+            col = __shfl_sync(kFullMask, v - v / nb * nb, 0);
             left = min(total, nb - col);
         }
     };
 
-    // The ring of this warp: slot s at ring + (s*NW + warp)*slot_bytes, its barrier at bar_w + 8s.
-    const uint32_t ring_w = smem_u32(ring) + warp * slot_bytes;
-    const uint32_t slot_stride = NW * slot_bytes;
-    const uint32_t bar_w = smem_u32(smem + kBarOffset) + warp * 16;
-    if (lane == 0) { mbar_init(bar_w, 1); mbar_init(bar_w + 8, 1); }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    __syncwarp();
-    // Issue cursor: this warp's chunks in order, one or two ahead of the decoding; a chunk does not cross a segment.
-    // Uniform over the warp, lane 0 issues the copies.
-    int i_left, i_total, i_col;
-    const uint8_t *i_ptr;
+    // The ring of this warp: slot s at ring + (s*NW + warp)*slot_bytes; the other slot of an address is ring_both - address.
+    const uint32_t ring_w = smem_u32(ring) + warp * slot_bytes, ring_both = 2 * ring_w + NW * slot_bytes;
+    // Issue cursor: this warp's chunks in order, one or two ahead of the decoding; a chunk does not cross a segment.  Uniform over the
+    // warp but for the pointers, which are this lane's (16 bytes of every 512).
+    int i_n, i_rest;                      // blocks left of the segment being requested, and after it
+    const uint8_t *i_ptr, *x_ptr = nullptr;
+    uint32_t i_slot = ring_w;
     const size_t i_jump = ((size_t)rstep * nb - seg_n) * kBlockBytes;
-    unsigned ichunk = 0;
     auto start_issue = [&]() {
-        int v;
-        run_of(v, i_col, i_left, i_total);
-        const int row = PIECES ? 0 : (v - i_col) / nb;             // pieces: the cursor runs on through all rounds
-        i_ptr = codes + ((size_t)(row0 + row * rstep) * nb + i_col) * kBlockBytes;
-        if (PIECES) i_total = rows_total * piece_n;
+        int v, col;
+        run_of(v, col, i_n, i_rest);
+        const int row = PIECES ? 0 : __shfl_sync(kFullMask, (v - col) / nb, 0);      // pieces: the cursor runs on through all rounds
+        if (PIECES) i_rest = rows_total * piece_n;
+        i_rest -= i_n;
+        i_ptr = codes + ((size_t)(row0 + row * rstep) * nb + col) * kBlockBytes + lane * 16;
+        if (!XS) x_ptr = reinterpret_cast<const uint8_t *>(x) + (size_t)col * xblk_bytes + lane * 16;
     };
-    // 0: issues the warp's copies.  From 32: a wait ran out, no more waits and no more copies (the results are meaningless); the chunk
-    // waited for (modulo 4) << 6 and how many are on their way << 8.  One register for all of it keeps the loop as short as it is.
-    unsigned role = lane;
-    // codes: the packed weights (any time); with x through the ring the x part follows separately for the chunk issued
-    // before the activations may be read
+    // x of nblk blocks, behind the codes of the slot
+    auto copy_x = [&](uint32_t slot, const uint8_t *src, int nblk) {
+        const int bytes = nblk * xblk_bytes;
+        const uint32_t dst = slot + C * kBlockBytes + lane * 16;
+        if (lane * 16 < bytes) copy16_async(dst, src);
+        if (C > 1 && lane * 16 + 512 < bytes) copy16_async(dst + 512, src + 512);      // plan_smem: bytes <= 1024
+    };
+    // One group of copies per call, empty when nothing is left.  Codes are weights and may be read any time; x follows separately for
+    // the chunk whose codes are requested before the activations may be read.
     auto issue = [&](bool with_x) {
-        if (i_left <= 0) return;
-        const int nblk = min(C, i_left);
-        if (role == 0) {
-            const uint32_t dst = ring_w + (ichunk & 1u) * slot_stride, bar = bar_w + (ichunk & 1u) * 8;
-            mbar_expect(bar, (uint32_t)(nblk * (kBlockBytes + xblk_bytes)));
-            bulk_copy(dst, i_ptr, (uint32_t)(nblk * kBlockBytes), bar);
-            if (!XS && with_x)
-                bulk_copy(dst + C * kBlockBytes, reinterpret_cast<const uint8_t *>(x) + (size_t)i_col * xblk_bytes,
-                          (uint32_t)(nblk * xblk_bytes), bar);
-        }
-        ichunk++;
-        i_left -= nblk;
-        i_total -= nblk;
-        i_ptr += nblk * kBlockBytes;
-        if (!XS) i_col += nblk;
-        if (i_left == 0) {
-            i_left = min(seg_n, i_total);
+        if (i_n == 0 && i_rest > 0) {
+            i_n = min(seg_n, i_rest);
+            i_rest -= i_n;
             i_ptr += i_jump;
-            i_col = PIECES ? piece_lo : 0;
+            if (!XS) x_ptr = reinterpret_cast<const uint8_t *>(x) + lane * 16;
         }
+        if (i_n > 0) {
+            const int nblk = min(C, i_n);
+            if (C == 1 || i_n >= C) {
+#pragma unroll
+                for (int o = 0; o < C * kBlockBytes; o += 512)
+                    if (o + 512 <= C * kBlockBytes || lane * 16 < C * kBlockBytes - o) copy16_async(i_slot + lane * 16 + o, i_ptr + o);
+            } else {
+#pragma unroll
+                for (int o = 0; o < (C - 1) * kBlockBytes; o += 512)
+                    if (o + lane * 16 < nblk * kBlockBytes) copy16_async(i_slot + lane * 16 + o, i_ptr + o);
+            }
+            if (!XS) {
+                if (with_x) copy_x(i_slot, x_ptr, nblk);
+                x_ptr += nblk * xblk_bytes;
+            }
+            i_ptr += nblk * kBlockBytes;
+            i_n -= nblk;
+            i_slot = ring_both - i_slot;
+        }
+        if (XS || with_x) copies_commit();
     };
     start_issue();
-    const int first_n = min(C, i_left), first_col = i_col;
+    const int first_n = min(C, i_n);
+    const uint8_t *const first_x = x_ptr;
     // First chunk of this warp: packed codes are weights, so the copy starts before the table build and before
     // waiting for the previous kernel of the stream.
     issue(false);
@@ -853,14 +848,11 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
     }
     else {
         // the x part of the chunk whose codes were requested above
-        if (lane == 0 && first_n > 0)
-            bulk_copy(ring_w + C * kBlockBytes, reinterpret_cast<const uint8_t *>(x) + (size_t)first_col * xblk_bytes,
-                      (uint32_t)(first_n * xblk_bytes), bar_w);
+        copy_x(ring_w, first_x, first_n);
+        copies_commit();
     }
-    // a scratch over ring slot 1 has been read and written by plain accesses, which the copy below must not overtake
-    if (scratch_offset <= 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
-    if (ichunk < 2) issue(true);        // second chunk: x may be read now, and the scratch no longer lies over ring slot 1
+    if (!XS || scratch_offset <= 0) issue(true);        // second chunk: x may be read now, and the scratch no longer lies over ring slot 1
 
     const int g = lane >> 2, t = lane & 3;
     const int xg = g < bs ? g : 0;      // lanes of unused batch columns alias row 0; their results are never stored
@@ -869,9 +861,9 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
     const uint32_t lut_lane = smem_u32(lut) + lane * 4;
     const uint32_t own_off = lane * (4 * K), nxt_off = ((lane + 1) & 31) * (4 * K);   // lane 31 wraps to lane 0: tail-biting
 
-    unsigned cchunk = 0;       // chunks consumed so far: slot cchunk & 1, barrier phase (cchunk >> 1) & 1
+    uint32_t slot = ring_w;        // of the next chunk
     for (;;) {
-        if (!PIECES) {      // the parts of a sum are added to the slot; what a warp without a block does not write counts as zero
+        if (!PIECES && e - p < NW) {      // fewer blocks than warps: what a warp without a block does not write counts as zero
             for (int i = threadIdx.x; i < (NW + (e - 1) / nb - rbase) * stride; i += kThreads) red[i] = 0.f;
             __syncthreads();
         }
@@ -880,55 +872,53 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
         float *slot_out = red + (PIECES ? warp : warp + (v - col) / nb - rbase) * stride;
         uint32_t xsp = xs_base + (uint32_t)col * xs_step;
         const uint32_t xs_next = PIECES ? xsp : xs_base;           // x at the start of the segments that follow
-        float acc[2][4] = {};
+        float acc[2][4] = {}, sum[2][4] = {};
         // the part being decoded, and what follows it in its segment and in all
         int part = PIECES ? left : min(part_n, left);
         left -= part;
         total -= part;
         while (part > 0) {
-            const int nblk = min(C, part);
-            uint32_t slot = ring_w + (cchunk & 1u) * slot_stride;
-            if (role < 32) {
-                const uint32_t bar = bar_w + (cchunk & 1u) * 8, parity = (cchunk >> 1) & 1u;
-                unsigned spins = 0;
-                while (!mbar_try_wait(bar, parity)) {
-                    if (++spins > kRingSpinLimit) {
-                        if (lane == 0) atomicOr(done_counter + 1, 1u);
-                        role = 32u + ((cchunk & 3u) << 6) + ((ichunk - cchunk) << 8);
-                        break;
-                    }
-                }
-            }
-            uint32_t xa = XS ? xsp : slot + C * kBlockBytes + xlane;
+            int nblk = min(C, part);
+            part -= nblk;
+            copies_wait_but_one();
+            __syncwarp();      // the other lanes' copies of the chunk
+            uint32_t xa = XS ? xsp : slot + C * kBlockBytes + xlane, blk = slot;
             // One block per trip, not unrolled: the body (about 95 instructions) stays in the instruction buffers of the
-            // sub-partitions; four blocks unrolled ran 17 % slower on the same data (32.6 against 28 cycles per block and SM).
+            // sub-partitions.
 #pragma unroll 1
-            for (int i = 0; i < nblk; i++) {
-                const LaneCodes<K> own = lds_lane_codes<K>(slot + own_off);
-                const LaneCodes<K> nxt = lds_lane_codes<K>(slot + nxt_off);
+            do {
+                const LaneCodes<K> own = lds_lane_codes<K>(blk + own_off);
+                const LaneCodes<K> nxt = lds_lane_codes<K>(blk + nxt_off);
                 uint32_t xb[4];
                 asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(xb[0]), "=r"(xb[1]), "=r"(xb[2]), "=r"(xb[3]) : "r"(xa));
                 xa += xs_step;
-                slot += kBlockBytes;
+                blk += kBlockBytes;
                 decode_block<K>(own, nxt, xb, acc, lut_lane);
-            }
+            } while (C > 1 && --nblk > 0);
             xsp = xa;
-            part -= nblk;
+            slot = ring_both - slot;
             __syncwarp();      // every lane has read the slot before it is filled again
             issue(true);
-            cchunk++;
             if (part == 0) {
-                // accumulator (ms, i): row = 16*ms + g + 8*(i>>1), batch = 2*t + (i&1); slot word = batch*32 + row
+                if (!PIECES) {
 #pragma unroll
-                for (int ms = 0; ms < 2; ms++)
+                    for (int ms = 0; ms < 2; ms++)
 #pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        const int b = 2 * t + (i & 1);
-                        float *word = slot_out + b * 32 + 16 * ms + g + 8 * (i >> 1);
-                        if (b < bs) *word = PIECES ? acc[ms][i] : *word + acc[ms][i];
-                        acc[ms][i] = 0.f;
-                    }
+                        for (int i = 0; i < 4; i++) {
+                            sum[ms][i] += acc[ms][i];
+                            acc[ms][i] = 0.f;
+                        }
+                }
                 if (PIECES || left == 0) {
+                    // accumulator (ms, i): row = 16*ms + g + 8*(i>>1), batch = 2*t + (i&1); slot word = batch*32 + row
+#pragma unroll
+                    for (int ms = 0; ms < 2; ms++)
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            const int b = 2 * t + (i & 1);
+                            if (b < bs) slot_out[b * 32 + 16 * ms + g + 8 * (i >> 1)] = PIECES ? acc[ms][i] : sum[ms][i];
+                            (PIECES ? acc : sum)[ms][i] = 0.f;
+                        }
                     slot_out += PIECES ? NW * stride : stride;
                     left = min(seg_n, total);
                     xsp = xs_next;
@@ -962,10 +952,6 @@ __global__ void __launch_bounds__(kConsumerWarps * 32, 1)
         __syncthreads();       // the slots are read before the next round writes them
     }
 
-    if (role >= 32) {          // nothing may land after the CTA has gone: what was on its way, with a limit again
-        for (unsigned c = (role >> 6) & 3u, end = c + (role >> 8); c != end; c++)
-            for (unsigned spins = 0; spins < kRingSpinLimit && !mbar_try_wait(bar_w + (c & 1u) * 8, (c >> 1) & 1u); spins++) {}
-    }
     if (TP && P.sig.seq) {
         // row-parallel partial result: the values are already on their way to every GPU (stamped); the CTA that
         // finishes last advances the sequence counter that the stamps of the next launch are derived from
@@ -1193,6 +1179,7 @@ bool plan_smem(int n, int bs, int cta_rows, bool pieces, int cap, bool xs, bool 
     plan.scratch_offset = 0;
     for (int c = kMaxChunkBytes / BB; c >= 1; c >>= 1) {          // 4, 2, 1: the instantiated chunk sizes
         const int slot = NW * c * (BB + ring_x);                        // one ring slot, all warps
+        if (c * ring_x > 1024) continue;                                // copy_x: at most two 16-byte words per lane
         if (2 * slot + red_bytes + x_bytes + scratch_bytes <= avail) {  // room for a scratch area of its own
             plan.chunk_blocks = c;
             plan.xs_offset = kCtrlBytes + kLutBytes + 2 * slot + red_bytes;
