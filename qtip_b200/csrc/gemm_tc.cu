@@ -5,30 +5,35 @@
 // One CTA owns 128 output rows (four 32-row blocks) and a contiguous range of input columns.  The
 // weights are the A operand: D[128 x N] += A[128 x 16] * B[16 x N] with D AND A in tensor memory, B in
 // shared memory, K-major, 128-byte swizzle; N = batch rounded up to 16.
-//   * 24 decode warps turn packed codes into fp16 and store them with tcgen05.st into the A part of a ring stage (128 rows x
-//     64 columns = 8 tile blocks, one per warp; three stages are filled concurrently).  A kernel-layout tile block in its lanes IS
+//   * 24 decode warps turn packed codes into fp16 and store them with tcgen05.st into a stage of weights (128 rows x 128
+//     columns = 16 tile blocks, two per warp; three stages are filled concurrently).  A kernel-layout tile block in its lanes IS
 //     the 16x128b store shape, so the weights never pass through shared memory, whose wavefronts the table lookups need.
-//     The same warps copy the 64-column slice of X into the B tile of the stage.
-//   * one thread issues four tcgen05.mma (K = 16 each) per stage and commits them to the stage's
-//     "empty" barrier; a last commit signals the epilogue.
+//   * one thread copies the slices of X with tiled TMA loads (no multicast; rows beyond the batch are filled with zeros) into a ring
+//     of its own, as deep as the memory beside the table allows;
+//   * one thread issues eight tcgen05.mma (K = 16 each) per step and commits them to the stages'
+//     "empty" barriers; a last commit signals the epilogue.
 //   * warps 0-3 read the accumulator with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31 = rows) and
 //     write out (coalesced along rows); when the row ranges leave SMs idle the columns are split over the
 //     2, 4 or 8 CTAs of a cluster, which leave their parts in shared memory and add them in order.
 // The compute codes (3INST / 1MAD, V = 1, plain layout) use the same kernel with another producer: a lane decodes one row of a
 // tile (its own 2K bytes and the start of the next row), lanes 2r and 2r + 1 row r of two tiles, and stores a row per
 // tensor-memory lane; the accumulator's lanes are mapped back to rows when they are read.
-// Bound: instruction issue of the decode warps (8192 x 8192, 27 rows: 190 instructions per warp and stage HYB, 295 3INST, issued in
-// 64 and 66 % of the cycles; the tensor pipe is busy 7 to 10 % of the time, and leaving out three of the four MMAs, the loads or half of the ring's depth changes nothing).  Hence the loop unrolled
-// by two with fixed stages and buffers, and x through asynchronous copies issued a step ahead.  Measured, K = 2, A through shared
-// memory and x through registers -> now:  HYB 8192 x 8192, 27 rows 28.7 -> 20.2 us; 8192 x 28672, 120 rows 123.5 -> 72.1 us;
-// 3INST 8192 x 8192, 27 rows 36.9 -> 29.4 us, 120 rows of 28672 155.7 -> 103.7 us; 1MAD 37.5 -> 29.4 us, 163.7 -> 102.7 us (of
-// which windows as byte permutes: 3INST 33.5 -> 31.3, 115.9 -> 108.8).
+// Bound: instruction issue of the decode warps up to about 64 rows (8192 x 28672, 27 rows: leaving out three of four MMAs 45.6 -> 43.0 us,
+// the lookups 35.4), the MMAs above (120 rows: 57.8 -> 48.9 and 54.4 us).  Hence two blocks per warp and step between the barriers, x
+// through TMA instead of copies by the decode warps, scalar control (the warp index through a shuffle), control threads that sleep
+// between polls, and codes requested two steps ahead.  Warp instructions per block of weights, HYB 27 rows 190 -> 157, 3INST 295 -> 254.
+// Measured, one block per warp and step with x copied by the decode warps -> now (microseconds, K = 2 unless stated): HYB 8192 x 8192
+// 27 rows 20.5 -> 17.5; 8192 x 28672 120 rows 73 -> 57.2; 14336 x 4096 K = 3 27 rows 19.7 -> 16.3; 28672 x 8192 K = 4 64 rows 70 -> 58;
+// 3INST 8192 x 8192 16 rows 30.5 -> 26.0, 8192 x 28672 120 rows 107 -> 83; 1MAD 8192 x 8192 K = 3 32 rows 33.0 -> 29.4.  A second
+// accumulator for every other MMA changes nothing.
 // This replaces decode-to-HBM + dense GEMM of BitshiftLinearKernelAG upstream
 // (lib/codebook/bitshift.py:476-489), which writes and re-reads 16x the packed bytes at 2 bits.
 //
 // Every mbarrier wait is bounded: after kSpinLimit polls the waiter records an error code in
 // `status`, raises a CTA-wide abort flag that makes every later wait fall through, and the kernel
 // still runs to its end, frees its tensor memory and returns (with meaningless results).
+#include <cuda.h>
+
 #include <mutex>
 
 #include "common.cuh"
@@ -38,18 +43,30 @@ namespace {
 
 constexpr int kGroups = 3;                               // groups of 8 decode warps; a group fills one stage
 constexpr int kDecodeWarps = 8 * kGroups;
-constexpr int kGemmThreads = (kDecodeWarps + 1) * 32;   // + one control warp (TMEM allocation, MMA issue)
-constexpr int kStages = 2 * kGroups;                    // ring stages: every group may be one step ahead of the MMA
+constexpr int kMmaWarp = kDecodeWarps, kCopyWarp = kDecodeWarps + 1;      // TMEM allocation and MMA issue; copies of x
+constexpr int kGemmThreads = (kDecodeWarps + 2) * 32;
+constexpr int kStages = 2 * kGroups;                    // stages of weights: every group may be one step ahead of the MMA
 constexpr int kRows = 128;                               // output rows per CTA
-constexpr int kStageCols = 64;                           // input columns per stage (128 bytes of fp16 per row)
-constexpr int kAStageCols = kStageCols / 2;              // 32-bit tensor-memory columns of an A stage: two weights each
+constexpr int kStageCols = 128;                          // input columns per step: two blocks per decode warp, two tiles of x
+constexpr int kTileCols = 64;                            // 128 bytes of fp16: the swizzle span
+constexpr int kAStageCols = kStageCols / 2;              // 32-bit tensor-memory columns of a stage of weights: two weights each
 constexpr int kLut512Bytes = 1024 * 32 * 4;              // (512 entries + sign-flipped twins) x 32 lane-private copies
 constexpr int kMaxN = 128;
+constexpr int kXRingBytes = 96 * 1024;                   // at most, beside the table
 constexpr unsigned kSpinLimit = 1u << 22;
+// A warp that polls takes issue slots from the decode warps of its sub-partition, so the two control threads sleep between polls; both
+// are one or more stages ahead of what they wait for.
+constexpr unsigned kMmaSleepNs = 40, kCopySleepNs = 200;
+
+// stages of x: a step's tiles are npad x 128 columns
+__host__ __device__ __forceinline__ int x_stages(int npad) {
+    const int fit = kXRingBytes / (npad * kStageCols * 2);
+    return fit < kStages ? fit : kStages;
+}
 
 struct GemmCtrl {
-    unsigned long long full[kStages];
-    unsigned long long empty[kStages];
+    unsigned long long full[kStages], empty[kStages];        // weights
+    unsigned long long xfull[kStages], xempty[kStages];      // x
     unsigned long long done;
     uint32_t tmem_base;
     int abort_flag;
@@ -74,10 +91,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     return ok != 0;
 }
 // false: the wait gave up (its own limit, or another waiter raised the abort flag)
+template <unsigned kSleepNs = 0>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, unsigned *status,
                                           unsigned code) {
     if (mbar_try_wait(bar, parity)) return true;
     for (unsigned spin = 0; spin < kSpinLimit; spin++) {
+        if (kSleepNs > 0) __nanosleep(kSleepNs);
         if (mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
     }
@@ -89,6 +108,15 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity) {
     for (unsigned spin = 0; spin < kSpinLimit; spin++)
         if (mbar_try_wait(bar, parity)) return;
+}
+
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Box of x at column c (a multiple of 64), row 0: rows beyond the tensor are filled with zeros
+__device__ __forceinline__ void copy_x_tile(uint32_t dst, const CUtensorMap *map, int c, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(dst), "l"(map), "r"(c), "r"(0), "r"(bar) : "memory");
 }
 
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 bytes apart.
@@ -201,10 +229,9 @@ __device__ __forceinline__ uint32_t pair_1mad(uint32_t s0, uint32_t s1, uint32_t
     return __byte_perm(w0, w1, 0x5410);
 }
 
-// SMALL: batches up to 64, whose slice of x is at most two copies per thread and whose accumulator leaves half of tensor memory free
-template <int K, int CODE, bool SMALL>
+template <int K, int CODE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
-    decompress_gemm_kernel(float *__restrict__ out, const uint8_t *__restrict__ codes, const __half *__restrict__ x,
+    decompress_gemm_kernel(float *__restrict__ out, const uint8_t *__restrict__ codes, const __grid_constant__ CUtensorMap xmap,
                            const uint32_t *__restrict__ tlut, int m, int n, int bs, int npad, int splitk,
                            unsigned *__restrict__ status) {
     constexpr int kBlockBytes = 128 * K;
@@ -213,27 +240,30 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const uint32_t raw = smem_addr(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;                 // swizzled tiles need 1024-byte alignment
     uint8_t *smem = smem_raw + (base - raw);
-    const int b_stage_bytes = npad * 128;
-    // layout: B stages | LUT | control
+    const int xstages = x_stages(npad), tile_bytes = npad * kTileCols * 2, x_stage_bytes = 2 * tile_bytes;
+    // layout: stages of x | LUT | control
     const uint32_t b_base = base;
-    uint32_t *lut = reinterpret_cast<uint32_t *>(smem + kStages * b_stage_bytes);
-    GemmCtrl *ctl = reinterpret_cast<GemmCtrl *>(smem + kStages * b_stage_bytes + kLut512Bytes);
+    uint32_t *lut = reinterpret_cast<uint32_t *>(smem + xstages * x_stage_bytes);
+    GemmCtrl *ctl = reinterpret_cast<GemmCtrl *>(smem + xstages * x_stage_bytes + kLut512Bytes);
     volatile int *abort_flag = &ctl->abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // tensor memory: kStages A stages, then the accumulator's npad columns
-    constexpr int kTmemD = kStages * kAStageCols, kTmemCols = SMALL ? 256 : 512;
+    // through a shuffle: known to be the same in all lanes, so that the control of a warp's steps is scalar
+    const int warp = __shfl_sync(kFullMask, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    // tensor memory: kStages stages of weights, then the accumulator's npad columns
+    constexpr int kTmemD = kStages * kAStageCols, kTmemCols = 512;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; s++) {
             mbar_init(smem_addr(&ctl->full[s]), 8);     // eight decode warps fill a stage
             mbar_init(smem_addr(&ctl->empty[s]), 1);    // one tcgen05.commit frees it
+            mbar_init(smem_addr(&ctl->xfull[s]), 1);    // the copying thread, and the bytes it announces
+            mbar_init(smem_addr(&ctl->xempty[s]), 1);
         }
         mbar_init(smem_addr(&ctl->done), 1);
         ctl->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == kDecodeWarps) {
+    if (warp == kMmaWarp) {
         // 128 lanes x kTmemCols 32-bit columns
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&ctl->tmem_base)),
                      "r"(kTmemCols)
@@ -255,6 +285,43 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             reinterpret_cast<uint4 *>(lut)[i] = make_uint4(e, e, e, e);
         }
     }
+    const int nb = n >> 5;                                  // 32-column blocks per row block
+    const int r0 = blockIdx.x * kRows;                      // first output row of this CTA
+    // 64-column tiles of this CTA: split over the CTAs of the cluster, not necessarily evenly; the last step may have one tile
+    const int all_tiles = n / kTileCols;
+    const int tile0 = all_tiles * (int)blockIdx.y / splitk, ntiles = all_tiles * ((int)blockIdx.y + 1) / splitk - tile0;
+    const int nsteps = (ntiles + 1) >> 1, c0 = tile0 * kTileCols;
+
+    // decode warps: this group fills steps group, group + kGroups, ...; a warp decodes two blocks of a step, rows 32 rb .. of the tile half
+    const int group = warp >> 3, rb = warp & 3, half = (warp >> 2) & 1;
+    const uint8_t *src = codes + ((size_t)(r0 / 32 + rb) * nb + (c0 / 32 + 2 * half + 4 * group)) * kBlockBytes + lane * (4 * K);
+    // plain layout (V = 1 codes): tile (tile row, tile column) = 16K words at ((row/16)*(n/16) + col/16)*16K; this
+    // lane decodes row lane >> 1 of tile row 2rb + (lane & 1), tile columns 4 half .. + 3 of the step
+    const uint16_t *prow = reinterpret_cast<const uint16_t *>(codes) +
+                           ((size_t)(r0 / 16 + 2 * rb + (lane & 1)) * (n >> 4) + (size_t)(c0 / 16 + 4 * half + 8 * group)) * (16 * K) +
+                           (lane >> 1) * K;
+    // codes of the current step and of the one after it
+    struct StepCodes {
+        LaneCodes<K> blk[2];
+        PlainRow<K> rows[2][2];
+    };
+    StepCodes now = {}, ahead = {};
+    auto load_codes = [&](StepCodes &c, int step) {
+        if (2 * step + half >= ntiles) return;
+        if constexpr (kHyb) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) c.blk[h] = load_lane_codes<K>(src + h * kBlockBytes);
+            src += kGroups * 4 * kBlockBytes;
+        } else {
+#pragma unroll
+            for (int h = 0; h < 4; h++) c.rows[h >> 1][h & 1] = load_plain_row<K>(prow + h * (16 * K));
+            prow += kGroups * (kStageCols / 16) * (16 * K);
+        }
+    };
+    if (warp < kDecodeWarps) {      // weights: before the wait for the launch that makes x
+        load_codes(now, group);
+        load_codes(ahead, group + kGroups);
+    }
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -262,135 +329,104 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     const uint32_t tmem = ctl->tmem_base, tmem_d = tmem + kTmemD;
     asm volatile("griddepcontrol.wait;" ::: "memory");      // everything above touches weights only
 
-    const int nb = n >> 5;                                  // 32-column blocks per row block
-    const int r0 = blockIdx.x * kRows;                      // first output row of this CTA
-    const int all_steps = n / kStageCols;                   // split over the CTAs of the cluster, not necessarily evenly
-    const int step0 = all_steps * (int)blockIdx.y / splitk, nsteps = all_steps * ((int)blockIdx.y + 1) / splitk - step0;
-    const int c0 = step0 * kStageCols;                      // first input column
-
     if (warp < kDecodeWarps) {
         // ---------------------------------- decode warps ------------------------------------------------
-        const int group = warp >> 3;                        // this group fills steps group, group + kGroups, ...
-        const int w8 = warp & 7, rb = w8 & 3, cb = w8 >> 2; // row block (of 4) and column block (of 2) of the stage
         const uint32_t lut_lane = smem_addr(lut) + lane * 4;
-        // this warp's 32 rows and 16 words of an A stage (a warp reaches the 32 lanes of its index modulo four)
-        const uint32_t tmem_warp = tmem + ((uint32_t)(32 * rb) << 16) + 16u * cb;
-        // The 64-column slice of x goes into the B tile of the stage: chunk ch of the tile = batch row ch >> 3, columns
-        // 8*(ch & 7) .. +7, rows beyond bs zero, 16-byte chunks swizzled by row % 8.  Thread tid8 of the stage's eight warps copies chunks
-        // tid8 + 256 i.  The copies of the warp's NEXT step are issued after the current step is decoded and awaited a step later.
-        const int tid8 = w8 * 32 + lane, brow = tid8 >> 3;
-        const __half *xsrc = x + (size_t)brow * n + c0 + group * kStageCols + (tid8 & 7) * 8;
-        const uint32_t xdst = b_base + (uint32_t)(brow * 128 + (((tid8 & 7) ^ (brow & 7)) << 4));
-        auto copy_x = [&](int s) {
+        // this warp's 32 rows and 32 words of a stage (a warp reaches the 32 lanes of its index modulo four)
+        const uint32_t tmem_warp = tmem + ((uint32_t)(32 * rb) << 16) + 32u * half;
+        uint32_t s = group, parity = 1;                     // stage group, then group + kGroups, in turn
+        for (int step = group; step < nsteps; step += kGroups) {
+            const uint32_t ast = tmem_warp + s * kAStageCols;
 #pragma unroll
-            for (int i = 0; i < (SMALL ? 2 : 4); i++)
-                if (brow + 32 * i < npad) {
-                    const bool live = brow + 32 * i < bs;
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(xdst + (uint32_t)(s * b_stage_bytes + 4096 * i)),
-                                 "l"(live ? xsrc + (size_t)(32 * i) * n : x), "r"(live ? 16 : 0)
-                                 : "memory");
-                }
-            xsrc += kGroups * kStageCols;
-        };
-        // codes: two steps of this warp ahead (the warp's steps are kGroups apart), in two buffers that the two steps of the loop take in turn
-        const uint8_t *src = codes + ((size_t)(r0 / 32 + rb) * nb + (c0 / 32 + cb + 2 * group)) * kBlockBytes + lane * (4 * K);
-        LaneCodes<K> own[2] = {};
-        // plain layout (V = 1 codes): tile (tile row, tile column) = 16K words at ((row/16)*(n/16) + col/16)*16K; this
-        // lane decodes row lane >> 1 of tile row 2rb + (lane & 1), in the step's tile columns 2cb and 2cb + 1
-        const uint16_t *prow = reinterpret_cast<const uint16_t *>(codes) +
-                               ((size_t)(r0 / 16 + 2 * rb + (lane & 1)) * (n >> 4) + (size_t)(c0 / 16 + 2 * cb + 4 * group)) * (16 * K) +
-                               (lane >> 1) * K;
-        PlainRow<K> prows[2][2] = {};
-        auto load_codes = [&](int buf) {
-            if constexpr (kHyb) {
-                own[buf] = load_lane_codes<K>(src);
-                src += kGroups * 2 * kBlockBytes;
-            } else {
+            for (int h = 0; h < 2; h++) {
+                uint32_t wv[16];
+                if constexpr (kHyb) {
+                    LaneCodes<K> nxt = {};
 #pragma unroll
-                for (int ks = 0; ks < 2; ks++) prows[buf][ks] = load_plain_row<K>(prow + ks * (16 * K));
-                prow += kGroups * (kStageCols / 16) * (16 * K);
-            }
-        };
-        if (group < nsteps) {
-            load_codes(0);
-            copy_x(group);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        if (group + kGroups < nsteps) load_codes(1);
-        // one step; buf and the stage group + kGroups * buf alternate
-        auto decode_step = [&](int step, int buf, int round) {
-            const int s = group + kGroups * buf, snext = group + kGroups * (buf ^ 1);
-            // the weights are decoded into registers first, so only the stores wait for the stage
-            uint32_t wv[16];
-            if constexpr (kHyb) {
-                LaneCodes<K> nxt = {};
+                    for (int i = 0; i < K; i++) nxt.w[i] = __shfl_sync(kFullMask, now.blk[h].w[i], lane + 1);
 #pragma unroll
-                for (int i = 0; i < K; i++) nxt.w[i] = __shfl_sync(kFullMask, own[buf].w[i], lane + 1);
+                    for (int tt = 0; tt < 4; tt++) {
+                        const int ks = tt >> 1, ms = tt & 1;
+                        uint32_t st[4];
+                        tile_states<K>(now.blk[h], nxt, tt, st);
 #pragma unroll
-                for (int tt = 0; tt < 4; tt++) {
-                    const int ks = tt >> 1, ms = tt & 1;
-                    uint32_t st[4];
-                    tile_states<K>(own[buf], nxt, tt, st);
+                        for (int q = 0; q < 4; q++)       // q = 2c + d: column half, row half of the 16x16 tile
+                            wv[8 * ms + 4 * ks + q] = hyb_lookup(st[q], lut_lane);
+                    }
+                } else {
 #pragma unroll
-                    for (int q = 0; q < 4; q++)       // q = 2c + d: column half, row half of the 16x16 tile
-                        wv[8 * ms + 4 * ks + q] = hyb_lookup(st[q], lut_lane);
-                }
-            } else {
+                    for (int ks = 0; ks < 2; ks++) {
+                        const uint32_t next = __shfl_sync(kFullMask, now.rows[h][ks].a, lane + 2);      // row 15 -> row 0: tail-biting
 #pragma unroll
-                for (int ks = 0; ks < 2; ks++) {
-                    const uint32_t next = __shfl_sync(kFullMask, prows[buf][ks].a, lane + 2);      // row 15 -> row 0: tail-biting
-#pragma unroll
-                    for (int j = 0; j < 8; j++) {
-                        const uint32_t s0 = plain_state<K>(prows[buf][ks], next, 2 * j), s1 = plain_state<K>(prows[buf][ks], next, 2 * j + 1);
-                        wv[8 * ks + j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1) : pair_1mad(s0, s1, lut_lane);
+                        for (int j = 0; j < 8; j++) {
+                            const uint32_t s0 = plain_state<K>(now.rows[h][ks], next, 2 * j), s1 = plain_state<K>(now.rows[h][ks], next, 2 * j + 1);
+                            wv[8 * ks + j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1) : pair_1mad(s0, s1, lut_lane);
+                        }
                     }
                 }
-            }
 #pragma unroll
-            for (int i = 0; i < 16; i++) asm volatile("" : "+r"(wv[i]));
-            if (step + 2 * kGroups < nsteps) load_codes(buf);
-            if (step + kGroups < nsteps) {
-                // the next step's stage: its last use was kStages - kGroups steps ago (round 0 of the second half: never)
-                if (buf || round > 0) mbar_wait(smem_addr(&ctl->empty[snext]), (buf ? round : round - 1) & 1, abort_flag, status, 1u);
-                copy_x(snext);
+                for (int i = 0; i < 16; i++) asm volatile("" : "+r"(wv[i]));
+                if (h == 0) {
+                    // the first block is decoded before the stage is waited for; its last use was kStages steps ago (or none)
+                    if (step >= kStages) mbar_wait(smem_addr(&ctl->empty[s]), parity, abort_flag, status, 1u);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    __syncwarp();
+                }
+                if constexpr (kHyb) {
+                    tmem_st_16x128b_x4(ast + 16u * h, wv);
+                    tmem_st_16x128b_x4(ast + 16u * h + (16u << 16), wv + 8);
+                } else tmem_st_32x32b_x16(ast + 16u * h, wv);
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            __syncwarp();
-            const uint32_t ast = tmem_warp + (uint32_t)(s * kAStageCols);
-            if constexpr (kHyb) {
-                tmem_st_16x128b_x4(ast, wv);
-                tmem_st_16x128b_x4(ast + (16u << 16), wv + 8);
-            } else tmem_st_32x32b_x16(ast, wv);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");            // this step's slice of x
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // -> visible to the MMA
+            now = ahead;
+            load_codes(ahead, step + 2 * kGroups);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_addr(&ctl->full[s]));
-        };
-        for (int step = group, round = 0; step < nsteps; step += kStages, round++) {
-            decode_step(step, 0, round);
-            if (step + kGroups < nsteps) decode_step(step + kGroups, 1, round);
+            parity ^= s >= kGroups;                         // both stages have been used once more
+            s = 2 * group + kGroups - s;
         }
-    } else if (elect_one()) {
+    } else if (warp == kMmaWarp && elect_one()) {
         // ------------------------------------ MMA issue ---------------------------------------------------
         // instruction descriptor: D fp32, A/B fp16, both K-major, N = npad, M = 128
         const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
-        int s = 0, round = 0;
+        int s = 0, round = 0, xs = 0, xround = 0;
         for (int step = 0; step < nsteps; step++) {
             // a wait that gave up ends the issue loop: no further MMA is started, and the commit below still
             // covers everything issued so far
-            if (!mbar_wait(smem_addr(&ctl->full[s]), round & 1, abort_flag, status, 2u)) break;
+            if (!mbar_wait<kMmaSleepNs>(smem_addr(&ctl->xfull[xs]), xround & 1, abort_flag, status, 4u)) break;
+            if (!mbar_wait<kMmaSleepNs>(smem_addr(&ctl->full[s]), round & 1, abort_flag, status, 2u)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint64_t bdesc = umma_desc(b_base + s * b_stage_bytes);
 #pragma unroll
-            for (int kk = 0; kk < 4; kk++)   // 16 columns = 32 bytes further inside the 128-byte swizzled row
-                umma_f16(tmem_d, tmem + (uint32_t)(s * kAStageCols + kk * 8), bdesc + (uint64_t)(kk * 2), idesc, (step | kk) != 0);
+            for (int tile = 0; tile < 2; tile++) {
+                if (2 * step + tile < ntiles) {
+                    const uint64_t bdesc = umma_desc(b_base + xs * x_stage_bytes + tile * tile_bytes);
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++)   // 16 columns = 32 bytes further inside the 128-byte swizzled row
+                        umma_f16(tmem_d, tmem + (uint32_t)(s * kAStageCols + tile * 32 + kk * 8), bdesc + (uint64_t)(kk * 2), idesc,
+                                 (step | tile | kk) != 0);
+                }
+            }
             umma_commit(smem_addr(&ctl->empty[s]));
+            umma_commit(smem_addr(&ctl->xempty[xs]));
             if (++s == kStages) { s = 0; round++; }
+            if (++xs == xstages) { xs = 0; xround++; }
         }
         umma_commit(smem_addr(&ctl->done));
+    } else if (warp == kCopyWarp && elect_one()) {
+        // ------------------------------------ copies of x -------------------------------------------------
+        int xs = 0, xround = 0, step = 0;
+        for (; step < nsteps; step++) {
+            if (xround > 0 && !mbar_wait<kCopySleepNs>(smem_addr(&ctl->xempty[xs]), (xround - 1) & 1, abort_flag, status, 5u)) break;
+            const uint32_t bar = smem_addr(&ctl->xfull[xs]), dst = b_base + xs * x_stage_bytes;
+            const int c = c0 + step * kStageCols, tiles = min(2, ntiles - 2 * step);
+            mbar_expect(bar, (uint32_t)(tiles * tile_bytes));
+            copy_x_tile(dst, &xmap, c, bar);
+            if (tiles > 1) copy_x_tile(dst + tile_bytes, &xmap, c + kTileCols, bar);
+            if (++xs == xstages) { xs = 0; xround++; }
+        }
+        // nothing may be on its way when the CTA ends, whatever the other roles did: the last copy of each stage, with a limit
+        for (int k = step - 1; k >= 0 && k >= step - xstages; k--) mbar_wait_bounded(smem_addr(&ctl->xfull[k % xstages]), (k / xstages) & 1);
     }
 
     if (warp < 4) {
@@ -421,7 +457,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == kDecodeWarps) {
+    if (warp == kMmaWarp) {
         // tensor memory is released only after the last commit has arrived, i.e. after every MMA that was issued has
         // completed - also on the abort path, where the epilogue warps did not wait for it
         if (lane == 0) mbar_wait_bounded(smem_addr(&ctl->done), 0u);
@@ -449,10 +485,37 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     }
 }
 
-template <int K, int CODE, bool SMALL>
-int launch_gemm_size(float *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, int npad,
-                       int splitk, unsigned *status, cudaStream_t s) {
-    const int smem = 1024 + kStages * npad * 128 + kLut512Bytes + 256;
+// Tensor map of x (bs, n) fp16 in boxes of npad rows x 64 columns, 128-byte swizzle
+int encode_x(CUtensorMap *map, const __half *x, int n, int bs, int npad) {
+    using Encode = decltype(&cuTensorMapEncodeTiled);
+    static std::mutex mutex;
+    static Encode encode = nullptr;
+    Encode f;
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        if (!encode) {
+            void *p = nullptr;
+            cudaDriverEntryPointQueryResult found;
+            QTIP_CUDA_TRY(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found));
+            if (found != cudaDriverEntryPointSuccess) return QTIP_ERR_CUDA;
+            encode = reinterpret_cast<Encode>(p);
+        }
+        f = encode;
+    }
+    const cuuint64_t dims[2] = {(cuuint64_t)n, (cuuint64_t)bs}, strides[1] = {(cuuint64_t)n * sizeof(__half)};
+    const cuuint32_t box[2] = {kTileCols, (cuuint32_t)npad}, step[2] = {1, 1};
+    const CUresult r = f(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(x), dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r == CUDA_SUCCESS) return QTIP_OK;
+    set_last_cuda_error(cudaErrorInvalidValue);
+    return QTIP_ERR_CUDA;
+}
+
+template <int K, int CODE>
+int launch_gemm(float *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, int npad,
+                int splitk, unsigned *status, cudaStream_t s) {
+    const int smem = 1024 + x_stages(npad) * npad * kStageCols * 2 + kLut512Bytes + 256;
+    static_assert(sizeof(GemmCtrl) <= 256 && 1024 + kXRingBytes + kLut512Bytes + 256 <= 227 * 1024, "shared memory");
     static bool attr_set[64] = {};
     static std::mutex attr_mutex;
     int dev = 0;
@@ -461,11 +524,13 @@ int launch_gemm_size(float *out, const uint8_t *codes, const __half *x, const ui
     {
         std::lock_guard<std::mutex> lock(attr_mutex);
         if (!attr_set[dev]) {
-            QTIP_CUDA_TRY(cudaFuncSetAttribute(decompress_gemm_kernel<K, CODE, SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               227 * 1024));
+            QTIP_CUDA_TRY(cudaFuncSetAttribute(decompress_gemm_kernel<K, CODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
             attr_set[dev] = true;
         }
     }
+    CUtensorMap xmap;
+    const int st = encode_x(&xmap, x, n, bs, npad);
+    if (st != QTIP_OK) return st;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(m / kRows, splitk);
     cfg.blockDim = dim3(kGemmThreads);
@@ -480,21 +545,14 @@ int launch_gemm_size(float *out, const uint8_t *codes, const __half *x, const ui
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = splitk > 1 ? 2 : 1;
-    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decompress_gemm_kernel<K, CODE, SMALL>, out, codes, x, tlut, m, n, bs, npad, splitk, status));
+    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decompress_gemm_kernel<K, CODE>, out, codes, xmap, tlut, m, n, bs, npad, splitk, status));
     return check_launch();
-}
-
-template <int K, int CODE>
-int launch_gemm(float *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, int npad,
-                int splitk, unsigned *status, cudaStream_t s) {
-    if (npad > 64) return launch_gemm_size<K, CODE, false>(out, codes, x, tlut, m, n, bs, npad, splitk, status, s);
-    return launch_gemm_size<K, CODE, true>(out, codes, x, tlut, m, n, bs, npad, splitk, status, s);
 }
 
 // CTAs per row range: as many as still fit the chip at once, in a cluster (at most the portable eight), each with a few steps
 int column_splits(int m, int n) {
     int s = 1;
-    while (s < kMaxSplit && (m / kRows) * s * 2 <= sm_count() && n / kStageCols >= 8 * s) s *= 2;
+    while (s < kMaxSplit && (m / kRows) * s * 2 <= sm_count() && n / kTileCols >= 8 * s) s *= 2;
     return s;
 }
 
@@ -514,7 +572,7 @@ using namespace qtip;
 extern "C" int qtip_decompress_gemm(float *out, const void *codes, const void *x, const void *tlut, int K, int m, int n,
                                     int bs, unsigned *status, void *stream) {
     if (!out || !codes || !x || !tlut || !status || K < 2 || K > 4 || bs < 1 || bs > kMaxN) return QTIP_ERR_BAD_ARG;
-    if (m <= 0 || n <= 0 || (m % kRows) || (n % kStageCols)) return QTIP_ERR_BAD_SHAPE;
+    if (m <= 0 || n <= 0 || (m % kRows) || (n % kTileCols)) return QTIP_ERR_BAD_SHAPE;
     if ((long)(m >> 5) * (n >> 5) >= (1L << 30)) return QTIP_ERR_BAD_SHAPE;
     if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, 4) || !aligned(tlut, 4) || !aligned(status, 4))
         return QTIP_ERR_ALIGNMENT;
@@ -531,7 +589,7 @@ extern "C" int qtip_decompress_gemm_plain(float *out, const void *codes, const v
                                           unsigned *status, void *stream) {
     if (!out || !codes || !x || !status || K < 2 || K > 4 || bs < 1 || bs > kMaxN) return QTIP_ERR_BAD_ARG;
     if (code != QTIP_CODE_3INST && code != QTIP_CODE_1MAD) return QTIP_ERR_BAD_ARG;
-    if (m <= 0 || n <= 0 || (m % kRows) || (n % kStageCols)) return QTIP_ERR_BAD_SHAPE;
+    if (m <= 0 || n <= 0 || (m % kRows) || (n % kTileCols)) return QTIP_ERR_BAD_SHAPE;
     if ((long)(m >> 5) * (n >> 5) >= (1L << 30)) return QTIP_ERR_BAD_SHAPE;
     if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, 4) || !aligned(status, 4)) return QTIP_ERR_ALIGNMENT;
     const int npad = (bs + 15) & ~15;

@@ -535,6 +535,18 @@ def test_decompress_gemm_ring_edges(K, code, m, n, bs):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("bs", [33, 75, 97, 113])
+def test_decompress_gemm_x_ring_depths(bs):
+    """The depths of the ring of x (6, 4, 4 and 3 stages) with several rounds in one CTA and a last step of one tile."""
+    K, m, n = 2, 9600, 1600
+    lay = synth.make_layer(m, n, K, seed=3700 + bs, bs=bs, device=DEV)
+    y, W = ops.decompress_gemm(lay["codes"], lay["x"], lay["tlut"], K, m, n), ops.decode_hyb(lay["codes"], lay["tlut"], K, m, n)
+    want = lay["x"].double() @ W.double().T
+    assert ops.gemm_status(DEV) == 0
+    assert rel_l2(y.cpu().numpy(), want.cpu().numpy()) < 1e-5      # 1600 fp32 additions, the bound of the tests above
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("ctx", [1, 7, 200, 257, 2048, 2049, 5000])
 @pytest.mark.parametrize("heads", [(8, 8), (16, 2)])
 def test_attn_decode_matches_fp32_softmax(ctx, heads):
