@@ -121,33 +121,6 @@ __device__ __forceinline__ LaneCodes<K> shfl_next_lane(const LaneCodes<K> &c, in
     return o;
 }
 
-// Slice t (= ks*2 + ms) of a lane: K bytes read as a little-endian integer, i.e. 8K stream bits
-// with the first bit as MSB.
-template <int K>
-__device__ __forceinline__ uint32_t lane_slice(const LaneCodes<K> &c, int t) {
-    if constexpr (K == 2) {
-        return (t & 1) ? (c.w[t >> 1] >> 16) : (c.w[t >> 1] & 0xFFFFu);
-    } else if constexpr (K == 3) {
-        switch (t) {
-            case 0: return c.w[0] & 0xFFFFFFu;
-            case 1: return __funnelshift_r(c.w[0], c.w[1], 24) & 0xFFFFFFu;
-            case 2: return __funnelshift_r(c.w[1], c.w[2], 16) & 0xFFFFFFu;
-            default: return c.w[2] >> 8;
-        }
-    } else {
-        return c.w[t];
-    }
-}
-
-// The four 16-bit states of (lane, tile t): windows at bit offsets 0, 2K, 4K, 6K of own-slice || next-slice.
-// Only the low 16 bits of each returned value are meaningful.
-template <int K>
-__device__ __forceinline__ void lane_states(uint32_t own, uint32_t next, uint32_t (&st)[4]) {
-    uint64_t win = ((uint64_t)own << (8 * K)) | next;
-#pragma unroll
-    for (int q = 0; q < 4; q++) st[q] = (uint32_t)(win >> (16 * K - 16 - 2 * K * q));
-}
-
 // The four states of tile tt (= ks*2 + ms) of a lane, from the lane's own words and those of lane+1.
 // Only the low 16 bits of each st[q] are meaningful (the hash ignores the rest), which saves the
 // masks and, for the state that already sits in the low half of a word, the shift.  Shifts are
