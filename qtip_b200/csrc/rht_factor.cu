@@ -20,6 +20,10 @@
 // (two wavefronts per mma) and the mma.sync rate together; few rows by the chain load, barrier, product, exchange, store.
 // fp16 rows without statistics and conversions (HALVES): 11008 x 1000 rows 55 -> 45, x 120 10.3 -> 9.3, x 1 6.4 -> 4.6;
 // 28672 x 1000 with signs 98 -> 67; 14336 x 1000 43 -> 30.
+// They are bound by instruction issue at few resident warps (20 000 warp instructions per row of 11008, a quarter of them in the last pass at
+// two values per thread).  Up to eight values per thread there, and a multiply-add instead of two predicated adds per shuffle: fp16 rows,
+// signs after the transform, 11008 x 1000 39.8 -> 33.6, x 120 8.4 -> 7.2, x 1 4.5 -> 3.2; 14336 x 1000 40.2 -> 27.9; 28672 x 1000
+// 88.6 -> 59.7, x 120 12.4 -> 8.6; 53248 x 1000 270 -> 224.  (A variant of 64 registers with more resident warps spilled: slower.)
 #include <algorithm>
 
 #include "rht.cuh"
@@ -52,7 +56,7 @@ struct ClusterShape {
 
 // Walsh-Hadamard stages over the columns a warp's accumulator holds: bit 0 is the register pair, bits 1-2 the lane's
 // position in its group of four, the others the n-tile.
-template <int NTL>
+template <int NTL, bool FMA>
 __device__ __forceinline__ void fwht_fragment(float (&acc)[NTL][4], int lane) {
 #pragma unroll
     for (int nt = 0; nt < NTL; nt++)
@@ -63,14 +67,17 @@ __device__ __forceinline__ void fwht_fragment(float (&acc)[NTL][4], int lane) {
             acc[nt][h + 1] = x - y;
         }
 #pragma unroll
-    for (int bit = 1; bit < 4; bit <<= 1)
+    for (int bit = 1; bit < 4; bit <<= 1) {
+        const float mine = (lane & bit) ? -1.f : 1.f;        // FMA: o +- x as one multiply-add (the product is exact), for a register
 #pragma unroll
         for (int nt = 0; nt < NTL; nt++)
 #pragma unroll
             for (int h = 0; h < 4; h++) {
                 const float o = __shfl_xor_sync(kFullMask, acc[nt][h], bit);
-                acc[nt][h] = (lane & bit) ? o - acc[nt][h] : acc[nt][h] + o;
+                if constexpr (FMA) acc[nt][h] = fmaf(acc[nt][h], mine, o);
+                else acc[nt][h] = (lane & bit) ? o - acc[nt][h] : acc[nt][h] + o;
             }
+    }
 #pragma unroll
     for (int s = 1; s < NTL; s <<= 1)
 #pragma unroll
@@ -84,20 +91,55 @@ __device__ __forceinline__ void fwht_fragment(float (&acc)[NTL][4], int lane) {
                 }
 }
 
-// butterflies over the register index of E column pairs
-template <int E>
-__device__ __forceinline__ void pair_butterflies(float (&v)[E][2]) {
+// butterflies over the register index of E groups of W columns
+template <int E, int W>
+__device__ __forceinline__ void butterflies(float (&v)[E][W]) {
 #pragma unroll
     for (int s = 1; s < E; s <<= 1)
 #pragma unroll
         for (int k = 0; k < E; k++)
             if (!(k & s))
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
+                for (int h = 0; h < W; h++) {
                     const float x = v[k][h], y = v[k | s][h];
                     v[k][h] = x + y;
                     v[k | s][h] = x - y;
                 }
+}
+// W = 2, 4 or 8 consecutive values, W values aligned
+template <int W>
+__device__ __forceinline__ void load_row(const float *p, float (&v)[W]) {
+    if constexpr (W == 2) {
+        const float2 q = __ldg(reinterpret_cast<const float2 *>(p));
+        v[0] = q.x; v[1] = q.y;
+    } else {
+#pragma unroll
+        for (int c = 0; c < W; c += 4) {
+            const float4 q = __ldg(reinterpret_cast<const float4 *>(p + c));
+            v[c] = q.x; v[c + 1] = q.y; v[c + 2] = q.z; v[c + 3] = q.w;
+        }
+    }
+}
+template <int W>
+__device__ __forceinline__ void store_row(const RhtArgs &a, size_t e, const float (&v)[W]) {
+    if (a.out_dtype == QTIP_F16) {
+        uint32_t h[W / 2];
+#pragma unroll
+        for (int c = 0; c < W; c += 2) {
+            const __half2 q = __floats2half2_rn(v[c], v[c + 1]);
+            h[c / 2] = *reinterpret_cast<const uint32_t *>(&q);
+        }
+        __half *o = static_cast<__half *>(a.out) + e;
+        if constexpr (W == 8) *reinterpret_cast<uint4 *>(o) = make_uint4(h[0], h[1], h[2], h[3]);
+        else if constexpr (W == 4) *reinterpret_cast<uint2 *>(o) = make_uint2(h[0], h[1]);
+        else *reinterpret_cast<uint32_t *>(o) = h[0];
+    } else {
+        float *o = static_cast<float *>(a.out) + e;
+        if constexpr (W == 2) *reinterpret_cast<float2 *>(o) = make_float2(v[0], v[1]);
+        else
+#pragma unroll
+            for (int c = 0; c < W; c += 4) *reinterpret_cast<float4 *>(o + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+    }
 }
 __device__ __forceinline__ void store_pair(const RhtArgs &a, size_t e, float y0, float y1) {
     if (a.out_dtype == QTIP_F16) *reinterpret_cast<__half2 *>(static_cast<__half *>(a.out) + e) = __floats2half2_rn(y0, y1);
@@ -252,32 +294,43 @@ __device__ __forceinline__ void factor_product_bits(float (&acc)[NTL][4], const 
     }
 }
 
-// The stages above the fragment's, scale, sign and store: a thread owns columns lo, lo + 1 and their 2^R partners.
-template <int R>
+// The stages above the fragment's, scale, sign and store: a thread owns columns lo .. lo + W - 1 and their 2^R partners.  WIDE: up to
+// eight columns with partners too (14336 x 1000 rows 40 -> 28 us); the general variant's registers are full (wider there: 2 to 4 % slower).
+template <int R, bool WIDE>
 __device__ __forceinline__ void row_finish(const RhtArgs &a, const float *obuf, int ostride, int cw_log, int rows_here, size_t sign_at,
                                            size_t out_at, float inv) {
-    constexpr int E = 1 << R;
-    const int pairs_log = cw_log - 1;
-    for (int it = threadIdx.x; it < (rows_here << pairs_log); it += blockDim.x) {
-        const int i = it >> pairs_log, lo = (it & ((1 << pairs_log) - 1)) * 2;
+    constexpr int E = 1 << R, W_log = R <= 1 ? 3 : WIDE && R <= 3 ? 2 : 1, W = 1 << W_log;
+    const int items_log = cw_log - W_log;
+    for (int it = threadIdx.x; it < (rows_here << items_log); it += blockDim.x) {
+        const int i = it >> items_log, lo = (it & ((1 << items_log) - 1)) * W;
         const float *src = obuf + i * ostride + lo;
         const size_t e0 = ((size_t)i << a.p) + lo;
-        float v[E][2];
+        float v[E][W];
 #pragma unroll
-        for (int k = 0; k < E; k++) {
-            const float2 q = *reinterpret_cast<const float2 *>(src + (k << cw_log));
-            v[k][0] = q.x; v[k][1] = q.y;
-        }
-        pair_butterflies<E>(v);
+        for (int k = 0; k < E; k++)
+#pragma unroll
+            for (int c = 0; c < W; c += 4) {
+                if constexpr (W == 2) {
+                    const float2 q = *reinterpret_cast<const float2 *>(src + (k << cw_log));
+                    v[k][0] = q.x; v[k][1] = q.y;
+                } else {
+                    const float4 q = *reinterpret_cast<const float4 *>(src + (k << cw_log) + c);
+                    v[k][c] = q.x; v[k][c + 1] = q.y; v[k][c + 2] = q.z; v[k][c + 3] = q.w;
+                }
+            }
+        butterflies<E, W>(v);
 #pragma unroll
         for (int k = 0; k < E; k++) {
             const size_t e = e0 + ((size_t)k << cw_log);
-            float y0 = v[k][0] * inv * a.scale, y1 = v[k][1] * inv * a.scale;
+#pragma unroll
+            for (int c = 0; c < W; c++) v[k][c] = v[k][c] * inv * a.scale;
             if (a.sign_out) {
-                const float2 s = *reinterpret_cast<const float2 *>(a.sign_out + sign_at + e);
-                y0 *= s.x; y1 *= s.y;
+                float s[W];
+                load_row<W>(a.sign_out + sign_at + e, s);
+#pragma unroll
+                for (int c = 0; c < W; c++) v[k][c] *= s[c];
             }
-            store_pair(a, out_at + e, y0, y1);
+            store_row<W>(a, out_at + e, v[k]);
         }
     }
 }
@@ -448,7 +501,7 @@ __global__ void __launch_bounds__(kRowMaxThreads) rht_row_kernel(const RhtArgs a
         for (int q = 0; q < TPW; q++) {
             const int task = warp + q * nwarps, tile = task >> chunks_log, c0 = (task & ((1 << chunks_log) - 1)) << cw_log;
             if (tile >= mt_here) continue;     // uniform over the warp
-            fwht_fragment<NTL>(acc[q], lane);
+            fwht_fragment<NTL, HALVES>(acc[q], lane);
             float *o = obuf + (tile * 16 + g) * stride + c0 + 2 * t;
 #pragma unroll
             for (int nt = 0; nt < NTL; nt++) {
@@ -459,12 +512,12 @@ __global__ void __launch_bounds__(kRowMaxThreads) rht_row_kernel(const RhtArgs a
         __syncthreads();
         const size_t first = (size_t)m0 << a.p, s_at = sign_off + first, o_at = (size_t)row * n + first;
         switch (chunks_log) {
-            case 0: row_finish<0>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
-            case 1: row_finish<1>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
-            case 2: row_finish<2>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
-            case 3: row_finish<3>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
-            case 4: row_finish<4>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
-            default: row_finish<5>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
+            case 0: row_finish<0, HALVES>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
+            case 1: row_finish<1, HALVES>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
+            case 2: row_finish<2, HALVES>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
+            case 3: row_finish<3, HALVES>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
+            case 4: row_finish<4, HALVES>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
+            default: row_finish<5, HALVES>(a, obuf, stride, cw_log, rows_here, s_at, o_at, inv); break;
         }
     }
 }
@@ -500,7 +553,7 @@ __device__ __forceinline__ void cluster_finish(const RhtArgs &a, uint32_t obuf, 
             const float2 q = peer_load2(peer_smem(obuf + (uint32_t)(i * ostride + lo + ((k & ((1 << lb) - 1)) << cw_log)) * 4u, k >> lb));
             v[k][0] = q.x; v[k][1] = q.y;
         }
-        pair_butterflies<E>(v);
+        butterflies<E, 2>(v);
         if (a.sign_out && it != first) signs(it);
 #pragma unroll
         for (int k = 0; k < E; k++) {
@@ -593,7 +646,7 @@ __global__ void __launch_bounds__(kClusterThreads, 2) rht_cluster_kernel(const R
         if (tile >= S.mt) continue;              // uniform over the warp
         float acc[NTL][4] = {};
         factor_product_bits<NTL>(acc, bits, wpr, kfac, a.transpose, tile * 16, b0p + c0 + g, S.kt, k2n, stride, plane, remainder);
-        fwht_fragment<NTL>(acc, lane);
+        fwht_fragment<NTL, false>(acc, lane);
         float *o = obuf + (tile * 16 + g) * stride + c0 + 2 * t;
 #pragma unroll
         for (int nt = 0; nt < NTL; nt++) {

@@ -40,7 +40,8 @@ def test_decode_hyb_golden(golden, K, shape):
 
 
 @pytest.mark.parametrize("K", [2, 3, 4])
-@pytest.mark.parametrize("m,n", [(256, 256), (4096, 4096), (4096, 11008), (11008, 4096)])
+@pytest.mark.parametrize("m,n", [(256, 256), (4096, 4096), (4096, 11008), (11008, 4096),
+                                 (2048, 2048), (2080, 2048), (131104, 32), (32, 160000)])     # both sides of the small kernel; steps over rows
 def test_decode_hyb_vs_oracle(K, m, n):
     lay = synth.make_layer(m, n, K, seed=2000 + K)
     W = ops.decode_hyb(dev(lay["codes"]), dev(lay["tlut"]), K, m, n)
@@ -424,6 +425,17 @@ def test_rht_factor_rows(n, rows, kind):
         got = ops.rht(x, sign_in=su, sign_out=sv, hadk_bits=bits, kfac=k, transpose=transpose, scale=1 / n**0.5, out_dtype=torch.float32)
         err = (got.double() - want).norm(dim=1) / want.norm(dim=1)
         assert float(err.max()) < 1e-6
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1376, 11008, 13824, 7168, 14336, 28672, 24576])
+def test_rht_factor_fp16_results(n):
+    """Every width of the stores (rows of the view of 8 to 2048 columns), with and without signs: the fp32 results rounded once."""
+    bits, k = ops.pack_hadk(ops.get_hadK(n)[0].to(DEV)), ops.had_factor(n)
+    x, sv = torch.randn(200, n, device=DEV).half(), torch.randn(n, device=DEV)
+    for sign in (None, sv):
+        y = [ops.rht(x, sign_out=sign, hadk_bits=bits, kfac=k, scale=1 / n**0.5, out_dtype=t) for t in (torch.float16, torch.float32)]
+        assert torch.equal(y[0], y[1].half())
 
 
 @pytest.mark.parametrize("n", [1024, 2048, 4096, 8192, 16384, 32768, 65536])
