@@ -151,6 +151,15 @@ int qtip_decompress_gemm(float *out, const void *codes, const void *x, const voi
 int qtip_decompress_gemm_plain(float *out, const void *codes, const void *x, int code, int K, int m, int n, int bs,
                                unsigned *status, void *stream);
 
+/* The same product for any number of rows, out (bs, m) fp16 (fp32 accumulation, rounded once): what the dense branch's fp16
+ * matmul returns (lib/codebook/bitshift.py:454-463, 476-489), for prompts of more than 128 rows.  code: QTIP_CODE_HYB (kernel layout,
+ * tlut required) or a compute code (plain layout, tlut ignored).  Same shape and status rules. */
+int qtip_decompress_gemm_f16(void *out, const void *codes, const void *x, const void *tlut, int code, int K, int m, int n, int bs,
+                             unsigned *status, void *stream);
+/* 1 if that is estimated to be faster on this device than qtip_decode_hyb / qtip_decode_plain and a dense product, else 0 (also for shapes
+ * it does not take). */
+int qtip_decompress_gemm_f16_faster(int code, int m, int n, int bs);
+
 /* One to four QTIP linears of the same shape in ONE launch (e.g. q/k/v, or gate/up), each optionally with
  * its input-side and output-side transforms fused into the matvec kernel, i.e. the whole of
  * BitshiftLinear.forward (lib/codebook/bitshift.py:428-472) for a decode step in one kernel:

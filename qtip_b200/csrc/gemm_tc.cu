@@ -34,6 +34,7 @@
 // still runs to its end, frees its tensor memory and returns (with meaningless results).
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -113,10 +114,10 @@ __device__ __forceinline__ void mbar_wait_bounded(uint32_t bar, uint32_t parity)
 __device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Box of x at column c (a multiple of 64), row 0: rows beyond the tensor are filled with zeros
-__device__ __forceinline__ void copy_x_tile(uint32_t dst, const CUtensorMap *map, int c, uint32_t bar) {
+// Box of x at column c (a multiple of 64) and row r: rows beyond the tensor are filled with zeros
+__device__ __forceinline__ void copy_x_tile(uint32_t dst, const CUtensorMap *map, int c, int r, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(dst), "l"(map), "r"(c), "r"(0), "r"(bar) : "memory");
+                 ::"r"(dst), "l"(map), "r"(c), "r"(r), "r"(bar) : "memory");
 }
 
 // Shared-memory matrix descriptor: K-major, 128-byte swizzle, rows of 128 bytes, 8-row groups 1024 bytes apart.
@@ -229,6 +230,64 @@ __device__ __forceinline__ uint32_t pair_1mad(uint32_t s0, uint32_t s1, uint32_t
     return __byte_perm(w0, w1, 0x5410);
 }
 
+// A decode warp's codes of a step: two blocks (HYB), or rows of 2 x 2 tiles each (V = 1).
+template <int K>
+struct StepCodes {
+    LaneCodes<K> blk[2];
+    PlainRow<K> rows[2][2];
+};
+template <int K, int CODE>
+__device__ __forceinline__ void load_step(StepCodes<K> &c, const uint8_t *src, const uint16_t *prow) {
+    if constexpr (CODE == QTIP_CODE_HYB) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) c.blk[h] = load_lane_codes<K>(src + h * (128 * K));
+    } else {
+#pragma unroll
+        for (int h = 0; h < 4; h++) c.rows[h >> 1][h & 1] = load_plain_row<K>(prow + h * (16 * K));
+    }
+}
+// Block h as the words that its tensor-memory stores take (HYB: 8 per 16 rows; V = 1: a row per lane)
+template <int K, int CODE>
+__device__ __forceinline__ void decode_half(const StepCodes<K> &c, int h, uint32_t lut_lane, int lane, uint32_t (&wv)[16]) {
+    if constexpr (CODE == QTIP_CODE_HYB) {
+        LaneCodes<K> nxt = {};
+#pragma unroll
+        for (int i = 0; i < K; i++) nxt.w[i] = __shfl_sync(kFullMask, c.blk[h].w[i], lane + 1);
+#pragma unroll
+        for (int tt = 0; tt < 4; tt++) {
+            const int ks = tt >> 1, ms = tt & 1;
+            uint32_t st[4];
+            tile_states<K>(c.blk[h], nxt, tt, st);
+#pragma unroll
+            for (int q = 0; q < 4; q++)       // q = 2c + d: column half, row half of the 16x16 tile
+                wv[8 * ms + 4 * ks + q] = hyb_lookup(st[q], lut_lane);
+        }
+    } else {
+#pragma unroll
+        for (int ks = 0; ks < 2; ks++) {
+            const uint32_t next = __shfl_sync(kFullMask, c.rows[h][ks].a, lane + 2);      // row 15 -> row 0: tail-biting
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const uint32_t s0 = plain_state<K>(c.rows[h][ks], next, 2 * j), s1 = plain_state<K>(c.rows[h][ks], next, 2 * j + 1);
+                wv[8 * ks + j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1) : pair_1mad(s0, s1, lut_lane);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i++) asm volatile("" : "+r"(wv[i]));
+}
+// lane-private copies of the table: entry e = sign << 9 | index, copy l at byte e*128 + l*4; the sign bit of
+// the hash flips the first weight of the pair, so it is folded into the table (no per-state sign op)
+// 1MAD: the weight of every byte sum (decode_1mad's own arithmetic) in the same form, 1021 entries used
+template <int CODE>
+__device__ __forceinline__ void build_table(uint32_t *lut, const uint32_t *__restrict__ tlut) {
+    for (int i = threadIdx.x; CODE != QTIP_CODE_3INST && i < 1024 * 8; i += blockDim.x) {
+        const uint32_t e = CODE == QTIP_CODE_1MAD ? (uint32_t)__half_as_ushort(__float2half_rn(__fdiv_rn((float)((i >> 3) - 510), 147.800537109375f)))
+                                                  : __ldg(tlut + ((i >> 3) & 511)) ^ ((uint32_t)(i >> 12) << 15);
+        reinterpret_cast<uint4 *>(lut)[i] = make_uint4(e, e, e, e);
+    }
+}
+
 template <int K, int CODE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     decompress_gemm_kernel(float *__restrict__ out, const uint8_t *__restrict__ codes, const __grid_constant__ CUtensorMap xmap,
@@ -270,21 +329,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    // lane-private copies of the table: entry e = sign << 9 | index, copy l at byte e*128 + l*4; the sign bit of
-    // the hash flips the first weight of the pair, so it is folded into the table (no per-state sign op)
-    // 1MAD: the weight of every byte sum (decode_1mad's own arithmetic) in the same form, 1021 entries used
-    if constexpr (CODE == QTIP_CODE_1MAD) {
-        for (int i = threadIdx.x; i < 1024 * 8; i += kGemmThreads) {
-            const uint32_t e = __half_as_ushort(__float2half_rn(__fdiv_rn((float)((i >> 3) - 510), 147.800537109375f)));
-            reinterpret_cast<uint4 *>(lut)[i] = make_uint4(e, e, e, e);
-        }
-    }
-    if constexpr (kHyb) {
-        for (int i = threadIdx.x; i < 1024 * 8; i += kGemmThreads) {
-            const uint32_t e = __ldg(tlut + ((i >> 3) & 511)) ^ ((uint32_t)(i >> 12) << 15);
-            reinterpret_cast<uint4 *>(lut)[i] = make_uint4(e, e, e, e);
-        }
-    }
+    build_table<CODE>(lut, tlut);
     const int nb = n >> 5;                                  // 32-column blocks per row block
     const int r0 = blockIdx.x * kRows;                      // first output row of this CTA
     // 64-column tiles of this CTA: split over the CTAs of the cluster, not necessarily evenly; the last step may have one tile
@@ -301,22 +346,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                            ((size_t)(r0 / 16 + 2 * rb + (lane & 1)) * (n >> 4) + (size_t)(c0 / 16 + 4 * half + 8 * group)) * (16 * K) +
                            (lane >> 1) * K;
     // codes of the current step and of the one after it
-    struct StepCodes {
-        LaneCodes<K> blk[2];
-        PlainRow<K> rows[2][2];
-    };
-    StepCodes now = {}, ahead = {};
-    auto load_codes = [&](StepCodes &c, int step) {
+    StepCodes<K> now = {}, ahead = {};
+    auto load_codes = [&](StepCodes<K> &c, int step) {
         if (2 * step + half >= ntiles) return;
-        if constexpr (kHyb) {
-#pragma unroll
-            for (int h = 0; h < 2; h++) c.blk[h] = load_lane_codes<K>(src + h * kBlockBytes);
-            src += kGroups * 4 * kBlockBytes;
-        } else {
-#pragma unroll
-            for (int h = 0; h < 4; h++) c.rows[h >> 1][h & 1] = load_plain_row<K>(prow + h * (16 * K));
-            prow += kGroups * (kStageCols / 16) * (16 * K);
-        }
+        load_step<K, CODE>(c, src, prow);
+        src += kGroups * 4 * kBlockBytes;
+        prow += kGroups * (kStageCols / 16) * (16 * K);
     };
     if (warp < kDecodeWarps) {      // weights: before the wait for the launch that makes x
         load_codes(now, group);
@@ -340,32 +375,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 uint32_t wv[16];
-                if constexpr (kHyb) {
-                    LaneCodes<K> nxt = {};
-#pragma unroll
-                    for (int i = 0; i < K; i++) nxt.w[i] = __shfl_sync(kFullMask, now.blk[h].w[i], lane + 1);
-#pragma unroll
-                    for (int tt = 0; tt < 4; tt++) {
-                        const int ks = tt >> 1, ms = tt & 1;
-                        uint32_t st[4];
-                        tile_states<K>(now.blk[h], nxt, tt, st);
-#pragma unroll
-                        for (int q = 0; q < 4; q++)       // q = 2c + d: column half, row half of the 16x16 tile
-                            wv[8 * ms + 4 * ks + q] = hyb_lookup(st[q], lut_lane);
-                    }
-                } else {
-#pragma unroll
-                    for (int ks = 0; ks < 2; ks++) {
-                        const uint32_t next = __shfl_sync(kFullMask, now.rows[h][ks].a, lane + 2);      // row 15 -> row 0: tail-biting
-#pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            const uint32_t s0 = plain_state<K>(now.rows[h][ks], next, 2 * j), s1 = plain_state<K>(now.rows[h][ks], next, 2 * j + 1);
-                            wv[8 * ks + j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1) : pair_1mad(s0, s1, lut_lane);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < 16; i++) asm volatile("" : "+r"(wv[i]));
+                decode_half<K, CODE>(now, h, lut_lane, lane, wv);
                 if (h == 0) {
                     // the first block is decoded before the stage is waited for; its last use was kStages steps ago (or none)
                     if (step >= kStages) mbar_wait(smem_addr(&ctl->empty[s]), parity, abort_flag, status, 1u);
@@ -421,8 +431,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             const uint32_t bar = smem_addr(&ctl->xfull[xs]), dst = b_base + xs * x_stage_bytes;
             const int c = c0 + step * kStageCols, tiles = min(2, ntiles - 2 * step);
             mbar_expect(bar, (uint32_t)(tiles * tile_bytes));
-            copy_x_tile(dst, &xmap, c, bar);
-            if (tiles > 1) copy_x_tile(dst + tile_bytes, &xmap, c + kTileCols, bar);
+            copy_x_tile(dst, &xmap, c, 0, bar);
+            if (tiles > 1) copy_x_tile(dst + tile_bytes, &xmap, c + kTileCols, 0, bar);
             if (++xs == xstages) { xs = 0; xround++; }
         }
         // nothing may be on its way when the CTA ends, whatever the other roles did: the last copy of each stage, with a limit
@@ -482,6 +492,215 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             out[(size_t)(i / kRows) * m + r0 + (i & (kRows - 1))] = t;
         }
         cluster_barrier();                                   // the parts are read
+    }
+}
+
+__device__ __forceinline__ uint32_t b_tile(uint32_t base, int stage, int bytes) { return base + (uint32_t)(stage * bytes); }
+
+// ---- more than 128 rows --------------------------------------------------------------------------------------------------
+// The same roles over tiles of 128 output rows x up to 256 batch rows, fp16 results: a CTA per SM walks over the tiles (all row ranges of
+// one batch group before the next), four more warps read the accumulator of a finished tile and write it.  Four stages of weights
+// (tensor memory: 256 columns beside the accumulator's 256); x in a ring of single 64-column tiles.  Every batch group decodes the
+// matrix again: a tile's 16 columns take the MMA about 100 + 0.15 N cycles and the decode warps 100, so up to 256 rows share a decode
+// at the price of one.  Measured against decode_hyb / decode_plain and
+// a library product, HYB K = 2 unless stated (microseconds): 11008 x 4096 129 rows 44.7 -> 26.6, 512 rows 59.8 -> 50.7, 1000 rows
+// 86.5 -> 81.1; 28672 x 8192 256 rows 214 -> 107, 1000 rows 450 -> 400; K = 4 4096 x 4096 1000 rows 37.8 -> 33.1; 1MAD K = 4 8192 x 8192
+// 256 rows 116 -> 56.  Bound: the MMAs (half of the tensor pipe's cycles are busy: a tensor-memory A operand takes twice the ideal interval),
+// then the lookups (left out: 80.3 -> 69.6) and the copies of x (74.2); hence no sleeping between the control threads' polls here.
+constexpr int kWideN = 256, kWideStages = 4, kWideXMax = 8, kEpilogueWarp = kCopyWarp + 1;
+constexpr int kWideThreads = (kEpilogueWarp + 4) * 32;
+
+struct WideCtrl {
+    unsigned long long full[kWideStages], empty[kWideStages];
+    unsigned long long xfull[kWideXMax], xempty[kWideXMax];
+    unsigned long long done, drained;      // the accumulator of a tile: complete; read
+    uint32_t tmem_base;
+    int abort_flag;
+    int committed;                         // tiles whose last commit was issued
+};
+__host__ __device__ __forceinline__ int wide_x_stages(int npad) {
+    const int fit = kXRingBytes / (npad * kTileCols * 2);
+    return fit < kWideXMax ? fit : kWideXMax;
+}
+
+template <int K, int CODE>
+__global__ void __launch_bounds__(kWideThreads, 1)
+    decompress_gemm_wide_kernel(__half *__restrict__ out, const uint8_t *__restrict__ codes, const __grid_constant__ CUtensorMap xmap,
+                                const uint32_t *__restrict__ tlut, int m, int n, int bs, int npad, int tiles, unsigned *__restrict__ status) {
+    constexpr int kBlockBytes = 128 * K;
+    constexpr bool kHyb = CODE == QTIP_CODE_HYB;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_addr(smem_raw);
+    const uint32_t base = (raw + 1023u) & ~1023u;
+    uint8_t *smem = smem_raw + (base - raw);
+    const int xstages = wide_x_stages(npad), xtile_bytes = npad * kTileCols * 2;
+    uint32_t *lut = reinterpret_cast<uint32_t *>(smem + xstages * xtile_bytes);
+    WideCtrl *ctl = reinterpret_cast<WideCtrl *>(smem + xstages * xtile_bytes + kLut512Bytes);
+    volatile int *abort_flag = &ctl->abort_flag;
+    const int warp = __shfl_sync(kFullMask, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    constexpr int kTmemD = kWideStages * kAStageCols, kTmemCols = 512;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kWideStages; s++) {
+            mbar_init(smem_addr(&ctl->full[s]), 8);
+            mbar_init(smem_addr(&ctl->empty[s]), 1);
+        }
+        for (int s = 0; s < kWideXMax; s++) {
+            mbar_init(smem_addr(&ctl->xfull[s]), 1);
+            mbar_init(smem_addr(&ctl->xempty[s]), 1);
+        }
+        mbar_init(smem_addr(&ctl->done), 1);
+        mbar_init(smem_addr(&ctl->drained), 4);
+        ctl->abort_flag = 0;
+        ctl->committed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&ctl->tmem_base)),
+                     "r"(kTmemCols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    build_table<CODE>(lut, tlut);
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = ctl->tmem_base, tmem_d = tmem + kTmemD;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    const int nb = n >> 5, ntiles = n / kTileCols, nsteps = (ntiles + 1) >> 1, row_tiles = m / kRows;
+    const int mine = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;      // tiles blockIdx.x, + gridDim.x, ...
+    auto tile_at = [&](int i) { return (int)blockIdx.x + i * (int)gridDim.x; };
+
+    if (warp < kDecodeWarps) {
+        // the steps of all tiles in one sequence, which the groups take in turn
+        const int group = warp >> 3, rb = warp & 3, half = (warp >> 2) & 1;
+        const uint32_t lut_lane = smem_addr(lut) + lane * 4;
+        const uint32_t tmem_warp = tmem + ((uint32_t)(32 * rb) << 16) + 32u * half;
+        int li = 0, lj = group;                             // tile and step of the next codes to be requested, and where they lie
+        const uint8_t *src = nullptr;
+        const uint16_t *prow = nullptr;
+        auto seek = [&]() {
+            while (lj >= nsteps) { lj -= nsteps; li++; }
+            const int r0 = __shfl_sync(kFullMask, tile_at(li) % row_tiles * kRows, 0);
+            if constexpr (kHyb) src = codes + ((size_t)(r0 / 32 + rb) * nb + 4 * lj + 2 * half) * kBlockBytes + lane * (4 * K);
+            else prow = reinterpret_cast<const uint16_t *>(codes) +
+                        ((size_t)(r0 / 16 + 2 * rb + (lane & 1)) * (n >> 4) + 8 * lj + 4 * half) * (16 * K) + (lane >> 1) * K;
+        };
+        auto load_codes = [&](StepCodes<K> &c) {
+            if (lj >= nsteps) seek();
+            if (li < mine && 2 * lj + half < ntiles) load_step<K, CODE>(c, src, prow);
+            lj += kGroups;
+            if constexpr (kHyb) src += kGroups * 4 * kBlockBytes;
+            else prow += kGroups * (kStageCols / 16) * (16 * K);
+        };
+        seek();
+        StepCodes<K> now = {}, ahead = {};
+        load_codes(now);
+        load_codes(ahead);
+        const int total = mine * nsteps;
+        for (int step = group; step < total; step += kGroups) {
+            const uint32_t s = step % kWideStages;
+            const uint32_t ast = tmem_warp + s * kAStageCols;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                uint32_t wv[16];
+                decode_half<K, CODE>(now, h, lut_lane, lane, wv);
+                if (h == 0) {
+                    if (step >= kWideStages) mbar_wait(smem_addr(&ctl->empty[s]), (step / kWideStages - 1) & 1, abort_flag, status, 1u);
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    __syncwarp();
+                }
+                if constexpr (kHyb) {
+                    tmem_st_16x128b_x4(ast + 16u * h, wv);
+                    tmem_st_16x128b_x4(ast + 16u * h + (16u << 16), wv + 8);
+                } else tmem_st_32x32b_x16(ast + 16u * h, wv);
+            }
+            now = ahead;
+            load_codes(ahead);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_addr(&ctl->full[s]));
+        }
+    } else if (warp == kMmaWarp && elect_one()) {
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(npad >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
+        int s = 0, round = 0, xs = 0, xround = 0;
+        bool ok = true;
+        for (int i = 0; i < mine && ok; i++) {
+            // the accumulator of the tile before has been read
+            if (i > 0 && !mbar_wait(smem_addr(&ctl->drained), (i - 1) & 1, abort_flag, status, 6u)) break;
+            for (int step = 0; step < nsteps && ok; step++) {
+                ok = mbar_wait(smem_addr(&ctl->full[s]), round & 1, abort_flag, status, 2u);
+                for (int tile = 0; tile < 2 && ok && 2 * step + tile < ntiles; tile++) {
+                    ok = mbar_wait(smem_addr(&ctl->xfull[xs]), xround & 1, abort_flag, status, 4u);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t bdesc = umma_desc(b_tile(base, xs, xtile_bytes));
+#pragma unroll
+                    for (int kk = 0; kk < 4; kk++)
+                        umma_f16(tmem_d, tmem + (uint32_t)(s * kAStageCols + tile * 32 + kk * 8), bdesc + (uint64_t)(kk * 2), idesc,
+                                 (step | tile | kk) != 0);
+                    umma_commit(smem_addr(&ctl->xempty[xs]));
+                    if (++xs == xstages) { xs = 0; xround++; }
+                }
+                umma_commit(smem_addr(&ctl->empty[s]));
+                if (++s == kWideStages) { s = 0; round++; }
+            }
+            umma_commit(smem_addr(&ctl->done));
+            ctl->committed = i + 1;
+        }
+    } else if (warp == kCopyWarp && elect_one()) {
+        const int total = mine * ntiles;
+        int xs = 0, xround = 0, k = 0, i = 0, t = 0;
+        for (; k < total; k++) {
+            if (xround > 0 && !mbar_wait(smem_addr(&ctl->xempty[xs]), (xround - 1) & 1, abort_flag, status, 5u)) break;
+            const uint32_t bar = smem_addr(&ctl->xfull[xs]);
+            mbar_expect(bar, (uint32_t)xtile_bytes);
+            copy_x_tile(b_tile(base, xs, xtile_bytes), &xmap, t * kTileCols, tile_at(i) / row_tiles * npad, bar);
+            if (++t == ntiles) { t = 0; i++; }
+            if (++xs == xstages) { xs = 0; xround++; }
+        }
+        // nothing may be on its way when the CTA ends: the last copy of each stage, with a limit
+        for (int j = k - 1; j >= 0 && j >= k - xstages; j--) mbar_wait_bounded(smem_addr(&ctl->xfull[j % xstages]), (j / xstages) & 1);
+    } else if (warp >= kEpilogueWarp) {
+        const int sub = warp & 3;                           // the tensor-memory lanes that a warp reaches: 32 sub ..
+        const int row = sub * 32 + (kHyb ? lane : 16 * (lane & 1) + (lane >> 1));
+        for (int i = 0; i < mine; i++) {
+            const int tile = tile_at(i), r0 = tile % row_tiles * kRows, b0 = tile / row_tiles * npad, count = min(npad, bs - b0);
+            if (!mbar_wait<kCopySleepNs>(smem_addr(&ctl->done), i & 1, abort_flag, status, 3u)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            __syncwarp();
+            __half *dst = out + (size_t)b0 * m + r0 + row;
+            for (int col = 0; col < npad; col += 16) {
+                uint32_t r[16];
+                asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+                               "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                             : "r"(tmem_d + ((uint32_t)(sub * 32) << 16) + (uint32_t)col)
+                             : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (col + 16 >= npad) {                     // the last words are in registers: the next tile may begin
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_addr(&ctl->drained));
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    if (col + j < count) dst[(size_t)(col + j) * m] = __float2half_rn(__uint_as_float(r[j]));
+            }
+        }
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        // tensor memory is released only after the last commit has arrived, on the abort path too (see above)
+        if (lane == 0 && ctl->committed > 0) mbar_wait_bounded(smem_addr(&ctl->done), (ctl->committed - 1) & 1);
+        __syncwarp();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
     }
 }
 
@@ -556,6 +775,65 @@ int column_splits(int m, int n) {
     return s;
 }
 
+// Time of a wide product on the busiest SM in cycles per 16 columns and wave of tiles: the MMA, or the decode warps.  (From timings: 11008 x 4096 129 rows
+// 26.6 us, 256 rows 32.3, 1000 rows in five groups 81.1, in four 86; 1MAD 8192 x 8192 129 rows 54.)
+double wide_cycles(int code, int npad) { return std::max(100 + 0.5 * npad, code == QTIP_CODE_HYB ? 140.0 : 188.0); }
+// Batch groups: as many as give the least time
+int wide_groups(int code, int m, int bs, double *cost = nullptr) {
+    const long row_tiles = m / kRows, sms = sm_count();
+    int best = 0;
+    double least = 0;
+    for (int g = (bs + kWideN - 1) / kWideN; g <= (bs + 127) / 128; g++) {
+        const int npad = ((bs + g - 1) / g + 15) & ~15;
+        const double waves = (double)((row_tiles * ((bs + npad - 1) / npad) + sms - 1) / sms), t = waves * wide_cycles(code, npad);
+        if (best == 0 || t < least) { best = g; least = t; }
+    }
+    if (cost) *cost = least;
+    return best;
+}
+
+template <int K, int CODE>
+int launch_gemm_wide(__half *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, unsigned *status,
+                     cudaStream_t s) {
+    static bool attr_set[64] = {};
+    static std::mutex attr_mutex;
+    int dev = 0;
+    QTIP_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return QTIP_ERR_BAD_ARG;
+    {
+        std::lock_guard<std::mutex> lock(attr_mutex);
+        if (!attr_set[dev]) {
+            QTIP_CUDA_TRY(cudaFuncSetAttribute(decompress_gemm_wide_kernel<K, CODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+            attr_set[dev] = true;
+        }
+    }
+    const int g = wide_groups(CODE, m, bs), npad = ((bs + g - 1) / g + 15) & ~15, groups = (bs + npad - 1) / npad;
+    const long tiles = (long)(m / kRows) * groups;
+    if (tiles >= 1L << 30) return QTIP_ERR_BAD_SHAPE;
+    static_assert(sizeof(WideCtrl) <= 256, "control block");
+    CUtensorMap xmap;
+    const int st = encode_x(&xmap, x, n, bs, npad);
+    if (st != QTIP_OK) return st;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(tiles < sm_count() ? tiles : sm_count()));
+    cfg.blockDim = dim3(kWideThreads);
+    cfg.dynamicSmemBytes = 1024 + wide_x_stages(npad) * npad * kTileCols * 2 + kLut512Bytes + 256;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decompress_gemm_wide_kernel<K, CODE>, out, codes, xmap, tlut, m, n, bs, npad, (int)tiles, status));
+    return check_launch();
+}
+template <int CODE>
+int launch_gemm_wide_k(__half *out, const uint8_t *c, const __half *x, const uint32_t *t, int K, int m, int n, int bs, unsigned *status, cudaStream_t s) {
+    if (K == 2) return launch_gemm_wide<2, CODE>(out, c, x, t, m, n, bs, status, s);
+    if (K == 3) return launch_gemm_wide<3, CODE>(out, c, x, t, m, n, bs, status, s);
+    return launch_gemm_wide<4, CODE>(out, c, x, t, m, n, bs, status, s);
+}
+
 template <int CODE>
 int launch_gemm_k(float *out, const uint8_t *c, const __half *xh, const uint32_t *t, int K, int m, int n, int bs, int npad,
                   int splitk, unsigned *status, cudaStream_t s) {
@@ -599,4 +877,35 @@ extern "C" int qtip_decompress_gemm_plain(float *out, const void *codes, const v
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (code == QTIP_CODE_3INST) return launch_gemm_k<QTIP_CODE_3INST>(out, c, xh, nullptr, K, m, n, bs, npad, splitk, status, s);
     return launch_gemm_k<QTIP_CODE_1MAD>(out, c, xh, nullptr, K, m, n, bs, npad, splitk, status, s);
+}
+
+extern "C" int qtip_decompress_gemm_f16(void *out, const void *codes, const void *x, const void *tlut, int code, int K, int m, int n, int bs,
+                                        unsigned *status, void *stream) {
+    if (!out || !codes || !x || !status || K < 2 || K > 4 || bs < 1) return QTIP_ERR_BAD_ARG;
+    if (code != QTIP_CODE_HYB && code != QTIP_CODE_3INST && code != QTIP_CODE_1MAD) return QTIP_ERR_BAD_ARG;
+    if (code == QTIP_CODE_HYB && !tlut) return QTIP_ERR_BAD_ARG;
+    if (m <= 0 || n <= 0 || (m % kRows) || (n % kTileCols)) return QTIP_ERR_BAD_SHAPE;
+    if ((long)(m >> 5) * (n >> 5) >= (1L << 30)) return QTIP_ERR_BAD_SHAPE;
+    if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, 2) || (tlut && !aligned(tlut, 4)) || !aligned(status, 4)) return QTIP_ERR_ALIGNMENT;
+    auto *o = static_cast<__half *>(out);
+    auto *c = static_cast<const uint8_t *>(codes);
+    auto *xh = static_cast<const __half *>(x);
+    auto *t = static_cast<const uint32_t *>(tlut);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (code == QTIP_CODE_HYB) return launch_gemm_wide_k<QTIP_CODE_HYB>(o, c, xh, t, K, m, n, bs, status, s);
+    if (code == QTIP_CODE_3INST) return launch_gemm_wide_k<QTIP_CODE_3INST>(o, c, xh, nullptr, K, m, n, bs, status, s);
+    return launch_gemm_wide_k<QTIP_CODE_1MAD>(o, c, xh, nullptr, K, m, n, bs, status, s);
+}
+
+// Rule: estimates of both ways in microseconds.  Wide: 6 to start and end, the cycles above at 1.965 GHz.  Dense: 5 for the launches, the
+// decode at its write rate (3.9 TB/s HYB, 2.8 3INST, 1.6 1MAD), the product at the rate of reading the matrix (4.2 TB/s) or 1430 TFLOP/s.
+// It errs by up to 10 %, on either side of the line (4096 x 4096: dense up to 512 rows, 26.2 against 27.0 us; 11008 x 4096: wide up to about 2000).
+extern "C" int qtip_decompress_gemm_f16_faster(int code, int m, int n, int bs) {
+    if (m <= 0 || n <= 0 || bs < 1 || (m % kRows) || (n % kTileCols)) return 0;
+    double cycles;
+    wide_groups(code, m, bs, &cycles);
+    const double bytes = 2.0 * m * n, wide = 6 + cycles * (n / 16) / 1965;
+    const double write = code == QTIP_CODE_HYB ? 3.9e6 : code == QTIP_CODE_3INST ? 2.8e6 : 1.6e6;
+    const double dense = 5 + bytes / write + std::max(bytes / 4.2e6, bytes * bs / 1.43e9);
+    return wide < dense;
 }

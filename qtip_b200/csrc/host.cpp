@@ -166,13 +166,16 @@ at::Tensor linear_forward(const at::Tensor &input, Layer &L, int &launches) {
     // compute codes: the tensor-core kernel decodes eight states per 44-bit window and is the faster one at every batch
     // size it takes; HYB: above 8 rows the matvec's single B fragment is full
     const bool gemm = whole_tiles && bs <= kMaxGemmBatch && (v1 || (L.kernel_layout && bs > kMaxMatvecBatch));
-    const bool dense = !gemm && bs > kMaxMatvecBatch;
+    // long prompts: the tensor-core kernel again where it is the faster way, else decoded once and a dense product
+    const bool wide = whole_tiles && bs > kMaxGemmBatch && (v1 || L.kernel_layout) && reinterpret_cast<uintptr_t>(trellis.data_ptr()) % 16 == 0 &&
+                      qtip_decompress_gemm_f16_faster(L.code, (int)m, (int)n, (int)bs);
+    const bool dense = !gemm && !wide && bs > kMaxMatvecBatch;
 
     // one allocation for both intermediates: the transformed activation (fp16) and, unless the dense product makes its
-    // own, the raw result (fp32)
+    // own, the raw result (fp32; fp16 of a long prompt, as from the dense product)
     const int64_t xh_bytes = (bs * n * 2 + 255) / 256 * 256;
     // (straight from the caching allocator, on the current stream: a tensor around it costs half a microsecond)
-    const c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate(xh_bytes + (dense ? 0 : bs * m * 4));
+    const c10::DataPtr scratch = c10::cuda::CUDACachingAllocator::get()->allocate(xh_bytes + (dense ? 0 : bs * m * (wide ? 2 : 4)));
     char *base = static_cast<char *>(scratch.get());
     void *xh = base;
     float *y = reinterpret_cast<float *>(base + xh_bytes);
@@ -194,6 +197,11 @@ at::Tensor linear_forward(const at::Tensor &input, Layer &L, int &launches) {
         else
             check(qtip_decompress_gemm(y, trellis.data_ptr(), xh, tlut.data_ptr(), L.K, (int)m, (int)n, (int)bs, st, stream),
                   "qtip_decompress_gemm");
+    } else if (wide) {
+        check(qtip_decompress_gemm_f16(y, trellis.data_ptr(), xh, v1 ? nullptr : tlut.data_ptr(), L.code, L.K, (int)m, (int)n, (int)bs,
+                                       static_cast<unsigned *>(gemm_status(dev).data_ptr()), stream),
+              "qtip_decompress_gemm_f16");
+        y_type = QTIP_F16;
     } else if (!dense) {
         at::Tensor ws = L.workspace.defined() ? L.workspace : matvec_workspace(dev, m, n, bs, stream);
         if (L.kernel_layout)

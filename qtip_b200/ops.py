@@ -597,5 +597,25 @@ def decompress_gemm_plain(codes, x, code, K, m, n, out=None):
     return out
 
 
+def decompress_gemm_f16(codes, x, code, K, m, n, tlut=None, out=None):
+    """out (bs, m) fp16 = x (bs, n) fp16 @ decode(codes)^T, any number of rows; HYB (kernel layout, with its table) or a compute code."""
+    _require_cuda(codes, x)
+    code = CODE_IDS.get(code, code)
+    if x.dtype != torch.float16:
+        x = x.to(torch.float16)
+    x = x.reshape(-1, n).contiguous()
+    bs = x.shape[0]
+    if out is None:
+        out = torch.empty(bs, m, dtype=torch.float16, device=x.device)
+    status = _lib.host().gemm_status(x.device.index)
+    with torch.cuda.device(x.device):
+        st = _lib.load().qtip_decompress_gemm_f16(out.data_ptr(), codes.data_ptr(), x.data_ptr(), None if tlut is None else tlut.data_ptr(),
+                                                  code, K, m, n, bs, status.data_ptr(), _stream())
+    _lib.check(st, "qtip_decompress_gemm_f16")
+    global launch_count
+    launch_count += 1
+    return out
+
+
 def gemm_plain_supported(m, n, bs):
     return 1 <= bs <= MAX_GEMM_BATCH and m % 128 == 0 and n % 64 == 0

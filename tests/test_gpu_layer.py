@@ -730,3 +730,24 @@ def test_native_layer_call_from_threads_while_allocations_call_into_python():
     from conftest import ROOT
     r = subprocess.run([sys.executable, "-c", _THREADS], capture_output=True, text=True, cwd=ROOT, timeout=300)
     assert r.returncode == 0 and "threads ok" in r.stdout, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("code,mode,K", [("hyb", "quantlut_sym", 2), ("hyb", "quantlut_sym", 4), ("3inst", "3inst", 3), ("1mad", "1mad", 2)])
+def test_long_prompt_on_the_tensor_core_path(code, mode, K):
+    """More rows than one accumulator holds, where the wide kernel is chosen: the rows of the short-prompt path, whose product stays in
+    fp32 where this one is rounded to fp16 (2^-11 of a value at most)."""
+    from qtip_b200 import _lib
+    m, n, bs = 22016, 1024, 389
+    assert _lib.load().qtip_decompress_gemm_f16_faster(ops.CODE_IDS[code], m, n, bs) == 1
+    lay = synth.make_layer(m, n, K, seed=77 + K, bs=bs, code=code, device=DEV)
+    q = QuantizedLinear(n, m, 16, 16, 16, K, 2 if code == "hyb" else 1, 9, mode).to(DEV)
+    q.trellis.copy_(lay["codes"].view(torch.int16))
+    q.SU.copy_(lay["SU"])
+    q.SV.copy_(lay["SV"])
+    if code == "hyb":
+        q.tlut.data.copy_(lay["tlut"])
+    y, x = q(lay["x"]), lay["x"]
+    want = torch.cat([q(x[i:i + 100]) for i in range(0, bs, 100)])
+    assert y.dtype == torch.float16 and y.shape == (bs, m)
+    assert float((y.double() - want.double()).norm() / want.double().norm()) < 2.0**-11
+    assert ops.gemm_status(DEV) == 0
