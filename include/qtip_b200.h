@@ -35,7 +35,8 @@ enum {
 };
 
 enum { QTIP_CODE_HYB = 0, QTIP_CODE_3INST = 1, QTIP_CODE_1MAD = 2 };
-enum { QTIP_F16 = 0, QTIP_F32 = 1 };
+enum { QTIP_F16 = 0, QTIP_F32 = 1,
+       QTIP_F16_FRAGMENTS = 2 };   /* output of qtip_rht / qtip_rht_fused only: see qtip_matvec_x_fragments */
 
 /* Human-readable text for a status code; never NULL. */
 const char *qtip_status_string(int status);
@@ -131,6 +132,15 @@ size_t qtip_matvec_workspace_bytes(int m, int n, int bs);
  * need separate workspaces. */
 int qtip_decompress_matvec(float *out, const void *codes, const void *x, const void *tlut, int K, int m, int n,
                            int bs, void *workspace, size_t workspace_bytes, void *stream);
+
+/* x in the order in which the matvec's lanes take it ("fragments"): block of 32 columns, row, four threads, four pairs of columns
+ * { 2t, 2t + 8, 2t + 16, 2t + 24 } (+ 1) of thread t.  When a call's rows are too long for shared memory, qtip_decompress_matvec puts x into
+ * that order with a launch of its own; a transform with out_dtype QTIP_F16_FRAGMENTS writes it so at once.
+ * qtip_matvec_x_fragments: 1 if a call of this shape takes x so and the transform can write it, else 0.
+ * qtip_decompress_matvec_fragments: qtip_decompress_matvec on such an x (any shape; bs rows interleaved as written by bs rows' transform). */
+int qtip_matvec_x_fragments(int K, int m, int n, int bs);
+int qtip_decompress_matvec_fragments(float *out, const void *codes, const void *x, const void *tlut, int K, int m, int n, int bs,
+                                     void *workspace, size_t workspace_bytes, void *stream);
 
 /* Decompress-GEMM for batches up to 128 on the tcgen05 tensor cores (accumulator in tensor memory):
  * out (bs, m) fp32 = x (bs, n) fp16 @ decode(codes)^T, HYB code, kernel layout.  Replaces
@@ -260,7 +270,8 @@ int qtip_decompress_matvec_plain(float *out, const void *codes, const void *x, i
  *   hadk_bits     : NULL when kfac == 1, else kfac rows of ceil(kfac/32) uint32 words, bit j of
  *                   word w of row i set when hadK[i][32w+j] == +1.
  *   kfac in {1,12,20,28,36,52,60,108,116,124,140,156,172}; n/kfac a power of two, 2 <= n/kfac,
- *   n <= 65536. */
+ *   n <= 65536.
+ *   out_dtype QTIP_F16_FRAGMENTS: at most 8 rows, n = 8192, 16384, 32768 or 65536, 16-byte aligned buffers. */
 int qtip_rht(void *out, int out_dtype, const void *in, int in_dtype, long rows, int n, const void *sign_in,
              int sign_in_dtype, const float *sign_out, long n_signs, const uint32_t *hadk_bits, int kfac,
              int transpose, float scale, void *stream);

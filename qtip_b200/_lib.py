@@ -11,7 +11,7 @@ SO_PATH = os.path.join(_HERE, "libqtip_b200.so")
 
 OK, ERR_BAD_ARG, ERR_BAD_SHAPE, ERR_WORKSPACE, ERR_CUDA, ERR_ALIGNMENT, ERR_TOO_LARGE = range(7)
 CODE_HYB, CODE_3INST, CODE_1MAD = 0, 1, 2
-F16, F32 = 0, 1
+F16, F32, F16_FRAGMENTS = 0, 1, 2
 
 _vp, _i, _l, _sz, _f = ctypes.c_void_p, ctypes.c_int, ctypes.c_long, ctypes.c_size_t, ctypes.c_float
 
@@ -44,6 +44,8 @@ SIGNATURES = {
     "qtip_kernel_to_plain_layout": (_i, [_vp, _vp, _i, _i, _i, _vp]),
     "qtip_matvec_workspace_bytes": (_sz, [_i, _i, _i]),
     "qtip_decompress_matvec": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp]),
+    "qtip_matvec_x_fragments": (_i, [_i, _i, _i, _i]),
+    "qtip_decompress_matvec_fragments": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _sz, _vp]),
     "qtip_decompress_matvec_static": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp]),
     "qtip_decompress_gemm": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp]),
     "qtip_decompress_gemm_plain": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp]),

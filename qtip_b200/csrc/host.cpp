@@ -129,6 +129,8 @@ struct Layer {
     bool kernel_layout;
 };
 
+bool aligned16(const at::Tensor &t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+
 at::Tensor linear_forward(const at::Tensor &input, Layer &L, int &launches) {
     const int64_t n = L.SU.numel(), m = L.SV.numel();
     for (const at::Tensor *t : {&input, &L.trellis, &L.SU, &L.SV, (const at::Tensor *)&L.tlut, (const at::Tensor *)&L.bits_left,
@@ -167,7 +169,7 @@ at::Tensor linear_forward(const at::Tensor &input, Layer &L, int &launches) {
     // size it takes; HYB: above 8 rows the matvec's single B fragment is full
     const bool gemm = whole_tiles && bs <= kMaxGemmBatch && (v1 || (L.kernel_layout && bs > kMaxMatvecBatch));
     // long prompts: the tensor-core kernel again where it is the faster way, else decoded once and a dense product
-    const bool wide = whole_tiles && bs > kMaxGemmBatch && (v1 || L.kernel_layout) && reinterpret_cast<uintptr_t>(trellis.data_ptr()) % 16 == 0 &&
+    const bool wide = whole_tiles && bs > kMaxGemmBatch && (v1 || L.kernel_layout) && aligned16(trellis) &&
                       qtip_decompress_gemm_f16_faster(L.code, (int)m, (int)n, (int)bs);
     const bool dense = !gemm && !wide && bs > kMaxMatvecBatch;
 
@@ -182,7 +184,10 @@ at::Tensor linear_forward(const at::Tensor &input, Layer &L, int &launches) {
 
     // input side: x * SU -> Hadamard^T (per chunk when row-parallel) -> / 32 -> fp16
     const int64_t seg_n = L.rcp == 1 ? n / L.tp : n;
-    check(qtip_rht(xh, QTIP_F16, x.data_ptr(), dtype_id(x), bs * (n / seg_n), (int)seg_n, SU.data_ptr(), dtype_id(SU), nullptr,
+    // rows that the matvec takes in fragment order are written so by the transform
+    const bool fragments = !gemm && !wide && !dense && L.kernel_layout && seg_n == n && aligned16(x) && aligned16(SU) &&
+                           qtip_matvec_x_fragments(L.K, (int)m, (int)n, (int)bs);
+    check(qtip_rht(xh, fragments ? QTIP_F16_FRAGMENTS : QTIP_F16, x.data_ptr(), dtype_id(x), bs * (n / seg_n), (int)seg_n, SU.data_ptr(), dtype_id(SU), nullptr,
                    n, bl, L.k_left, 1, (float)(1.0 / (std::sqrt((double)seg_n) * kInternalScale)), stream),
           "qtip_rht");
     launches = 3;
@@ -204,7 +209,11 @@ at::Tensor linear_forward(const at::Tensor &input, Layer &L, int &launches) {
         y_type = QTIP_F16;
     } else if (!dense) {
         at::Tensor ws = L.workspace.defined() ? L.workspace : matvec_workspace(dev, m, n, bs, stream);
-        if (L.kernel_layout)
+        if (fragments)
+            check(qtip_decompress_matvec_fragments(y, trellis.data_ptr(), xh, tlut.data_ptr(), L.K, (int)m, (int)n, (int)bs, ws.data_ptr(),
+                                                   (size_t)ws.nbytes(), stream),
+                  "qtip_decompress_matvec_fragments");
+        else if (L.kernel_layout)
             check(qtip_decompress_matvec(y, trellis.data_ptr(), xh, tlut.data_ptr(), L.K, (int)m, (int)n, (int)bs, ws.data_ptr(),
                                          (size_t)ws.nbytes(), stream),
                   "qtip_decompress_matvec");

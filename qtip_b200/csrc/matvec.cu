@@ -1222,22 +1222,51 @@ int launch_fragments(const FragmentArgs &a, int nprob, int n, int bs, cudaStream
     return check_launch();
 }
 
-// fused_in: the batch uses the fused input transform (needs x staged in shared memory plus fp32 scratch)
+// How a call runs with x staged in shared memory; false if x does not fit.  fused_in: the batch uses the fused input transform (fp32
+// scratch beside x)
+struct HybPlan {
+    Partition p;
+    int cta_rows;
+    bool pieces;
+    SmemPlan smem;
+};
 template <int K>
-int launch_hyb_batch(const MatvecBatch &batch, int nprob, int m, int n, int bs, bool fused_in, cudaStream_t s) {
+bool plan_staged(int nprob, int m, int n, int bs, bool fused_in, HybPlan &h) {
     // shared memory: control + table are fixed; then the ring, the partial-sum slots and, when it fits, x.
-    const Partition p = make_partition(m, n, nprob);
+    const Partition p = h.p = make_partition(m, n, nprob);
     const int mb = m >> 5, nb = n >> 5;
-    const int cta_rows = p.mode == kModeRows ? (mb + p.grid - 1) / p.grid : (int)((((long)mb * nb + p.grid - 1) / p.grid + nb - 2) / nb) + 1;
+    const int cta_rows = h.cta_rows = p.mode == kModeRows ? (mb + p.grid - 1) / p.grid : (int)((((long)mb * nb + p.grid - 1) / p.grid + nb - 2) / nb) + 1;
     // More rows of x need several times the slots, which the ring then lacks (22016 x 4096, 5 rows: 24.6 us with pieces, 19.8
     // with runs); with one row block per CTA the slots are few and pieces save the run arithmetic (4096 x 4096: 7.1 against 8.2)
-    const bool pieces = (bs == 1 || cta_rows == 1) && p.mode == kModeRows && nb >= kConsumerWarps;
-    SmemPlan plan;
+    const bool pieces = h.pieces = (bs == 1 || cta_rows == 1) && p.mode == kModeRows && nb >= kConsumerWarps;
     // slots of up to four row blocks at once, fewer where memory is short
     for (int rows = pieces ? 4 : kMaxRowBlocks; rows >= 1; rows = pieces ? rows >> 1 : 0)
-        if (plan_smem<K>(n, bs, cta_rows, pieces, rows, true, fused_in, plan))
-            return pieces ? launch_hyb_variant<K, kStagedX | kPieces>(batch, nprob, m, n, bs, p, plan, s)
-                          : launch_hyb_variant<K, kStagedX>(batch, nprob, m, n, bs, p, plan, s);
+        if (plan_smem<K>(n, bs, cta_rows, pieces, rows, true, fused_in, h.smem)) return true;
+    return false;
+}
+
+// x of every problem in fragment order, through the ring
+template <int K>
+int launch_hyb_ring(const MatvecBatch &batch, int nprob, int m, int n, int bs, const HybPlan &h, bool make_fragments, const FragmentArgs &a,
+                    cudaStream_t s) {
+    SmemPlan plan;
+    // the ring takes all of the memory at K = 4 and 8 rows but for the slots of two row blocks (7 rows: 11; K = 3, 8 rows: 10)
+    int rows = kMaxRowBlocks;
+    while (rows >= 1 && !plan_smem<K>(n, bs, h.cta_rows, false, rows, false, false, plan)) rows >>= 1;
+    if (rows < 1) return QTIP_ERR_BAD_SHAPE;
+    if (make_fragments) {
+        const int st = launch_fragments(a, nprob, n, bs, s);
+        if (st != QTIP_OK) return st;
+    }
+    return launch_hyb_variant<K, 0>(batch, nprob, m, n, bs, h.p, plan, s);
+}
+
+template <int K>
+int launch_hyb_batch(const MatvecBatch &batch, int nprob, int m, int n, int bs, bool fused_in, cudaStream_t s) {
+    HybPlan h;
+    if (plan_staged<K>(nprob, m, n, bs, fused_in, h))
+        return h.pieces ? launch_hyb_variant<K, kStagedX | kPieces>(batch, nprob, m, n, bs, h.p, h.smem, s)
+                        : launch_hyb_variant<K, kStagedX>(batch, nprob, m, n, bs, h.p, h.smem, s);
     if (fused_in) return QTIP_ERR_BAD_SHAPE;      // the fused input side leaves x in shared memory
     MatvecBatch ring = batch;
     FragmentArgs a = {};
@@ -1246,13 +1275,14 @@ int launch_hyb_batch(const MatvecBatch &batch, int nprob, int m, int n, int bs, 
         a.frag[i] = reinterpret_cast<uint32_t *>(batch.p[i].workspace + partials_end(m, n));
         ring.p[i].x = reinterpret_cast<const __half *>(a.frag[i]);
     }
-    // the ring takes all of the memory at K = 4 and 8 rows but for the slots of two row blocks (7 rows: 11; K = 3, 8 rows: 10)
-    int rows = kMaxRowBlocks;
-    while (rows >= 1 && !plan_smem<K>(n, bs, cta_rows, false, rows, false, false, plan)) rows >>= 1;
-    if (rows < 1) return QTIP_ERR_BAD_SHAPE;
-    const int st = launch_fragments(a, nprob, n, bs, s);
-    if (st != QTIP_OK) return st;
-    return launch_hyb_variant<K, 0>(ring, nprob, m, n, bs, p, plan, s);
+    return launch_hyb_ring<K>(ring, nprob, m, n, bs, h, true, a, s);
+}
+
+template <int K>
+int launch_hyb_fragments(const MatvecBatch &batch, int m, int n, int bs, cudaStream_t s) {
+    HybPlan h;
+    (void)plan_staged<K>(1, m, n, bs, false, h);       // the partition; x is in its order already
+    return launch_hyb_ring<K>(batch, 1, m, n, bs, h, false, FragmentArgs{}, s);
 }
 
 template <int K>
@@ -1288,6 +1318,27 @@ extern "C" int qtip_decompress_matvec(float *out, const void *codes, const void 
     if (K == 2) return launch_hyb<2>(out, c, xh, t, m, n, bs, ws, s);
     if (K == 3) return launch_hyb<3>(out, c, xh, t, m, n, bs, ws, s);
     return launch_hyb<4>(out, c, xh, t, m, n, bs, ws, s);
+}
+
+extern "C" int qtip_matvec_x_fragments(int K, int m, int n, int bs) {
+    if (K < 2 || K > 4 || m < 32 || (m & 31) || bs < 1 || bs > kMaxBatch || (n != 8192 && n != 16384 && n != 32768 && n != 65536)) return 0;
+    HybPlan h;
+    return !(K == 2 ? plan_staged<2>(1, m, n, bs, false, h) : K == 3 ? plan_staged<3>(1, m, n, bs, false, h) : plan_staged<4>(1, m, n, bs, false, h));
+}
+
+extern "C" int qtip_decompress_matvec_fragments(float *out, const void *codes, const void *x, const void *tlut, int K, int m, int n, int bs,
+                                                void *workspace, size_t workspace_bytes, void *stream) {
+    if (!tlut) return QTIP_ERR_BAD_ARG;
+    const int st = check_common(out, codes, x, K, m, n, bs, workspace, workspace_bytes);
+    if (st != QTIP_OK) return st;
+    if (!aligned(tlut, 4)) return QTIP_ERR_ALIGNMENT;
+    MatvecBatch batch = {};
+    batch.p[0].out = out; batch.p[0].codes = static_cast<const uint8_t *>(codes); batch.p[0].x = static_cast<const __half *>(x);
+    batch.p[0].tlut = static_cast<const uint32_t *>(tlut); batch.p[0].workspace = static_cast<uint8_t *>(workspace);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (K == 2) return launch_hyb_fragments<2>(batch, m, n, bs, s);
+    if (K == 3) return launch_hyb_fragments<3>(batch, m, n, bs, s);
+    return launch_hyb_fragments<4>(batch, m, n, bs, s);
 }
 
 extern "C" int qtip_decompress_matvec_plain(float *out, const void *codes, const void *x, int code, int K, int m, int n,

@@ -330,6 +330,11 @@ int launch_rht(RhtArgs a, long rows, void *stream) {
     }
     int status = QTIP_OK;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    // the fragment order: written by the cluster kernels of the powers of two
+    if (a.out_dtype == QTIP_F16_FRAGMENTS) {
+        if (a.kfac != 1 || p < 13 || p > 16 || rows > 8) return QTIP_ERR_BAD_SHAPE;
+        if (!a.vec_ok) return QTIP_ERR_ALIGNMENT;
+    }
     if (launch_rht_pow2(a, rows, s, status) || launch_rht_cluster(a, rows, s, status) || launch_rht_rows(a, rows, s, status)) return status;
     // rows of the factor matrix per CTA: 8, or 4 when a row is long - a thread keeps at most 4 x 4 products
     // in registers, so (rpc / 4) * len <= 4 * kRhtThreads
@@ -372,7 +377,7 @@ int launch_rht(RhtArgs a, long rows, void *stream) {
 int check_rht(const void *out, int out_dtype, const void *in, int in_dtype, long rows, int n, const void *sign_in,
               int sign_in_dtype, const float *sign_out, long n_signs, const uint32_t *hadk_bits, int kfac) {
     if (!out || !in || rows < 0) return QTIP_ERR_BAD_ARG;
-    if ((out_dtype != QTIP_F16 && out_dtype != QTIP_F32) || (in_dtype != QTIP_F16 && in_dtype != QTIP_F32))
+    if ((out_dtype != QTIP_F16 && out_dtype != QTIP_F32 && out_dtype != QTIP_F16_FRAGMENTS) || (in_dtype != QTIP_F16 && in_dtype != QTIP_F32))
         return QTIP_ERR_BAD_ARG;
     if (sign_in && sign_in_dtype != QTIP_F16 && sign_in_dtype != QTIP_F32) return QTIP_ERR_BAD_ARG;
     if (!valid_kfac(kfac) || (kfac > 1 && !hadk_bits)) return QTIP_ERR_BAD_ARG;

@@ -64,6 +64,12 @@ __device__ __forceinline__ void finish_row_vec(const RhtArgs &a, size_t in_off, 
     }
 }
 
+// Where the pair of columns e, e + 1 of a row lies in the matvec's fragment order (32-bit words)
+__device__ __forceinline__ size_t fragment_word(long rows, long row, size_t e) {
+    const size_t w = e >> 1;
+    return ((w >> 4) * rows + row) * 16 + (w & 3) * 4 + ((w >> 2) & 3);
+}
+
 // ---- thread-block clusters ----------------------------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
     uint32_t r;

@@ -189,11 +189,12 @@ __global__ void __launch_bounds__(Pow2Cfg<P, CL>::kThreads) rht_pow2_kernel(cons
             if (a.sign_out && it != first) signs(it);
 #pragma unroll
             for (int k = 0; k < E; k++) {
-                const size_t e = (size_t)row * n + ((size_t)k << LP) + 2 * it;
+                const size_t col = ((size_t)k << LP) + 2 * it, e = (size_t)row * n + col;
                 float y0 = w[k][0] * a.scale, y1 = w[k][1] * a.scale;
                 if (a.sign_out) { y0 *= sg[k].x; y1 *= sg[k].y; }
                 if (a.out_dtype == QTIP_F16) *reinterpret_cast<__half2 *>(static_cast<__half *>(a.out) + e) = __floats2half2_rn(y0, y1);
-                else *reinterpret_cast<float2 *>(static_cast<float *>(a.out) + e) = make_float2(y0, y1);
+                else if (a.out_dtype == QTIP_F32) *reinterpret_cast<float2 *>(static_cast<float *>(a.out) + e) = make_float2(y0, y1);
+                else static_cast<__half2 *>(a.out)[fragment_word(rows, row, col)] = __floats2half2_rn(y0, y1);
             }
         }
         cluster_sync();                                    // no CTA leaves while others read its part

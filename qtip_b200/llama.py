@@ -433,10 +433,11 @@ class QtipLlama:
         """One QTIP linear on B rows: transform in (optionally residual add / RMSNorm / SwiGLU), matvec, transform out."""
         B, n, m = self.B, lin.n, lin.m
         xh, y = self.b_xh.view(-1)[:B * n].view(B, n), self.b_y.view(-1)[:B * m].view(B, m)
+        frag = ops.matvec_takes_fragments(lin.K, m, n, B) and all(t is None or t.data_ptr() % 16 == 0 for t in (lin.SU, norm))
         ops.rht_fused(src, B, n, xh, residual=residual, residual_out=residual_out, norm_weight=norm, eps=self.shape.rms_eps,
                       gate=gate, sign_in=lin.SU, hadk_bits=self.bits[kf_in], kfac=kf_in, transpose=True,
-                      scale=1 / math.sqrt(n) / 32)
-        ops.decompress_matvec(lin.codes, xh, lin.tlut, lin.K, m, n, out=y, workspace=self.b_workspace)
+                      scale=1 / math.sqrt(n) / 32, fragments=frag)
+        ops.decompress_matvec(lin.codes, xh, lin.tlut, lin.K, m, n, out=y, workspace=self.b_workspace, fragments=frag)
         if all_reduce:
             self._all_reduce(y)
         ops.rht_fused(y, B, m, out, sign_out=lin.SV32, hadk_bits=self.bits[kf_out], kfac=kf_out, scale=1 / math.sqrt(m))

@@ -10,7 +10,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import CODE_1MAD, CODE_3INST, CODE_HYB, F16, F32  # noqa: F401
+from ._lib import CODE_1MAD, CODE_3INST, CODE_HYB, F16, F16_FRAGMENTS, F32  # noqa: F401
 
 CODE_IDS = {"quantlut_sym": CODE_HYB, "hyb": CODE_HYB, "3inst": CODE_3INST, "1mad": CODE_1MAD}
 HAD_FACTORS = (172, 156, 140, 124, 116, 108, 60, 52, 36, 28, 20, 12)
@@ -248,8 +248,14 @@ def kernel_to_plain_layout(codes, K, m, n):
     return out
 
 
-def decompress_matvec(codes, x, tlut, K, m, n, out=None, workspace=None):
-    """out (bs, m) fp32 = x (bs, n) fp16 @ decode(codes)^T, HYB kernel layout, bs <= 8."""
+def matvec_takes_fragments(K, m, n, bs):
+    """True when the input transform should write x in the matvec's fragment order (one launch less)."""
+    return bool(_lib.load().qtip_matvec_x_fragments(K, m, n, bs))
+
+
+def decompress_matvec(codes, x, tlut, K, m, n, out=None, workspace=None, fragments=False):
+    """out (bs, m) fp32 = x (bs, n) fp16 @ decode(codes)^T, HYB kernel layout, bs <= 8.  fragments: x holds its rows in fragment
+    order (rht_fused(..., fragments=True))."""
     _require_cuda(codes, x, tlut)
     if x.dtype != torch.float16:
         x = x.to(torch.float16)
@@ -260,8 +266,9 @@ def decompress_matvec(codes, x, tlut, K, m, n, out=None, workspace=None):
     if workspace is None:
         workspace = matvec_workspace(m, n, bs, x.device)
     with torch.cuda.device(x.device):
-        st = _lib.load().qtip_decompress_matvec(out.data_ptr(), codes.data_ptr(), x.data_ptr(), tlut.data_ptr(), K, m,
-                                                n, bs, workspace.data_ptr(), workspace.numel(), _stream())
+        lib = _lib.load()
+        call = lib.qtip_decompress_matvec_fragments if fragments else lib.qtip_decompress_matvec
+        st = call(out.data_ptr(), codes.data_ptr(), x.data_ptr(), tlut.data_ptr(), K, m, n, bs, workspace.data_ptr(), workspace.numel(), _stream())
     _lib.check(st, "qtip_decompress_matvec")
     global launch_count
     launch_count += 1
@@ -332,8 +339,9 @@ def hadamard(x, hadK=None, K=1, transpose=False):
 
 
 def rht_fused(x, rows, n, out, *, in_row_stride=None, residual=None, residual_out=None, norm_weight=None, eps=1e-5,
-              gate=None, sign_in=None, sign_out=None, hadk_bits=None, kfac=1, transpose=False, scale=1.0):
-    """qtip_rht_fused on preallocated tensors (no allocation, graph-capturable); see include/qtip_b200.h."""
+              gate=None, sign_in=None, sign_out=None, hadk_bits=None, kfac=1, transpose=False, scale=1.0, fragments=False):
+    """qtip_rht_fused on preallocated tensors (no allocation, graph-capturable); see include/qtip_b200.h.  fragments: fp16 rows in the
+    order that decompress_matvec(..., fragments=True) takes."""
     _check_device(x, out, residual, residual_out, norm_weight, gate, sign_in, sign_out, hadk_bits)
     n_signs = n
     if sign_in is not None:
@@ -341,7 +349,7 @@ def rht_fused(x, rows, n, out, *, in_row_stride=None, residual=None, residual_ou
     if sign_out is not None:
         n_signs = sign_out.numel()
     p = lambda t: None if t is None else t.data_ptr()  # noqa: E731
-    st = _lib.load().qtip_rht_fused(out.data_ptr(), _dtype_id(out), x.data_ptr(), _dtype_id(x), rows,
+    st = _lib.load().qtip_rht_fused(out.data_ptr(), F16_FRAGMENTS if fragments else _dtype_id(out), x.data_ptr(), _dtype_id(x), rows,
                                     n if in_row_stride is None else in_row_stride, n, p(residual), p(residual_out),
                                     p(norm_weight), float(eps), p(gate), p(sign_in),
                                     F16 if sign_in is None else _dtype_id(sign_in), p(sign_out), n_signs, p(hadk_bits),

@@ -547,6 +547,26 @@ def test_decompress_gemm_ring_edges(K, code, m, n, bs):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("K", [2, 3, 4])
+@pytest.mark.parametrize("m,n,bs", [(64, 8192, 8), (4096, 8192, 5), (1024, 16384, 3), (320, 32768, 8), (32, 65536, 1)])
+def test_transform_in_fragment_order(K, m, n, bs):
+    """The transform's fragment order and the matvec that takes it: the bits of the row-major transform and its own re-ordering."""
+    lay = synth.make_layer(m, n, K, seed=3900 + K, bs=bs, device=DEV)
+    assert ops.matvec_takes_fragments(K, m, n, bs)
+    x, su = lay["x"].to(torch.float16), lay["SU"].to(torch.float16)
+    rows, frag = (torch.empty(bs, n, dtype=torch.float16, device=DEV) for _ in range(2))
+    ops.rht_fused(x, bs, n, rows, sign_in=su, scale=n**-0.5)
+    ops.rht_fused(x, bs, n, frag, sign_in=su, scale=n**-0.5, fragments=True)
+    # block of 32 columns, row, thread t, pairs 2t + 8i
+    want = rows.view(bs, n // 32, 4, 4, 2).permute(1, 0, 3, 2, 4).reshape(bs, n)
+    assert torch.equal(frag, want)
+    y = ops.decompress_matvec(lay["codes"], frag, lay["tlut"], K, m, n, fragments=True)
+    assert torch.equal(y, ops.decompress_matvec(lay["codes"], rows, lay["tlut"], K, m, n))
+    with pytest.raises(RuntimeError):
+        ops.rht_fused(x[:, :4096].contiguous(), bs, 4096, frag, fragments=True)      # a width whose kernel does not write it
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bs", [33, 75, 97, 113])
 def test_decompress_gemm_x_ring_depths(bs):
     """The depths of the ring of x (6, 4, 4 and 3 stages) with several rounds in one CTA and a last step of one tile."""
