@@ -21,7 +21,8 @@
 // Bound: instruction issue of the decode warps up to about 64 rows (8192 x 28672, 27 rows: leaving out three of four MMAs 45.6 -> 43.0 us,
 // the lookups 35.4), the MMAs above (120 rows: 57.8 -> 48.9 and 54.4 us).  Hence two blocks per warp and step between the barriers, x
 // through TMA instead of copies by the decode warps, scalar control (the warp index through a shuffle), control threads that sleep
-// between polls, and codes requested two steps ahead.  Warp instructions per block of weights, HYB 27 rows 190 -> 157, 3INST 295 -> 254.
+// between polls, and codes requested two steps ahead.  Warp instructions per block of weights, HYB 27 rows 190 -> 157, 3INST 295 -> 254,
+// and 222 with the mask of mask_3inst.
 // Measured, one block per warp and step with x copied by the decode warps -> now (microseconds, K = 2 unless stated): HYB 8192 x 8192
 // 27 rows 20.5 -> 17.5; 8192 x 28672 120 rows 73 -> 57.2; 14336 x 4096 K = 3 27 rows 19.7 -> 16.3; 28672 x 8192 K = 4 64 rows 70 -> 58;
 // 3INST 8192 x 8192 16 rows 30.5 -> 26.0, 8192 x 28672 120 rows 107 -> 83; 1MAD 8192 x 8192 K = 3 32 rows 33.0 -> 29.4.  A second
@@ -217,8 +218,11 @@ __device__ __forceinline__ float cluster_load(uint32_t addr, int rank) {
 // Two weights of the compute codes, packed.  3INST: each state's two fp16 terms are added by a half2 instruction that takes them
 // from one register (the multiply pipe has room; gathering both states' terms for one addition costs a permute more, 31.3 against
 // 29.4 us at 8192 x 8192, 27 rows).  1MAD: byte sums of the LCG values by dot product, weights from the lane's copy of the table.
-__device__ __forceinline__ uint32_t pair_3inst(uint32_t s0, uint32_t s1) {
-    const uint32_t r0 = ((s0 * 89226354u + 64248484u) & 0x8FFF8FFFu) ^ 0x3B603B60u, r1 = ((s1 * 89226354u + 64248484u) & 0x8FFF8FFFu) ^ 0x3B603B60u;
+// `mask` is 0x8FFF8FFF as a run-time value: a three-input logic instruction takes one literal, so with two it becomes two
+// instructions (8192 x 8192, 16 rows, 26.0 -> 21.6; 8192 x 28672, 120 rows, 83 -> 69.6 us).
+__device__ __forceinline__ uint32_t mask_3inst(int npad) { return 0x8FFF8FFFu | (uint32_t)npad >> 16; }
+__device__ __forceinline__ uint32_t pair_3inst(uint32_t s0, uint32_t s1, uint32_t mask) {
+    const uint32_t r0 = ((s0 * 89226354u + 64248484u) & mask) ^ 0x3B603B60u, r1 = ((s1 * 89226354u + 64248484u) & mask) ^ 0x3B603B60u;
     const __half2 h0 = *reinterpret_cast<const __half2 *>(&r0), h1 = *reinterpret_cast<const __half2 *>(&r1);
     const __half2 w0 = __hadd2(__low2half2(h0), __high2half2(h0)), w1 = __hadd2(__low2half2(h1), __high2half2(h1));
     return __byte_perm(*reinterpret_cast<const uint32_t *>(&w0), *reinterpret_cast<const uint32_t *>(&w1), 0x5410);
@@ -246,7 +250,8 @@ __device__ __forceinline__ void load_step(StepCodes<K> &c, const uint8_t *src, c
         for (int h = 0; h < 4; h++) c.rows[h >> 1][h & 1] = load_plain_row<K>(prow + h * (16 * K));
     }
 }
-// Block h as the words that its tensor-memory stores take (HYB: 8 per 16 rows; V = 1: a row per lane)
+// Block h as the words that its tensor-memory stores take (HYB: 8 per 16 rows; V = 1: a row per lane).  lut_lane: the lane's copy of the
+// table; 3INST, which has none: the mask
 template <int K, int CODE>
 __device__ __forceinline__ void decode_half(const StepCodes<K> &c, int h, uint32_t lut_lane, int lane, uint32_t (&wv)[16]) {
     if constexpr (CODE == QTIP_CODE_HYB) {
@@ -269,7 +274,7 @@ __device__ __forceinline__ void decode_half(const StepCodes<K> &c, int h, uint32
 #pragma unroll
             for (int j = 0; j < 8; j++) {
                 const uint32_t s0 = plain_state<K>(c.rows[h][ks], next, 2 * j), s1 = plain_state<K>(c.rows[h][ks], next, 2 * j + 1);
-                wv[8 * ks + j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1) : pair_1mad(s0, s1, lut_lane);
+                wv[8 * ks + j] = CODE == QTIP_CODE_3INST ? pair_3inst(s0, s1, lut_lane) : pair_1mad(s0, s1, lut_lane);
             }
         }
     }
@@ -366,7 +371,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 
     if (warp < kDecodeWarps) {
         // ---------------------------------- decode warps ------------------------------------------------
-        const uint32_t lut_lane = smem_addr(lut) + lane * 4;
+        const uint32_t lut_lane = CODE == QTIP_CODE_3INST ? mask_3inst(npad) : smem_addr(lut) + lane * 4;
         // this warp's 32 rows and 32 words of a stage (a warp reaches the 32 lanes of its index modulo four)
         const uint32_t tmem_warp = tmem + ((uint32_t)(32 * rb) << 16) + 32u * half;
         uint32_t s = group, parity = 1;                     // stage group, then group + kGroups, in turn
@@ -576,7 +581,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     if (warp < kDecodeWarps) {
         // the steps of all tiles in one sequence, which the groups take in turn
         const int group = warp >> 3, rb = warp & 3, half = (warp >> 2) & 1;
-        const uint32_t lut_lane = smem_addr(lut) + lane * 4;
+        const uint32_t lut_lane = CODE == QTIP_CODE_3INST ? mask_3inst(npad) : smem_addr(lut) + lane * 4;
         const uint32_t tmem_warp = tmem + ((uint32_t)(32 * rb) << 16) + 32u * half;
         int li = 0, lj = group;                             // tile and step of the next codes to be requested, and where they lie
         const uint8_t *src = nullptr;
@@ -776,8 +781,8 @@ int column_splits(int m, int n) {
 }
 
 // Time of a wide product on the busiest SM in cycles per 16 columns and wave of tiles: the MMA, or the decode warps.  (From timings: 11008 x 4096 129 rows
-// 26.6 us, 256 rows 32.3, 1000 rows in five groups 81.1, in four 86; 1MAD 8192 x 8192 129 rows 54.)
-double wide_cycles(int code, int npad) { return std::max(100 + 0.5 * npad, code == QTIP_CODE_HYB ? 140.0 : 188.0); }
+// 26.6 us, 256 rows 32.3, 1000 rows in five groups 81.1, in four 86; 8192 x 8192 129 rows 3INST 52, 1MAD 56.)
+double wide_cycles(int code, int npad) { return std::max(100 + 0.5 * npad, code == QTIP_CODE_HYB ? 140.0 : code == QTIP_CODE_3INST ? 165.0 : 188.0); }
 // Batch groups: as many as give the least time
 int wide_groups(int code, int m, int bs, double *cost = nullptr) {
     const long row_tiles = m / kRows, sms = sm_count();

@@ -306,9 +306,12 @@ __device__ __forceinline__ void v1_errors(uint32_t x, f2 nx, float minus_zero, f
     f2 r[2];
     float *rs = reinterpret_cast<float *>(r);
     if constexpr (CODE == QTIP_CODE_3INST) {
+        // 0x8FFF8FFF, made at run time: a three-input logic instruction takes one literal, with two it becomes two instructions (K = 3 and 4
+        // 3 % faster, K = 2 the same)
+        const uint32_t mask = __float_as_uint(minus_zero) | 0x0FFF8FFFu;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            uint32_t v = ((x + (uint32_t)j * k3instA) & 0x8FFF8FFFu) ^ 0x3B603B60u;
+            uint32_t v = ((x + (uint32_t)j * k3instA) & mask) ^ 0x3B603B60u;
             const __half2 h = *reinterpret_cast<__half2 *>(&v);
             rs[j] = __half2float(__hadd(__low2half(h), __high2half(h)));
         }
