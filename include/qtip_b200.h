@@ -150,7 +150,7 @@ int qtip_decompress_matvec_fragments(float *out, const void *codes, const void *
  * uint32 in device memory; the kernel leaves it 0, or a non-zero code if one of its (bounded) waits on
  * a shared-memory barrier gave up - the results are then meaningless, but the kernel still terminates
  * and frees its tensor memory.  When the row ranges leave SMs idle the input columns are split over
- * two CTAs and `out` is zeroed on the stream first (allocation-free, capturable). */
+ * the CTAs of a cluster, which add their parts in order (allocation-free, capturable). */
 int qtip_decompress_gemm(float *out, const void *codes, const void *x, const void *tlut, int K, int m, int n, int bs,
                          unsigned *status, void *stream);
 

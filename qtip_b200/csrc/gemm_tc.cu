@@ -21,11 +21,11 @@
 // Bound: instruction issue of the decode warps up to about 64 rows (8192 x 28672, 27 rows: leaving out three of four MMAs 45.6 -> 43.0 us,
 // the lookups 35.4), the MMAs above (120 rows: 57.8 -> 48.9 and 54.4 us).  Hence two blocks per warp and step between the barriers, x
 // through TMA instead of copies by the decode warps, scalar control (the warp index through a shuffle), control threads that sleep
-// between polls, and codes requested two steps ahead.  Warp instructions per block of weights, HYB 27 rows 190 -> 157, 3INST 295 -> 254,
-// and 222 with the mask of mask_3inst.
+// between polls, and codes requested two steps ahead.  Warp instructions per block of weights, HYB 27 rows 190 -> 145, 3INST 295 -> 217
+// (of which the mask of mask_3inst 32).
 // Measured, one block per warp and step with x copied by the decode warps -> now (microseconds, K = 2 unless stated): HYB 8192 x 8192
 // 27 rows 20.5 -> 17.5; 8192 x 28672 120 rows 73 -> 57.2; 14336 x 4096 K = 3 27 rows 19.7 -> 16.3; 28672 x 8192 K = 4 64 rows 70 -> 58;
-// 3INST 8192 x 8192 16 rows 30.5 -> 26.0, 8192 x 28672 120 rows 107 -> 83; 1MAD 8192 x 8192 K = 3 32 rows 33.0 -> 29.4.  A second
+// 3INST 8192 x 8192 16 rows 30.5 -> 21.6, 8192 x 28672 120 rows 107 -> 69.6; 1MAD 8192 x 8192 K = 3 32 rows 33.0 -> 29.4.  A second
 // accumulator for every other MMA changes nothing.
 // This replaces decode-to-HBM + dense GEMM of BitshiftLinearKernelAG upstream
 // (lib/codebook/bitshift.py:476-489), which writes and re-reads 16x the packed bytes at 2 bits.
@@ -509,7 +509,7 @@ __device__ __forceinline__ uint32_t b_tile(uint32_t base, int stage, int bytes) 
 // matrix again: a tile's 16 columns take the MMA about 100 + 0.15 N cycles and the decode warps 100, so up to 256 rows share a decode
 // at the price of one.  Measured against decode_hyb / decode_plain and
 // a library product, HYB K = 2 unless stated (microseconds): 11008 x 4096 129 rows 44.7 -> 26.6, 512 rows 59.8 -> 50.7, 1000 rows
-// 86.5 -> 81.1; 28672 x 8192 256 rows 214 -> 107, 1000 rows 450 -> 400; K = 4 4096 x 4096 1000 rows 37.8 -> 33.1; 1MAD K = 4 8192 x 8192
+// 86.5 -> 81.1; 28672 x 8192 256 rows 214 -> 107, 512 rows 287 -> 230; K = 4 4096 x 4096 1000 rows 37.8 -> 33.1; 1MAD K = 4 8192 x 8192
 // 256 rows 116 -> 56.  Bound: the MMAs (half of the tensor pipe's cycles are busy: a tensor-memory A operand takes twice the ideal interval),
 // then the lookups (left out: 80.3 -> 69.6) and the copies of x (74.2); hence no sleeping between the control threads' polls here.
 constexpr int kWideN = 256, kWideStages = 4, kWideXMax = 8, kEpilogueWarp = kCopyWarp + 1;
@@ -721,7 +721,10 @@ int encode_x(CUtensorMap *map, const __half *x, int n, int bs, int npad) {
             void *p = nullptr;
             cudaDriverEntryPointQueryResult found;
             QTIP_CUDA_TRY(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &found));
-            if (found != cudaDriverEntryPointSuccess) return QTIP_ERR_CUDA;
+            if (found != cudaDriverEntryPointSuccess) {
+                set_last_cuda_error(cudaErrorSymbolNotFound);
+                return QTIP_ERR_CUDA;
+            }
             encode = reinterpret_cast<Encode>(p);
         }
         f = encode;
@@ -904,12 +907,15 @@ extern "C" int qtip_decompress_gemm_f16(void *out, const void *codes, const void
 
 // Rule: estimates of both ways in microseconds.  Wide: 6 to start and end, the cycles above at 1.965 GHz.  Dense: 5 for the launches, the
 // decode at its write rate (3.9 TB/s HYB, 2.8 3INST, 1.6 1MAD), the product at the rate of reading the matrix (4.2 TB/s) or 1430 TFLOP/s.
+// Products of several hundred microseconds run at the power cap (28672 x 8192, 1000 rows: 400 to 458 us in three runs, dense 432 to 450): 10 % more.
 // It errs by up to 10 %, on either side of the line (4096 x 4096: dense up to 512 rows, 26.2 against 27.0 us; 11008 x 4096: wide up to about 2000).
 extern "C" int qtip_decompress_gemm_f16_faster(int code, int m, int n, int bs) {
     if (m <= 0 || n <= 0 || bs < 1 || (m % kRows) || (n % kTileCols)) return 0;
     double cycles;
     wide_groups(code, m, bs, &cycles);
-    const double bytes = 2.0 * m * n, wide = 6 + cycles * (n / 16) / 1965;
+    const double bytes = 2.0 * m * n;
+    double wide = 6 + cycles * (n / 16) / 1965;
+    if (wide > 300) wide *= 1.1;
     const double write = code == QTIP_CODE_HYB ? 3.9e6 : code == QTIP_CODE_3INST ? 2.8e6 : 1.6e6;
     const double dense = 5 + bytes / write + std::max(bytes / 4.2e6, bytes * bs / 1.43e9);
     return wide < dense;

@@ -14,7 +14,7 @@
 // 64 KiB in flight per SM, no registers held).  The kernel is bound by instruction issue, so what controls the ring is kept short: the
 // group wait has no polling loop, no lane is elected, and every count is the same in all lanes in a way the compiler can see (warp
 // index and division results through a shuffle), which makes the control scalar and spares the reconvergence code.  A bulk copy per
-// chunk with an mbarrier wait, issued by one lane, took 137 warp instructions per block against 123 at 1 row, 210 against 138 at 8 rows
+// chunk with an mbarrier wait, issued by one lane, took 137 warp instructions per block against 124 at 1 row, 210 against 139 at 8 rows
 // through the ring.  A lane
 // reads its 4K bytes of a block and those of lane+1 (the wrap-around bits of the tail-biting stream) from the ring, so the loop
 // has no shuffles.  A lane decodes its 16 trellis states into four mma.m16n8k16 A fragments in registers - HYB: h = s*(s+1),
@@ -29,7 +29,7 @@
 // 6.2e-6, 6.7e-6).  The parts are added in registers.
 //
 // The kernel is instruction-issue bound, not HBM bound (about 5 instructions per state are irreducible: shift, multiply-add
-// hash, mask, multiply-add address, shared load).  K = 2, 1 row: 123 warp instructions per block with everything that surrounds the
+// hash, mask, multiply-add address, shared load).  K = 2, 1 row: 124 warp instructions per block with everything that surrounds the
 // loop, 31 issue cycles of the four schedulers; the loop alone on resident data (100 instructions) runs at 83 % of the issue slots,
 // 30 cycles per block and SM, whichever pipe the address arithmetic is given to (integer or float multiply-add, adds).  A launch
 // takes about 4000 cycles before the loop (table, x) and, for shared row blocks, 4500 after it.  Measured, K = 2 unless stated, the
