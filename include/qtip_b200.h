@@ -276,6 +276,10 @@ int qtip_rht(void *out, int out_dtype, const void *in, int in_dtype, long rows, 
              int sign_in_dtype, const float *sign_out, long n_signs, const uint32_t *hadk_bits, int kfac,
              int transpose, float scale, void *stream);
 
+/* CTAs that share a row of n values (1024 to 65536, a power of two; 16-byte aligned buffers) in qtip_rht / qtip_rht_fused on a device of
+ * `sms` multiprocessors: 1, or 8 (a cluster; the only kernels that write QTIP_F16_FRAGMENTS); 0 for other widths.  No device is touched. */
+int qtip_rht_ctas_per_row(int n, long rows, int out_dtype, int sms);
+
 /* qtip_rht with the element-wise neighbours of a QTIP linear in a decoder layer fused into the load:
  *   v = in (+ residual)            the sum rounded to fp16, written to residual_out when given
  *   v = RMSNorm(v) * norm_weight   LlamaRMSNorm, model/llama.py:129-136 (fp32 statistics, fp16 product)

@@ -55,6 +55,7 @@ SIGNATURES = {
     "qtip_linear_desc_layout": (_i, [ctypes.POINTER(ctypes.c_size_t), _i]),
     "qtip_decompress_matvec_plain": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _sz, _vp]),
     "qtip_rht": (_i, [_vp, _i, _vp, _i, _l, _i, _vp, _i, _vp, _l, _vp, _i, _i, _f, _vp]),
+    "qtip_rht_ctas_per_row": (_i, [_i, _l, _i, _i]),
     "qtip_rht_fused": (_i, [_vp, _i, _vp, _i, _l, _l, _i, _vp, _vp, _vp, _f, _vp, _vp, _i, _vp, _l, _vp, _i, _i, _f,
                             _vp]),
     "qtip_mlp_mid_supported": (_i, [_i, _i]),

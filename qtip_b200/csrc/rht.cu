@@ -334,6 +334,7 @@ int launch_rht(RhtArgs a, long rows, void *stream) {
     if (a.out_dtype == QTIP_F16_FRAGMENTS) {
         if (a.kfac != 1 || p < 13 || p > 16 || rows > 8) return QTIP_ERR_BAD_SHAPE;
         if (!a.vec_ok) return QTIP_ERR_ALIGNMENT;
+        return launch_rht_pow2(a, rows, s, status) ? status : QTIP_ERR_BAD_SHAPE;
     }
     if (launch_rht_pow2(a, rows, s, status) || launch_rht_cluster(a, rows, s, status) || launch_rht_rows(a, rows, s, status)) return status;
     // rows of the factor matrix per CTA: 8, or 4 when a row is long - a thread keeps at most 4 x 4 products

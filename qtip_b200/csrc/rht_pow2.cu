@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(Pow2Cfg<P, CL>::kThreads) rht_pow2_kernel(cons
                 else
 #pragma unroll
                     for (int c = 0; c < W; c += 2) *reinterpret_cast<__half2 *>(o + c) = __floats2half2_rn(y[c], y[c + 1]);
-            } else {
+            } else if (a.out_dtype == QTIP_F32) {          // (fragments: never here, see pow2_cluster_log)
                 float *o = static_cast<float *>(a.out) + out_off + e;
                 if constexpr (W == 1) *o = y[0];
                 else
@@ -231,11 +231,18 @@ int launch_pow2(const RhtArgs &a, long rows, cudaStream_t s) {
     return check_launch();
 }
 
+// log2 of the CTAs that share a row.  Short rows: one CTA, long ones: a cluster of eight.  In between a cluster while all of them
+// run at once (three clusters of eight per sixteen SMs); fragments by the cluster kernels always: they alone write that order.
+int pow2_cluster_log(int p, long rows, int out_dtype, int sms) {
+    if (p < 13) return 0;
+    return p > 14 || out_dtype == QTIP_F16_FRAGMENTS || rows <= (3 * sms / 2) >> 3 ? 3 : 0;
+}
+
 }  // namespace
 
 bool launch_rht_pow2(const RhtArgs &a, long rows, cudaStream_t s, int &status) {
     if (a.kfac != 1 || !a.vec_ok) return false;
-    const bool cluster = rows <= (3 * sm_count() / 2) >> 3;
+    const bool cluster = pow2_cluster_log(a.p, rows, a.out_dtype, sm_count()) > 0;
     switch (a.p) {
         case 10: status = launch_pow2<10, 0>(a, rows, s); return true;
         case 11: status = launch_pow2<11, 0>(a, rows, s); return true;
@@ -249,3 +256,10 @@ bool launch_rht_pow2(const RhtArgs &a, long rows, cudaStream_t s, int &status) {
 }
 
 }  // namespace qtip
+
+extern "C" int qtip_rht_ctas_per_row(int n, long rows, int out_dtype, int sms) {
+    int p = 0;
+    while (p < 17 && (1 << p) < n) p++;
+    if (n != 1 << p || p < 10 || p > 16 || rows < 1 || sms < 1) return 0;
+    return 1 << qtip::pow2_cluster_log(p, rows, out_dtype, sms);
+}

@@ -128,6 +128,22 @@ def test_argument_validation_without_device():
     assert lib.qtip_pipe_rate_count() == 10 and lib.qtip_pipe_rate_name(0).startswith(b"IMAD") and lib.qtip_pipe_rate_name(99) == b""
 
 
+@pytest.mark.parametrize("sms", [8, 18, 42, 148])
+def test_fragment_order_goes_to_the_kernels_that_write_it(sms):
+    """Whatever part of the GPU is visible: rows in fragment order (up to 8 of them) take the cluster kernels, the others as many CTAs
+    as fill the device."""
+    rule = _lib.load().qtip_rht_ctas_per_row
+    for rows in range(1, 9):
+        for n in (8192, 16384, 32768, 65536):
+            assert rule(n, rows, _lib.F16_FRAGMENTS, sms) == 8, (n, rows)
+            for dtype in (_lib.F16, _lib.F32):
+                assert rule(n, rows, dtype, sms) == (8 if n > 16384 or 16 * rows <= 3 * sms else 1), (n, rows)
+    for n in (1024, 2048, 4096):
+        assert rule(n, 1, _lib.F16, sms) == 1
+    for n in (0, 512, 1025, 11008, 131072):
+        assert rule(n, 1, _lib.F16, sms) == 0
+
+
 def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(_lib, "_lib", None)
     monkeypatch.setattr(_lib, "SO_PATH", os.path.join(ROOT, "does_not_exist.so"))
