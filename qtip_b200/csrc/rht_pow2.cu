@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(Pow2Cfg<P, CL>::kThreads) rht_pow2_kernel(cons
                 else
 #pragma unroll
                     for (int c = 0; c < W; c += 2) *reinterpret_cast<__half2 *>(o + c) = __floats2half2_rn(y[c], y[c + 1]);
-            } else if (a.out_dtype == QTIP_F32) {          // (fragments: never here, see pow2_cluster_log)
+            } else {      // fp32 (launch_pow2 refuses fragments here; a test of the type in this loop costs 2.5 us per launch)
                 float *o = static_cast<float *>(a.out) + out_off + e;
                 if constexpr (W == 1) *o = y[0];
                 else
@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(Pow2Cfg<P, CL>::kThreads) rht_pow2_kernel(cons
 template <int P, int CL>
 int launch_pow2(const RhtArgs &a, long rows, cudaStream_t s) {
     using C = Pow2Cfg<P, CL>;
+    if (CL == 0 && a.out_dtype == QTIP_F16_FRAGMENTS) return QTIP_ERR_BAD_SHAPE;
     static bool attr_set[64] = {};
     int dev = 0;
     QTIP_CUDA_TRY(cudaGetDevice(&dev));
