@@ -32,6 +32,11 @@ template <int K>
 __global__ void __launch_bounds__(kHybThreads, 1) decode_hyb_kernel(__half *__restrict__ W, const uint8_t *__restrict__ codes,
                                                                     const uint32_t *__restrict__ tlut, int m, int n) {
     extern __shared__ __align__(128) uint8_t smem[];
+    // codes and table may come from the launch before (a conversion, the layout shuffle), so nothing is read ahead of the wait (through
+    // the pointers: read-only loads are not moved either), and the next launch starts its own reads of weights only when everything
+    // before this one is complete
+    asm volatile("griddepcontrol.wait;" : "+l"(codes), "+l"(tlut) : : "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // the warp index through a shuffle: the same in all lanes, so the loop control is scalar
     const int warp = __shfl_sync(kFullMask, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int nb = n >> 5, blocks = (m >> 5) * nb, warps = (int)gridDim.x * (kHybThreads / 32);
@@ -44,9 +49,7 @@ __global__ void __launch_bounds__(kHybThreads, 1) decode_hyb_kernel(__half *__re
         const uint32_t e = __ldg(tlut + ((i >> 3) & 511)) ^ ((uint32_t)(i >> 12) << 15);
         reinterpret_cast<uint4 *>(smem)[i] = make_uint4(e, e, e, e);
     }
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __syncthreads();
-    asm volatile("griddepcontrol.wait;" ::: "memory");      // W may still be read by an earlier launch of the stream
 
     const uint32_t lut_lane = (uint32_t)__cvta_generic_to_shared(smem) + lane * 4;
     const uint32_t stage = (uint32_t)__cvta_generic_to_shared(smem) + kHybLutBytes + warp * (32 * kStageStride);

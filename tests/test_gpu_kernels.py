@@ -48,6 +48,27 @@ def test_decode_hyb_vs_oracle(K, m, n):
     assert np.array_equal(u16(W), u16(C.decode_kernel(lay["codes"], m, n, K, lay["tlut"])))
 
 
+def _write_early(dst, seed):
+    """fp16 values into dst by a launch that lets the one after it start before it has written anything: 4096 or 1024 a row."""
+    half = dst.view(torch.float16).view(-1)
+    n = 4096 if half.numel() % 4096 == 0 else 1024
+    x = torch.randn(half.numel() // n, n, device=DEV, generator=torch.Generator(DEV).manual_seed(seed)).half()
+    torch.cuda.synchronize()
+    ops.rht_fused(x, x.shape[0], n, half, scale=n**-0.5)
+
+
+@pytest.mark.parametrize("K", [2, 3, 4])
+@pytest.mark.parametrize("m,n", [(1024, 1024), (8192, 4096)])
+@pytest.mark.parametrize("operand", ["codes", "tlut"])
+def test_decode_hyb_reads_what_the_launch_before_wrote(K, m, n, operand):
+    for seed in range(3):
+        codes = torch.full((K * m * n // 16,), -1, dtype=torch.int16, device=DEV)
+        tlut = torch.full((512, 2), 7.0, dtype=torch.float16, device=DEV)
+        _write_early(codes if operand == "codes" else tlut, seed)
+        W = ops.decode_hyb(codes, tlut, K, m, n)
+        assert torch.equal(W.view(torch.int16), ops.decode_hyb(codes, tlut, K, m, n).view(torch.int16))
+
+
 # ---- producers of the packed formats: bit exact ---------------------------------------------------------
 @pytest.mark.parametrize("K", [2, 3, 4])
 @pytest.mark.parametrize("V", [1, 2])
