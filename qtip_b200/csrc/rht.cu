@@ -86,8 +86,7 @@ __global__ void __launch_bounds__(kRhtThreads) rht_kernel(const RhtArgs a) {
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + c * 16), "l"(src + c * 4) : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    rht_wait(a);
 
     const bool write_res = a.residual_out && blockIdx.x == 0 && (a.in_row_stride != 0 || row == 0);
     float ss = 0.f;
@@ -408,6 +407,7 @@ extern "C" int qtip_rht(void *out, int out_dtype, const void *in, int in_dtype, 
     a.in_row_stride = n; a.out_dtype = out_dtype; a.in_dtype = in_dtype; a.sign_in_dtype = sign_in_dtype;
     a.n = n; a.sign_rep = (sign_in || sign_out) ? (int)(n_signs / n) : 1; a.kfac = kfac; a.transpose = transpose;
     a.scale = scale;
+    a.settle = 1;
     return launch_rht(a, rows, stream);
 }
 

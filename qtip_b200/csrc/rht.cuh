@@ -15,8 +15,19 @@ struct RhtArgs {
     int part_offset;     // float offset in shared memory of the partial-product buffer (short rows only)
     int sgn_offset;      // float offset of the staged sign_out slice (short rows only, else 0)
     int vec_ok;          // every buffer is 16-byte aligned and n, strides are multiples of 8: 8-wide loads / stores
+    int settle;          // the next launch may start only when everything before this one is complete (see rht_wait)
     float scale, eps;
 };
+
+// Waits for the launch before and lets the next one start: at once (the decode loop, whose weights are old), or with `settle` (qtip_rht)
+// only after the wait.  A product that reads its weights while the transform before it runs is then safe whatever wrote them before
+// that.  It also measured faster where layer calls follow one another (28672 x 8192 K = 4, 1 row: 60.1 -> 50.8 us a call; 8192 x 8192,
+// 5 rows 22.8 -> 22.1; 8192 x 8192 3INST, 16 rows 30.7 -> 31.1).
+__device__ __forceinline__ void rht_wait(const RhtArgs &a) {
+    if (!a.settle) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (a.settle) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 __device__ __forceinline__ float load_elem(const void *p, int dtype, size_t i) {
     return dtype == QTIP_F16 ? __half2float(static_cast<const __half *>(p)[i]) : static_cast<const float *>(p)[i];

@@ -353,8 +353,7 @@ __global__ void __launch_bounds__(kRowMaxThreads) rht_row_kernel(const RhtArgs a
     uint32_t *b0p = afrag + S.mt_cta * S.kq * 32;
     float *obuf = reinterpret_cast<float *>(b0p);
     build_fragments(a, afrag, b0p, m0, mt_here, S.kq);
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    rht_wait(a);
 
     const int j8_log = a.p - 3, npairs = k2n << j8_log;
     constexpr int cw_log = NTL == 8 ? 6 : NTL == 4 ? 5 : NTL == 2 ? 4 : 3;
@@ -579,8 +578,7 @@ __global__ void __launch_bounds__(kClusterThreads, 2) rht_cluster_kernel(const R
     uint32_t *b0p = bits + nbits;
     float *obuf = reinterpret_cast<float *>(b0p + 2 * plane);
     for (int i = threadIdx.x; i < kfac * wpr; i += kClusterThreads) bits[i] = __ldg(a.hadk_bits + i);
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    rht_wait(a);
 
     const long row = blockIdx.y;
     const size_t sign_off = (size_t)(row % a.sign_rep) * n, in_off = (size_t)row * a.in_row_stride;

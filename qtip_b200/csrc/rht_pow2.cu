@@ -54,8 +54,7 @@ __global__ void __launch_bounds__(Pow2Cfg<P, CL>::kThreads) rht_pow2_kernel(cons
     const int sub = threadIdx.x / C::kRowThreads, tid = threadIdx.x % C::kRowThreads, lane = threadIdx.x & 31;
     float *scratch = sm;                                   // 64 floats
     float *buf = sm + 64 + sub * C::kRowFloats;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    rht_wait(a);
     const long row = CL ? (long)blockIdx.y : (long)blockIdx.x * C::kRows + sub;
     const bool live = row < rows;
     const long r = live ? row : rows - 1;                  // idle threads of the last CTA repeat the last row and store nothing

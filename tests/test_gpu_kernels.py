@@ -48,7 +48,7 @@ def test_decode_hyb_vs_oracle(K, m, n):
     assert np.array_equal(u16(W), u16(C.decode_kernel(lay["codes"], m, n, K, lay["tlut"])))
 
 
-def _write_early(dst, seed):
+def write_early(dst, seed):
     """fp16 values into dst by a launch that lets the one after it start before it has written anything: 4096 or 1024 a row."""
     half = dst.view(torch.float16).view(-1)
     n = 4096 if half.numel() % 4096 == 0 else 1024
@@ -64,7 +64,7 @@ def test_decode_hyb_reads_what_the_launch_before_wrote(K, m, n, operand):
     for seed in range(3):
         codes = torch.full((K * m * n // 16,), -1, dtype=torch.int16, device=DEV)
         tlut = torch.full((512, 2), 7.0, dtype=torch.float16, device=DEV)
-        _write_early(codes if operand == "codes" else tlut, seed)
+        write_early(codes if operand == "codes" else tlut, seed)
         W = ops.decode_hyb(codes, tlut, K, m, n)
         assert torch.equal(W.view(torch.int16), ops.decode_hyb(codes, tlut, K, m, n).view(torch.int16))
 

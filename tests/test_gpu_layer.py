@@ -751,3 +751,21 @@ def test_long_prompt_on_the_tensor_core_path(code, mode, K):
     assert y.dtype == torch.float16 and y.shape == (bs, m)
     assert float((y.double() - want.double()).norm() / want.double().norm()) < 2.0**-11
     assert ops.gemm_status(DEV) == 0
+
+
+@pytest.mark.parametrize("code,mode,K", [("hyb", "quantlut_sym", 2), ("3inst", "3inst", 2)])
+@pytest.mark.parametrize("m,n,bs", [(4096, 4096, 1), (2048, 8192, 5), (4096, 4096, 27), (22016, 1024, 300), (1024, 2752, 3)])
+def test_weights_written_by_the_launch_before_the_call(code, mode, K, m, n, bs):
+    """Codes (and a table) from a launch that lets its successor start before it has written them: the product behind the first
+    transform, which reads its weights early, must find them."""
+    from test_gpu_kernels import write_early
+    q = QuantizedLinear(n, m, 16, 16, 16, K, 2 if code == "hyb" else 1, 9, mode).to(DEV)
+    q.SU.fill_(1), q.SV.fill_(1)
+    x = torch.randn(bs, n, device=DEV, generator=torch.Generator(DEV).manual_seed(5)).half()
+    q(x)                # the workspace and the packed factors exist
+    for seed in range(3):
+        for t in (q.trellis, q.tlut) if code == "hyb" else (q.trellis,):
+            q.trellis.fill_(-1)
+            write_early(t.data, seed)
+            y = q(x)
+            assert torch.isfinite(y).all() and torch.equal(y, q(x))
