@@ -8,6 +8,14 @@
  * otherwise an entry point allocates nothing, so it may be called while a stream is captured
  * into a CUDA graph.
  *
+ * Order.  Activations, workspaces and outputs are touched only after everything before the call on its stream is complete.  The launches
+ * of a decode loop or a layer call, however, read their WEIGHTS (codes, tables, sign vectors, norm weights, hadk_bits, the head's
+ * matrix) while the launch before them may still run: qtip_decompress_matvec and its forms for HYB, qtip_linear_fused,
+ * qtip_rht (hadk_bits, sign_out), qtip_rht_fused, qtip_mlp_mid, qtip_rope_kv_append_fused, qtip_lm_head, and whatever says so below.
+ * Weights of these must not be written by the launch directly before, nor by one further back with only such launches since.  qtip_rht
+ * and qtip_decode_hyb end that: the launch behind one of them starts when everything before it is complete.  All others
+ * (the decoders, qtip_decompress_gemm*, the packing and layout calls, the quantizer) follow plain stream order for every operand.
+ *
  * Naming: K = bits per weight (the upstream CUDA template parameter R), m = out_features
  * (upstream M), n = in_features (upstream template K), bs = batch rows.  fp16 buffers are IEEE
  * binary16 (uint16_t storage).  "kernel layout" is the packed trellis format written by
@@ -166,7 +174,11 @@ int qtip_decompress_gemm_plain(float *out, const void *codes, const void *x, int
  * tlut required) or a compute code (plain layout, tlut ignored).  Same shape and status rules. */
 int qtip_decompress_gemm_f16(void *out, const void *codes, const void *x, const void *tlut, int code, int K, int m, int n, int bs,
                              unsigned *status, void *stream);
-/* 1 if that is estimated to be faster on this device than qtip_decode_hyb / qtip_decode_plain and a dense product, else 0 (also for shapes
+/* These three for weights (codes, table) that were complete before the launch before this one began: they are read while it still runs.
+ * out_dtype QTIP_F32: qtip_decompress_gemm (QTIP_CODE_HYB) or _plain (compute codes), at most 128 rows; QTIP_F16: _f16. */
+int qtip_decompress_gemm_settled(void *out, int out_dtype, const void *codes, const void *x, const void *tlut, int code, int K, int m, int n,
+                                 int bs, unsigned *status, void *stream);
+/* 1 if qtip_decompress_gemm_f16 is estimated to be faster on this device than qtip_decode_hyb / qtip_decode_plain and a dense product, else 0 (also for shapes
  * it does not take). */
 int qtip_decompress_gemm_f16_faster(int code, int m, int n, int bs);
 

@@ -50,6 +50,7 @@ SIGNATURES = {
     "qtip_decompress_gemm": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _vp]),
     "qtip_decompress_gemm_plain": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp]),
     "qtip_decompress_gemm_f16": (_i, [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp]),
+    "qtip_decompress_gemm_settled": (_i, [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp]),
     "qtip_decompress_gemm_f16_faster": (_i, [_i, _i, _i, _i]),
     "qtip_linear_fused": (_i, [ctypes.POINTER(LinearDesc), _i, _i, _i, _i, _i, _vp]),
     "qtip_linear_desc_layout": (_i, [ctypes.POINTER(ctypes.c_size_t), _i]),

@@ -740,9 +740,18 @@ int encode_x(CUtensorMap *map, const __half *x, int n, int bs, int npad) {
     return QTIP_ERR_CUDA;
 }
 
+// The launch may start while the one before it runs.  Both kernels read weights before they wait for it, so only where the caller says
+// that those are settled; otherwise a plain launch (8192 x 8192, 27 rows, K = 2, after a transform: 19.7 -> 21.8 us for the two).
+cudaLaunchAttribute overlap_attribute() {
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    return a;
+}
+
 template <int K, int CODE>
 int launch_gemm(float *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, int npad,
-                int splitk, unsigned *status, cudaStream_t s) {
+                int splitk, unsigned *status, bool settled, cudaStream_t s) {
     const int smem = 1024 + x_stages(npad) * npad * kStageCols * 2 + kLut512Bytes + 256;
     static_assert(sizeof(GemmCtrl) <= 256 && 1024 + kXRingBytes + kLut512Bytes + 256 <= 227 * 1024, "shared memory");
     static bool attr_set[64] = {};
@@ -766,14 +775,14 @@ int launch_gemm(float *out, const uint8_t *codes, const __half *x, const uint32_
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 1;
-    attr[1].val.clusterDim.y = splitk;
-    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = splitk > 1 ? 2 : 1;
+    if (settled) attr[cfg.numAttrs++] = overlap_attribute();
+    if (splitk > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 1;
+        attr[cfg.numAttrs].val.clusterDim.y = splitk;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
     QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decompress_gemm_kernel<K, CODE>, out, codes, xmap, tlut, m, n, bs, npad, splitk, status));
     return check_launch();
 }
@@ -804,7 +813,7 @@ int wide_groups(int code, int m, int bs, double *cost = nullptr) {
 
 template <int K, int CODE>
 int launch_gemm_wide(__half *out, const uint8_t *codes, const __half *x, const uint32_t *tlut, int m, int n, int bs, unsigned *status,
-                     cudaStream_t s) {
+                     bool settled, cudaStream_t s) {
     static bool attr_set[64] = {};
     static std::mutex attr_mutex;
     int dev = 0;
@@ -829,27 +838,44 @@ int launch_gemm_wide(__half *out, const uint8_t *codes, const __half *x, const u
     cfg.blockDim = dim3(kWideThreads);
     cfg.dynamicSmemBytes = 1024 + wide_x_stages(npad) * npad * kTileCols * 2 + kLut512Bytes + 256;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr = overlap_attribute();
+    cfg.attrs = &attr;
+    cfg.numAttrs = settled ? 1 : 0;
     QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decompress_gemm_wide_kernel<K, CODE>, out, codes, xmap, tlut, m, n, bs, npad, (int)tiles, status));
     return check_launch();
 }
 template <int CODE>
-int launch_gemm_wide_k(__half *out, const uint8_t *c, const __half *x, const uint32_t *t, int K, int m, int n, int bs, unsigned *status, cudaStream_t s) {
-    if (K == 2) return launch_gemm_wide<2, CODE>(out, c, x, t, m, n, bs, status, s);
-    if (K == 3) return launch_gemm_wide<3, CODE>(out, c, x, t, m, n, bs, status, s);
-    return launch_gemm_wide<4, CODE>(out, c, x, t, m, n, bs, status, s);
+int launch_gemm_k(void *out, bool wide, const uint8_t *c, const __half *x, const uint32_t *t, int K, int m, int n, int bs, unsigned *status,
+                  bool settled, cudaStream_t s) {
+    if (wide) {
+        auto *o = static_cast<__half *>(out);
+        if (K == 2) return launch_gemm_wide<2, CODE>(o, c, x, t, m, n, bs, status, settled, s);
+        if (K == 3) return launch_gemm_wide<3, CODE>(o, c, x, t, m, n, bs, status, settled, s);
+        return launch_gemm_wide<4, CODE>(o, c, x, t, m, n, bs, status, settled, s);
+    }
+    auto *o = static_cast<float *>(out);
+    const int npad = (bs + 15) & ~15, splitk = column_splits(m, n);
+    if (K == 2) return launch_gemm<2, CODE>(o, c, x, t, m, n, bs, npad, splitk, status, settled, s);
+    if (K == 3) return launch_gemm<3, CODE>(o, c, x, t, m, n, bs, npad, splitk, status, settled, s);
+    return launch_gemm<4, CODE>(o, c, x, t, m, n, bs, npad, splitk, status, settled, s);
 }
 
-template <int CODE>
-int launch_gemm_k(float *out, const uint8_t *c, const __half *xh, const uint32_t *t, int K, int m, int n, int bs, int npad,
-                  int splitk, unsigned *status, cudaStream_t s) {
-    if (K == 2) return launch_gemm<2, CODE>(out, c, xh, t, m, n, bs, npad, splitk, status, s);
-    if (K == 3) return launch_gemm<3, CODE>(out, c, xh, t, m, n, bs, npad, splitk, status, s);
-    return launch_gemm<4, CODE>(out, c, xh, t, m, n, bs, npad, splitk, status, s);
+int gemm(void *out, bool wide, const void *codes, const void *x, const void *tlut, int code, int K, int m, int n, int bs, unsigned *status,
+         bool settled, void *stream) {
+    if (!out || !codes || !x || !status || K < 2 || K > 4 || bs < 1 || (!wide && bs > kMaxN)) return QTIP_ERR_BAD_ARG;
+    if (code != QTIP_CODE_HYB && code != QTIP_CODE_3INST && code != QTIP_CODE_1MAD) return QTIP_ERR_BAD_ARG;
+    if (code == QTIP_CODE_HYB && !tlut) return QTIP_ERR_BAD_ARG;
+    if (m <= 0 || n <= 0 || (m % kRows) || (n % kTileCols)) return QTIP_ERR_BAD_SHAPE;
+    if ((long)(m >> 5) * (n >> 5) >= (1L << 30)) return QTIP_ERR_BAD_SHAPE;
+    if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, wide ? 2 : 4) || (tlut && !aligned(tlut, 4)) || !aligned(status, 4))
+        return QTIP_ERR_ALIGNMENT;
+    auto *c = static_cast<const uint8_t *>(codes);
+    auto *xh = static_cast<const __half *>(x);
+    auto *t = static_cast<const uint32_t *>(tlut);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (code == QTIP_CODE_HYB) return launch_gemm_k<QTIP_CODE_HYB>(out, wide, c, xh, t, K, m, n, bs, status, settled, s);
+    if (code == QTIP_CODE_3INST) return launch_gemm_k<QTIP_CODE_3INST>(out, wide, c, xh, nullptr, K, m, n, bs, status, settled, s);
+    return launch_gemm_k<QTIP_CODE_1MAD>(out, wide, c, xh, nullptr, K, m, n, bs, status, settled, s);
 }
 
 }  // namespace
@@ -857,54 +883,26 @@ int launch_gemm_k(float *out, const uint8_t *c, const __half *xh, const uint32_t
 
 using namespace qtip;
 
-extern "C" int qtip_decompress_gemm(float *out, const void *codes, const void *x, const void *tlut, int K, int m, int n,
-                                    int bs, unsigned *status, void *stream) {
-    if (!out || !codes || !x || !tlut || !status || K < 2 || K > 4 || bs < 1 || bs > kMaxN) return QTIP_ERR_BAD_ARG;
-    if (m <= 0 || n <= 0 || (m % kRows) || (n % kTileCols)) return QTIP_ERR_BAD_SHAPE;
-    if ((long)(m >> 5) * (n >> 5) >= (1L << 30)) return QTIP_ERR_BAD_SHAPE;
-    if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, 4) || !aligned(tlut, 4) || !aligned(status, 4))
-        return QTIP_ERR_ALIGNMENT;
-    const int npad = (bs + 15) & ~15;
-    const int splitk = column_splits(m, n);
-    auto *c = static_cast<const uint8_t *>(codes);
-    auto *xh = static_cast<const __half *>(x);
-    auto *t = static_cast<const uint32_t *>(tlut);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return launch_gemm_k<QTIP_CODE_HYB>(out, c, xh, t, K, m, n, bs, npad, splitk, status, s);
+extern "C" int qtip_decompress_gemm(float *out, const void *codes, const void *x, const void *tlut, int K, int m, int n, int bs,
+                                    unsigned *status, void *stream) {
+    return gemm(out, false, codes, x, tlut, QTIP_CODE_HYB, K, m, n, bs, status, false, stream);
 }
 
 extern "C" int qtip_decompress_gemm_plain(float *out, const void *codes, const void *x, int code, int K, int m, int n, int bs,
                                           unsigned *status, void *stream) {
-    if (!out || !codes || !x || !status || K < 2 || K > 4 || bs < 1 || bs > kMaxN) return QTIP_ERR_BAD_ARG;
-    if (code != QTIP_CODE_3INST && code != QTIP_CODE_1MAD) return QTIP_ERR_BAD_ARG;
-    if (m <= 0 || n <= 0 || (m % kRows) || (n % kTileCols)) return QTIP_ERR_BAD_SHAPE;
-    if ((long)(m >> 5) * (n >> 5) >= (1L << 30)) return QTIP_ERR_BAD_SHAPE;
-    if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, 4) || !aligned(status, 4)) return QTIP_ERR_ALIGNMENT;
-    const int npad = (bs + 15) & ~15;
-    const int splitk = column_splits(m, n);
-    auto *c = static_cast<const uint8_t *>(codes);
-    auto *xh = static_cast<const __half *>(x);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (code == QTIP_CODE_3INST) return launch_gemm_k<QTIP_CODE_3INST>(out, c, xh, nullptr, K, m, n, bs, npad, splitk, status, s);
-    return launch_gemm_k<QTIP_CODE_1MAD>(out, c, xh, nullptr, K, m, n, bs, npad, splitk, status, s);
+    if (code == QTIP_CODE_HYB) return QTIP_ERR_BAD_ARG;
+    return gemm(out, false, codes, x, nullptr, code, K, m, n, bs, status, false, stream);
 }
 
 extern "C" int qtip_decompress_gemm_f16(void *out, const void *codes, const void *x, const void *tlut, int code, int K, int m, int n, int bs,
                                         unsigned *status, void *stream) {
-    if (!out || !codes || !x || !status || K < 2 || K > 4 || bs < 1) return QTIP_ERR_BAD_ARG;
-    if (code != QTIP_CODE_HYB && code != QTIP_CODE_3INST && code != QTIP_CODE_1MAD) return QTIP_ERR_BAD_ARG;
-    if (code == QTIP_CODE_HYB && !tlut) return QTIP_ERR_BAD_ARG;
-    if (m <= 0 || n <= 0 || (m % kRows) || (n % kTileCols)) return QTIP_ERR_BAD_SHAPE;
-    if ((long)(m >> 5) * (n >> 5) >= (1L << 30)) return QTIP_ERR_BAD_SHAPE;
-    if (!aligned(codes, 16) || !aligned(x, 16) || !aligned(out, 2) || (tlut && !aligned(tlut, 4)) || !aligned(status, 4)) return QTIP_ERR_ALIGNMENT;
-    auto *o = static_cast<__half *>(out);
-    auto *c = static_cast<const uint8_t *>(codes);
-    auto *xh = static_cast<const __half *>(x);
-    auto *t = static_cast<const uint32_t *>(tlut);
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    if (code == QTIP_CODE_HYB) return launch_gemm_wide_k<QTIP_CODE_HYB>(o, c, xh, t, K, m, n, bs, status, s);
-    if (code == QTIP_CODE_3INST) return launch_gemm_wide_k<QTIP_CODE_3INST>(o, c, xh, nullptr, K, m, n, bs, status, s);
-    return launch_gemm_wide_k<QTIP_CODE_1MAD>(o, c, xh, nullptr, K, m, n, bs, status, s);
+    return gemm(out, true, codes, x, tlut, code, K, m, n, bs, status, false, stream);
+}
+
+extern "C" int qtip_decompress_gemm_settled(void *out, int out_dtype, const void *codes, const void *x, const void *tlut, int code, int K, int m,
+                                            int n, int bs, unsigned *status, void *stream) {
+    if (out_dtype != QTIP_F16 && out_dtype != QTIP_F32) return QTIP_ERR_BAD_ARG;
+    return gemm(out, out_dtype == QTIP_F16, codes, x, tlut, code, K, m, n, bs, status, true, stream);
 }
 
 // Rule: estimates of both ways in microseconds.  Wide: 6 to start and end, the cycles above at 1.965 GHz.  Dense: 5 for the launches, the

@@ -194,19 +194,12 @@ at::Tensor linear_forward(const at::Tensor &input, Layer &L, int &launches) {
     at::Tensor dense_y;
     const void *y_in = y;
     int y_type = QTIP_F32;
-    if (gemm) {
-        unsigned *st = static_cast<unsigned *>(gemm_status(dev).data_ptr());
-        if (v1)
-            check(qtip_decompress_gemm_plain(y, trellis.data_ptr(), xh, L.code, L.K, (int)m, (int)n, (int)bs, st, stream),
-                  "qtip_decompress_gemm_plain");
-        else
-            check(qtip_decompress_gemm(y, trellis.data_ptr(), xh, tlut.data_ptr(), L.K, (int)m, (int)n, (int)bs, st, stream),
-                  "qtip_decompress_gemm");
-    } else if (wide) {
-        check(qtip_decompress_gemm_f16(y, trellis.data_ptr(), xh, v1 ? nullptr : tlut.data_ptr(), L.code, L.K, (int)m, (int)n, (int)bs,
-                                       static_cast<unsigned *>(gemm_status(dev).data_ptr()), stream),
-              "qtip_decompress_gemm_f16");
-        y_type = QTIP_F16;
+    if (gemm || wide) {
+        // (qtip_rht starts it when the weights, whatever wrote them, are complete)
+        y_type = wide ? QTIP_F16 : QTIP_F32;
+        check(qtip_decompress_gemm_settled(y, y_type, trellis.data_ptr(), xh, v1 ? nullptr : tlut.data_ptr(), L.code, L.K, (int)m, (int)n, (int)bs,
+                                           static_cast<unsigned *>(gemm_status(dev).data_ptr()), stream),
+              "qtip_decompress_gemm_settled");
     } else if (!dense) {
         at::Tensor ws = L.workspace.defined() ? L.workspace : matvec_workspace(dev, m, n, bs, stream);
         if (fragments)

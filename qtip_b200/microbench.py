@@ -30,11 +30,11 @@ def _sets(m, n, K, bs, code, device, min_bytes=400e6, max_sets=48):
 
 def _launch(lay, code, K, m, n, out, ws):
     if code == "hyb" and lay["x"].shape[0] > ops.MAX_MATVEC_BATCH:
-        ops.decompress_gemm(lay["codes"], lay["x"], lay["tlut"], K, m, n, out=out)      # tcgen05 path, batches 9..128
+        ops.decompress_gemm(lay["codes"], lay["x"], lay["tlut"], K, m, n, out=out, settled=True)      # tcgen05 path, batches 9..128
     elif code == "hyb":
         ops.decompress_matvec(lay["codes"], lay["x"], lay["tlut"], K, m, n, out=out, workspace=ws)
     elif ops.gemm_plain_supported(m, n, lay["x"].shape[0]) and not _PLAIN_MATVEC:
-        ops.decompress_gemm_plain(lay["codes"], lay["x"], code, K, m, n, out=out)      # compute codes on the tcgen05 path
+        ops.decompress_gemm_plain(lay["codes"], lay["x"], code, K, m, n, out=out, settled=True)      # compute codes on the tcgen05 path
     else:
         ops.decompress_matvec_plain(lay["codes"], lay["x"], code, K, m, n, out=out, workspace=ws)
 

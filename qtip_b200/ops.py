@@ -566,8 +566,9 @@ def gemm_status(device):
     return int(_lib.host().gemm_status(torch.cuda.current_device() if index is None else index).item())
 
 
-def decompress_gemm(codes, x, tlut, K, m, n, out=None):
-    """out (bs, m) fp32 = x (bs, n) fp16 @ decode(codes)^T on the tcgen05 tensor cores, 1 <= bs <= 128."""
+def decompress_gemm(codes, x, tlut, K, m, n, out=None, settled=False):
+    """out (bs, m) fp32 = x (bs, n) fp16 @ decode(codes)^T on the tcgen05 tensor cores, 1 <= bs <= 128.  settled: codes and table were
+    complete before the launch before this one began, so they may be read while that one runs."""
     _require_cuda(codes, x, tlut)
     if x.dtype != torch.float16:
         x = x.to(torch.float16)
@@ -577,15 +578,20 @@ def decompress_gemm(codes, x, tlut, K, m, n, out=None):
         out = torch.empty(bs, m, dtype=torch.float32, device=x.device)
     status = _lib.host().gemm_status(x.device.index)
     with torch.cuda.device(x.device):
-        st = _lib.load().qtip_decompress_gemm(out.data_ptr(), codes.data_ptr(), x.data_ptr(), tlut.data_ptr(), K, m, n, bs,
-                                              status.data_ptr(), _stream())
+        lib = _lib.load()
+        if settled:
+            st = lib.qtip_decompress_gemm_settled(out.data_ptr(), F32, codes.data_ptr(), x.data_ptr(), tlut.data_ptr(), CODE_HYB, K, m, n, bs,
+                                                  status.data_ptr(), _stream())
+        else:
+            st = lib.qtip_decompress_gemm(out.data_ptr(), codes.data_ptr(), x.data_ptr(), tlut.data_ptr(), K, m, n, bs, status.data_ptr(),
+                                          _stream())
     _lib.check(st, "qtip_decompress_gemm")
     global launch_count
     launch_count += 1
     return out
 
 
-def decompress_gemm_plain(codes, x, code, K, m, n, out=None):
+def decompress_gemm_plain(codes, x, code, K, m, n, out=None, settled=False):
     """decompress_gemm for the 3INST / 1MAD compute codes (plain layout, V = 1), 1 <= bs <= 128."""
     _require_cuda(codes, x)
     code = CODE_IDS.get(code, code)
@@ -597,8 +603,12 @@ def decompress_gemm_plain(codes, x, code, K, m, n, out=None):
         out = torch.empty(bs, m, dtype=torch.float32, device=x.device)
     status = _lib.host().gemm_status(x.device.index)
     with torch.cuda.device(x.device):
-        st = _lib.load().qtip_decompress_gemm_plain(out.data_ptr(), codes.data_ptr(), x.data_ptr(), code, K, m, n, bs,
-                                                    status.data_ptr(), _stream())
+        lib = _lib.load()
+        if settled:
+            st = lib.qtip_decompress_gemm_settled(out.data_ptr(), F32, codes.data_ptr(), x.data_ptr(), None, code, K, m, n, bs, status.data_ptr(),
+                                                  _stream())
+        else:
+            st = lib.qtip_decompress_gemm_plain(out.data_ptr(), codes.data_ptr(), x.data_ptr(), code, K, m, n, bs, status.data_ptr(), _stream())
     _lib.check(st, "qtip_decompress_gemm_plain")
     global launch_count
     launch_count += 1

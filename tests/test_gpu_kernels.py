@@ -588,6 +588,34 @@ def test_transform_in_fragment_order(K, m, n, bs):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("K", [2, 3, 4])
+@pytest.mark.parametrize("code", [O.CODE_HYB, O.CODE_3INST, O.CODE_1MAD])
+@pytest.mark.parametrize("m,n,bs", [(1024, 1024, 9), (8192, 4096, 27), (8192, 4096, 200)])
+def test_decompress_gemm_reads_what_the_launch_before_wrote(K, code, m, n, bs):
+    hyb = code == O.CODE_HYB
+    x = torch.randn(bs, n, device=DEV, generator=torch.Generator(DEV).manual_seed(9)).half()
+    codes = torch.zeros(K * m * n // 16, dtype=torch.int16, device=DEV)
+    tlut = torch.zeros(512, 2, dtype=torch.float16, device=DEV)
+
+    def product():
+        if bs > ops.MAX_GEMM_BATCH:
+            return ops.decompress_gemm_f16(codes, x, code, K, m, n, tlut=tlut if hyb else None)
+        return ops.decompress_gemm(codes, x, tlut, K, m, n) if hyb else ops.decompress_gemm_plain(codes, x, code, K, m, n)
+
+    product()
+    for seed in range(3):
+        for t in (codes, tlut) if hyb else (codes,):
+            codes.fill_(-1)
+            write_early(t, seed)
+            y = product()
+            assert torch.equal(y, product())
+            if bs <= ops.MAX_GEMM_BATCH:
+                assert torch.equal(y, ops.decompress_gemm(codes, x, tlut, K, m, n, settled=True) if hyb
+                                   else ops.decompress_gemm_plain(codes, x, code, K, m, n, settled=True))
+    assert ops.gemm_status(DEV) == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("bs", [33, 75, 97, 113])
 def test_decompress_gemm_x_ring_depths(bs):
     """The depths of the ring of x (6, 4, 4 and 3 stages) with several rounds in one CTA and a last step of one tile."""
