@@ -617,7 +617,7 @@ def decompress_gemm_plain(codes, x, code, K, m, n, out=None, settled=False):
 
 def decompress_gemm_f16(codes, x, code, K, m, n, tlut=None, out=None):
     """out (bs, m) fp16 = x (bs, n) fp16 @ decode(codes)^T, any number of rows; HYB (kernel layout, with its table) or a compute code."""
-    _require_cuda(codes, x)
+    _require_cuda(codes, x, tlut)
     code = CODE_IDS.get(code, code)
     if x.dtype != torch.float16:
         x = x.to(torch.float16)

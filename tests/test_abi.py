@@ -158,3 +158,23 @@ def test_ops_refuse_cpu_tensors():
         ops.decode_hyb(torch.zeros(32 * 32 * 2 // 16, dtype=torch.int16), torch.zeros(512, 2, dtype=torch.float16), 2, 32, 32)
     with pytest.raises(RuntimeError, match="CUDA"):
         ops.rht(torch.zeros(1, 64))
+
+
+def test_products_check_the_table_too(monkeypatch):
+    """A table in host memory is refused like any other operand (seen on the list that the check is given: no GPU here)."""
+    import torch
+    from qtip_b200 import ops
+
+    class Checked(Exception):
+        pass
+
+    def check(*tensors):
+        raise Checked(tensors)
+
+    monkeypatch.setattr(ops, "_require_cuda", check)
+    codes, x, tlut = torch.zeros(128 * 64 // 8, dtype=torch.int16), torch.zeros(1, 64), torch.zeros(512, 2, dtype=torch.float16)
+    for call in (lambda: ops.decompress_gemm_f16(codes, x, "hyb", 2, 128, 64, tlut=tlut), lambda: ops.decompress_gemm(codes, x, tlut, 2, 128, 64),
+                 lambda: ops.decompress_matvec(codes, x, tlut, 2, 128, 64)):
+        with pytest.raises(Checked) as e:
+            call()
+        assert any(t is tlut for t in e.value.args[0])
