@@ -630,10 +630,12 @@ def test_decompress_gemm_x_ring_depths(bs):
 @pytest.mark.gpu
 @pytest.mark.parametrize("K", [2, 3, 4])
 @pytest.mark.parametrize("code", [O.CODE_HYB, O.CODE_3INST, O.CODE_1MAD])
-@pytest.mark.parametrize("m,n,bs", [(128, 64, 129), (384, 320, 256), (256, 832, 257), (19200, 192, 300), (2560, 1216, 1000)])
+@pytest.mark.parametrize("m,n,bs", [(128, 64, 129), (384, 320, 256), (256, 832, 257), (19200, 192, 300), (2560, 1216, 1000),
+                                    (38016, 704, 1), (38016, 704, 16), (38016, 704, 17), (38016, 704, 128)])
 def test_decompress_gemm_f16(K, code, m, n, bs):
-    """One to several batch groups and tiles per CTA, an odd number of 64-column tiles, one step per tile, ragged last groups; against
-    the dense product of the (bit-exact) decoded matrix in 64 bits: rounding to fp16 is 2^-11 of a value at most, uniform."""
+    """One to several batch groups and tiles per CTA, an odd number of 64-column tiles, one step per tile, ragged last groups, few rows
+    (all eight stages of x, several times round); against the dense product of the (bit-exact) decoded
+    matrix in 64 bits: rounding to fp16 is 2^-11 of a value at most, uniform."""
     lay = synth.make_layer(m, n, K, seed=3800 + K, bs=bs, device=DEV, **({} if code == O.CODE_HYB else {"code": "none"}))
     hyb = code == O.CODE_HYB
     y = ops.decompress_gemm_f16(lay["codes"], lay["x"], code, K, m, n, tlut=lay["tlut"] if hyb else None)

@@ -769,3 +769,53 @@ def test_weights_written_by_the_launch_before_the_call(code, mode, K, m, n, bs):
             write_early(t.data, seed)
             y = q(x)
             assert torch.isfinite(y).all() and torch.equal(y, q(x))
+
+
+def _offset(t):
+    """The same values one element into a buffer: contiguous, but not on a 16-byte boundary."""
+    out = torch.empty(t.numel() + 8, dtype=t.dtype, device=t.device)[1:1 + t.numel()].view(t.shape)
+    assert out.data_ptr() % 16
+    return out.copy_(t)
+
+
+@pytest.mark.parametrize("K", [2, 4])
+@pytest.mark.parametrize("which", ["x", "SU"])
+def test_unaligned_rows_of_a_width_whose_transform_writes_fragments(K, which):
+    """x or SU off the 16-byte boundary: the general transform, row-major, and the matvec's own re-ordering.  Only the order of the
+    transform's sums differs, which shows where a value of x rounds to the other fp16 neighbour."""
+    m, n, bs = 2048, 8192, 5
+    assert ops.matvec_takes_fragments(K, m, n, bs)
+    lay = synth.make_layer(m, n, K, seed=90 + K, bs=bs, device=DEV)
+    q = QuantizedLinear(n, m, 16, 16, 16, K, 2, 9, "quantlut_sym").to(DEV)
+    q.trellis.copy_(lay["codes"].view(torch.int16))
+    q.SU.copy_(lay["SU"]), q.SV.copy_(lay["SV"]), q.tlut.data.copy_(lay["tlut"])
+    x = lay["x"].half()
+    want = q(x)
+    if which == "x":
+        x = _offset(x)
+    else:
+        q.SU = _offset(q.SU)
+    y = q(x)
+    assert float((y.double() - want.double()).norm() / want.double().norm()) < 1e-3
+
+
+@pytest.mark.parametrize("code,mode,K", [("hyb", "quantlut_sym", 2), ("3inst", "3inst", 3)])
+def test_long_prompt_with_unaligned_codes(code, mode, K):
+    """Codes off the 16-byte boundary: decoded densely where the decoder takes them, refused where it does not (HYB)."""
+    from qtip_b200 import _lib
+    m, n, bs = 22016, 1024, 389
+    assert _lib.load().qtip_decompress_gemm_f16_faster(ops.CODE_IDS[code], m, n, bs) == 1
+    lay = synth.make_layer(m, n, K, seed=60 + K, bs=bs, code=code, device=DEV)
+    q = QuantizedLinear(n, m, 16, 16, 16, K, 2 if code == "hyb" else 1, 9, mode).to(DEV)
+    q.trellis.copy_(lay["codes"].view(torch.int16))
+    q.SU.copy_(lay["SU"]), q.SV.copy_(lay["SV"])
+    if code == "hyb":
+        q.tlut.data.copy_(lay["tlut"])
+    want = q(lay["x"])
+    q.trellis = _offset(q.trellis)
+    if code == "hyb":
+        with pytest.raises(RuntimeError, match="align"):
+            q(lay["x"])
+        return
+    y = q(lay["x"])
+    assert float((y.double() - want.double()).norm() / want.double().norm()) < 2.0**-10      # two products rounded to fp16
