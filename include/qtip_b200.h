@@ -13,7 +13,7 @@
  * matrix) while the launch before them may still run: qtip_decompress_matvec and its forms for HYB, qtip_linear_fused,
  * qtip_rht (hadk_bits, sign_out), qtip_rht_fused, qtip_mlp_mid, qtip_rope_kv_append_fused, qtip_lm_head, and whatever says so below.
  * Weights of these must not be written by the launch directly before, nor by one further back with only such launches since.  qtip_rht
- * and qtip_decode_hyb end that: the launch behind one of them starts when everything before it is complete.  All others
+ * and every plain launch end that: the launch behind one of them starts when everything before it is complete.  All others
  * (the decoders, qtip_decompress_gemm*, the packing and layout calls, the quantizer) follow plain stream order for every operand.
  *
  * Naming: K = bits per weight (the upstream CUDA template parameter R), m = out_features
@@ -61,6 +61,8 @@ int qtip_version(void);
  * BitshiftLinear.get_hatW_kernel (lib/codebook/bitshift.py:383-387); bit-exact with them.
  * codes: K*m*n/8 bytes, 16-byte aligned; W 16-byte aligned; tlut: 512x2 fp16; m, n multiples of 32; K in {2,3,4}. */
 int qtip_decode_hyb(void *W, const void *codes, const void *tlut, int K, int m, int n, void *stream);
+/* The same for codes and a table that were complete before the launch before this one began: they are read while it still runs. */
+int qtip_decode_hyb_settled(void *W, const void *codes, const void *tlut, int K, int m, int n, void *stream);
 
 /* Plain layout, any of the three codes.  Replaces unpack_trellis + recons + get_hatW
  * (lib/codebook/bitshift.py:329-353, 199-201, 378-381).  HYB uses V=2 and needs tlut; 3INST and

@@ -31,6 +31,7 @@ SIGNATURES = {
     "qtip_last_cuda_error": (_i, []),
     "qtip_version": (_i, []),
     "qtip_decode_hyb": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
+    "qtip_decode_hyb_settled": (_i, [_vp, _vp, _vp, _i, _i, _i, _vp]),
     "qtip_decode_plain": (_i, [_vp, _vp, _i, _vp, _i, _i, _i, _vp]),
     "qtip_pipe_rate_count": (_i, []),
     "qtip_pipe_rate_name": (ctypes.c_char_p, [_i]),

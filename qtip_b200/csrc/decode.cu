@@ -6,10 +6,17 @@
 //                     Bound: writing 2 bytes per weight.  With the 512 entries once per CTA the lookups' bank conflicts were the
 //                     bound (shared-memory pipe at 77 %, issue at 35 %), so a persistent CTA of 32 warps keeps the matvec's 1024
 //                     entries in 32 lane-private copies, and a tile's fragments go to the staging tile as matrices.
-//                     11008 x 4096, K = 2: 28 -> 23 us = 3.9 TB/s of writes (a fill of the same size takes 26.7 us); 4096 x 4096, K = 4
-//                     12.0 -> 10.4.
-// decode_hyb_small_kernel  the same for matrices of at most kSmallBlocks blocks, where building the 128 KiB table costs more than the
-//                     conflicts (1024 x 1024: 2.6 against 3.5 us, 2048 x 2048: 4.4 against 4.5, 3072 x 2048: 5.7 against 5.6).
+//                     Back to back, several matrices, microseconds at K = 2, 3, 4, the small kernel / this one / this one with settled
+//                     weights, whose reads and table overlap the launch before:
+//                       11008 x 4096  27.6 28.9 28.6 / 25.6 29.6 26.8 / 23.0 26.4 24.0 (3.9 TB/s of writes at K = 2)
+//                       8192 x 8192   40.0 41.8 41.9 / 34.4 40.1 35.9 / 32.5 37.2 33.9
+//                       28672 x 8192  131 138 137 / 109 130 114 / 106 127 111
+// decode_hyb_small_kernel  the same with one copy of the table, for matrices of at most small_blocks() blocks, where building the
+//                     128 KiB table costs more than the conflicts:
+//                       2048 x 2048   5.0 5.0 5.1 / 5.9 6.2 6.1 / 4.8 5.0 5.0
+//                       3072 x 2048   6.2 6.4 6.3 / 8.0 8.7 8.3 / 5.9 6.3 6.0
+//                       4096 x 4096   11.7 12.2 12.3 / 12.3 14.0 12.8 / 10.4 11.6 10.8
+//                       8192 x 4096   21.2 22.2 22.4 / 18.9 21.5 19.8 / 17.5 19.8 18.3
 // decode_plain_kernel any code, plain layout (lib/codebook/bitshift.py:329-353, 378-381): one warp
 //                     per tile, each lane decodes 8 consecutive sequence elements of one tile row half.
 #include <mutex>
@@ -32,11 +39,6 @@ template <int K>
 __global__ void __launch_bounds__(kHybThreads, 1) decode_hyb_kernel(__half *__restrict__ W, const uint8_t *__restrict__ codes,
                                                                     const uint32_t *__restrict__ tlut, int m, int n) {
     extern __shared__ __align__(128) uint8_t smem[];
-    // codes and table may come from the launch before (a conversion, the layout shuffle), so nothing is read ahead of the wait (through
-    // the pointers: read-only loads are not moved either), and the next launch starts its own reads of weights only when everything
-    // before this one is complete
-    asm volatile("griddepcontrol.wait;" : "+l"(codes), "+l"(tlut) : : "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // the warp index through a shuffle: the same in all lanes, so the loop control is scalar
     const int warp = __shfl_sync(kFullMask, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int nb = n >> 5, blocks = (m >> 5) * nb, warps = (int)gridDim.x * (kHybThreads / 32);
@@ -49,7 +51,9 @@ __global__ void __launch_bounds__(kHybThreads, 1) decode_hyb_kernel(__half *__re
         const uint32_t e = __ldg(tlut + ((i >> 3) & 511)) ^ ((uint32_t)(i >> 12) << 15);
         reinterpret_cast<uint4 *>(smem)[i] = make_uint4(e, e, e, e);
     }
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __syncthreads();
+    asm volatile("griddepcontrol.wait;" ::: "memory");      // W may still be read by an earlier launch of the stream
 
     const uint32_t lut_lane = (uint32_t)__cvta_generic_to_shared(smem) + lane * 4;
     const uint32_t stage = (uint32_t)__cvta_generic_to_shared(smem) + kHybLutBytes + warp * (32 * kStageStride);
@@ -89,7 +93,8 @@ __global__ void __launch_bounds__(kHybThreads, 1) decode_hyb_kernel(__half *__re
     }
 }
 
-constexpr long kSmallBlocks = 4096;
+// where the two kernels meet (the figures above)
+constexpr long small_blocks(bool settled) { return settled ? 4 << 10 : 16 << 10; }
 constexpr int kSmallStride = kStageStride / 4;      // words
 
 template <int K>
@@ -142,9 +147,9 @@ int decode_grid(long warps_needed) {
 }
 
 template <int K>
-int launch_decode_hyb(__half *W, const uint8_t *codes, const uint32_t *tlut, int m, int n, cudaStream_t s) {
+int launch_decode_hyb(__half *W, const uint8_t *codes, const uint32_t *tlut, int m, int n, bool settled, cudaStream_t s) {
     const long blocks = (long)(m >> 5) * (n >> 5);
-    if (blocks <= kSmallBlocks) {
+    if (blocks <= small_blocks(settled)) {
         decode_hyb_small_kernel<K><<<decode_grid(blocks), kDecodeThreads, 0, s>>>(W, codes, tlut, m, n);
         return check_launch();
     }
@@ -170,7 +175,7 @@ int launch_decode_hyb(__half *W, const uint8_t *codes, const uint32_t *tlut, int
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = settled ? 1 : 0;       // codes and table are read before the wait
     QTIP_CUDA_TRY(cudaLaunchKernelEx(&cfg, decode_hyb_kernel<K>, W, codes, tlut, m, n));
     return check_launch();
 }
@@ -232,12 +237,7 @@ __global__ void __launch_bounds__(kDecodeThreads) decode_plain_kernel(__half *__
     }
 }
 
-}  // namespace
-}  // namespace qtip
-
-using namespace qtip;
-
-extern "C" int qtip_decode_hyb(void *W, const void *codes, const void *tlut, int K, int m, int n, void *stream) {
+int decode_hyb(void *W, const void *codes, const void *tlut, int K, int m, int n, bool settled, void *stream) {
     if (!W || !codes || !tlut || K < 2 || K > 4) return QTIP_ERR_BAD_ARG;
     if (m <= 0 || n <= 0 || (m & 31) || (n & 31)) return QTIP_ERR_BAD_SHAPE;
     if (!aligned(codes, 16) || !aligned(W, 16) || !aligned(tlut, 4)) return QTIP_ERR_ALIGNMENT;
@@ -245,9 +245,22 @@ extern "C" int qtip_decode_hyb(void *W, const void *codes, const void *tlut, int
     auto *Wh = static_cast<__half *>(W);
     auto *c = static_cast<const uint8_t *>(codes);
     auto *t = static_cast<const uint32_t *>(tlut);
-    if (K == 2) return launch_decode_hyb<2>(Wh, c, t, m, n, s);
-    if (K == 3) return launch_decode_hyb<3>(Wh, c, t, m, n, s);
-    return launch_decode_hyb<4>(Wh, c, t, m, n, s);
+    if (K == 2) return launch_decode_hyb<2>(Wh, c, t, m, n, settled, s);
+    if (K == 3) return launch_decode_hyb<3>(Wh, c, t, m, n, settled, s);
+    return launch_decode_hyb<4>(Wh, c, t, m, n, settled, s);
+}
+
+}  // namespace
+}  // namespace qtip
+
+using namespace qtip;
+
+extern "C" int qtip_decode_hyb(void *W, const void *codes, const void *tlut, int K, int m, int n, void *stream) {
+    return decode_hyb(W, codes, tlut, K, m, n, false, stream);
+}
+
+extern "C" int qtip_decode_hyb_settled(void *W, const void *codes, const void *tlut, int K, int m, int n, void *stream) {
+    return decode_hyb(W, codes, tlut, K, m, n, true, stream);
 }
 
 extern "C" int qtip_decode_plain(void *W, const void *codes, int code, const void *tlut, int K, int m, int n,

@@ -219,7 +219,8 @@ at::Tensor linear_forward(const at::Tensor &input, Layer &L, int &launches) {
         // product goes to the output transform as it is
         at::Tensor W = at::empty({m, n}, opts.dtype(at::kHalf));
         if (L.kernel_layout)
-            check(qtip_decode_hyb(W.data_ptr(), trellis.data_ptr(), tlut.data_ptr(), L.K, (int)m, (int)n, stream), "qtip_decode_hyb");
+            check(qtip_decode_hyb_settled(W.data_ptr(), trellis.data_ptr(), tlut.data_ptr(), L.K, (int)m, (int)n, stream),
+                  "qtip_decode_hyb_settled");
         else
             check(qtip_decode_plain(W.data_ptr(), trellis.data_ptr(), L.code, tlut.defined() ? tlut.data_ptr() : nullptr, L.K, (int)m,
                                     (int)n, stream),

@@ -120,8 +120,9 @@ def matvec_workspace(m, n, bs, device):
 # ---------------------------------------------------------------------------------------------
 # ops
 # ---------------------------------------------------------------------------------------------
-def decode_hyb(codes, tlut, K, m, n, out=None):
-    """Kernel-layout HYB codes -> (m, n) fp16 (decode_compressed upstream)."""
+def decode_hyb(codes, tlut, K, m, n, out=None, settled=False):
+    """Kernel-layout HYB codes -> (m, n) fp16 (decode_compressed upstream).  settled: codes and table (fp16, contiguous) were complete
+    before the launch before this one began, so they may be read while that one runs."""
     _require_cuda(codes, tlut)
     codes = codes.contiguous()
     tlut = tlut.to(torch.float16).contiguous()
@@ -130,7 +131,9 @@ def decode_hyb(codes, tlut, K, m, n, out=None):
     if out is None:
         out = torch.empty(m, n, dtype=torch.float16, device=codes.device)
     with torch.cuda.device(codes.device):
-        st = _lib.load().qtip_decode_hyb(out.data_ptr(), codes.data_ptr(), tlut.data_ptr(), K, m, n, _stream())
+        lib = _lib.load()
+        call = lib.qtip_decode_hyb_settled if settled else lib.qtip_decode_hyb
+        st = call(out.data_ptr(), codes.data_ptr(), tlut.data_ptr(), K, m, n, _stream())
     _lib.check(st, "qtip_decode_hyb")
     global launch_count
     launch_count += 1

@@ -41,11 +41,16 @@ def test_decode_hyb_golden(golden, K, shape):
 
 @pytest.mark.parametrize("K", [2, 3, 4])
 @pytest.mark.parametrize("m,n", [(256, 256), (4096, 4096), (4096, 11008), (11008, 4096),
-                                 (2048, 2048), (2080, 2048), (131104, 32), (32, 160000)])     # both sides of the small kernel; steps over rows
+                                 (2048, 2048), (2080, 2048), (131104, 32), (32, 160000),
+                                 # and of the one chosen for unsettled weights (16384 blocks)
+                                 (4128, 4096), (524832, 32), (32, 524832)])
 def test_decode_hyb_vs_oracle(K, m, n):
     lay = synth.make_layer(m, n, K, seed=2000 + K)
-    W = ops.decode_hyb(dev(lay["codes"]), dev(lay["tlut"]), K, m, n)
+    codes, tlut = dev(lay["codes"]), dev(lay["tlut"])
+    W = ops.decode_hyb(codes, tlut, K, m, n)
     assert np.array_equal(u16(W), u16(C.decode_kernel(lay["codes"], m, n, K, lay["tlut"])))
+    torch.cuda.synchronize()
+    assert torch.equal(W.view(torch.int16), ops.decode_hyb(codes, tlut, K, m, n, settled=True).view(torch.int16))
 
 
 def write_early(dst, seed):
@@ -58,7 +63,7 @@ def write_early(dst, seed):
 
 
 @pytest.mark.parametrize("K", [2, 3, 4])
-@pytest.mark.parametrize("m,n", [(1024, 1024), (8192, 4096)])
+@pytest.mark.parametrize("m,n", [(1024, 1024), (16384, 4096)])
 @pytest.mark.parametrize("operand", ["codes", "tlut"])
 def test_decode_hyb_reads_what_the_launch_before_wrote(K, m, n, operand):
     for seed in range(3):
