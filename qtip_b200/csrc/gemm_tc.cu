@@ -19,13 +19,13 @@
 // tile (its own 2K bytes and the start of the next row), lanes 2r and 2r + 1 row r of two tiles, and stores a row per
 // tensor-memory lane; the accumulator's lanes are mapped back to rows when they are read.
 // Bound: instruction issue of the decode warps up to about 64 rows (8192 x 28672, 27 rows: leaving out three of four MMAs 45.6 -> 43.0 us,
-// the lookups 35.4), the MMAs above (120 rows: 57.8 -> 48.9 and 54.4 us).  Hence two blocks per warp and step between the barriers, x
+// the lookups 35.4), the MMAs above (120 rows: 58.3 -> 48.9 and 54.4 us).  Hence two blocks per warp and step between the barriers, x
 // through TMA instead of copies by the decode warps, scalar control (the warp index through a shuffle), control threads that sleep
 // between polls, and codes requested two steps ahead.  Warp instructions per block of weights, HYB 27 rows 190 -> 145, 3INST 295 -> 217
 // (of which the mask of mask_3inst 32).
 // Measured, one block per warp and step with x copied by the decode warps -> now (microseconds, K = 2 unless stated): HYB 8192 x 8192
-// 27 rows 20.5 -> 17.5; 8192 x 28672 120 rows 73 -> 57.2; 14336 x 4096 K = 3 27 rows 19.7 -> 16.3; 28672 x 8192 K = 4 64 rows 70 -> 58;
-// 3INST 8192 x 8192 16 rows 30.5 -> 21.6, 8192 x 28672 120 rows 107 -> 69.6; 1MAD 8192 x 8192 K = 3 32 rows 33.0 -> 29.4.  A second
+// 27 rows 20.5 -> 17.2; 8192 x 28672 120 rows 73 -> 58.5; 14336 x 4096 K = 3 27 rows 19.7 -> 15.8; 28672 x 8192 K = 4 64 rows 70 -> 57;
+// 3INST 8192 x 8192 16 rows 30.5 -> 21.6, 8192 x 28672 120 rows 107 -> 69.5; 1MAD 8192 x 8192 K = 3 32 rows 33.0 -> 29.2.  A second
 // accumulator for every other MMA changes nothing.
 // This replaces decode-to-HBM + dense GEMM of BitshiftLinearKernelAG upstream
 // (lib/codebook/bitshift.py:476-489), which writes and re-reads 16x the packed bytes at 2 bits.
@@ -219,7 +219,7 @@ __device__ __forceinline__ float cluster_load(uint32_t addr, int rank) {
 // from one register (the multiply pipe has room; gathering both states' terms for one addition costs a permute more, 31.3 against
 // 29.4 us at 8192 x 8192, 27 rows).  1MAD: byte sums of the LCG values by dot product, weights from the lane's copy of the table.
 // `mask` is 0x8FFF8FFF as a run-time value: a three-input logic instruction takes one literal, so with two it becomes two
-// instructions (8192 x 8192, 16 rows, 26.0 -> 21.6; 8192 x 28672, 120 rows, 83 -> 69.6 us).
+// instructions (8192 x 8192, 16 rows, 26.0 -> 21.6; 8192 x 28672, 120 rows, 83 -> 69.5 us).
 __device__ __forceinline__ uint32_t mask_3inst(int npad) { return 0x8FFF8FFFu | (uint32_t)npad >> 16; }
 __device__ __forceinline__ uint32_t pair_3inst(uint32_t s0, uint32_t s1, uint32_t mask) {
     const uint32_t r0 = ((s0 * 89226354u + 64248484u) & mask) ^ 0x3B603B60u, r1 = ((s1 * 89226354u + 64248484u) & mask) ^ 0x3B603B60u;
@@ -506,8 +506,8 @@ __device__ __forceinline__ uint32_t b_tile(uint32_t base, int stage, int bytes) 
 // The same roles over tiles of 128 output rows x up to 256 batch rows, fp16 results: a CTA per SM walks over the tiles (all row ranges of
 // one batch group before the next), four more warps read the accumulator of a finished tile and write it.  Four stages of weights
 // (tensor memory: 256 columns beside the accumulator's 256); x in a ring of single 64-column tiles.  Every batch group decodes the
-// matrix again: a tile's 16 columns take the MMA about 100 + 0.15 N cycles and the decode warps 100, so up to 256 rows share a decode
-// at the price of one.  Measured against decode_hyb / decode_plain and
+// matrix again; 16 columns of a tile take the MMA 100 + 0.5 N cycles and the decode warps 140 (3INST 165, 1MAD 188; fitted, wide_cycles), so one
+// group of 256 rows takes 228 where two of 128 take 328.  Measured against decode_hyb / decode_plain and
 // a library product, HYB K = 2 unless stated (microseconds): 11008 x 4096 129 rows 44.7 -> 26.6, 512 rows 59.8 -> 50.7, 1000 rows
 // 86.5 -> 81.1; 28672 x 8192 256 rows 214 -> 107, 512 rows 287 -> 230; K = 4 4096 x 4096 1000 rows 37.8 -> 33.1; 1MAD K = 4 8192 x 8192
 // 256 rows 116 -> 56.  Bound: the MMAs (half of the tensor pipe's cycles are busy: a tensor-memory A operand takes twice the ideal interval),
@@ -906,7 +906,7 @@ extern "C" int qtip_decompress_gemm_settled(void *out, int out_dtype, const void
 }
 
 // Rule: estimates of both ways in microseconds.  Wide: 6 to start and end, the cycles above at 1.965 GHz.  Dense: 5 for the launches, the
-// decode at its write rate (3.9 TB/s HYB, 2.8 3INST, 1.6 1MAD), the product at the rate of reading the matrix (4.2 TB/s) or 1430 TFLOP/s.
+// decode at its write rate (3.9 TB/s HYB, settled weights, 2.8 3INST, 1.6 1MAD), the product at the rate of reading the matrix (4.2 TB/s) or 1430 TFLOP/s.
 // Products of several hundred microseconds run at the power cap (28672 x 8192, 1000 rows: 400 to 458 us in three runs, dense 432 to 450): 10 % more.
 // It errs by up to 10 %, on either side of the line (4096 x 4096: dense up to 512 rows, 26.2 against 27.0 us; 11008 x 4096: wide up to about 2000).
 extern "C" int qtip_decompress_gemm_f16_faster(int code, int m, int n, int bs) {

@@ -20,8 +20,9 @@
 // (two wavefronts per mma) and the mma.sync rate together; few rows by the chain load, barrier, product, exchange, store.
 // fp16 rows without statistics and conversions (HALVES): 11008 x 1000 rows 55 -> 45, x 120 10.3 -> 9.3, x 1 6.4 -> 4.6;
 // 28672 x 1000 with signs 98 -> 67; 14336 x 1000 43 -> 30.
-// They are bound by instruction issue at few resident warps (20 000 warp instructions per row of 11008, a quarter of them in the last pass at
-// two values per thread).  Up to eight values per thread there, and a multiply-add instead of two predicated adds per shuffle: fp16 rows,
+// Nothing is full there: a CTA's rows are strictly serial (load, barrier, product, exchange, store) at 16 resident warps, so the time is the
+// chain's, in which instructions count (20 000 per row of 11008, a quarter of them in the last pass at two values per thread; now 15 900,
+// issued in 36 % of the slots).  Up to eight values per thread there, and a multiply-add instead of two predicated adds per shuffle: fp16 rows,
 // signs after the transform, 11008 x 1000 39.8 -> 33.6, x 120 8.4 -> 7.2, x 1 4.5 -> 3.2; 14336 x 1000 40.2 -> 27.9; 28672 x 1000
 // 88.6 -> 59.7, x 120 12.4 -> 8.6; 53248 x 1000 270 -> 224.  (A variant of 64 registers with more resident warps spilled: slower.)
 #include <algorithm>

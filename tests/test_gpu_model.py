@@ -250,6 +250,37 @@ def test_batched_decode_at_large_widths_matches_64_bits(hidden, heads, kv, mlp, 
     assert err < 4.5e-3, err
 
 
+def test_batched_decode_with_unaligned_vectors():
+    """Sign and norm vectors off the 16-byte boundary at a width whose transform writes fragment order otherwise: the same step by the
+    general transform and the matvec's own re-ordering, within the bound above."""
+    shape = LlamaShape(n_layers=1, hidden=8192, n_heads=64, n_kv_heads=8, head_dim=128, mlp=8192, vocab=2048, K=2)
+    model = QtipLlama(shape, max_positions=64, device=DEV, seed=61)
+    B = 5
+    assert ops.matvec_takes_fragments(2, 8192, 8192, B)
+    model.enable_batch(B)
+
+    def offset(t):
+        return torch.empty(t.numel() + 8, dtype=t.dtype, device=DEV)[1:1 + t.numel()].view(t.shape).copy_(t)
+
+    L = model.layers[0]
+    for name in ("o", "down"):
+        L[name].SU = offset(L[name].SU)
+    L["ln1"], L["ln2"] = offset(L["ln1"]), offset(L["ln2"])
+    assert all(t.data_ptr() % 16 for t in (L["o"].SU, L["down"].SU, L["ln1"], L["ln2"]))
+    g = torch.Generator(device=DEV).manual_seed(62)
+    for c in (model.b_cache_k, model.b_cache_v):
+        c[:, :, :20].normal_(generator=g)
+    model.b_pos.fill_(20)
+    tokens = torch.randint(0, shape.vocab, (2, B), generator=g, device=DEV)
+    want = reference_batch_logits(model, tokens)
+    for ids in tokens:
+        model.b_token.copy_(ids)
+        model.step_batch()
+    model.check_status()
+    err = float((model.b_logits.double() - want).norm() / want.norm())
+    assert err < 4.5e-3, err
+
+
 def test_state_dict_round_trip_into_decode_model():
     """A synthetic checkpoint with upstream's keys, shapes and dtypes (lib/linear/quantized_linear.py:41-67) loaded into
     a differently seeded model reproduces the source model's logits bit for bit; wrong shapes and tensor-parallel
